@@ -202,3 +202,25 @@ def test_tree_build_bit_exact_near_the_origin():
     O, G = build_both(xyz, st, leaf_max_points=16, leaf_density=0.0)
     assert O.accepted and G is not None
     assert_same_tree(O, G)
+
+
+@pytest.mark.parametrize("sizes", [
+    [1024, 1025, 2048, 2049, 1023] * 60,   # 300 roots around one and two chunks: several list batches per block
+    [300_001, 7, 1025, 65_537],            # one root of many chunks beside ragged small ones
+])
+def test_large_node_chunk_lists(scene, sizes):
+    """The large-node lists at their edges: roots of one chunk and one point more, more large
+    roots than a block has threads, and chunk counts far above a block's threads."""
+    import kd_slam2_b200 as kds
+    xyz, st = make_scan(scene, 2450, beams=128, cols=4096, elev=(-22.5, 22.5))
+    rng = np.random.default_rng(7)
+    clouds = []
+    for n in sizes:
+        k = np.sort(rng.choice(len(xyz), n, replace=False))
+        clouds.append((np.ascontiguousarray(xyz[k]), np.ascontiguousarray(st[k])))
+    trees = kds.TreeGeneratorB2003D(leaf_max_points=16).make_trees(clouds)
+    for (x, s), T in zip(clouds, trees):
+        if len(x) < 100:
+            assert T is None
+            continue
+        assert_same_tree(orc.OTree.build(x, s, orc.tree_params(leaf_max_points=16)), T)
