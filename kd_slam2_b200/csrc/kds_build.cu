@@ -5,10 +5,10 @@
 // Replaces TreeGenerator_::makeTree (kd/tree/tree_generator_impl_.h:7-19), which the
 // reference runs on the CPU only.  The tree is built level by level for all trees of
 // the batch together:
-//   * per-node moments [xx,xy,xz,yy,yz,zz,x,y,z,dt,dt^2] are exact, order-free 128-bit
-//     fixed-point sums: each product of two floats (or double stamp term) is decomposed
-//     into sign/mantissa/exponent and its floor(v * 2^64) is formed with integer shifts,
-//     so warps, blocks and atomics may add them in any order;
+//   * per-node moments [xx,xy,xz,yy,yz,zz,x,y,z] are exact, order-free 128-bit
+//     fixed-point sums: floor(v * 2^64) of each product of two floats (or double stamp
+//     term) is formed and added in integers, so warps, blocks and atomics may add them in
+//     any order;
 //   * FP64 covariance, cyclic Jacobi eigensolver, FlatLeafPolicy_ decision
 //     (kd/tree/flat_leaf_policy_.h:52-108) in FP64;
 //   * stable partition by Node_::whichSide in float (kd/tree/node_.h:53-56);
@@ -42,7 +42,9 @@ constexpr int kLevelBlocks = 148 * 3;  // k_decide: 3 blocks per SM at its regis
 constexpr int kLevelsPerSync = 4;
 constexpr int kMaxDepth = 64;
 constexpr int kUnroll = 2;  // rounds of 32 points in flight per lane in the warp-per-node partition
-constexpr int kSmallBlocks = 148 * 4;  // two waves: other streams' kernels interleave at block boundaries
+constexpr int kScatterPerSM = 2;  // 122 registers: the lanes' 21 64-bit parts and four points in flight
+constexpr int kSmallPerSM = 3;
+constexpr int kSmallBlocks = 148 * kSmallPerSM * 2;  // two waves: other streams' kernels interleave at block boundaries
 
 // ---------------------------------------------------------------------------
 // 128-bit two's complement fixed point (units of 2^-64)
@@ -54,12 +56,6 @@ __host__ __device__ __forceinline__ U128 u128_add(U128 a, U128 b) {
   U128 r;
   r.lo = a.lo + b.lo;
   r.hi = a.hi + b.hi + (r.lo < a.lo ? 1ull : 0ull);
-  return r;
-}
-__device__ __forceinline__ U128 shfl_xor_u128(U128 v, int m) {
-  U128 r;
-  r.lo = __shfl_xor_sync(0xffffffffu, v.lo, m);
-  r.hi = __shfl_xor_sync(0xffffffffu, v.hi, m);
   return r;
 }
 __device__ __forceinline__ void atomic_add_u128(U128* dst, U128 v) {
@@ -122,37 +118,16 @@ __device__ __forceinline__ void f_parts(float f, unsigned& s, unsigned& m, int& 
     e = (int)E - 150;
   }
 }
-__device__ __forceinline__ U128 fx_f(float a) {
-  unsigned s, m;
-  int e;
-  f_parts(a, s, m, e);
-  return fx_parts(s, m, e);
-}
-__device__ __forceinline__ U128 fx_ff(float a, float b) {
+// floor(a * b * 2^64) of any two floats
+__device__ __noinline__ U128 fx_ff(float a, float b) {
   unsigned sa, ma, sb, mb;
   int ea, eb;
   f_parts(a, sa, ma, ea);
   f_parts(b, sb, mb, eb);
   return fx_parts(sa ^ sb, (unsigned long long)ma * (unsigned long long)mb, ea + eb);
 }
-__device__ __forceinline__ U128 fx_d(double d) {
-  unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  unsigned s = (unsigned)(b >> 63);
-  int E = (int)((b >> 52) & 0x7ffull);
-  unsigned long long m = b & ((1ull << 52) - 1ull);
-  int e;
-  if (E == 0) {
-    e = -1074;
-  } else {
-    m |= 1ull << 52;
-    e = E - 1075;
-  }
-  return fx_parts(s, m, e);
-}
-
-// floor(d * 2^64) for a non-negative double below 2^52 (the stamp terms dt and dt^2: dt >= 0
-// by construction, dt < 2^16 checked): two clamped shifts instead of fx_parts' branches,
-// the same bits.
+// floor(d * 2^64) for a double 0 <= d < 2^52 (the stamp terms dt and dt^2: dt >= 0 by
+// construction, dt < 2^16 checked): shifts that clamp, no branch.
 __device__ __forceinline__ unsigned long long shl_c(unsigned long long v, unsigned n) {
   unsigned long long r;
   asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));  // n >= 64 gives 0
@@ -165,77 +140,246 @@ __device__ __forceinline__ unsigned long long shr_c(unsigned long long v, unsign
 }
 __device__ __forceinline__ U128 fx_d_nonneg(double d) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const int E = (int)((b >> 52) & 0x7ffull);
-  if ((b >> 63) || E >= 1075) return fx_d(d);  // negative, >= 2^52 or not finite: general path
-  unsigned long long m = b & ((1ull << 52) - 1ull);
-  int sh;  // d * 2^64 = m * 2^sh
-  if (E == 0) {
-    sh = -1074 + 64;
-  } else {
-    m |= 1ull << 52;
-    sh = E - 1075 + 64;
-  }
-  U128 r;  // sh < 64 here
-  r.lo = sh >= 0 ? shl_c(m, (unsigned)sh) : shr_c(m, (unsigned)(-sh));
+  const unsigned long long m = (b & ((1ull << 52) - 1ull)) | (1ull << 52);  // below 2^-63 all bits are shifted out
+  const int sh = (int)(b >> 52) - 1011;                                     // d * 2^64 = m * 2^sh, sh < 64
+  U128 r;
+  r.lo = shl_c(m, (unsigned)sh) | shr_c(m, (unsigned)(-sh));  // one of them is 0, or both are m
   r.hi = shr_c(m, (unsigned)(64 - sh));
   return r;
 }
 
-struct Moments {
-  U128 s[11];
-};
-
-// Fast path of the same floors.  A float x with x == 0 or 2^-25 <= |x| < 2^15 has no
-// bit below 2^-48, so x = X * 2^-48 with an integer |X| < 2^63.  Then
-// floor(x * y * 2^64) = floor(X * Y / 2^32) (an arithmetic shift of the 128-bit
-// product) and floor(x * 2^64) = X * 2^16, both exact.
-__device__ __forceinline__ bool fx_grid48(float x, long long& X) {
-  X = __float2ll_rn(x * 0x1p48f);
+// ---- exact sums of points --------------------------------------------------------------
+// A node's nine sums are floor(v * 2^64) over its points of v = xx, xy, xz, yy, yz, zz, x, y, z:
+// products of two of the four numbers x, y, z, 1.
+//
+// A coordinate that is 0 or at least 2^-17 in magnitude (below 2^15) has no bit below 2^-40:
+// x * 2^40 = h * 2^28 + l with |h|, |l| <= 2^27, both exact.  A product is then
+// (h h') 2^56 + (h l' + l h') 2^28 + l l' in units of 2^-80; only l l' has bits below 2^-64, and
+// clearing its low 16 bits floors the product.  Each part is one multiply-add into a 64-bit
+// sum; 64 points, on the grid or off it, stay below 2^63.  The rare point with a nonzero coordinate below 2^-17
+// takes fx_ff.
+constexpr int kSums = 9;
+// the two factors of product c
+__device__ __forceinline__ int sum_fa(int c) { return c < 6 ? (c < 3 ? 0 : (c < 5 ? 1 : 2)) : c - 6; }
+__device__ __forceinline__ int sum_fb(int c) { return c < 6 ? (c < 3 ? c : (c < 5 ? c - 2 : 2)) : 3; }
+__device__ __forceinline__ bool limbs40(float x, int2& w) {
+  const float y = x * 4096.0f;  // exact
+  w.x = __float2int_rn(y);
+  w.y = __float2int_rn((y - (float)w.x) * 0x1p28f);  // the difference is exact
   const float a = fabsf(x);
-  return a == 0.0f || a >= 0x1p-25f;
+  return a == 0.0f || a >= 0x1p-17f;
 }
-__device__ __forceinline__ U128 fx_prod48(long long X, long long Y) {
-  const unsigned long long lo = (unsigned long long)X * (unsigned long long)Y;
-  const long long hi = __mul64hi(X, Y);
-  U128 r;
-  r.lo = (lo >> 32) | ((unsigned long long)hi << 32);
-  r.hi = (unsigned long long)(hi >> 32);
-  return r;
-}
-__device__ __forceinline__ U128 fx_single48(long long X) {
-  U128 r;
-  r.lo = (unsigned long long)X << 16;
-  r.hi = (unsigned long long)(X >> 48);
-  return r;
+// (hh 2^56 + mid 2^28 + ll) / 2^16, ll a multiple of 2^16
+__device__ __forceinline__ U128 limb_total(long long hh, long long mid, long long ll) {
+  U128 q, m;
+  q.lo = (unsigned long long)hh << 40;
+  q.hi = (unsigned long long)(hh >> 24);
+  m.lo = (unsigned long long)mid << 12;
+  m.hi = (unsigned long long)(mid >> 52);
+  q = u128_add(q, m);
+  m.lo = (unsigned long long)(ll >> 16);
+  m.hi = (unsigned long long)(ll >> 63);
+  return u128_add(q, m);
 }
 
-__device__ __forceinline__ void moments_add_point(Moments& M, float4 p, double st, double ts0) {
-  long long X, Y, Z;
-  const bool gx = fx_grid48(p.x, X), gy = fx_grid48(p.y, Y), gz = fx_grid48(p.z, Z);
-  if (gx && gy && gz) {
-    M.s[0] = u128_add(M.s[0], fx_prod48(X, X));
-    M.s[1] = u128_add(M.s[1], fx_prod48(X, Y));
-    M.s[2] = u128_add(M.s[2], fx_prod48(X, Z));
-    M.s[3] = u128_add(M.s[3], fx_prod48(Y, Y));
-    M.s[4] = u128_add(M.s[4], fx_prod48(Y, Z));
-    M.s[5] = u128_add(M.s[5], fx_prod48(Z, Z));
-    M.s[6] = u128_add(M.s[6], fx_single48(X));
-    M.s[7] = u128_add(M.s[7], fx_single48(Y));
-    M.s[8] = u128_add(M.s[8], fx_single48(Z));
-  } else {
-    M.s[0] = u128_add(M.s[0], fx_ff(p.x, p.x));
-    M.s[1] = u128_add(M.s[1], fx_ff(p.x, p.y));
-    M.s[2] = u128_add(M.s[2], fx_ff(p.x, p.z));
-    M.s[3] = u128_add(M.s[3], fx_ff(p.y, p.y));
-    M.s[4] = u128_add(M.s[4], fx_ff(p.y, p.z));
-    M.s[5] = u128_add(M.s[5], fx_ff(p.z, p.z));
-    M.s[6] = u128_add(M.s[6], fx_f(p.x));
-    M.s[7] = u128_add(M.s[7], fx_f(p.y));
-    M.s[8] = u128_add(M.s[8], fx_f(p.z));
+// Sums of small sets by one warp: the set's points are staged in shared memory as limbs, lane
+// c < 27 forms product c % 9 of every third point, so a lane holds one sum, not nine, only
+// points of the set cost anything, and the warp total is two exchanges.  Points off the grid
+// are staged as they are, from the other end.
+constexpr int kStage = 64;  // points staged per warp
+struct __align__(16) SumStage {  // a point's first two limb pairs are stored as one 16 B word
+  int2 w[kStage][4];  // limbs (h, l) of x, y, z, 1
+};
+struct WarpSums {
+  U128 v;   // lane c < 27: its product's sum
+  int cnt;  // points staged as limbs
+  int odd;  // and as floats
+};
+__device__ __forceinline__ void stage_init(SumStage& sg, int lane) {
+  for (int k = lane; k < kStage; k += 32) sg.w[k][3] = make_int2(1 << 12, 0);
+  __syncwarp();
+}
+__device__ __forceinline__ void sums_zero(WarpSums& S) {
+  S.v = u128_zero();
+  S.cnt = S.odd = 0;
+}
+// Adds the staged points to the lanes' sums (whole warp, staged points visible).
+__device__ __forceinline__ void sums_flush(WarpSums& S, const SumStage& sg, int lane) {
+  const int c = lane % 9;
+  const int2* pa = &sg.w[0][sum_fa(c)];
+  const int2* pb = &sg.w[0][sum_fb(c)];
+  long long hh = 0, mid = 0, ll = 0;
+#pragma unroll 2
+  for (int i = lane < 27 ? lane / 9 : S.cnt; i < S.cnt; i += 3) {
+    const int2 a = pa[4 * i], b = pb[4 * i];
+    hh += (long long)a.x * b.x;
+    mid += (long long)a.x * b.y;
+    mid += (long long)a.y * b.x;
+    ll += ((long long)a.y * b.y) & ~0xffffll;
   }
-  double dt = st - ts0;
-  M.s[9] = u128_add(M.s[9], fx_d_nonneg(dt));
-  M.s[10] = u128_add(M.s[10], fx_d_nonneg(dt * dt));
+  S.v = u128_add(S.v, limb_total(hh, mid, ll));
+  for (int k = lane < 27 ? lane / 9 : S.odd; k < S.odd; k += 3) {
+    const float4 f = *reinterpret_cast<const float4*>(sg.w[kStage - 1 - k]);
+    const int a = sum_fa(c), b = sum_fb(c);
+    S.v = u128_add(S.v, fx_ff(a == 0 ? f.x : (a == 1 ? f.y : f.z),
+                              b == 0 ? f.x : (b == 1 ? f.y : (b == 2 ? f.z : 1.0f))));
+  }
+  S.cnt = S.odd = 0;
+}
+// Adds the points p of the lanes with add set (whole warp; room for 32 more staged points is
+// the caller's to keep).
+__device__ __forceinline__ void sums_add(WarpSums& S, SumStage& sg, bool add, float4 p, int lane) {
+  int2 wx, wy, wz;
+  const bool ox = limbs40(p.x, wx), oy = limbs40(p.y, wy), oz = limbs40(p.z, wz);
+  const bool on = ox && oy && oz;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned bm = __ballot_sync(0xffffffffu, add && on), bo = __ballot_sync(0xffffffffu, add && !on);
+  if (add) {
+    int2* w = sg.w[on ? S.cnt + __popc(bm & lt) : kStage - 1 - S.odd - __popc(bo & lt)];
+    *reinterpret_cast<int4*>(w) = on ? make_int4(wx.x, wx.y, wy.x, wy.y)
+                                     : make_int4(__float_as_int(p.x), __float_as_int(p.y), __float_as_int(p.z), 0);
+    if (on) w[2] = wz;
+  }
+  S.cnt += __popc(bm);
+  S.odd += __popc(bo);
+}
+// Flushes if more than `most` points are staged.
+__device__ __forceinline__ void sums_room(WarpSums& S, const SumStage& sg, int most, int lane) {
+  if (S.cnt + S.odd <= most) return;
+  __syncwarp();
+  sums_flush(S, sg, lane);
+  __syncwarp();
+}
+// The warp's totals: lane k < 9 returns sum k.  S starts anew.
+__device__ __forceinline__ U128 sums_total(WarpSums& S, const SumStage& sg, int lane) {
+  __syncwarp();
+  sums_flush(S, sg, lane);
+  __syncwarp();
+  const U128 q = S.v;  // lanes c, c + 9 and c + 18 hold product c
+  U128 r, u;
+  r.lo = __shfl_down_sync(0xffffffffu, q.lo, 9);
+  r.hi = __shfl_down_sync(0xffffffffu, q.hi, 9);
+  u.lo = __shfl_down_sync(0xffffffffu, q.lo, 18);
+  u.hi = __shfl_down_sync(0xffffffffu, q.hi, 18);
+  sums_zero(S);
+  return u128_add(q, u128_add(r, u));
+}
+
+// Sums of large sets: each lane keeps the three parts of its own points' products (no
+// staging, nine independent chains), folded into the warp's totals every kLanePoints points
+// per lane at most.
+constexpr int kLanePoints = 64;
+struct LaneSums {
+  long long hh[6], mid[6], ll[6];
+  long long s[3];   // x, y, z in units of 2^-40
+  unsigned sl[3];   // and what lies below, in units of 2^-64 (points off the grid)
+  U128 tot;         // lane k < 9: the warp's sum k
+};
+__device__ __forceinline__ void lane_zero(LaneSums& S) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) S.hh[k] = S.mid[k] = S.ll[k] = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    S.s[k] = 0;
+    S.sl[k] = 0u;
+  }
+}
+// Adds the point p of the lanes with add set (whole warp).
+__device__ __forceinline__ void lane_add(LaneSums& S, bool add, float4 p, int lane) {
+  int2 w[3];
+  const bool ox = limbs40(p.x, w[0]), oy = limbs40(p.y, w[1]), oz = limbs40(p.z, w[2]);
+  const bool on = ox && oy && oz;
+  unsigned odd = __ballot_sync(0xffffffffu, add && !on);
+  if (add && on) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const int2 a = w[c < 3 ? 0 : (c < 5 ? 1 : 2)], b = w[c < 3 ? c : (c < 5 ? c - 2 : 2)];
+      S.hh[c] += (long long)a.x * b.x;
+      if (c == 0 || c == 3 || c == 5) {
+        S.mid[c] += (long long)a.x * (2 * b.y);
+      } else {
+        S.mid[c] += (long long)a.x * b.y;
+        S.mid[c] += (long long)a.y * b.x;
+      }
+      S.ll[c] += ((long long)a.y * b.y) & ~0xffffll;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      S.s[k] += (long long)w[k].x * (1 << 28);
+      S.s[k] += w[k].y;
+    }
+  }
+  if (!odd) return;
+  // Off the grid.  A few points (a map's ground near z = 0): one by one, lane c < 9 forming
+  // product c.
+  if (__popc(odd) <= 4) {
+    while (odd) {
+      const int src = __ffs(odd) - 1;
+      odd &= odd - 1;
+      const float f0 = __shfl_sync(0xffffffffu, p.x, src), f1 = __shfl_sync(0xffffffffu, p.y, src);
+      const float f2 = __shfl_sync(0xffffffffu, p.z, src);
+      if (lane < 9) {
+        const int a = sum_fa(lane), b = sum_fb(lane);
+        S.tot = u128_add(S.tot, fx_ff(a == 0 ? f0 : (a == 1 ? f1 : f2),
+                                      b == 0 ? f0 : (b == 1 ? f1 : (b == 2 ? f2 : 1.0f))));
+      }
+    }
+    return;
+  }
+  // Many (a scan's column along an axis brings 128 in a row): the lanes together, whole
+  // values split over the same parts.
+  if (!add || on) return;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const U128 v = fx_ff(c < 3 ? p.x : (c < 5 ? p.y : p.z), c == 0 ? p.x : (c == 1 || c == 3 ? p.y : p.z));
+    S.hh[c] += (long long)((v.lo >> 40) | (v.hi << 24));
+    S.ll[c] += (long long)((v.lo & 0xffffffffffull) << 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const U128 v = fx_ff(k == 0 ? p.x : (k == 1 ? p.y : p.z), 1.0f);
+    S.s[k] += (long long)((v.lo >> 24) | (v.hi << 40));
+    S.sl[k] += (unsigned)v.lo & 0xffffffu;
+  }
+}
+__device__ __forceinline__ U128 shfl_xor_u128(U128 v, int m) {
+  U128 r;
+  r.lo = __shfl_xor_sync(0xffffffffu, v.lo, m);
+  r.hi = __shfl_xor_sync(0xffffffffu, v.hi, m);
+  return r;
+}
+// Folds the lanes' parts into the warp's totals.  Reduce-scatter: 16 slots (9 used) halved
+// over lane bits 4..1, then added with lane ^ 1, so lanes 2k and 2k + 1 hold total k.
+__device__ __forceinline__ void lane_fold(LaneSums& S, int lane) {
+  U128 v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = u128_zero();
+#pragma unroll
+  for (int k = 0; k < 6; ++k) v[k] = limb_total(S.hh[k], S.mid[k], S.ll[k]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // x * 2^40 to units of 2^-64
+    U128 q;
+    q.lo = S.sl[k];
+    q.hi = 0ull;
+    v[6 + k].lo = (unsigned long long)S.s[k] << 24;
+    v[6 + k].hi = (unsigned long long)(S.s[k] >> 40);
+    v[6 + k] = u128_add(v[6 + k], q);
+  }
+  U128 w8[8], w4[4], w2[2];
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w8[j] = u128_add(b4 ? v[8 + j] : v[j], shfl_xor_u128(b4 ? v[j] : v[8 + j], 16));
+#pragma unroll
+  for (int j = 0; j < 4; ++j) w4[j] = u128_add(b3 ? w8[4 + j] : w8[j], shfl_xor_u128(b3 ? w8[j] : w8[4 + j], 8));
+#pragma unroll
+  for (int j = 0; j < 2; ++j) w2[j] = u128_add(b2 ? w4[2 + j] : w4[j], shfl_xor_u128(b2 ? w4[j] : w4[2 + j], 4));
+  U128 w1 = u128_add(b1 ? w2[1] : w2[0], shfl_xor_u128(b1 ? w2[0] : w2[1], 2));
+  w1 = u128_add(w1, shfl_xor_u128(w1, 1));
+  U128 q;
+  q.lo = __shfl_sync(0xffffffffu, w1.lo, (2 * lane) & 31);
+  q.hi = __shfl_sync(0xffffffffu, w1.hi, (2 * lane) & 31);
+  if (lane < kSums) S.tot = u128_add(S.tot, q);
+  lane_zero(S);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,7 +395,6 @@ struct BNode {
   int32_t has_prop;   // propagated normal handed to the children
   int32_t parent;     // parent node, -1 for a root
   float mean[3], dir[3];
-  double dts_mean, dts_cov;
   double prop[3];
   double par_prop[3];
 };
@@ -343,23 +486,19 @@ __device__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
 // FlatLeafPolicy_::fillMetadata over CountLeafPolicy_ and LabelPolicyBase_
 // (kd/tree/flat_leaf_policy_.h:52-108, count_leaf_policy_.h:27-43,
 // label_policy_base_impl_.h:12-97) on FP64 statistics.
-// Sd: the node's 11 moment sums converted to double (fx_to_d of the exact sums).
+// Sd: the node's nine moment sums converted to double (fx_to_d of the exact sums).
 // root (nullable): for a root node, its frame as TreeCPU_'s constructor stores it
 // (kd/tree/tree_cpu_.h:72-86): [0..2] eigenvalues ascending, [3..11] eigenvectors
 // column-major (columns 0 and 2 reoriented as in fillMetadata, then column 0 negated if
 // the determinant is negative), [12..14] mean; zero where the node has < 3 points.
 __device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, const BuildParams& P, double* root) {
   for (int i = 0; i < 3; ++i) { nd.mean[i] = 0.f; nd.dir[i] = 0.f; }
-  nd.dts_mean = 0.0;
-  nd.dts_cov = 0.0;
   double mean_d[3] = {0, 0, 0};
   double e0[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
   double lam[3] = {0, 0, 0};
   bool is_bad = true;
   if (n > 0) {
     double dn = (double)n;
-    nd.dts_mean = Sd[9] / dn;
-    nd.dts_cov = Sd[10] / dn - nd.dts_mean * nd.dts_mean;
     for (int i = 0; i < 3; ++i) mean_d[i] = Sd[6 + i] / dn;
     for (int i = 0; i < 3; ++i) nd.mean[i] = (float)mean_d[i];
     if (n >= 3) {
@@ -511,14 +650,11 @@ __device__ __forceinline__ void level_range(const LevelState* ls, int& b, int& e
 // ---------------------------------------------------------------------------
 // Kernels
 
-__global__ void k_ingest(const float* xyz, const double* st, int64_t n, float4* pts, double* sts, LevelState* ls) {
+__global__ void k_ingest(const float* xyz, int64_t n, float4* pts, LevelState* ls) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
-    double s = st ? st[i] : 0.0;
-    bool ok = fabsf(x) < 32768.f && fabsf(y) < 32768.f && fabsf(z) < 32768.f && isfinite(s);
-    if (!ok) ls->error = 2;
+    if (!(fabsf(x) < 32768.f && fabsf(y) < 32768.f && fabsf(z) < 32768.f)) ls->error = 2;
     pts[i] = make_float4(x, y, z, __int_as_float((int32_t)i));
-    sts[i] = s;
   }
 }
 
@@ -543,15 +679,19 @@ __global__ void k_tree_min(const double* sts, const int64_t* off, unsigned long 
   if ((threadIdx.x & 31) == 0 && m != ~0ull) atomicMin(&tsmin[r], m);
 }
 
-// decodes ts_start and checks the dt range of every point; blockIdx.y = tree.
+// decodes ts_start, checks every point's stamp and writes its dt; blockIdx.y = tree.
 __global__ void k_tree_check(const double* sts, const int64_t* off, const unsigned long long* tsmin, double* ts0,
-                             LevelState* ls) {
+                             double* dt, LevelState* ls) {
   const int r = blockIdx.y;
   const int64_t b = off[r], e = off[r + 1];
   const double t0 = (e > b) ? dkey_inv(tsmin[r]) : 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) ts0[r] = t0;
-  for (int64_t i = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e; i += (int64_t)gridDim.x * blockDim.x)
-    if (!(sts[i] - t0 < 65536.0)) ls->error = 2;
+  for (int64_t i = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e; i += (int64_t)gridDim.x * blockDim.x) {
+    const double s = sts[i];
+    const double d = s - t0;
+    if (!(isfinite(s) && d < 65536.0)) ls->error = 2;
+    dt[i] = d;
+  }
 }
 
 __global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState* ls, int32_t* level_begin) {
@@ -578,15 +718,15 @@ __global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState
 }
 
 // A point moves through the levels as one 16 B record (x, y, z, w = its input index as int
-// bits), double-buffered by level parity; its stamp stays in input order and is read by
-// index where a sum needs it.
+// bits), double-buffered by level parity.  The stamps stay out of the levels: no decision
+// needs them, and once the final point order is known every node's dt sums are differences
+// of prefix sums over it (k_dt_prefix).
 struct PointBufs {
   float4* p[2];
-  double* st;     // stamps, input order
   int32_t* perm;  // final point order (global indices)
 };
 
-// Every node's 11 exact moment sums are kept in mom[node].  The roots' sums are
+// Every node's nine exact moment sums are kept in mom[node].  The roots' sums are
 // computed from their points; a split node hands its children their sums: the smaller
 // child's from one pass over its points after the partition, the other's as the
 // parent's minus the smaller's (exact integer arithmetic).  So below the roots each point
@@ -595,63 +735,25 @@ struct PointBufs {
 // L1 prefetch of the line holding p (no register, no effect on results).
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-// Warp-cooperative exact sums of points [b, e) of one point buffer.
-// Warp total of the 11 sums in reduce-scatter form: the 16 slots (11 used) are halved
-// over lane bits 4..1 (8 + 4 + 2 + 1 exchanges instead of 5 x 11), then added with
-// lane ^ 1.  Lanes 2k and 2k + 1 return the total of sum k (k < 11; slots 11-15 are 0).
-__device__ __forceinline__ U128 warp_sum_moments(const Moments& M, int lane) {
-  U128 v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = k < 11 ? M.s[k] : u128_zero();
-  U128 w8[8], w4[4], w2[2];
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) w8[j] = u128_add(b4 ? v[8 + j] : v[j], shfl_xor_u128(b4 ? v[j] : v[8 + j], 16));
-#pragma unroll
-  for (int j = 0; j < 4; ++j) w4[j] = u128_add(b3 ? w8[4 + j] : w8[j], shfl_xor_u128(b3 ? w8[j] : w8[4 + j], 8));
-#pragma unroll
-  for (int j = 0; j < 2; ++j) w2[j] = u128_add(b2 ? w4[2 + j] : w4[j], shfl_xor_u128(b2 ? w4[j] : w4[2 + j], 4));
-  U128 w1 = u128_add(b1 ? w2[1] : w2[0], shfl_xor_u128(b1 ? w2[0] : w2[1], 2));
-  return u128_add(w1, shfl_xor_u128(w1, 1));
-}
-
-// Sums of the points [b, e) by one warp; returns warp_sum_moments of them.
-__device__ __forceinline__ U128 warp_moments(const float4* p, const double* st, int b, int e, double t0, int lane) {
-  constexpr int U = 2;  // loads in flight per lane (the 11 sums already hold 44 registers)
-  Moments M;
-  for (int k = 0; k < 11; ++k) M.s[k] = u128_zero();
-  for (int k0 = b; k0 < e; k0 += 32 * U) {
-    float4 pv[U];
-    double sv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = k0 + u * 32 + lane;
-      if (i < e) pv[u] = p[i];
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = k0 + u * 32 + lane;
-      if (i < e) sv[u] = st[__float_as_int(pv[u].w)];
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = k0 + u * 32 + lane;
-      if (i < e) moments_add_point(M, pv[u], sv[u], t0);
-    }
-  }
-  return warp_sum_moments(M, lane);
-}
-
 // Level 0: warp per root of at most kBig points.
-__global__ void __launch_bounds__(kThreads) k_root_moments(const BNode* nodes, int R, PointBufs B, const double* ts0,
-                                                           U128* mom) {
+__global__ void __launch_bounds__(kThreads) k_root_moments(const BNode* nodes, int R, PointBufs B, U128* mom) {
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
+  static_assert(kBig <= 32 * kLanePoints, "a root's points fit the lanes' sums");
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < R; r += nw) {
     const int s = nodes[r].start, e = nodes[r].end;
     if (e - s > kBig) continue;
-    const U128 q = warp_moments(B.p[0], B.st, s, e, ts0[nodes[r].tree], lane);
-    if (!(lane & 1) && lane < 22) mom[(size_t)r * 11 + (lane >> 1)] = q;
+    LaneSums S;
+    lane_zero(S);
+    S.tot = u128_zero();
+    for (int k0 = s; k0 < e; k0 += 32) {
+      const int i = k0 + lane;
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < e) p = B.p[0][i];
+      lane_add(S, i < e, p, lane);
+    }
+    lane_fold(S, lane);
+    if (lane < kSums) mom[(size_t)r * kSums + lane] = S.tot;
   }
 }
 
@@ -667,8 +769,8 @@ __global__ void k_decide(BNode* nodes, const LevelState* ls, const U128* mom, Bu
   for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
     BNode nd = nodes[i];
     const int n = nd.end - nd.start;
-    double Sd[11];
-    for (int k = 0; k < 11; ++k) Sd[k] = fx_to_d(mom[(size_t)i * 11 + k]);
+    double Sd[kSums];
+    for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(mom[(size_t)i * kSums + k]);
     decide(Sd, n, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
     nodes[i] = nd;
     v += nd.split ? 1 : 0;
@@ -736,31 +838,37 @@ static_assert(offsetof(BNode, start) == 0 && offsetof(BNode, end) == 4 && offset
 // Warp per node of at most kBig points, after its children are numbered: stable
 // partition by whichSide (or leaf point order), the children's ranges and sums.
 // Latency-bound at deep levels (many small nodes per warp), so each node's record
-// and sums are fetched in one round of loads, one node ahead.
-__global__ void __launch_bounds__(kThreads, 2) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
-                                                         const double* ts0, U128* mom, const int32_t* bsum,
-                                                         int nblocks, int32_t* level_begin, unsigned* done) {
+// and sums are fetched in one round of loads, one node ahead.  The staged sums
+// (SumStage) leave room for 24 warps per SM: a level of 11.4M points in small nodes takes
+// 298 us at most; with eleven 128-bit terms per lane (124 registers, 16 warps) it took 510.
+__global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
+                                                         U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin,
+                                                         unsigned* done) {
   const int lb = ls->lb, le = ls->le, cur = ls->cur;
   const float4* pin = B.p[cur];
-  const double* sts = B.st;
   float4* pout = B.p[cur ^ 1];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int wslot = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // consecutive nodes on different SMs
-  const bool sum_lane = !(lane & 1) && lane < 22;                  // holds sum lane / 2
+  const bool sum_lane = lane < kSums;                              // holds sum lane
+  __shared__ SumStage stage[kThreads / 32];
+  SumStage& sg = stage[threadIdx.x >> 5];
+  stage_init(sg, lane);
+  WarpSums S;
+  sums_zero(S);
   int maxc = 0;
   int word = 0;
   U128 pm = u128_zero();
   auto fetch = [&](int ni) {
     if (ni < le) {
       if (lane < kNodeHeadWords) word = reinterpret_cast<const int*>(nodes + ni)[lane];
-      if (sum_lane) pm = mom[(size_t)ni * 11 + (lane >> 1)];
+      if (sum_lane) pm = mom[(size_t)ni * kSums + lane];
     }
   };
   fetch(lb + wslot);
   for (int ni = lb + wslot; ni < le; ni += nwarps) {
     const int s = __shfl_sync(0xffffffffu, word, 0), e = __shfl_sync(0xffffffffu, word, 1);
-    const int tree = __shfl_sync(0xffffffffu, word, 3), split = __shfl_sync(0xffffffffu, word, 4);
+    const int split = __shfl_sync(0xffffffffu, word, 4);
     const int li = __shfl_sync(0xffffffffu, word, 6), ri = __shfl_sync(0xffffffffu, word, 7);
     float mean[3], dir[3];
 #pragma unroll
@@ -796,7 +904,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_part(BNode* nodes, LevelS
       for (int u = 0; u < kUnroll; ++u) {
         int i = s + ((k0 + u) << 5) + lane;
         if (i < e) {
-          prefetch_l1(sts + __float_as_int(pv[u].w));  // the stamp, if this point lands in the smaller child
           if (which_side_f(mean, dir, pv[u])) bits |= 1u << (k0 + u);
         }
       }
@@ -806,9 +913,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_part(BNode* nodes, LevelS
     const int mid = s + nl;
     // the smaller child is summed while its points move; the other is the parent minus it
     const bool small_left = mid - s <= e - mid;
-    const double t0 = ts0[tree];
-    Moments MS;
-    for (int k = 0; k < 11; ++k) MS.s[k] = u128_zero();
     const unsigned lt = (1u << lane) - 1u;
     int cl = 0, cr = 0;
     for (int k0 = 0; k0 < K; k0 += kUnroll) {
@@ -827,18 +931,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_part(BNode* nodes, LevelS
         if (valid) {
           int dst = left ? (s + cl + __popc(bl & lt)) : (s + nl + cr + __popc(br & lt));
           pout[dst] = pv[u];
-          if (left == small_left) moments_add_point(MS, pv[u], sts[__float_as_int(pv[u].w)], t0);
         }
+        sums_add(S, sg, valid && left == small_left, pv[u], lane);
         cl += __popc(bl);
         cr += __popc(br);
       }
+      sums_room(S, sg, kStage - 32 * kUnroll, lane);
     }
-    const U128 q = warp_sum_moments(MS, lane);
+    const U128 q = sums_total(S, sg, lane);
     if (sum_lane) {
-      const int k = lane >> 1;
       const U128 other = u128_sub(psum, q);
-      mom[(size_t)li * 11 + k] = small_left ? q : other;
-      mom[(size_t)ri * 11 + k] = small_left ? other : q;
+      mom[(size_t)li * kSums + lane] = small_left ? q : other;
+      mom[(size_t)ri * kSums + lane] = small_left ? other : q;
     }
     if (lane == 0) {
       nodes[ni].mid = mid;
@@ -941,9 +1045,9 @@ __global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bb
       node_chunk0[carry_b + ob] = carry_c + oc;
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < tb * 11; k += blockDim.x) {
-      acc[(size_t)carry_b * 11 + k] = u128_zero();
-      accl[(size_t)carry_b * 11 + k] = u128_zero();
+    for (int k = threadIdx.x; k < tb * kSums; k += blockDim.x) {
+      acc[(size_t)carry_b * kSums + k] = u128_zero();
+      accl[(size_t)carry_b * kSums + k] = u128_zero();
     }
     for (int c = threadIdx.x; c < tc; c += blockDim.x) {
       int lo = 0, hi = tb;  // the last listed node whose first chunk is at or before c
@@ -973,13 +1077,19 @@ __global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bb
   }
 }
 
-// Block sum of per-thread sums into one 128-bit accumulator set (any order: exact).
-__device__ __forceinline__ void block_add_moments(const Moments& M, U128 (*sm)[11], U128* dst) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const U128 q = warp_sum_moments(M, lane);
-  if (!(lane & 1) && lane < 22) sm[w][lane >> 1] = q;
+// Block sum of the warps' sums into one 128-bit accumulator set (any order: exact).
+// alone: the block has one chunk only (a small level, where latency counts): each warp adds
+// its own.
+__device__ __forceinline__ void block_add_sums(LaneSums& S, int lane, U128 (*sm)[kSums], U128* dst, bool alone) {
+  lane_fold(S, lane);
+  if (alone) {
+    if (lane < kSums) atomic_add_u128(&dst[lane], S.tot);
+    return;
+  }
+  if (lane < kSums) sm[threadIdx.x >> 5][lane] = S.tot;
+  S.tot = u128_zero();
   __syncthreads();
-  if (threadIdx.x < 11) {
+  if (threadIdx.x < kSums) {
     U128 t = u128_zero();
     for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) t = u128_add(t, sm[ww][threadIdx.x]);
     atomic_add_u128(&dst[threadIdx.x], t);
@@ -987,58 +1097,97 @@ __device__ __forceinline__ void block_add_moments(const Moments& M, U128 (*sm)[1
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) k_big_moments(const Chunk* chunks, const LevelState* ls,
-                                                          const PointBufs B, const double* ts0, const BNode* nodes,
-                                                          U128* acc) {
-  __shared__ U128 sm[kThreads / 32][11];
-  const int nc = ls->num_chunks, cur = ls->cur;
-  const float4* pts = B.p[cur];
-  const double* st = B.st;
-  for (int ci = blockIdx.x; ci < nc; ci += gridDim.x) {
-    Chunk c = chunks[ci];
-    double t0 = ts0[nodes[c.node].tree];
-    Moments M;
-    for (int k = 0; k < 11; ++k) M.s[k] = u128_zero();
-    for (int i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) {
-      const float4 pp = pts[i];
-      moments_add_point(M, pp, st[__float_as_int(pp.w)], t0);
+constexpr int kSegs = kThreads / 32;     // 128-point segments per chunk, one per warp of a block
+constexpr int kPer = kChunk / kThreads;  // rounds of 32 points per segment
+constexpr int kFoldChunks = kLanePoints / kPer;
+static_assert(kPer * kThreads == kChunk && kSegs == 8, "a chunk is eight segments, its counts one 16 B word");
+
+// Level 0: the large roots' sums; a block takes a contiguous range of chunks and adds its
+// sums once per root.
+__global__ void __launch_bounds__(kThreads, 2) k_big_moments(const Chunk* chunks, const LevelState* ls,
+                                                             const PointBufs B, U128* acc) {
+  __shared__ U128 sm[kSegs][kSums];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  LaneSums S;
+  lane_zero(S);
+  S.tot = u128_zero();
+  const int nc = ls->num_chunks;
+  const float4* pts = B.p[ls->cur];
+  const int per = (nc + gridDim.x - 1) / gridDim.x;
+  const int c0 = blockIdx.x * per, c1 = min(c0 + per, nc);
+  int big = -1, held = 0;
+  for (int ci = c0; ci < c1; ++ci) {
+    const Chunk c = chunks[ci];
+    if (c.big != big) {
+      if (big >= 0) block_add_sums(S, lane, sm, acc + (size_t)big * kSums, false);
+      big = c.big;
+      held = 0;
+    } else if (++held == kFoldChunks) {
+      lane_fold(S, lane);
+      held = 0;
     }
-    block_add_moments(M, sm, acc + (size_t)c.big * 11);
+    float4 pv[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = c.begin + (w * kPer + u) * 32 + lane;
+      if (i < c.end) pv[u] = pts[i];
+    }
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int u = 0; u < kPer / 2; ++u)
+        lane_add(S, c.begin + (w * kPer + 2 * h + u) * 32 + lane < c.end, h ? pv[2 + u] : pv[u], lane);
+    }
   }
+  if (big >= 0) block_add_sums(S, lane, sm, acc + (size_t)big * kSums, per == 1);
 }
 
 // Level 0: the sums of the large roots, from the chunk accumulators.
 __global__ void k_big_to_mom(const LevelState* ls, const int32_t* big_list, const U128* acc, U128* mom) {
   const int nb = ls->num_big;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * 11; t += gridDim.x * blockDim.x)
-    mom[(size_t)big_list[t / 11] * 11 + t % 11] = acc[t];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * kSums; t += gridDim.x * blockDim.x)
+    mom[(size_t)big_list[t / kSums] * kSums + t % kSums] = acc[t];
 }
 
-__global__ void k_big_count(const Chunk* chunks, const LevelState* ls, const BNode* nodes, const PointBufs B,
-                            int32_t* chunk_nl) {
-  __shared__ int cnt;
+// Left points of each chunk's eight 128-point segments; a warp per segment, no barrier.
+struct __align__(16) SegCounts {
+  uint16_t n[kSegs];
+};
+__global__ void __launch_bounds__(kThreads) k_big_count(const Chunk* chunks, const LevelState* ls, const BNode* nodes,
+                                                        const PointBufs B, SegCounts* seg) {
   const int nc = ls->num_chunks;
   const float4* pts = B.p[ls->cur];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int ci = blockIdx.x; ci < nc; ci += gridDim.x) {
-    Chunk c = chunks[ci];
+    const Chunk c = chunks[ci];
     const BNode& nd = nodes[c.node];
-    if (threadIdx.x == 0) cnt = 0;
-    __syncthreads();
-    int local = 0;
-    if (nd.split)
-      for (int i = c.begin + threadIdx.x; i < c.end; i += blockDim.x)
-        local += which_side_f(nd.mean, nd.dir, pts[i]) ? 1 : 0;
-    atomicAdd(&cnt, local);
-    __syncthreads();
-    if (threadIdx.x == 0) chunk_nl[ci] = cnt;
-    __syncthreads();
+    int nl = 0;
+    if (nd.split) {
+      const int wb = c.begin + w * 32 * kPer;
+      float4 pv[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        if (wb + u * 32 + lane < c.end) pv[u] = pts[wb + u * 32 + lane];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        nl += __popc(__ballot_sync(0xffffffffu, wb + u * 32 + lane < c.end && which_side_f(nd.mean, nd.dir, pv[u])));
+    }
+    if (lane == 0) seg[ci].n[w] = (uint16_t)nl;
   }
+}
+// The eight counts of a chunk, and their sum before segment w (w = 8: of all).
+__device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < kSegs; ++k)
+    if (k < w) n += s.n[k];
+  return n;
 }
 
 // Block per large node: the exclusive scan of its chunks' left counts (each chunk's left
 // offset inside the node), then the node's split point and its children's ranges.
 __global__ void k_big_offsets(BNode* nodes, LevelState* ls, const int32_t* big_list,
-                              const int32_t* node_chunk0, const int32_t* chunk_nl, int32_t* chunk_loff) {
+                              const int32_t* node_chunk0, const SegCounts* seg, int32_t* chunk_loff) {
   __shared__ int sm[32];
   const int nb = ls->num_big, nc = ls->num_chunks;
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -1047,7 +1196,7 @@ __global__ void k_big_offsets(BNode* nodes, LevelState* ls, const int32_t* big_l
     int carry = 0;
     for (int base = c0; base < c1; base += blockDim.x) {
       const int c = base + threadIdx.x;
-      const int v = c < c1 ? chunk_nl[c] : 0;
+      const int v = c < c1 ? seg_before(seg[c], kSegs) : 0;
       int tot;
       const int ex = block_scan(v, sm, &tot);
       if (c < c1) chunk_loff[c] = carry + ex;
@@ -1067,107 +1216,95 @@ __global__ void k_big_offsets(BNode* nodes, LevelState* ls, const int32_t* big_l
   }
 }
 
-// Stable scatter of one chunk by warp ballots: warp w of the block moves points
-// [begin + 128 w, begin + 128 (w + 1)) in four rounds of 32, so left and right runs are
-// written contiguously.  The points that go to the node's smaller child are summed on
-// the way (the sums of the large node's smaller child).  A block takes a contiguous range
-// of chunks and keeps each thread's sums in registers until the range reaches another
-// node, so the warp reduction and the 128-bit atomics come once per block and node
-// (a reduction and 22 atomics per warp and chunk before: 711 us on the 11.4M-point root,
-// where every warp hits the same 22 words, and 235-310 us on the levels below).
-__global__ void __launch_bounds__(kThreads) k_big_scatter(const Chunk* chunks, const LevelState* ls,
-                                                          const BNode* nodes, PointBufs B,
-                                                          const int32_t* chunk_loff, const double* ts0, U128* accl) {
-  constexpr int kPer = kChunk / kThreads;  // rounds of 32 points per warp
-  constexpr int kWarpsB = kThreads / 32;
-  static_assert(kPer * kThreads == kChunk, "chunk = block x rounds");
-  __shared__ int swl[2][kWarpsB];  // left counts of the chunk's warps, by chunk parity
+// Stable scatter by warp ballots: warp w of a block moves segment w of each of its chunks, in
+// four rounds of 32 points, so left and right runs are written contiguously.  The points
+// that go to the node's smaller child are summed on the way (the sums of the large node's
+// smaller child).  A block takes a contiguous range of chunks and its warps keep their sums
+// until the range reaches another node: only there do they meet, for one block total and 9
+// atomics.  Bound by issue and memory together: a level of 11.4M points takes 100 us (3.6 TB/s
+// of records read and written).  With eleven 128-bit terms per lane, reduced per warp and
+// chunk and added with 22 atomics each, it took 235-310 us, and 691 us on the root, where
+// every warp hits the same words; three blocks per SM spill and take 118 us.
+__global__ void __launch_bounds__(kThreads, kScatterPerSM)
+    k_big_scatter(const Chunk* chunks, const LevelState* ls, const BNode* nodes, PointBufs B, const SegCounts* seg,
+                  const int32_t* chunk_loff, U128* accl) {
+  __shared__ U128 smm[kSegs][kSums];
   const int nc = ls->num_chunks, cur = ls->cur;
   const float4* pin = B.p[cur];
-  const double* sts = B.st;
   float4* pout = B.p[cur ^ 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  __shared__ U128 smm[kWarpsB][11];
-  int par = 0;
+  LaneSums S;
+  lane_zero(S);
+  S.tot = u128_zero();
   const int per = (nc + gridDim.x - 1) / gridDim.x;
   const int c0 = blockIdx.x * per, c1 = min(c0 + per, nc);
-  Moments M;
-  for (int k = 0; k < 11; ++k) M.s[k] = u128_zero();
-  int sum_big = -1;  // large node that M belongs to (block-uniform)
+  // the current large node (block-uniform); its points' sums are in S
+  int big = -1, held = 0;
+  float mean[3], dir[3];
+  int nstart = 0, nmid = 0;
+  bool split = false, small_left = false;
   for (int ci = c0; ci < c1; ++ci) {
     const Chunk c = chunks[ci];
-    if (c.big != sum_big) {
-      if (sum_big >= 0) {
-        block_add_moments(M, smm, accl + (size_t)sum_big * 11);
-        for (int k = 0; k < 11; ++k) M.s[k] = u128_zero();
-      }
-      sum_big = -1;
-    }
-    const BNode& nd = nodes[c.node];
-    if (!nd.split) {
-      for (int i = c.begin + threadIdx.x; i < c.end; i += blockDim.x) B.perm[i] = __float_as_int(pin[i].w);
-      continue;  // uniform per block
-    }
-    const float mean[3] = {nd.mean[0], nd.mean[1], nd.mean[2]};
-    const float dir[3] = {nd.dir[0], nd.dir[1], nd.dir[2]};
     const int wb = c.begin + w * 32 * kPer;  // this warp's first point
     float4 pv[kPer];
-    unsigned bl[kPer], bv[kPer];
-    int nl = 0;
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int i = wb + u * 32 + lane;
-      if (i < c.end) pv[u] = pin[i];
-    }
+    for (int u = 0; u < kPer; ++u)
+      if (wb + u * 32 + lane < c.end) pv[u] = pin[wb + u * 32 + lane];
+    const int loff = chunk_loff[ci] + seg_before(seg[ci], w);  // left points of the node before this segment
+    if (c.big != big) {
+      if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, false);
+      big = c.big;
+      held = 0;
+      const BNode& nd = nodes[c.node];
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int i = wb + u * 32 + lane;
-      bv[u] = __ballot_sync(0xffffffffu, i < c.end);
-      bl[u] = __ballot_sync(0xffffffffu, i < c.end && which_side_f(mean, dir, pv[u]));
-      nl += __popc(bl[u]);
-    }
-    if (lane == 0) swl[par][w] = nl;
-    __syncthreads();
-    int lpre = 0;  // left points of the chunk's earlier warps
-    for (int k = 0; k < w; ++k) lpre += swl[par][k];
-    const int nl_total = nd.mid - nd.start;
-    const int before = min(wb, c.end) - nd.start;  // the node's points before this warp's
-    int lo = nd.start + chunk_loff[ci] + lpre;
-    int ro = nd.mid + before - (chunk_loff[ci] + lpre);
-    const bool small_left = nl_total <= nd.end - nd.mid;
-    const double t0 = ts0[nd.tree];
-    sum_big = c.big;
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const unsigned br = bv[u] & ~bl[u];
-      if ((bv[u] >> lane) & 1u) {
-        const bool left = (bl[u] >> lane) & 1u;
-        const int dst = left ? lo + __popc(bl[u] & lt) : ro + __popc(br & lt);
-        pout[dst] = pv[u];
-        if (left == small_left) moments_add_point(M, pv[u], sts[__float_as_int(pv[u].w)], t0);
+      for (int k = 0; k < 3; ++k) {
+        mean[k] = nd.mean[k];
+        dir[k] = nd.dir[k];
       }
-      lo += __popc(bl[u]);
+      split = nd.split != 0;
+      nstart = nd.start;
+      nmid = nd.mid;
+      small_left = nd.mid - nd.start <= nd.end - nd.mid;
+    } else if (++held == kFoldChunks) {
+      lane_fold(S, lane);
+      held = 0;
+    }
+    if (!split) {
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        if (wb + u * 32 + lane < c.end) B.perm[wb + u * 32 + lane] = __float_as_int(pv[u].w);
+      continue;
+    }
+    int lo = nstart + loff;
+    int ro = nmid + min(wb, c.end) - nstart - loff;  // the node's points before this segment, less the left ones
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const bool valid = wb + u * 32 + lane < c.end;
+      const bool left = valid && which_side_f(mean, dir, pv[u]);
+      const unsigned bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, valid && !left);
+      if (valid) pout[left ? lo + __popc(bl & lt) : ro + __popc(br & lt)] = pv[u];
+      lane_add(S, valid && left == small_left, pv[u], lane);
+      lo += __popc(bl);
       ro += __popc(br);
     }
-    par ^= 1;  // the barrier above keeps warps within one split chunk of each other
   }
-  if (sum_big >= 0) block_add_moments(M, smm, accl + (size_t)sum_big * 11);
+  if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, per == 1);
 }
 
 // Children's sums of the large split nodes: the smaller from accl, the other = parent - it.
 __global__ void k_big_childmom(const BNode* nodes, LevelState* ls, const int32_t* big_list, const U128* accl,
                                U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin, unsigned* done) {
   const int nb = ls->num_big;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * 11; t += gridDim.x * blockDim.x) {
-    const int b = t / 11, k = t % 11;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * kSums; t += gridDim.x * blockDim.x) {
+    const int b = t / kSums, k = t % kSums;
     const int i = big_list[b];
     if (!nodes[i].split) continue;
     const U128 q = accl[t];  // the smaller child's sums
-    const U128 other = u128_sub(mom[(size_t)i * 11 + k], q);
+    const U128 other = u128_sub(mom[(size_t)i * kSums + k], q);
     const bool small_left = nodes[i].mid - nodes[i].start <= nodes[i].end - nodes[i].mid;
-    mom[(size_t)nodes[i].left * 11 + k] = small_left ? q : other;
-    mom[(size_t)nodes[i].right * 11 + k] = small_left ? other : q;
+    mom[(size_t)nodes[i].left * kSums + k] = small_left ? q : other;
+    mom[(size_t)nodes[i].right * kSums + k] = small_left ? other : q;
   }
   advance_if_last(ls, bsum, nblocks, level_begin, done);
 }
@@ -1253,7 +1390,6 @@ static_assert(2 * (kDeepMax / 3) <= kDeepNodes, "node capacity of one depth");
 
 struct DeepNode {
   float mean[3], dir[3];
-  double dts_mean, dts_cov;
   double prop[3];
   int32_t start, end;     // point offsets inside the subtree
   int32_t sub;            // subtree ordinal: its root is node lb + sub
@@ -1263,8 +1399,8 @@ struct DeepNode {
   int32_t parent_rank;    // rank of the parent at depth - 1
   int32_t has_prop;
 };
-static_assert(sizeof(DeepNode) == 96, "DeepNode layout");
-static_assert(sizeof(DeepNode) <= 11 * sizeof(U128), "a DeepNode fits the sums slot of one node");
+static_assert(sizeof(DeepNode) == 80, "DeepNode layout");
+static_assert(sizeof(DeepNode) <= kSums * sizeof(U128), "a DeepNode fits the sums slot of one node");
 
 struct DeepWarpSmem {                // one warp's slice
   float4 pts[2][kDeepMax];           // the 16 B point records (w = input index)
@@ -1272,10 +1408,11 @@ struct DeepWarpSmem {                // one warp's slice
   int32_t prank[2][kDeepNodes];      // parent's rank, by depth parity
   int32_t list[kDeepNodes];          // q -> rank of the q-th split node of the depth
   uint8_t split[kDeepNodes];
+  SumStage stage;
 };
 
 __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
-    k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const double* ts0, const U128* mom, BuildParams P,
+    k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, BuildParams P,
                  double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* ring, int32_t* counts,
                  int32_t dcap) {
   extern __shared__ __align__(16) unsigned char deep_smem_raw[];
@@ -1285,15 +1422,16 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
   const int nroots = le - lb;
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
   const int gw = blockIdx.x * kDeepWarpsPerBlock + wib, nw = gridDim.x * kDeepWarpsPerBlock;
-  U128* myring = ring + (size_t)gw * 2 * kDeepNodes * 11;
+  stage_init(S.stage, lane);
+  WarpSums W;
+  sums_zero(W);
+  U128* myring = ring + (size_t)gw * 2 * kDeepNodes * kSums;
   const float4* pin = B.p[cur0];
-  const double* sts = B.st;
   for (int sub = gw; sub < nroots; sub += nw) {
     const int R = lb + sub;
     const BNode root = nodes[R];
     const int n = root.end - root.start;
     const int pbase = root.start;
-    const double t0 = ts0[root.tree];
     for (int i = lane; i < n; i += 32) S.pts[0][i] = pin[pbase + i];
     if (lane == 0) {
       S.range[0][0] = (uint32_t)n << 16;
@@ -1313,7 +1451,7 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
           break;
         }
       }
-      const U128* psums = d == 0 ? mom + (size_t)R * 11 : myring + (size_t)(d & 1) * kDeepNodes * 11;
+      const U128* psums = d == 0 ? mom + (size_t)R * kSums : myring + (size_t)(d & 1) * kDeepNodes * kSums;
       for (int r = lane; r < cnt; r += 32) {
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
@@ -1334,9 +1472,9 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
             for (int k = 0; k < 3; ++k) nd.par_prop[k] = pn.prop[k];
           }
         }
-        double Sd[11];
-        const U128* ms = d == 0 ? psums : psums + (size_t)r * 11;
-        for (int k = 0; k < 11; ++k) Sd[k] = fx_to_d(ms[k]);
+        double Sd[kSums];
+        const U128* ms = d == 0 ? psums : psums + (size_t)r * kSums;
+        for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(ms[k]);
         decide(Sd, en - st, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
         S.split[r] = nd.split ? 1 : 0;
         if (d == 0) {
@@ -1348,8 +1486,6 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
             x.dir[k] = nd.dir[k];
             x.prop[k] = nd.prop[k];
           }
-          x.dts_mean = nd.dts_mean;
-          x.dts_cov = nd.dts_cov;
           x.start = st;
           x.end = en;
           x.sub = sub;
@@ -1411,8 +1547,6 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
         }
         const int mid = st + nl;
         const bool small_left = mid - st <= en - mid;
-        Moments MS;
-        for (int k = 0; k < 11; ++k) MS.s[k] = u128_zero();
         int cl = 0, cr = 0;
         for (int k0 = st; k0 < en; k0 += 32) {
           const int i = k0 + lane;
@@ -1425,19 +1559,20 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
           if (valid) {
             const int dst = left ? (st + cl + __popc(bl & lt)) : (mid + cr + __popc(br & lt));
             S.pts[c ^ 1][dst] = p;
-            if (left == small_left) moments_add_point(MS, p, sts[__float_as_int(p.w)], t0);
           }
+          sums_add(W, S.stage, valid && left == small_left, p, lane);
+          sums_room(W, S.stage, kStage - 32, lane);
           cl += __popc(bl);
           cr += __popc(br);
         }
-        const U128 qs = warp_sum_moments(MS, lane);
-        if (!(lane & 1) && lane < 22) {
-          const int k = lane >> 1;
-          const U128 ps = d == 0 ? psums[k] : psums[(size_t)r * 11 + k];
+        const U128 qs = sums_total(W, S.stage, lane);
+        if (lane < kSums) {
+          const int k = lane;
+          const U128 ps = d == 0 ? psums[k] : psums[(size_t)r * kSums + k];
           const U128 other = u128_sub(ps, qs);
-          U128* nxt = myring + (size_t)((d + 1) & 1) * kDeepNodes * 11;
-          nxt[(size_t)(2 * q) * 11 + k] = small_left ? qs : other;
-          nxt[(size_t)(2 * q + 1) * 11 + k] = small_left ? other : qs;
+          U128* nxt = myring + (size_t)((d + 1) & 1) * kDeepNodes * kSums;
+          nxt[(size_t)(2 * q) * kSums + k] = small_left ? qs : other;
+          nxt[(size_t)(2 * q + 1) * kSums + k] = small_left ? other : qs;
         }
         if (lane == 0) {
           S.range[c ^ 1][2 * q] = (uint32_t)st | ((uint32_t)mid << 16);
@@ -1498,8 +1633,6 @@ __global__ void k_deep_place(BNode* nodes, LevelState* ls, const DeepNode* dn, c
       o.dir[k] = x.dir[k];
       o.prop[k] = x.prop[k];
     }
-    o.dts_mean = x.dts_mean;
-    o.dts_cov = x.dts_cov;
     const int g = le + off[(size_t)d * nroots + s] + x.rank;
     if (g >= cap_nodes) {
       ls->error = 1;
@@ -1619,9 +1752,122 @@ __global__ void k_group_tables(int depth, int R, const int32_t* cnt, const int32
   }
 }
 
+// ---- stamps ----------------------------------------------------------------------------
+// Prefix sums of (dt, dt^2) over the final point order, exact: a node's sums are the
+// difference at the ends of its point range.  One pass at the end in place of the stamps'
+// share of every level (a 32 B sector per summed point and level, two 128-bit terms per
+// point, and two more sums to reduce per node).  Tiles of kDtTile points: their sums, the
+// scan of those by one block, then every position's exclusive prefix.
+struct __align__(16) DtSum {
+  U128 d, dd;
+};
+__host__ __device__ __forceinline__ DtSum dt_add(DtSum a, DtSum b) {
+  DtSum r;
+  r.d = u128_add(a.d, b.d);
+  r.dd = u128_add(a.dd, b.dd);
+  return r;
+}
+constexpr int kDtItems = 8;
+constexpr int kDtTile = kThreads * kDtItems;
+__device__ __forceinline__ DtSum dt_shfl_up(DtSum v, int off) {
+  DtSum r;
+  r.d.lo = __shfl_up_sync(0xffffffffu, v.d.lo, off);
+  r.d.hi = __shfl_up_sync(0xffffffffu, v.d.hi, off);
+  r.dd.lo = __shfl_up_sync(0xffffffffu, v.dd.lo, off);
+  r.dd.hi = __shfl_up_sync(0xffffffffu, v.dd.hi, off);
+  return r;
+}
+__device__ __forceinline__ DtSum dt_zero() {
+  DtSum r;
+  r.d = r.dd = u128_zero();
+  return r;
+}
+// Block-wide exclusive scan (kThreads threads); *total = block sum.
+__device__ __forceinline__ DtSum dt_block_scan(DtSum v, DtSum* sm, DtSum* total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  DtSum x = v;
+  for (int off = 1; off < 32; off <<= 1) {
+    const DtSum y = dt_shfl_up(x, off);
+    if (lane >= off) x = dt_add(x, y);
+  }
+  DtSum ex = dt_shfl_up(x, 1);
+  if (lane == 0) ex = dt_zero();
+  if (lane == 31) sm[w] = x;
+  __syncthreads();
+  DtSum pre = dt_zero(), tot = dt_zero();
+  for (int k = 0; k < kThreads / 32; ++k) {
+    if (k == w) pre = tot;
+    tot = dt_add(tot, sm[k]);
+  }
+  __syncthreads();
+  *total = tot;
+  return dt_add(pre, ex);
+}
+__device__ __forceinline__ void dt_load(const double* dt, const int32_t* perm, int64_t b, int64_t n, DtSum* t) {
+  double d[kDtItems];
+#pragma unroll
+  for (int k = 0; k < kDtItems; ++k) d[k] = b + k < n ? dt[perm[b + k]] : 0.0;
+#pragma unroll
+  for (int k = 0; k < kDtItems; ++k) {
+    t[k].d = fx_d_nonneg(d[k]);
+    t[k].dd = fx_d_nonneg(d[k] * d[k]);
+  }
+}
+__global__ void __launch_bounds__(kThreads) k_dt_tiles(const double* dt, const int32_t* perm, int64_t n, DtSum* tiles) {
+  __shared__ DtSum sm[kThreads / 32];
+  DtSum t[kDtItems], tot;
+  dt_load(dt, perm, (int64_t)blockIdx.x * kDtTile + threadIdx.x * kDtItems, n, t);
+  DtSum v = t[0];
+#pragma unroll
+  for (int k = 1; k < kDtItems; ++k) v = dt_add(v, t[k]);
+  dt_block_scan(v, sm, &tot);
+  if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
+}
+__global__ void __launch_bounds__(kThreads) k_dt_top(DtSum* tiles, int nt) {
+  __shared__ DtSum sm[kThreads / 32];
+  DtSum carry = dt_zero();
+  for (int b = 0; b < nt; b += kThreads) {
+    const int i = b + threadIdx.x;
+    DtSum tot;
+    const DtSum ex = dt_block_scan(i < nt ? tiles[i] : dt_zero(), sm, &tot);
+    if (i < nt) tiles[i] = dt_add(carry, ex);
+    carry = dt_add(carry, tot);
+  }
+}
+// pre[i] for i in [0, n].  tiles: the tiles' sums, scanned already or (at most kThreads of
+// them) not, then each block adds up those before it.
+__global__ void __launch_bounds__(kThreads) k_dt_prefix(const double* dt, const int32_t* perm, int64_t n,
+                                                        const DtSum* tiles, int scanned, DtSum* pre) {
+  __shared__ DtSum sm[kThreads / 32];
+  const int64_t b = (int64_t)blockIdx.x * kDtTile + threadIdx.x * kDtItems;
+  DtSum t[kDtItems], tot;
+  dt_load(dt, perm, b, n, t);
+  DtSum v = t[0];
+#pragma unroll
+  for (int k = 1; k < kDtItems; ++k) v = dt_add(v, t[k]);
+  DtSum x = dt_block_scan(v, sm, &tot);
+  if (scanned) {
+    x = dt_add(x, tiles[blockIdx.x]);
+  } else if (blockIdx.x > 0) {
+    dt_block_scan(threadIdx.x < blockIdx.x ? tiles[threadIdx.x] : dt_zero(), sm, &tot);
+    x = dt_add(x, tot);
+  }
+#pragma unroll
+  for (int k = 0; k < kDtItems; ++k) {
+    if (b + k <= n) {  // two 16 B stores
+      ulonglong2* o = reinterpret_cast<ulonglong2*>(pre + b + k);
+      o[0] = make_ulonglong2(x.d.lo, x.d.hi);
+      o[1] = make_ulonglong2(x.dd.lo, x.dd.hi);
+    }
+    x = dt_add(x, t[k]);
+  }
+}
+
+// pre: prefix sums of the stamps over the point order (nullptr: every dt is 0)
 __global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_t* alive, const int32_t* rank,
                                  const int32_t* leaf_flag, const int32_t* lrank, int R, const int32_t* gp,
-                                 const int32_t* lgp, const int32_t* to, const int32_t* lto, TreeDev* trees) {
+                                 const int32_t* lgp, const int32_t* to, const int32_t* lto, const DtSum* pre,
+                                 TreeDev* trees) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (!alive[i]) continue;
     const BNode& nd = nodes[i];
@@ -1636,9 +1882,16 @@ __global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_
     d.a = make_float4(nd.mean[0], nd.mean[1], nd.mean[2], nd.dir[0]);
     d.b = make_float4(nd.dir[1], nd.dir[2], __int_as_float(l), __int_as_float(r));
     T.nodes[o] = d;
-    T.dts_f[o] = (float)nd.dts_mean;
-    T.dts_mean[o] = nd.dts_mean;
-    T.dts_cov[o] = nd.dts_cov;
+    double dts_mean = 0.0, dts_cov = 0.0;
+    if (pre && nd.end > nd.start) {
+      const double dn = (double)(nd.end - nd.start);
+      const DtSum a = pre[nd.start], b = pre[nd.end];
+      dts_mean = fx_to_d(u128_sub(b.d, a.d)) / dn;
+      dts_cov = fx_to_d(u128_sub(b.dd, a.dd)) / dn - dts_mean * dts_mean;
+    }
+    T.dts_f[o] = (float)dts_mean;
+    T.dts_mean[o] = dts_mean;
+    T.dts_cov[o] = dts_cov;
     int64_t base = nd.start;  // ranges are global; made tree-relative below
     T.range[2 * o] = base;
     T.range[2 * o + 1] = nd.end;
@@ -1686,11 +1939,14 @@ struct BuildWs {
   BNode* nodes;
   int32_t *alive, *rank, *leaf_flag, *lrank, *tile_sums;
   Chunk* chunks;
-  int32_t *chunk_nl, *chunk_loff, *big_list, *node_chunk0;
+  SegCounts* seg;
+  int32_t *chunk_loff, *big_list, *node_chunk0;
   U128* acc;
   U128* accl;  // left-child sums of the level's large nodes
-  U128* mom;   // exact sums of every node (11 per node)
-  double* ts0;
+  U128* mom;   // exact sums of every node
+  double* ts0;   // per cloud
+  double* dt;    // stamps less ts0, input order
+  DtSum* dt_tiles;
   double* root_frame;  // kRootFrame per cloud (k_decide at level 0)
   unsigned long long* tsmin;
   int64_t* off;
@@ -1711,10 +1967,11 @@ size_t ws_bytes(int64_t n, int R) {
   const int64_t chunk_cap = n / kChunk + n / kBig + 16;
   const int64_t ntiles = cn / 4096 + 2;
   const int64_t G = (int64_t)(kMaxDepth + 2) * R;
-  return 2 * carve_size<float4>(n) + carve_size<double>(n) + carve_size<int32_t>(n) +
+  return carve_size<float4>(2 * n + 2) + carve_size<int32_t>(n) +
          carve_size<BNode>(cn) + 4 * carve_size<int32_t>(cn) + carve_size<int32_t>(ntiles) +
-         carve_size<Chunk>(chunk_cap) + 4 * carve_size<int32_t>(chunk_cap) +
-         2 * carve_size<U128>((size_t)11 * (n / kBig + 2)) + carve_size<U128>((size_t)11 * cn) + 2 * carve_size<double>(R) +
+         carve_size<Chunk>(chunk_cap) + carve_size<SegCounts>(chunk_cap) + 3 * carve_size<int32_t>(chunk_cap) +
+         2 * carve_size<U128>((size_t)kSums * (n / kBig + 2)) + carve_size<U128>((size_t)kSums * cn) + carve_size<unsigned long long>(R) + carve_size<double>(R) + carve_size<double>(n) +
+         carve_size<DtSum>(n / kDtTile + 1) +
          carve_size<double>((size_t)kRootFrame * R) + carve_size<int64_t>(R + 1) +
          carve_size<LevelState>(1) + carve_size<int32_t>(kMaxDepth + 2) + carve_size<unsigned>(1) +
          carve_size<int32_t>(kLevelBlocks) +
@@ -1738,9 +1995,8 @@ int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
     return KDS_ERR_OOM;
   }
   char* p = (char*)w.block;
-  w.B.p[0] = carve<float4>(p, n);
-  w.B.p[1] = carve<float4>(p, n);
-  w.B.st = carve<double>(p, n);
+  w.B.p[0] = carve<float4>(p, 2 * n + 2);  // later the n + 1 stamp prefixes of 32 B
+  w.B.p[1] = w.B.p[0] + n;
   w.B.perm = carve<int32_t>(p, n);
   w.nodes = carve<BNode>(p, cn);
   w.alive = carve<int32_t>(p, cn);
@@ -1749,14 +2005,16 @@ int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
   w.lrank = carve<int32_t>(p, cn);
   w.tile_sums = carve<int32_t>(p, ntiles);
   w.chunks = carve<Chunk>(p, w.chunk_cap);
-  w.chunk_nl = carve<int32_t>(p, w.chunk_cap);
+  w.seg = carve<SegCounts>(p, w.chunk_cap);
   w.chunk_loff = carve<int32_t>(p, w.chunk_cap);
   w.big_list = carve<int32_t>(p, w.chunk_cap);
   w.node_chunk0 = carve<int32_t>(p, w.chunk_cap);
-  w.acc = carve<U128>(p, (size_t)11 * (n / kBig + 2));
-  w.accl = carve<U128>(p, (size_t)11 * (n / kBig + 2));
-  w.mom = carve<U128>(p, (size_t)11 * cn);
+  w.acc = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
+  w.accl = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
+  w.mom = carve<U128>(p, (size_t)kSums * cn);
   w.ts0 = carve<double>(p, R);
+  w.dt = carve<double>(p, n);
+  w.dt_tiles = carve<DtSum>(p, n / kDtTile + 1);
   w.root_frame = carve<double>(p, (size_t)kRootFrame * R);
   w.tsmin = carve<unsigned long long>(p, R);
   w.off = carve<int64_t>(p, R + 1);
@@ -1792,8 +2050,8 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   const int nroots = le - lb;
   if (nroots <= 0) return KDS_OK;
   const int dcap = std::max(1, P.max_level - h.depth);
-  DeepNode* dn = reinterpret_cast<DeepNode*>(w.mom + (size_t)le * 11);
-  const int64_t dn_cap64 = ((w.cap_nodes - le) * (int64_t)(11 * sizeof(U128))) / (int64_t)sizeof(DeepNode);
+  DeepNode* dn = reinterpret_cast<DeepNode*>(w.mom + (size_t)le * kSums);
+  const int64_t dn_cap64 = ((w.cap_nodes - le) * (int64_t)(kSums * sizeof(U128))) / (int64_t)sizeof(DeepNode);
   const int32_t dn_cap = (int32_t)std::min<int64_t>(dn_cap64, INT32_MAX);
   const int grid = (int)std::min<int64_t>((nroots + kDeepWarpsPerBlock - 1) / kDeepWarpsPerBlock,
                                           148 * kDeepBlocksPerSM);
@@ -1801,7 +2059,7 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   const int64_t ncount = (int64_t)dcap * nroots;
   if (ncount > INT32_MAX / 2) { set_error("kds_tree_build: too many deep subtrees"); return KDS_ERR_CAPACITY; }
   const size_t bc = carve_size<int32_t>(ncount), bt = carve_size<int32_t>(ncount / 4096 + 2),
-               br = carve_size<U128>((size_t)nwarps * 2 * kDeepNodes * 11);
+               br = carve_size<U128>((size_t)nwarps * 2 * kDeepNodes * kSums);
   void* blk = nullptr;
   cudaError_t e = cudaMallocAsync(&blk, 2 * bc + bt + 3 * 256 + br, s);
   if (e != cudaSuccess) {
@@ -1816,7 +2074,7 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   int32_t* total = carve<int32_t>(p, 1);
   int32_t* dn_count = carve<int32_t>(p, 1);
   carve<int32_t>(p, 1);
-  U128* ring = carve<U128>(p, (size_t)nwarps * 2 * kDeepNodes * 11);
+  U128* ring = carve<U128>(p, (size_t)nwarps * 2 * kDeepNodes * kSums);
   int rc = KDS_OK;
   static std::atomic<bool> attr_set{false};  // a property of the kernel, per process (builds may run on two threads)
   if (!attr_set.load()) {
@@ -1827,7 +2085,7 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * ncount, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(dn_count, 0, sizeof(int32_t), s);
   if (e == cudaSuccess) {
-    k_deep_build<<<grid, kDeepThreads, sizeof(DeepWarpSmem) * kDeepWarpsPerBlock, s>>>(w.nodes, w.ls, w.B, w.ts0, w.mom, P, w.root_frame, dn,
+    k_deep_build<<<grid, kDeepThreads, sizeof(DeepWarpSmem) * kDeepWarpsPerBlock, s>>>(w.nodes, w.ls, w.B, w.mom, P, w.root_frame, dn,
                                                               dn_cap, dn_count, ring, counts, dcap);
     count_launch();
     rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
@@ -1935,16 +2193,17 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   KDS_CK(cudaMemsetAsync(w.ls, 0, sizeof(LevelState), s));
   KDS_CK(cudaMemsetAsync(w.done, 0, sizeof(unsigned), s));
   KDS_CK(cudaMemcpyAsync(w.off, off.data(), sizeof(int64_t) * (R + 1), cudaMemcpyHostToDevice, s));
-  k_ingest<<<nblk(N, kThreads), kThreads, 0, s>>>(d_xyz, d_st, N, w.B.p[0], w.B.st, w.ls);
+  k_ingest<<<nblk(N, kThreads), kThreads, 0, s>>>(d_xyz, N, w.B.p[0], w.ls);
   count_launch();
-  {
+  if (!d_st) KDS_CK(cudaMemsetAsync(w.ts0, 0, sizeof(double) * R, s));
+  if (d_st) {
     KDS_CK(cudaMemsetAsync(w.tsmin, 0xff, sizeof(unsigned long long) * R, s));
     // enough blocks to fill the machine whatever the number of clouds (64 per cloud before:
     // 370 + 200 us over the 11.4M stamps of one map)
     const int64_t gx = std::max<int64_t>(64, (148 * 8 + R - 1) / R);
     dim3 g((unsigned)std::min<int64_t>(std::max<int64_t>((max_size + kThreads - 1) / kThreads, 1), gx), (unsigned)R);
-    k_tree_min<<<g, kThreads, 0, s>>>(w.B.st, w.off, w.tsmin);
-    k_tree_check<<<g, kThreads, 0, s>>>(w.B.st, w.off, w.tsmin, w.ts0, w.ls);
+    k_tree_min<<<g, kThreads, 0, s>>>(d_st, w.off, w.tsmin);
+    k_tree_check<<<g, kThreads, 0, s>>>(d_st, w.off, w.tsmin, w.ts0, w.dt, w.ls);
     count_launch();
     count_launch();
   }
@@ -1962,6 +2221,9 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   double* h_dbl = reinterpret_cast<double*>(stage + st_ls + st_cnt);
   int32_t host_max = max_size;
   const int cb = std::min<int>(w.chunk_cap, kGridBlocks * 2);
+  // blocks that take a contiguous range of chunks each: one resident wave, so that no block
+  // starts when the others are done
+  const int sb = std::min<int>(w.chunk_cap, 148 * kScatterPerSM);
   // Grids of the level kernels sized to the level: a level has at most twice the nodes
   // of the one before, and the host learns the current level's size at each sync.  The
   // node-range kernels (k_decide, k_level_children, k_big_plan) share
@@ -1976,7 +2238,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       // every node of the current level fits one block: the rest of every subtree is
       // built in shared memory, then the host reads the final level state
       if (round == 0) {  // the roots' sums (every root has at most kBig points)
-        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.ts0, w.mom);
+        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
         count_launch();
       }
       global_levels = hls.depth;
@@ -1998,13 +2260,13 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       const int small_blocks =
           (int)std::max<int64_t>(1, std::min<int64_t>(kSmallBlocks, (nodes_bound + kThreads / 32 - 1) / (kThreads / 32)));
       if (level0) {  // the roots' sums
-        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.ts0, w.mom);
+        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
         count_launch();
         if (host_max > kBig) {
           k_big_sums<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig);
           k_big_plan<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list,
                                                      w.node_chunk0, w.acc, w.accl);
-          k_big_moments<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.ts0, w.nodes, w.acc);
+          k_big_moments<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.acc);
           k_big_to_mom<<<64, 256, 0, s>>>(w.ls, w.big_list, w.acc, w.mom);
           for (int c = 0; c < 4; ++c) count_launch();
         }
@@ -2012,7 +2274,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       k_decide<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, P, w.bsum, w.bbig, w.root_frame);
       k_level_children<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
       const bool big = host_max > kBig;  // the large-node kernels run after the partition
-      k_small_part<<<small_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.B, w.ts0, w.mom, w.bsum, lvl_blocks,
+      k_small_part<<<small_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks,
                                                      w.level_begin, big ? nullptr : w.done);
       for (int c = 0; c < 3; ++c) count_launch();
       if (big) {
@@ -2021,10 +2283,11 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
                                                      w.node_chunk0, w.acc, w.accl);
           count_launch();
         }
-        k_big_count<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.chunk_nl);
-        k_big_offsets<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, w.ls, w.big_list, w.node_chunk0, w.chunk_nl,
+        k_big_count<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg);
+        k_big_offsets<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, w.ls, w.big_list, w.node_chunk0, w.seg,
                                                        w.chunk_loff);
-        k_big_scatter<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.chunk_loff, w.ts0, w.accl);
+        k_big_scatter<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg, w.chunk_loff,
+                                                  w.accl);
         k_big_childmom<<<64, 256, 0, s>>>(w.nodes, w.ls, w.big_list, w.accl, w.mom, w.bsum, lvl_blocks,
                                           w.level_begin, w.done);
         for (int c = 0; c < 5; ++c) count_launch();
@@ -2095,8 +2358,23 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     td[r] = t->d;
   }
   KDS_CK(cudaMemcpyAsync(w.trees, td.data(), sizeof(TreeDev) * R, cudaMemcpyHostToDevice, s));
+  DtSum* pre = nullptr;
+  if (d_st) {  // the point buffers are free now
+    pre = reinterpret_cast<DtSum*>(w.B.p[0]);
+    const int nt = (int)(N / kDtTile + 1);  // tiles of the N + 1 positions
+    if (nt > 1) {
+      k_dt_tiles<<<nt, kThreads, 0, s>>>(w.dt, w.B.perm, N, w.dt_tiles);
+      count_launch();
+    }
+    if (nt > kThreads) {
+      k_dt_top<<<1, kThreads, 0, s>>>(w.dt_tiles, nt);
+      count_launch();
+    }
+    k_dt_prefix<<<nt, kThreads, 0, s>>>(w.dt, w.B.perm, N, w.dt_tiles, nt > kThreads ? 1 : 0, pre);
+    count_launch();
+  }
   k_compact_forest<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, w.rank, w.leaf_flag, w.lrank,
-                                                              R, w.gp, w.lgp, w.to, w.lto, w.trees);
+                                                              R, w.gp, w.lgp, w.to, w.lto, pre, w.trees);
   count_launch();
   dim3 fg((unsigned)std::min<int64_t>(nblk(max_size, kThreads), 256), (unsigned)R);
   k_finish_trees<<<fg, kThreads, 0, s>>>(w.trees, w.off, w.B.perm);

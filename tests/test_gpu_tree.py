@@ -224,3 +224,36 @@ def test_large_node_chunk_lists(scene, sizes):
             assert T is None
             continue
         assert_same_tree(orc.OTree.build(x, s, orc.tree_params(leaf_max_points=16)), T)
+
+
+@pytest.mark.parametrize("n", [1000, 1025, 40_000])
+def test_exact_sums_off_the_grid(n):
+    """Coordinates on both sides of the sums' 2^-40 grid (nonzero below 2^-17, down to
+    denormals), exact zeros and values up to the range limit, with and without stamps: every
+    node equals the oracle's bit for bit."""
+    import kd_slam2_b200 as kds
+    rng = np.random.default_rng(n)
+    xyz = (rng.normal(size=(n, 3)) * [20.0, 8.0, 0.01]).astype(np.float32)
+    k = rng.integers(0, n, n // 8)
+    xyz[k, 2] = np.ldexp(rng.uniform(-1, 1, len(k)), rng.integers(-150, -14, len(k))).astype(np.float32)
+    xyz[rng.integers(0, n, n // 16), 1] = 0.0
+    xyz[rng.integers(0, n, n // 16), 0] = np.float32(2.0**-17)
+    xyz[rng.integers(0, n, 5)] = [32767.996, -32767.0, 30000.5]
+    st = np.sort(rng.uniform(0, 40_000.0, n))
+    st[: n // 2] *= 1e-9
+    prm = dict(leaf_max_points=16, tree_min_good_leaves=1)
+    for s in (None, st, np.full(n, 7.25)):
+        O, G = build_both(xyz, s, **prm)
+        assert_same_tree(O, G)
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4096])
+def test_stamp_prefix_tiles(scene, n):
+    """Point counts at the edges of the stamp prefix's tiles, in one forest with differing
+    first stamps."""
+    import kd_slam2_b200 as kds
+    xyz, st = make_scan(scene, 2460, beams=32, vel=[8.0, 0, 0, 0, 0, 0.2])
+    clouds = [(xyz[:n], st[:n] + 5.0), (xyz[n:2 * n + 1], st[n:2 * n + 1])]
+    for (x, s), T in zip(clouds, kds.TreeGeneratorB2003D(leaf_max_points=16).make_trees(clouds)):
+        assert_same_tree(orc.OTree.build(x, s, orc.tree_params(leaf_max_points=16)), T)
+    assert_same_tree(*build_both(xyz[:n], st[:n], leaf_max_points=16))
