@@ -54,29 +54,36 @@ __device__ __forceinline__ F3 mv3(const float* A, F3 p) { return mat_vec_x(A, p)
 // column c of a row-major 3x3
 __device__ __forceinline__ F3 col3(const float* A, int c) { return f3(A[c], A[3 + c], A[6 + c]); }
 
+// C = A * skew(u): each coefficient's dot3x less its term with a zero factor
+__device__ __forceinline__ void mm3_skew(const float* A, F3 u, float* C) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    C[i * 3] = fa(fm(A[i * 3 + 1], u.z), fm(A[i * 3 + 2], -u.y));
+    C[i * 3 + 1] = fa(fm(A[i * 3], -u.z), fm(A[i * 3 + 2], u.x));
+    C[i * 3 + 2] = fa(fm(A[i * 3], u.y), fm(A[i * 3 + 1], -u.x));
+  }
+}
+
 // Pieces of dRxp (kd/utils/geometry_3d_impl_.h:143-174) shared by both of its calls:
-// R = rodrigues(w) and Q = n n^T + (R^T - I) S / angle, so that
+// with R = rodrigues(w), Q = n n^T + (R^T - I) S / angle, so that
 // d(R u)/dw = -R skew(u) Q.  small = angle < 1e-9 (then dR = -skew(u)).
 struct DRxp {
-  float R[9];
   float Q[9];
   bool small;
 };
-__device__ __forceinline__ void drxp_setup(F3 w, DRxp& d) {
+__device__ __forceinline__ void drxp_setup(F3 w, const float* R, DRxp& d) {
   float angle = __fsqrt_rn(dot3x(w, w));
   d.small = angle < 1e-9f;
   if (d.small) {
 #pragma unroll
-    for (int i = 0; i < 9; ++i) { d.R[i] = (i % 4 == 0) ? 1.f : 0.f; d.Q[i] = 0.f; }
+    for (int i = 0; i < 9; ++i) d.Q[i] = 0.f;
     return;
   }
-  rodrigues_x(w, d.R);
   float inv = __fdiv_rn(1.0f, angle);
   F3 n = f3(fm(w.x, inv), fm(w.y, inv), fm(w.z, inv));
-  float S[9] = {0.f, -n.z, n.y, n.z, 0.f, -n.x, -n.y, n.x, 0.f};
-  float RtmI[9] = {fs(d.R[0], 1.f), d.R[3], d.R[6], d.R[1], fs(d.R[4], 1.f), d.R[7], d.R[2], d.R[5], fs(d.R[8], 1.f)};
+  float RtmI[9] = {fs(R[0], 1.f), R[3], R[6], R[1], fs(R[4], 1.f), R[7], R[2], R[5], fs(R[8], 1.f)};
   float A[9];
-  mm3(RtmI, S, A);
+  mm3_skew(RtmI, n, A);
   float nn[3] = {n.x, n.y, n.z};
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -84,39 +91,35 @@ __device__ __forceinline__ void drxp_setup(F3 w, DRxp& d) {
     for (int j = 0; j < 3; ++j) d.Q[i * 3 + j] = fa(fm(nn[i], nn[j]), fm(A[i * 3 + j], inv));
 }
 // out = Ra * d(R u)/dw  (3x3)
-__device__ __forceinline__ void ra_drxp(const DRxp& d, const float* Ra, F3 u, float* out) {
-  float su[9] = {0.f, -u.z, u.y, u.z, 0.f, -u.x, -u.y, u.x, 0.f};
+__device__ __forceinline__ void ra_drxp(const DRxp& d, const float* R, const float* Ra, F3 u, float* out) {
   float dR[9];
   if (d.small) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) dR[i] = -su[i];
-  } else {
-    float Rs[9], P[9];
-    mm3(d.R, su, Rs);
-    mm3(Rs, d.Q, P);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) dR[i] = -P[i];
+    mm3_skew(Ra, f3(-u.x, -u.y, -u.z), out);
+    return;
   }
+  float Rs[9];
+  mm3_skew(R, u, Rs);
+  mm3(Rs, d.Q, dR);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) dR[i] = -dR[i];
   mm3(Ra, dR, out);
 }
 
-// errorAndJacobianVelocityA (kd/d3/cticp_impl_.h:10-39) -> J[0..5]
-__device__ __forceinline__ void jac_vel_A(const float* Xm, F3 pa_l, F3 na_l, F3 pb_g, F3 nb_g, const float* va, float dt,
-                                          float* J) {
-  F3 tm = f3(fm(va[0], dt), fm(va[1], dt), fm(va[2], dt));
+// errorAndJacobianVelocityA (kd/d3/cticp_impl_.h:10-39) -> J[0..5].  R = rodrigues(va_w dt);
+// pam, nam: the leaf warped by the velocities (applyVelocities).
+__device__ __forceinline__ void jac_vel_A(const float* Xm, F3 pa_l, F3 na_l, F3 pam, F3 nam, F3 pb_g, F3 nb_g,
+                                          const float* va, const float* R, float dt, float* J) {
   F3 wa = f3(fm(va[3], dt), fm(va[4], dt), fm(va[5], dt));
   DRxp d;
-  drxp_setup(wa, d);
+  drxp_setup(wa, R, d);
   float Ra[9] = {Xm[0], Xm[1], Xm[2], Xm[4], Xm[5], Xm[6], Xm[8], Xm[9], Xm[10]};
-  F3 pam = add3x(mv3(d.R, pa_l), tm);
-  F3 nam = mv3(d.R, na_l);
   F3 pag = add3x(mv3(Ra, pam), f3(Xm[3], Xm[7], Xm[11]));
   F3 nag = mv3(Ra, nam);
   F3 n = add3x(nag, nb_g);
   F3 dp = sub3x(pag, pb_g);
   float A[9], B[9];
-  ra_drxp(d, Ra, pa_l, A);
-  ra_drxp(d, Ra, na_l, B);
+  ra_drxp(d, R, Ra, pa_l, A);
+  ra_drxp(d, R, Ra, na_l, B);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     J[c] = fm(dot3x(n, col3(Ra, c)), dt);
@@ -127,21 +130,21 @@ __device__ __forceinline__ void jac_vel_A(const float* Xm, F3 pa_l, F3 na_l, F3 
 // errorAndJacobianVelocityB (kd/d3/cticp_impl_.h:43-73) -> J[0..5]
 __device__ __forceinline__ void jac_vel_B(const float* Xf, F3 pa_g, F3 na_g, F3 pb_l, F3 nb_l, const float* vb, float dt,
                                           float* J) {
-  F3 tm = f3(fm(vb[0], dt), fm(vb[1], dt), fm(vb[2], dt));
   F3 wb = f3(fm(vb[3], dt), fm(vb[4], dt), fm(vb[5], dt));
+  float R[9];
+  F3 pbm, nbm;
+  warp_x(vb, dt, pb_l, nb_l, pbm, nbm, R);
   DRxp d;
-  drxp_setup(wb, d);
+  drxp_setup(wb, R, d);
   float Rb[9] = {Xf[0], Xf[1], Xf[2], Xf[4], Xf[5], Xf[6], Xf[8], Xf[9], Xf[10]};
-  F3 pbm = add3x(mv3(d.R, pb_l), tm);
-  F3 nbm = mv3(d.R, nb_l);
   F3 pbg = add3x(mv3(Rb, pbm), f3(Xf[3], Xf[7], Xf[11]));
   F3 nbg = mv3(Rb, nbm);
   F3 n = add3x(na_g, nbg);
   F3 nn = f3(-n.x, -n.y, -n.z);
   F3 dp = sub3x(pa_g, pbg);
   float A[9], B[9];
-  ra_drxp(d, Rb, pb_l, A);
-  ra_drxp(d, Rb, nb_l, B);
+  ra_drxp(d, R, Rb, pb_l, A);
+  ra_drxp(d, R, Rb, nb_l, B);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     J[c] = fm(dot3x(nn, col3(Rb, c)), dt);
@@ -156,16 +159,16 @@ template <> struct KindDim<0> { static constexpr int D = 6; };
 template <> struct KindDim<1> { static constexpr int D = 12; };
 template <> struct KindDim<2> { static constexpr int D = 18; };
 
-// The query of one moving leaf: optional CT warp (applyVelocities) and the moving-to-
-// fixed transform Xmf.
+// The query of one moving leaf: optional CT warp (applyVelocities, its rotation in R) and
+// the moving-to-fixed transform Xmf.
 template <int KIND>
 __device__ __forceinline__ void leaf_query(const CacheF& C, float4 md, float4 nr, F3& m, F3& n, F3& mw, F3& nw,
-                                           F3& q) {
+                                           F3& q, float* R) {
   m = f3(md.x, md.y, md.z);
   n = f3(nr.x, nr.y, nr.z);
   mw = m;
   nw = n;
-  if (KIND != 0) warp_x(C.v, md.w, m, n, mw, nw);
+  if (KIND != 0) warp_x(C.v, md.w, m, n, mw, nw, R);
   q = apply_iso_x(C.Xmf, mw);
 }
 
@@ -217,8 +220,8 @@ __device__ __forceinline__ void descend2(const DNode* F, int fnn, const DNode* s
 
 // Gates, error, Jacobian and robust weight of one leaf whose descent ended at idx / nd.
 template <int KIND>
-__device__ __forceinline__ void leaf_math(const CacheF& C, F3 m, F3 n, float dt, F3 mw, F3 nw, int idx,
-                                          const DNode& nd, const float* fdts, const ParamsF& P, bool stats_mode,
+__device__ __forceinline__ void leaf_math(const CacheF& C, F3 m, F3 n, float dt, F3 mw, F3 nw, const float* R,
+                                          int idx, const DNode& nd, const float* fdts, const ParamsF& P, bool stats_mode,
                                           int& status, int& match, float& e_out, float& gamma_out, float* J) {
   constexpr int D = KindDim<KIND>::D;
 #pragma unroll
@@ -240,7 +243,7 @@ __device__ __forceinline__ void leaf_math(const CacheF& C, F3 m, F3 n, float dt,
   F3 c1 = cross3(pm, nfx), c2 = cross3(pfx, nm);
   J[0] = ns.x; J[1] = ns.y; J[2] = ns.z;
   J[3] = fa(c1.x, c2.x); J[4] = fa(c1.y, c2.y); J[5] = fa(c1.z, c2.z);
-  if (KIND != 0) jac_vel_A(C.Xm, m, n, pfx, nfx, C.v, dt, J + 6);
+  if (KIND != 0) jac_vel_A(C.Xm, m, n, mw, nw, pfx, nfx, C.v, R, dt, J + 6);
   float chi2 = fm(e, e);
   float kt = P.kernel_threshold;
   float gamma;
@@ -264,21 +267,44 @@ __device__ __forceinline__ void leaf_term(const CacheF& C, const DNode* F, int f
                                           float4 nr, const ParamsF& P, bool stats_mode, int& status, int& match,
                                           float& e_out, float& gamma_out, float* J) {
   F3 m, n, mw, nw, q;
-  leaf_query<KIND>(C, md, nr, m, n, mw, nw, q);
+  float R[9];
+  leaf_query<KIND>(C, md, nr, m, n, mw, nw, q, R);
   int idx;
   DNode nd;
   descend(F, fnn, staged, nstaged, q, idx, nd);
-  leaf_math<KIND>(C, m, n, md.w, mw, nw, idx, nd, fdts, P, stats_mode, status, match, e_out, gamma_out, J);
+  leaf_math<KIND>(C, m, n, md.w, mw, nw, R, idx, nd, fdts, P, stats_mode, status, match, e_out, gamma_out, J);
 }
 
-// entry k of the packed D(D+1)/2 + D vector -> (row, col); col == D means "e"
+// Entry k of the packed D(D+1)/2 + D vector (upper triangle row by row, then J_r e):
+// (row, col); col == D means "e".
+template <int D>
+struct alignas(4) EntryTable {
+  static constexpr int M = D * (D + 1) / 2 + D;
+  unsigned char rc[M][2];
+};
+template <int D>
+constexpr EntryTable<D> make_entry_table() {
+  EntryTable<D> t{};
+  int k = 0;
+  for (int r = 0; r < D; ++r)
+    for (int c = r; c < D; ++c, ++k) {
+      t.rc[k][0] = (unsigned char)r;
+      t.rc[k][1] = (unsigned char)c;
+    }
+  for (int r = 0; r < D; ++r, ++k) {
+    t.rc[k][0] = (unsigned char)r;
+    t.rc[k][1] = (unsigned char)D;
+  }
+  return t;
+}
+__device__ const EntryTable<6> g_rc6 = make_entry_table<6>();
+__device__ const EntryTable<12> g_rc12 = make_entry_table<12>();
+__device__ const EntryTable<18> g_rc18 = make_entry_table<18>();
 __device__ __forceinline__ void entry_rc(int D, int k, int& r, int& c) {
-  int T = D * (D + 1) / 2;
-  if (k >= T) { r = k - T; c = D; return; }
-  int rr = 0, off = 0;
-  while (off + (D - rr) <= k) { off += D - rr; ++rr; }
-  r = rr;
-  c = rr + (k - off);
+  const unsigned char* t = D == 6 ? g_rc6.rc[k] : (D == 12 ? g_rc12.rc[k] : g_rc18.rc[k]);
+  const uchar2 v = __ldg(reinterpret_cast<const uchar2*>(t));
+  r = v.x;
+  c = v.y;
 }
 
 constexpr int kBlock = 128;
@@ -315,24 +341,36 @@ __device__ __forceinline__ void tile_reduce(int status, float e, float gamma, co
     chi2k += __shfl_xor_sync(full, chi2k, off);
   }
   __syncwarp();
-  // warp-cooperative outer products: lane owns entries lane, lane+32, ...
+  // Warp-cooperative outer products: lane owns entries lane, lane + 32, ..., all of them summed
+  // side by side (one compensated sum is a chain of four dependent operations per leaf).
+  constexpr int NE = (M + 31) / 32;
   const float* wf = fac + w * 32 * kMaxFS;
   double* wp = wpart + w * kPStride;
-  for (int k = lane; k < M; k += 32) {
+  const float *pr[NE], *pc[NE];
+  float s[NE], comp[NE];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
     int r, c;
-    entry_rc(D, k, r, c);
-    float s = 0.f, comp = 0.f;
-#pragma unroll 8
-    for (int l = 0; l < 32; ++l) {
-      const float* fr = wf + l * kMaxFS;
-      float val = fm(fm(fr[r], fr[c]), fr[D + 1]);
-      float y = fs(val, comp);
-      float t = fa(s, y);
-      comp = fs(fs(t, s), y);
-      s = t;
-    }
-    wp[k] = (double)s - (double)comp;
+    entry_rc(D, min(lane + 32 * k, M - 1), r, c);
+    pr[k] = wf + r;
+    pc[k] = wf + c;
+    s[k] = comp[k] = 0.f;
   }
+#pragma unroll 4
+  for (int l = 0; l < 32; ++l) {
+    const float g = wf[l * kMaxFS + D + 1];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      float val = fm(fm(pr[k][l * kMaxFS], pc[k][l * kMaxFS]), g);
+      float y = fs(val, comp[k]);
+      float t = fa(s[k], y);
+      comp[k] = fs(fs(t, s[k]), y);
+      s[k] = t;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NE; ++k)
+    if (lane + 32 * k < M) wp[lane + 32 * k] = (double)s[k] - (double)comp[k];
   if (lane == 0) {
     wp[kPStats + 0] = c_in;
     wp[kPStats + 1] = c_out;
@@ -380,14 +418,15 @@ __device__ __forceinline__ void tile_body_pair(const JobIn& Jn, const LinDev& L,
   const bool va = ia < TA.leaf_end, vb = has_b && ib < TB.leaf_end;
   F3 ma, na, mwa, nwa, qa, mb, nb, mwb, nwb, qb;
   float dta = 0.f, dtb = 0.f;
+  float R[9];  // recomputed after the descents: two would not fit the registers
   if (va) {
     const float4 md = __ldg(Jn.m_md + ia), nr = __ldg(Jn.m_nrm + ia);
-    leaf_query<KIND>(C, md, nr, ma, na, mwa, nwa, qa);
+    leaf_query<KIND>(C, md, nr, ma, na, mwa, nwa, qa, R);
     dta = md.w;
   }
   if (vb) {
     const float4 md = __ldg(Jn.m_md + ib), nr = __ldg(Jn.m_nrm + ib);
-    leaf_query<KIND>(C, md, nr, mb, nb, mwb, nwb, qb);
+    leaf_query<KIND>(C, md, nr, mb, nb, mwb, nwb, qb, R);
     dtb = md.w;
   }
   int xa, xb;
@@ -399,7 +438,8 @@ __device__ __forceinline__ void tile_body_pair(const JobIn& Jn, const LinDev& L,
 #pragma unroll
     for (int k = 0; k < D; ++k) J[k] = 0.f;
     if (va) {
-      leaf_math<KIND>(C, ma, na, dta, mwa, nwa, xa, nda, L.fdts, Jn.P, Jn.stats_mode != 0, status, match, e, gamma, J);
+      if (KIND != 0) rodrigues_x(f3(fm(C.v[3], dta), fm(C.v[4], dta), fm(C.v[5], dta)), R);
+      leaf_math<KIND>(C, ma, na, dta, mwa, nwa, R, xa, nda, L.fdts, Jn.P, Jn.stats_mode != 0, status, match, e, gamma, J);
       if (dbg_match) { dbg_match[ia] = match; dbg_status[ia] = status; }
     }
     tile_reduce<KIND>(status, e, gamma, J, wpa, fac);
@@ -410,7 +450,8 @@ __device__ __forceinline__ void tile_body_pair(const JobIn& Jn, const LinDev& L,
 #pragma unroll
     for (int k = 0; k < D; ++k) J[k] = 0.f;
     if (vb) {
-      leaf_math<KIND>(C, mb, nb, dtb, mwb, nwb, xb, ndb, L.fdts, Jn.P, Jn.stats_mode != 0, status, match, e, gamma, J);
+      if (KIND != 0) rodrigues_x(f3(fm(C.v[3], dtb), fm(C.v[4], dtb), fm(C.v[5], dtb)), R);
+      leaf_math<KIND>(C, mb, nb, dtb, mwb, nwb, R, xb, ndb, L.fdts, Jn.P, Jn.stats_mode != 0, status, match, e, gamma, J);
       if (dbg_match) { dbg_match[ib] = match; dbg_status[ib] = status; }
     }
     tile_reduce<KIND>(status, e, gamma, J, wpb, fac);
@@ -433,12 +474,6 @@ __device__ void iso_mul_d(const double* A, const double* B, double* C) {
     C[i * 4 + 3] = da(ddot3(A[i * 4], A[i * 4 + 1], A[i * 4 + 2], B[3], B[7], B[11]), A[i * 4 + 3]);
   }
 }
-__device__ void iso_inv_d(const double* A, double* B) {
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) B[i * 4 + j] = A[j * 4 + i];
-  for (int i = 0; i < 3; ++i) B[i * 4 + 3] = -ddot3(A[i], A[4 + i], A[8 + i], A[3], A[7], A[11]);
-}
-
 // Canonical FP64 sine/cosine (this project's own, shared with the CPU oracle so that the
 // pose update is bit-identical there): Cody-Waite reduction by pi/2 with a three-part
 // constant (Cody & Waite 1980; parts of 33, 33 and 53 bits, so q * C1 and q * C2 are
@@ -479,7 +514,7 @@ __device__ void sincos_canon_d(double x, double* s_out, double* c_out) {
 }
 
 // rodrigues (kd/utils/geometry_3d_impl_.h:37-46) in FP64: I + sin(a) S + (1 - cos(a)) S^2
-__device__ void rodrigues_d(const double* w, double* R) {
+__device__ __forceinline__ void rodrigues_d(const double* w, double* R) {
   const double a = sqrt(ddot3(w[0], w[1], w[2], w[0], w[1], w[2]));
   if (a < 1e-9) {
     for (int i = 0; i < 9; ++i) R[i] = (i % 4 == 0) ? 1.0 : 0.0;
@@ -496,14 +531,6 @@ __device__ void rodrigues_d(const double* w, double* R) {
       const double s2 = ddot3(S[i * 3], S[i * 3 + 1], S[i * 3 + 2], S[j], S[3 + j], S[6 + j]);
       R[i * 3 + j] = da(da((i == j) ? 1.0 : 0.0, dm(s, S[i * 3 + j])), dm(omc, s2));
     }
-}
-__device__ void expmap_d(const double* v, double* X) {
-  double R[9];
-  rodrigues_d(v + 3, R);
-  for (int i = 0; i < 3; ++i) {
-    for (int j = 0; j < 3; ++j) X[i * 4 + j] = R[i * 3 + j];
-    X[i * 4 + 3] = v[i];
-  }
 }
 __device__ void logso3_d(const double* X, double* w) {
   double tr = X[0] + X[5] + X[10];
@@ -564,24 +591,6 @@ __device__ void dpose_d(const double* ZXi, const double* Xm, double* e, double J
     }
 }
 
-__device__ void refresh_caches(const JobState& S, LinDev* lins, int lb, int lc) {
-  for (int l = lb; l < lb + lc; ++l) {
-    LinDev& L = lins[l];
-    double iXf[12], Xmf[12];
-    iso_inv_d(L.Xf, iXf);
-    iso_mul_d(iXf, S.X, Xmf);
-    for (int k = 0; k < 12; ++k) {
-      L.cache.Xm[k] = (float)S.X[k];
-      L.cache.Xf[k] = (float)L.Xf[k];
-      L.cache.Xmf[k] = (float)Xmf[k];
-    }
-    for (int k = 0; k < 6; ++k) {
-      L.cache.v[k] = (float)S.v[k];
-      L.cache.fv[k] = (float)L.fv[k];
-    }
-  }
-}
-
 // Pose prior (posePriorBuildQuadraticForm, kd/icp/tree_aligner_base_.h:139-152): adds
 // J^T Omega J and J^T Omega e to the pose block.  Single thread, used by the localizer.
 __device__ __noinline__ void add_pose_prior(const JobIn& Jn, const double* X, double* H, double* b, int D) {
@@ -611,22 +620,16 @@ __device__ __noinline__ void add_pose_prior(const JobIn& Jn, const double* X, do
   }
 }
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
-
 // ---------------------------------------------------------------------------
-// The last block of a job: FP64 sum of the job's partials in tile order, then warp 0
-// runs ICP_::oneRound / CTICP_::oneRound (kd/icp/icp_impl_.h:72-89,
-// kd/cticp/cticp_impl_.h:67-91) with the D x D system in shared memory: Cholesky of
-// H + damping (SPD), warp-parallel trailing updates and triangular solves.
-__device__ void tail_warp(const JobIn& Jn, JobState& S, JobOut& O, kds_stats* log, LinDev* lins, double* red, int M);
+// The last block of a job: FP64 sum of the job's partials in tile order (a thread per entry),
+// then warp 0 runs ICP_::oneRound / CTICP_::oneRound (kd/icp/icp_impl_.h:72-89,
+// kd/cticp/cticp_impl_.h:67-91): Cholesky of H + damping (SPD) and the triangular solves with
+// a row per lane in registers, the pose update, the termination test and the float caches
+// of the next iteration.
 
 // Phase stamps (clock64) of the last launch, recorded only when profiling is on:
 // [0..3] block 0: entry, staged, tile done, partial published; [8..15] tail block:
-// entry, partials summed, state staged, solve start, factorized, solved, updated, done.
+// entry, partials summed, state staged, solve start, -, solved, updated, done.
 __device__ int g_phase_on;
 __device__ unsigned long long g_phase[16];
 // Error bits of a k_linearize launch whose caller passed no error slot of its own (the
@@ -652,241 +655,317 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int sp
   return false;
 }
 
-constexpr int kTailJobOff = 560;    // doubles into the tail's shared scratch
-constexpr int kTailStateOff = 680;
-static_assert(kTailJobOff + sizeof(JobIn) / 8 + 1 <= kTailStateOff, "tail scratch layout");
-static_assert(kTailStateOff + sizeof(JobState) / 8 + 1 <= 4 * kPStride, "tail scratch layout");
+// Shared scratch of a job's step, in doubles.
+constexpr int kTailH = 0;                           // H, D x D
+constexpr int kTailB = 144;                         // b
+constexpr int kTailStats = 156;                     // the 7 stats sums
+constexpr int kTailX = 164;                         // dx
+constexpr int kTailA = 176;                         // Cholesky factor (transposed read)
+constexpr int kTailP = 320;                         // 2 x 12: pose products
+constexpr int kTailLin = 344;                       // Xf (12), fv (6) of the first fixed entry
+constexpr int kTailJob = 362;                       // the job's inputs
+constexpr int kTailState = kTailJob + (int)(sizeof(JobIn) / 8);
+constexpr int kTailDoubles = kTailState + (int)(sizeof(JobState) / 8);
+static_assert(sizeof(JobIn) % 8 == 0 && sizeof(JobState) % 8 == 0, "staged as 8 B words");
+static_assert(kTailDoubles <= kWarps * kPStride, "the step's scratch reuses the warps' partials");
+static_assert(sizeof(JobIn) / 8 + sizeof(JobState) / 8 + 18 <= kBlock, "one staged word per thread");
 
-__device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O, kds_stats* log, LinDev* lins,
-                                      const double* partials, double* red, int M) {
-  const bool stamp = g_phase_on && threadIdx.x == 0;
-  if (stamp) g_phase[8] = clock64();
-  for (int k = threadIdx.x; k < kPStride; k += blockDim.x) {
-    if (k >= M && k < kPStats) { red[k] = 0.0; continue; }
-    double acc = 0.0;
-    const double* src = partials + (size_t)JnG.tile_begin * kPStride + k;
-    const int nt = JnG.tile_count;
+// Sums entry by entry over the nt partials at `partials`, in tile order over four interleaved
+// accumulators; H and b go to scr, the dual blocks to O.  Threads 0..kBlock-1 (tid).
+template <int KIND, bool SMEM>
+__device__ __forceinline__ void tail_sums(const double* partials, int stride, int nt, double* scr, JobOut& O, int tid) {
+  constexpr int DK = KindDim<KIND>::D;
+  constexpr int M = DK * (DK + 1) / 2 + DK;
+  constexpr int D = KIND == 0 ? 6 : 12;
+  auto load = [&](const double* p) { return SMEM ? *p : __ldcg(p); };
+  for (int e = tid; e < M + 7; e += kBlock) {
+    int r = 0, c = 0;
+    if (e < M) entry_rc(DK, e, r, c);
+    const double* src = partials + (SMEM || e < M ? e : kPStats + (e - M));
     double a4[4] = {0.0, 0.0, 0.0, 0.0};
     int t = 0;
-    for (; t + 4 <= nt; t += 4) {
+    for (; t + 16 <= nt; t += 16) {  // sixteen loads in flight
+      double v[16];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) a4[u] += __ldcg(src + (size_t)(t + u) * kPStride);
+      for (int u = 0; u < 16; ++u) v[u] = load(src + (size_t)(t + u) * stride);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) a4[u & 3] += v[u];
     }
-    for (; t < nt; ++t) a4[0] += __ldcg(src + (size_t)t * kPStride);
-    acc = (a4[0] + a4[1]) + (a4[2] + a4[3]);
-    red[k] = acc;
-  }
-  __syncthreads();
-  if (stamp) g_phase[9] = clock64();
-  if (threadIdx.x >= 32) return;
-  // the job's inputs and state move to shared memory in one parallel round trip
-  JobIn* sJn = reinterpret_cast<JobIn*>(red + kTailJobOff);
-  JobState* sS = reinterpret_cast<JobState*>(red + kTailStateOff);
-  {
-    typedef unsigned long long u64;
-    constexpr int NJ = sizeof(JobIn) / 8, NS = sizeof(JobState) / 8;
-    static_assert(sizeof(JobIn) % 8 == 0 && sizeof(JobState) % 8 == 0 && NJ <= 96 && NS <= 32, "staging");
-    const u64* a = reinterpret_cast<const u64*>(&JnG);
-    const u64* c = reinterpret_cast<const u64*>(&SG);
-    const int l = threadIdx.x;
-    u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;  // all loads issued before any store
-    if (l < NJ) r0 = a[l];
-    if (l + 32 < NJ) r1 = a[l + 32];
-    if (l + 64 < NJ) r2 = a[l + 64];
-    if (l < NS) r3 = c[l];
-    u64* b = reinterpret_cast<u64*>(sJn);
-    u64* d = reinterpret_cast<u64*>(sS);
-    if (l < NJ) b[l] = r0;
-    if (l + 32 < NJ) b[l + 32] = r1;
-    if (l + 64 < NJ) b[l + 64] = r2;
-    if (l < NS) d[l] = r3;
-  }
-  __syncwarp();
-  if (stamp) g_phase[10] = clock64();
-  tail_warp(*sJn, *sS, O, log, lins, red, M);
-  __syncwarp();
-  {
-    const unsigned long long* c = reinterpret_cast<const unsigned long long*>(sS);
-    unsigned long long* d = reinterpret_cast<unsigned long long*>(&SG);
-    if (threadIdx.x < (int)(sizeof(JobState) / 8)) d[threadIdx.x] = c[threadIdx.x];
-  }
-  if (stamp) g_phase[15] = clock64();
-}
-
-// Warp 0 of the last block: unpack, prior, solve, update, termination test.
-__device__ void tail_warp(const JobIn& Jn, JobState& S, JobOut& O, kds_stats* log, LinDev* lins, double* red, int M) {
-  const int lane = threadIdx.x;
-  const int kind = Jn.kind;
-  const int Dk = kind == 0 ? 6 : (kind == 1 ? 12 : 18);
-  const int D = kind == 0 ? 6 : 12;
-  double* sH = red + kPStride;  // D*D
-  double* sA = sH + 144;        // D*D
-  double* sb = sA + 144;        // D
-  double* sy = sb + 12;         // D
-  double* sx = sy + 12;         // D
-  // unpack the packed upper triangle
-  for (int k = lane; k < M; k += 32) {
-    int r, c;
-    entry_rc(Dk, k, r, c);
-    double v = red[k];
-    if (c == Dk) {
-      if (r < D) sb[r] = v;
+    for (; t + 4 <= nt; t += 4) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = load(src + (size_t)(t + u) * stride);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a4[u] += v[u];
+    }
+    for (; t < nt; ++t) a4[0] += load(src + (size_t)t * stride);
+    const double v = (a4[0] + a4[1]) + (a4[2] + a4[3]);
+    if (e >= M) {
+      scr[kTailStats + e - M] = v;
+    } else if (c == DK) {
+      if (r < D) scr[kTailB + r] = v;
       else O.b_vel_B[r - 12] = v;
     } else if (c < D) {
-      sH[r * D + c] = v;
-      sH[c * D + r] = v;
+      scr[kTailH + r * D + c] = v;
+      scr[kTailH + c * D + r] = v;
     } else {  // dual blocks, c >= 12
       if (r < 6) O.H_cross_pose_vel_B[r * 6 + (c - 12)] = v;
       else if (r < 12) O.H_cross_vel_AB[(r - 6) * 6 + (c - 12)] = v;
       else { O.H_vel_B[(r - 12) * 6 + (c - 12)] = v; O.H_vel_B[(c - 12) * 6 + (r - 12)] = v; }
     }
   }
+}
+
+__device__ __forceinline__ kds_stats tail_stats(const double* scr) {
   kds_stats st;
-  st.num_inliers = (int32_t)red[kPStats + 0];
-  st.num_outliers = (int32_t)red[kPStats + 1];
-  st.num_bad = (int32_t)red[kPStats + 2];
-  st.num_err_normal = (int32_t)red[kPStats + 3];
-  st.num_err_fn = (int32_t)red[kPStats + 4];
-  st.chi2 = (float)red[kPStats + 5];
-  st.chi2_kernelized = (float)red[kPStats + 6];
+  st.num_inliers = (int32_t)scr[kTailStats + 0];
+  st.num_outliers = (int32_t)scr[kTailStats + 1];
+  st.num_bad = (int32_t)scr[kTailStats + 2];
+  st.num_err_normal = (int32_t)scr[kTailStats + 3];
+  st.num_err_fn = (int32_t)scr[kTailStats + 4];
+  st.chi2 = (float)scr[kTailStats + 5];
+  st.chi2_kernelized = (float)scr[kTailStats + 6];
   st.pert_pose_norm = 0.f;
   st.pert_vel_norm = 0.f;
-  const int it = S.iter;
-  __syncwarp();
-  if (Jn.mode != KDS_JOB_COMPUTE) {
-    for (int i = lane; i < D * D; i += 32) O.H[i] = sH[i];
-    if (lane < D) O.b[lane] = sb[lane];
-    if (lane == 0) {
-      O.stats = st;
-      O.result = 0;
-      O.iterations = 1;
-      S.done = 1;
-      S.arrive = 0u;
-    }
-    return;
+  return st;
+}
+
+// dx = -(H + damping)^-1 b by one warp: lane i holds row i of the lower triangle (Cholesky by
+// columns, right-looking), then L y = -b and L^T x = y by column sweeps.  0 where H + damping
+// is not positive definite.  The rows in registers make a pivot a chain of one shuffle,
+// square root and division (350 cycles; 1,000 with the matrix in shared memory).
+template <int D>
+__device__ __forceinline__ void tail_solve(double* scr, float damping, float velocity_damping, int lane) {
+  double a[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    a[j] = lane < D ? scr[kTailH + lane * D + j] : 0.0;
+    if (lane == j) a[j] += j < 6 ? (double)damping : (double)velocity_damping;
   }
-  if (Jn.prior_enabled && lane == 0) add_pose_prior(Jn, S.X, sH, sb, D);
-  __syncwarp();
-  for (int i = lane; i < D * D; i += 32) {
-    O.H[i] = sH[i];
-    sA[i] = sH[i];
+  double myinv = 0.0;  // 1 / L(lane, lane)
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const double d = __shfl_sync(0xffffffffu, a[k], k);
+    ok = ok && (d > 0.0);
+    const double lkk = sqrt(fmax(d, 1e-300));
+    const double inv = 1.0 / lkk;
+    if (lane == k) {
+      a[k] = lkk;
+      myinv = inv;
+    } else if (lane > k) {
+      a[k] *= inv;
+    }
+#pragma unroll
+    for (int j = k + 1; j < D; ++j) {
+      const double ljk = __shfl_sync(0xffffffffu, a[k], j);
+      if (lane >= j) a[j] -= a[k] * ljk;
+    }
   }
   if (lane < D) {
-    O.b[lane] = sb[lane];
-    sA[lane * D + lane] += (lane < 6) ? (double)Jn.P.damping : (double)Jn.P.velocity_damping;
+#pragma unroll
+    for (int j = 0; j < D; ++j) scr[kTailA + lane * D + j] = a[j];
   }
+  double y = lane < D ? -scr[kTailB + lane] : 0.0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const double yk = __shfl_sync(0xffffffffu, y * myinv, k);
+    if (lane == k) y = yk;
+    if (lane > k) y -= a[k] * yk;
+  }
+  __syncwarp();
+  double lt[D];  // column `lane` of L
+#pragma unroll
+  for (int k = 0; k < D; ++k) lt[k] = lane < D && k > lane ? scr[kTailA + k * D + lane] : 0.0;
+#pragma unroll
+  for (int k = D - 1; k >= 0; --k) {
+    const double xk = __shfl_sync(0xffffffffu, y * myinv, k);
+    if (lane == k) y = xk;
+    if (lane < k) y -= lt[k] * xk;
+  }
+  if (lane < D) scr[kTailX + lane] = ok ? y : 0.0;
+  __syncwarp();
+}
+
+// The float caches of one (job, fixed entry) pair at pose X and velocities v (shared memory)
+// by one warp: element e of the caches through put(e, value).  Xf, fv: the entry's (shared);
+// tmp: 12 doubles.
+template <class Put>
+__device__ __forceinline__ void tail_caches(const double* X, const double* v, const double* Xf, const double* fv,
+                                            double* tmp, int lane, Put put) {
+  if (lane < 12) {  // inverse of Xf
+    const int i = lane >> 2, j = lane & 3;
+    tmp[lane] = j < 3 ? Xf[j * 4 + i] : -ddot3(Xf[i], Xf[4 + i], Xf[8 + i], Xf[3], Xf[7], Xf[11]);
+  }
+  __syncwarp();
+  if (lane < 12) {
+    const int i = lane >> 2, j = lane & 3;
+    double m = ddot3(tmp[i * 4], tmp[i * 4 + 1], tmp[i * 4 + 2], X[j], X[4 + j], X[8 + j]);
+    if (j == 3) m = da(m, tmp[i * 4 + 3]);
+    put(lane, (float)X[lane]);
+    put(12 + lane, (float)Xf[lane]);
+    put(24 + lane, (float)m);
+  } else if (lane < 18) {
+    put(36 + lane - 12, (float)v[lane - 12]);
+    put(42 + lane - 12, (float)fv[lane - 12]);
+  }
+  __syncwarp();
+}
+
+// A COMPUTE job's step by one warp, from H, b and the stats in scr: solve, update, test, then
+// caches() (unless the job is done), then the outputs.  Jn and S are in shared memory.
+template <int KIND, class Caches>
+__device__ __forceinline__ void tail_step(const JobIn& Jn, JobState& S, JobOut& O, kds_stats* log, double* scr,
+                                          int lane, Caches caches) {
+  constexpr int D = KIND == 0 ? 6 : 12;
+  kds_stats st = tail_stats(scr);
+  const int it = S.iter;
   if (st.num_inliers + st.num_outliers < Jn.P.min_good_measurements) {
+    __syncwarp();
     if (lane == 0) {
       if (log && it < kMaxLog) log[it] = st;
       O.stats = st;
       O.iterations = it + 1;
       S.done = 1;
       S.result = -it;
-      O.result = S.result;
+      O.result = -it;
       S.arrive = 0u;
     }
+    __syncwarp();
     return;
   }
-  __syncwarp();
   if (g_phase_on && lane == 0) g_phase[11] = clock64();
-  // Cholesky of the lower triangle of sA: per pivot one square root and reciprocal,
-  // the column scaled by the lanes, the trailing update spread over all lanes.
-  double* sinv = sx + 12;  // reciprocals of diag(L)
-  bool ok = true;
-  for (int k = 0; k < D; ++k) {
-    double d = sA[k * D + k];
-    ok = ok && (d > 0.0);
-    double lkk = sqrt(fmax(d, 1e-300));
-    double inv = 1.0 / lkk;
-    __syncwarp();
-    if (lane > k && lane < D) sA[lane * D + k] *= inv;
-    if (lane == k) {
-      sA[k * D + k] = lkk;
-      sinv[k] = inv;
+  tail_solve<D>(scr, Jn.P.damping, Jn.P.velocity_damping, lane);
+  if (g_phase_on && lane == 0) g_phase[13] = clock64();
+  const double* dx = scr + kTailX;
+  double pose = 0.0, vel = 0.0;  // this lane's element of the updated state
+  if (lane < 12) pose = S.X[lane];
+  else if (lane < 18) vel = S.v[lane - 12];
+  if (!Jn.stats_mode) {
+    // X <- expmap(dx) X, an element per lane
+    double R[9];
+    rodrigues_d(dx + 3, R);
+    if (lane < 12) {
+      const int i = lane >> 2, j = lane & 3;
+      const double r0 = i == 0 ? R[0] : (i == 1 ? R[3] : R[6]), r1 = i == 0 ? R[1] : (i == 1 ? R[4] : R[7]);
+      const double r2 = i == 0 ? R[2] : (i == 1 ? R[5] : R[8]);
+      pose = ddot3(r0, r1, r2, S.X[j], S.X[4 + j], S.X[8 + j]);
+      if (j == 3) pose = da(pose, dx[i]);
+    } else if (D == 12 && lane < 18) {
+      vel += dx[6 + lane - 12];
     }
-    __syncwarp();
-    // pairs (i, j), k < j <= i < D, enumerated row-major over the trailing triangle
-    const int m = D - k - 1;
-    const int npair = m * (m + 1) / 2;
-    for (int p = lane; p < npair; p += 32) {
-      int ii = 0;
-      while ((ii + 1) * (ii + 2) / 2 <= p) ++ii;
-      const int i = k + 1 + ii, j = k + 1 + (p - ii * (ii + 1) / 2);
-      sA[i * D + j] -= sA[i * D + k] * sA[j * D + k];
-    }
-    __syncwarp();
   }
-  if (g_phase_on && lane == 0) g_phase[12] = clock64();
-  // L y = -b and L^T x = y by column sweeps
-  if (lane < D) sy[lane] = -sb[lane];
-  __syncwarp();
-  for (int k = 0; k < D; ++k) {
-    const double yk = sy[k] * sinv[k];
-    __syncwarp();
-    if (lane == k) sy[k] = yk;
-    if (lane > k && lane < D) sy[lane] -= sA[lane * D + k] * yk;
-    __syncwarp();
-  }
-  if (lane < D) sx[lane] = sy[lane];
-  __syncwarp();
-  for (int k = D - 1; k >= 0; --k) {
-    const double xk = sx[k] * sinv[k];
-    __syncwarp();
-    if (lane == k) sx[k] = xk;
-    if (lane < k) sx[lane] -= sA[k * D + lane] * xk;
-    __syncwarp();
-  }
-  if (lane != 0) return;
-  if (g_phase_on) g_phase[13] = clock64();
-  double dx[12];
-  for (int i = 0; i < D; ++i) dx[i] = ok ? sx[i] : 0.0;
+  bool stop = false;
   double pp = 0.0, pv = 0.0;
+#pragma unroll
   for (int i = 0; i < 6; ++i) pp += dx[i] * dx[i];
   st.pert_pose_norm = (float)sqrt(pp);
   if (D == 12) {
-    for (int i = 6; i < 12; ++i) pv += dx[i] * dx[i];
+#pragma unroll
+    for (int i = 6; i < D; ++i) pv += dx[i] * dx[i];
     st.pert_vel_norm = (float)sqrt(pv);
   }
-  for (int i = 0; i < D; ++i) O.dx[i] = dx[i];
-  if (log && it < kMaxLog) log[it] = st;
-  O.stats = st;
-  O.iterations = it + 1;
-  if (!Jn.stats_mode) {
-    double dX[12], Xn[12];
-    expmap_d(dx, dX);
-    iso_mul_d(dX, S.X, Xn);
-    for (int i = 0; i < 12; ++i) S.X[i] = Xn[i];
-    if (D == 12)
-      for (int i = 0; i < 6; ++i) S.v[i] += dx[6 + i];
-  }
-  bool stop = false;
+  float score = 0.f;
   if (Jn.P.term_crit) {
     // ICPTerminationCriteriaScore_::hasToStop (kd/icp/icp_stats_.h:91-101)
     int nl = st.num_inliers + st.num_outliers + st.num_bad + st.num_err_normal + st.num_err_fn;
     float ratio = nl ? (float)st.num_inliers / (float)nl : 0.f;
-    float score = ratio / (st.chi2_kernelized / (float)st.num_inliers + 1e-6f);
+    score = ratio / (st.chi2_kernelized / (float)st.num_inliers + 1e-6f);
     if (it > 0) {
       bool pert_ok = st.pert_pose_norm < Jn.P.d_pert;
       float dsc = score - S.prev_score;
       bool score_ok = (dsc > 0.f) && ((double)dsc / ((double)S.prev_score + 1e-6) < (double)Jn.P.d_score);
       if (pert_ok && score_ok) stop = true;
     }
-    S.prev_score = score;
   }
-  S.iter = it + 1;
-  if (stop) {
-    S.done = 1;
-    S.result = it;
-  } else if (S.iter >= S.max_iter) {
-    S.done = 1;
-    S.result = Jn.P.max_iterations;
+  const bool last = it + 1 >= S.max_iter;
+  const int result = stop ? it : (last ? Jn.P.max_iterations : S.result);
+  __syncwarp();  // the state was read by every lane
+  if (lane < 12) S.X[lane] = pose;
+  else if (lane < 18) S.v[lane - 12] = vel;
+  if (lane == 0) {
+    if (Jn.P.term_crit) S.prev_score = score;
+    S.iter = it + 1;
+    S.result = result;
+    if (stop || last) S.done = 1;
+    S.arrive = 0u;
   }
-  O.result = S.result;
-  for (int i = 0; i < 12; ++i) O.X[i] = S.X[i];
-  for (int i = 0; i < 6; ++i) O.v[i] = S.v[i];
-  if (!S.done) refresh_caches(S, lins, Jn.lin_begin, Jn.lin_count);
-  if (g_phase_on) g_phase[14] = clock64();
-  S.arrive = 0u;
+  __syncwarp();
+  if (!stop && !last) caches();
+  if (lane < D) O.dx[lane] = dx[lane];
+  if (lane < 12) O.X[lane] = S.X[lane];
+  else if (lane < 18) O.v[lane - 12] = S.v[lane - 12];
+  if (lane == 0) {
+    if (log && it < kMaxLog) log[it] = st;
+    O.stats = st;
+    O.iterations = it + 1;
+    O.result = result;
+  }
+  if (g_phase_on && lane == 0) g_phase[14] = clock64();
+}
+
+// Threads 0..kBlock-1 of the job's last block.
+template <int KIND>
+__device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O, kds_stats* log, LinDev* lins,
+                                      const double* partials, double* scr) {
+  constexpr int D = KIND == 0 ? 6 : 12;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool stamp = g_phase_on && tid == 0;
+  if (stamp) g_phase[8] = clock64();
+  // the job's inputs, state and first fixed entry to shared memory, one word per thread,
+  // beside the partials' loads
+  typedef unsigned long long u64;
+  constexpr int NJ = sizeof(JobIn) / 8, NS = sizeof(JobState) / 8;
+  u64 word = 0;
+  if (tid < NJ) word = reinterpret_cast<const u64*>(&JnG)[tid];
+  else if (tid < NJ + NS) word = reinterpret_cast<const u64*>(&SG)[tid - NJ];
+  else if (tid < NJ + NS + 12) word = __double_as_longlong(lins[JnG.lin_begin].Xf[tid - NJ - NS]);
+  else if (tid < NJ + NS + 18) word = __double_as_longlong(lins[JnG.lin_begin].fv[tid - NJ - NS - 12]);
+  tail_sums<KIND, false>(partials + (size_t)JnG.tile_begin * kPStride, kPStride, JnG.tile_count, scr, O, tid);
+  u64* dst = reinterpret_cast<u64*>(scr);
+  if (tid < NJ + NS) dst[kTailJob + tid] = word;
+  else if (tid < NJ + NS + 18) dst[kTailLin + tid - NJ - NS] = word;
+  __syncthreads();
+  if (stamp) g_phase[9] = g_phase[10] = clock64();
+  const JobIn& Jn = *reinterpret_cast<const JobIn*>(scr + kTailJob);
+  JobState& S = *reinterpret_cast<JobState*>(scr + kTailState);
+  if (Jn.mode != KDS_JOB_COMPUTE) {
+    for (int i = tid; i < D * D; i += kBlock) O.H[i] = scr[kTailH + i];
+    if (tid < D) O.b[tid] = scr[kTailB + tid];
+    if (tid == 0) {
+      O.stats = tail_stats(scr);
+      O.result = 0;
+      O.iterations = 1;
+      SG.done = 1;
+      SG.arrive = 0u;
+    }
+    return;
+  }
+  if (Jn.prior_enabled) {
+    if (tid == 0) add_pose_prior(Jn, S.X, scr + kTailH, scr + kTailB, D);
+    __syncthreads();
+  }
+  if (tid >= 32) {
+    for (int i = tid - 32; i < D * D; i += kBlock - 32) O.H[i] = scr[kTailH + i];
+    if (tid - 32 < D) O.b[tid - 32] = scr[kTailB + tid - 32];
+    return;
+  }
+  tail_step<KIND>(Jn, S, O, log, scr, lane, [&]() {
+    for (int l = 0; l < Jn.lin_count; ++l) {
+      LinDev& L = lins[Jn.lin_begin + l];
+      if (l > 0) {
+        if (lane < 12) scr[kTailLin + lane] = L.Xf[lane];
+        else if (lane < 18) scr[kTailLin + lane] = L.fv[lane - 12];
+        __syncwarp();
+      }
+      float* c = reinterpret_cast<float*>(&L.cache);
+      tail_caches(S.X, S.v, scr + kTailLin, scr + kTailLin + 12, scr + kTailP, lane,
+                  [&](int e, float x) { c[e] = x; });
+    }
+  });
+  __syncwarp();
+  if (lane < NS) reinterpret_cast<u64*>(&SG)[lane] = reinterpret_cast<const u64*>(&S)[lane];
+  if (stamp) g_phase[15] = clock64();
 }
 
 // One Gauss-Newton iteration over the tiles [tile0, tile0 + gridDim.x) of one kind.
@@ -967,7 +1046,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize(const JobIn* __restrict
     return;
   }
   __threadfence();
-  job_tail(Jn, S, outs[T.job], logs ? logs + (size_t)T.job * kMaxLog : nullptr, lins, partials, swp, M);
+  job_tail<KIND>(Jn, S, outs[T.job], logs ? logs + (size_t)T.job * kMaxLog : nullptr, lins, partials, swp);
   settle();
 }
 
@@ -1046,7 +1125,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_pair(const JobIn* __res
     return;
   }
   __threadfence();
-  job_tail(Jn, S, outs[TA.job], logs ? logs + (size_t)TA.job * kMaxLog : nullptr, lins, partials, swp[0], M);
+  job_tail<KIND>(Jn, S, outs[TA.job], logs ? logs + (size_t)TA.job * kMaxLog : nullptr, lins, partials, swp[0]);
   settle();
 }
 
@@ -1184,8 +1263,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_persistent(const JobIn*
     __syncthreads();
     if (s_last) {
       __threadfence();
-      const int Mk = Jn.kind == 0 ? 27 : (Jn.kind == 1 ? 90 : 189);
-      job_tail(Jn, S, outs[T.job], logs ? logs + (size_t)T.job * kMaxLog : nullptr, lins, partials, swp, Mk);
+      kds_stats* log = logs ? logs + (size_t)T.job * kMaxLog : nullptr;
+      if (Jn.kind == 0) job_tail<0>(Jn, S, outs[T.job], log, lins, partials, swp);
+      else if (Jn.kind == 1) job_tail<1>(Jn, S, outs[T.job], log, lins, partials, swp);
+      else job_tail<2>(Jn, S, outs[T.job], log, lins, partials, swp);
       if (threadIdx.x < 32) {  // every lane that wrote the job's state makes it visible, then publish
         __threadfence();
         __syncwarp();
@@ -1199,47 +1280,74 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_persistent(const JobIn*
   }
 }
 
-// Resets control state, seeds state from the job inputs and writes the first caches.
-__device__ void init_job(int j, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins) {
+// Resets control state, seeds state from the job inputs and writes the first caches: a warp
+// per job (a thread per job took 7 us for one job, 20 us for 250: every store a sector of its
+// own, the pose algebra one element after the other).
+constexpr int kInitWarps = 4;
+struct InitScratch {
+  double X[12], v[6], Xf[12], fv[6], tmp[12];
+};
+__device__ __forceinline__ void init_job(int j, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
+                                         InitScratch& C, int lane) {
   const JobIn& Jn = jobs[j];
   JobState& S = states[j];
-  for (int i = 0; i < 12; ++i) S.X[i] = Jn.X0[i];
-  for (int i = 0; i < 6; ++i) S.v[i] = Jn.v0[i];
-  S.iter = 0;
-  S.done = 0;
-  S.result = 0;
-  S.arrive = 0u;
-  S.prev_score = 0.f;
-  S.max_iter = Jn.stats_mode ? 1 : Jn.P.max_iterations;
   JobOut& O = outs[j];
-  for (int i = 0; i < 12; ++i) O.X[i] = S.X[i];
-  for (int i = 0; i < 6; ++i) O.v[i] = S.v[i];
-  O.result = Jn.P.max_iterations;
-  O.iterations = 0;
-  if (Jn.tile_count == 0 || S.max_iter <= 0) {
+  const int max_iter = Jn.stats_mode ? 1 : Jn.P.max_iterations;
+  const bool idle = Jn.tile_count == 0 || max_iter <= 0;
+  if (lane < 12) {
+    C.X[lane] = S.X[lane] = O.X[lane] = Jn.X0[lane];
+  } else if (lane < 18) {
+    C.v[lane - 12] = S.v[lane - 12] = O.v[lane - 12] = Jn.v0[lane - 12];
+  } else if (lane == 18) {
+    S.iter = 0;
+    S.done = idle ? 1 : 0;
+    S.result = 0;
+    S.arrive = 0u;
+    S.prev_score = 0.f;
+    S.max_iter = max_iter;
+    O.result = Jn.P.max_iterations;
+    O.iterations = 0;
+  }
+  __syncwarp();
+  if (idle) {
     // no moving leaves: the round sees zero measurements and fails at iteration 0
-    kds_stats z;
-    memset(&z, 0, sizeof(z));
-    O.stats = z;
-    for (int i = 0; i < 144; ++i) O.H[i] = 0.0;
-    for (int i = 0; i < 12; ++i) { O.b[i] = 0.0; O.dx[i] = 0.0; }
-    S.done = 1;
-    O.result = (Jn.mode == KDS_JOB_COMPUTE && S.max_iter > 0 && Jn.P.min_good_measurements > 0) ? 0
-                                                                                                  : Jn.P.max_iterations;
-    if (Jn.mode != KDS_JOB_COMPUTE) O.result = 0;
+    for (int i = lane; i < 144; i += 32) O.H[i] = 0.0;
+    if (lane < 12) O.b[lane] = O.dx[lane] = 0.0;
+    if (lane == 0) {
+      kds_stats z;
+      memset(&z, 0, sizeof(z));
+      O.stats = z;
+      O.result = (Jn.mode == KDS_JOB_COMPUTE && max_iter > 0 && Jn.P.min_good_measurements > 0) ? 0
+                                                                                                : Jn.P.max_iterations;
+      if (Jn.mode != KDS_JOB_COMPUTE) O.result = 0;
+    }
     return;
   }
-  if (!Jn.keep_cache) refresh_caches(S, lins, Jn.lin_begin, Jn.lin_count);
+  if (Jn.keep_cache) return;
+  for (int l = Jn.lin_begin; l < Jn.lin_begin + Jn.lin_count; ++l) {
+    LinDev& L = lins[l];
+    if (lane < 12) C.Xf[lane] = L.Xf[lane];
+    else if (lane < 18) C.fv[lane - 12] = L.fv[lane - 12];
+    __syncwarp();
+    float* c = reinterpret_cast<float*>(&L.cache);
+    tail_caches(C.X, C.v, C.Xf, C.fv, C.tmp, lane, [&](int e, float x) { c[e] = x; });
+  }
 }
 
-__global__ void k_init_jobs(const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins, int num_jobs,
-                            int32_t* err, int32_t* ready = nullptr, unsigned int* queue = nullptr) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j == 0 && err) *err = 0;
-  if (j == 0 && queue) { queue[0] = 0u; queue[1] = 0u; }
-  if (j < num_jobs && ready) ready[j] = 0;
+__global__ void __launch_bounds__(32 * kInitWarps) k_init_jobs(const JobIn* jobs, JobState* states, JobOut* outs,
+                                                               LinDev* lins, int num_jobs, int32_t* err,
+                                                               int32_t* ready = nullptr,
+                                                               unsigned int* queue = nullptr) {
+  __shared__ InitScratch scratch[kInitWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = blockIdx.x * kInitWarps + w;
+  if (j == 0 && lane == 0) {
+    if (err) *err = 0;
+    if (queue) { queue[0] = 0u; queue[1] = 0u; }
+  }
   if (j >= num_jobs) return;
-  init_job(j, jobs, states, outs, lins);
+  if (ready && lane == 0) ready[j] = 0;
+  init_job(j, jobs, states, outs, lins, scratch[w], lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -1275,7 +1383,7 @@ __global__ void k_popc(const uint32_t* bitmap, int64_t words, unsigned long long
 int count_touched(Runner& R, int kind, int64_t fixed_nodes, int64_t* out, cudaStream_t s) {
   *out = 0;
   if (R.num_jobs < 1 || fixed_nodes <= 0) return KDS_OK;
-  k_init_jobs<<<1, 128, 0, s>>>(R.d_jobs, R.d_states, R.d_outs, R.d_lins, 1, R.d_err); ::kds::count_launch();
+  k_init_jobs<<<1, 32 * kInitWarps, 0, s>>>(R.d_jobs, R.d_states, R.d_outs, R.d_lins, 1, R.d_err); ::kds::count_launch();
   int64_t words = (fixed_nodes + 31) / 32;
   uint32_t* bm = nullptr;
   unsigned long long* cnt = nullptr;
@@ -1490,8 +1598,8 @@ static int persistent_grid(size_t smem, int64_t items) {
 int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   if (num_jobs == 0) return KDS_OK;
   if (persistent && !dbg_match) {
-    k_init_jobs<<<(num_jobs + 127) / 128, 128, 0, s>>>(d_jobs, d_states, d_outs, d_lins, num_jobs, d_err, d_ready,
-                                                       d_queue);
+    k_init_jobs<<<(num_jobs + kInitWarps - 1) / kInitWarps, 32 * kInitWarps, 0, s>>>(
+        d_jobs, d_states, d_outs, d_lins, num_jobs, d_err, d_ready, d_queue);
     ::kds::count_launch();
     const int L = max_launches();
     prof_launches = profiling ? 1 : 0;
@@ -1517,7 +1625,8 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
     KDS_CK(cudaGetLastError());
     return KDS_OK;
   }
-  k_init_jobs<<<(num_jobs + 127) / 128, 128, 0, s>>>(d_jobs, d_states, d_outs, d_lins, num_jobs, d_err);
+  k_init_jobs<<<(num_jobs + kInitWarps - 1) / kInitWarps, 32 * kInitWarps, 0, s>>>(d_jobs, d_states, d_outs, d_lins,
+                                                                                   num_jobs, d_err);
   ::kds::count_launch();
   int L = max_launches();
   int nk = (kind_count[0] ? 1 : 0) + (kind_count[1] ? 1 : 0) + (kind_count[2] ? 1 : 0);
@@ -1647,14 +1756,22 @@ int timeout_status(int32_t err) {
 // Served-loop helpers (kds_serve.cu): jobs addressed by slot.
 namespace {
 
-__global__ void k_admit_slots(const int32_t* slots, int n, const JobIn* new_jobs, const LinDev* new_lins,
-                              JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kInitWarps) k_admit_slots(const int32_t* slots, int n, const JobIn* new_jobs,
+                                                                 const LinDev* new_lins, JobIn* jobs,
+                                                                 JobState* states, JobOut* outs, LinDev* lins) {
+  __shared__ InitScratch scratch[kInitWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * kInitWarps + w;
   if (i >= n) return;
   const int slot = slots[i];
-  jobs[slot] = new_jobs[i];
-  lins[slot] = new_lins[i];
-  init_job(slot, jobs, states, outs, lins);
+  typedef unsigned long long u64;
+  static_assert(sizeof(LinDev) % 8 == 0, "copied as 8 B words");
+  for (int k = lane; k < (int)(sizeof(JobIn) / 8); k += 32)
+    reinterpret_cast<u64*>(jobs + slot)[k] = reinterpret_cast<const u64*>(new_jobs + i)[k];
+  for (int k = lane; k < (int)(sizeof(LinDev) / 8); k += 32)
+    reinterpret_cast<u64*>(lins + slot)[k] = reinterpret_cast<const u64*>(new_lins + i)[k];
+  __syncwarp();
+  init_job(slot, jobs, states, outs, lins, scratch[w], lane);
 }
 
 __global__ void k_collect(int n, const JobState* states, const JobOut* outs, const unsigned long long* touched,
@@ -1691,7 +1808,7 @@ int linearize_smem_setup() {
 int launch_admit_slots(const int32_t* d_slots, int n, const JobIn* new_jobs, const LinDev* new_lins, JobIn* jobs,
                        JobState* states, JobOut* outs, LinDev* lins, cudaStream_t s) {
   if (n <= 0) return KDS_OK;
-  k_admit_slots<<<(n + 127) / 128, 128, 0, s>>>(d_slots, n, new_jobs, new_lins, jobs, states, outs, lins);
+  k_admit_slots<<<(n + kInitWarps - 1) / kInitWarps, 32 * kInitWarps, 0, s>>>(d_slots, n, new_jobs, new_lins, jobs, states, outs, lins);
   count_launch();
   KDS_CK(cudaGetLastError());
   return KDS_OK;
@@ -1883,7 +2000,7 @@ int linearize_static(const TreeDev& fixed, const TreeDev& moving, int32_t type, 
   for (int i = 0; i < 6; ++i) L.fv[i] = fv ? fv[i] : 0.0;
   k_static_setup<<<1, 256, 0, s>>>(scr, J, L, (int)ntiles);
   count_launch();
-  k_init_jobs<<<1, 128, 0, s>>>(&scr->job, &scr->state, &scr->res.out, &scr->lin, 1, &scr->res.err);
+  k_init_jobs<<<1, 32 * kInitWarps, 0, s>>>(&scr->job, &scr->state, &scr->res.out, &scr->lin, 1, &scr->res.err);
   count_launch();
   if (ntiles > 0) {
     const size_t stage_bytes = (size_t)kStaticStage * sizeof(DNode);

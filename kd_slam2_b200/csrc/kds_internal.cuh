@@ -182,12 +182,10 @@ __device__ __forceinline__ void rodrigues_x(F3 w, float* R) {
   float inv = __fdiv_rn(1.0f, angle);
   F3 n = f3(fm(w.x, inv), fm(w.y, inv), fm(w.z, inv));
   float S[9] = {0.0f, -n.z, n.y, n.z, 0.0f, -n.x, -n.y, n.x, 0.0f};
-  float S2[9];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      S2[i * 3 + j] = dot3x(f3(S[i * 3], S[i * 3 + 1], S[i * 3 + 2]), f3(S[j], S[3 + j], S[6 + j]));
+  // S S, each entry's dot product less its terms with a zero factor
+  float S2[9] = {fa(fm(-n.z, n.z), fm(n.y, -n.y)), fm(n.y, n.x), fm(n.z, n.x),
+                 fm(n.x, n.y), fa(fm(n.z, -n.z), fm(-n.x, n.x)), fm(n.z, n.y),
+                 fm(n.x, n.z), fm(n.y, n.z), fa(fm(-n.y, n.y), fm(n.x, -n.x))};
   float s, c;
   sincos_canon(angle, &s, &c);
   float omc = fs(1.0f, c);
@@ -201,13 +199,16 @@ __device__ __forceinline__ F3 mat_vec_x(const float* R, F3 p) {
   return f3(dot3x(f3(R[0], R[1], R[2]), p), dot3x(f3(R[3], R[4], R[5]), p), dot3x(f3(R[6], R[7], R[8]), p));
 }
 // CTICP_3D_Traits::applyVelocities (kd/d3/cticp_impl_.h:75-85): m' = R(w dt) m + v dt, n' = R n
-__device__ __forceinline__ void warp_x(const float* v, float dt, F3 m, F3 n, F3& mo, F3& no) {
+__device__ __forceinline__ void warp_x(const float* v, float dt, F3 m, F3 n, F3& mo, F3& no, float* R) {
   F3 td = f3(fm(v[0], dt), fm(v[1], dt), fm(v[2], dt));
   F3 rd = f3(fm(v[3], dt), fm(v[4], dt), fm(v[5], dt));
-  float R[9];
   rodrigues_x(rd, R);
   mo = add3x(mat_vec_x(R, m), td);
   no = mat_vec_x(R, n);
+}
+__device__ __forceinline__ void warp_x(const float* v, float dt, F3 m, F3 n, F3& mo, F3& no) {
+  float R[9];
+  warp_x(v, dt, m, n, mo, no, R);
 }
 }  // namespace kds
 
