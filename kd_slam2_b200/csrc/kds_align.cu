@@ -19,6 +19,7 @@
 //      batch), adds the pose prior, solves (H + damping) dx = -b by FP64 LDL^T, applies
 //      X <- expmap(dx) X, v += dx_v, runs the termination test and refreshes the
 //      float caches for the next launch.  No host round trip inside compute().
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -309,23 +310,27 @@ __device__ __forceinline__ void entry_rc(int D, int k, int& r, int& c) {
 
 constexpr int kBlock = 128;
 constexpr int kWarps = kBlock / 32;
-constexpr int kMaxFS = 21;  // factor row stride (D + 2, padded to odd)
+// A warp's factors in shared memory: row r (J_0 .. J_{D-1}, e, gamma) holds the 32 leaves' values,
+// read four leaves at a time; the row stride of 36 floats spreads the rows over the banks.
+constexpr int kFacStride = 36;
+constexpr int kMaxFac = 20 * kFacStride;  // floats per warp, D = 18
 
 // One warp's share of a tile partial from its 32 leaves' terms (leaf = lane): stats by
 // ballots, chi2 sums by xor butterfly, and gamma J^T J, gamma J^T e as float Kahan sums
 // over the lanes (lane k owns packed entries k, k + 32, ...) stored as s - comp in FP64.
-template <int KIND>
+// A warp's partial takes STRIDE doubles, its 7 stats at STATS.
+template <int KIND, int STRIDE = kPStride, int STATS = kPStats>
 __device__ __forceinline__ void tile_reduce(int status, float e, float gamma, const float* J, double* wpart,
                                             float* fac) {
   constexpr int D = KindDim<KIND>::D;
   constexpr int M = D * (D + 1) / 2 + D;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   bool contrib = status == ST_INLIER || status == ST_OUTLIER;
-  float* row = fac + (w * 32 + lane) * kMaxFS;
+  float* wf = fac + w * (D + 2) * kFacStride;
 #pragma unroll
-  for (int k = 0; k < D; ++k) row[k] = contrib ? J[k] : 0.f;
-  row[D] = contrib ? e : 0.f;
-  row[D + 1] = contrib ? gamma : 0.f;
+  for (int k = 0; k < D; ++k) wf[k * kFacStride + lane] = contrib ? J[k] : 0.f;
+  wf[D * kFacStride + lane] = contrib ? e : 0.f;
+  wf[(D + 1) * kFacStride + lane] = contrib ? gamma : 0.f;
   // stats (ICPStats_::pack, kd/icp/icp_stats_.h:57-59)
   unsigned full = 0xffffffffu;
   int c_in = __popc(__ballot_sync(full, status == ST_INLIER));
@@ -344,52 +349,63 @@ __device__ __forceinline__ void tile_reduce(int status, float e, float gamma, co
   // Warp-cooperative outer products: lane owns entries lane, lane + 32, ..., all of them summed
   // side by side (one compensated sum is a chain of four dependent operations per leaf).
   constexpr int NE = (M + 31) / 32;
-  const float* wf = fac + w * 32 * kMaxFS;
-  double* wp = wpart + w * kPStride;
-  const float *pr[NE], *pc[NE];
+  double* wp = wpart + w * STRIDE;
+  const float4 *pr[NE], *pc[NE];
   float s[NE], comp[NE];
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     int r, c;
     entry_rc(D, min(lane + 32 * k, M - 1), r, c);
-    pr[k] = wf + r;
-    pc[k] = wf + c;
+    pr[k] = reinterpret_cast<const float4*>(wf + r * kFacStride);
+    pc[k] = reinterpret_cast<const float4*>(wf + c * kFacStride);
     s[k] = comp[k] = 0.f;
   }
-#pragma unroll 4
-  for (int l = 0; l < 32; ++l) {
-    const float g = wf[l * kMaxFS + D + 1];
+  const float4* pg = reinterpret_cast<const float4*>(wf + (D + 1) * kFacStride);
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q) {
+    const float4 g4 = pg[q];
+    const float g[4] = {g4.x, g4.y, g4.z, g4.w};
+    float4 r4[NE], c4[NE];
 #pragma unroll
     for (int k = 0; k < NE; ++k) {
-      float val = fm(fm(pr[k][l * kMaxFS], pc[k][l * kMaxFS]), g);
-      float y = fs(val, comp[k]);
-      float t = fa(s[k], y);
-      comp[k] = fs(fs(t, s[k]), y);
-      s[k] = t;
+      r4[k] = pr[k][q];
+      c4[k] = pc[k][q];
     }
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {
+        const float rv = l == 0 ? r4[k].x : (l == 1 ? r4[k].y : (l == 2 ? r4[k].z : r4[k].w));
+        const float cv = l == 0 ? c4[k].x : (l == 1 ? c4[k].y : (l == 2 ? c4[k].z : c4[k].w));
+        float val = fm(fm(rv, cv), g[l]);
+        float y = fs(val, comp[k]);
+        float t = fa(s[k], y);
+        comp[k] = fs(fs(t, s[k]), y);
+        s[k] = t;
+      }
   }
 #pragma unroll
   for (int k = 0; k < NE; ++k)
     if (lane + 32 * k < M) wp[lane + 32 * k] = (double)s[k] - (double)comp[k];
   if (lane == 0) {
-    wp[kPStats + 0] = c_in;
-    wp[kPStats + 1] = c_out;
-    wp[kPStats + 2] = c_bad;
-    wp[kPStats + 3] = c_nrm;
-    wp[kPStats + 4] = c_fn;
-    wp[kPStats + 5] = chi2;
-    wp[kPStats + 6] = chi2k;
+    wp[STATS + 0] = c_in;
+    wp[STATS + 1] = c_out;
+    wp[STATS + 2] = c_bad;
+    wp[STATS + 3] = c_nrm;
+    wp[STATS + 4] = c_fn;
+    wp[STATS + 5] = chi2;
+    wp[STATS + 6] = chi2k;
   }
   __syncwarp();  // the warp's rows may be rewritten after this
 }
 
-template <int KIND>
+template <int KIND, int STRIDE = kPStride, int STATS = kPStats>
 __device__ __forceinline__ void tile_body(const JobIn& Jn, const LinDev& L, const CacheF& C, const TileDev& T,
                                           const DNode* staged, int nstaged,
-                                          double* wpart /* [kWarps][kPStride] */, float* fac /* [kWarps][32][kMaxFS] */,
+                                          double* wpart /* [kWarps][STRIDE] */, float* fac /* [kWarps][(D + 2) * kFacStride] */,
                                           int32_t* dbg_match, int32_t* dbg_status) {
   constexpr int D = KindDim<KIND>::D;
-  const int i = T.leaf_begin + threadIdx.x;
+  const int i = T.leaf_begin + (threadIdx.x & (kBlock - 1));
   int status = ST_NONE, match = -1;
   float e = 0.f, gamma = 0.f;
   float J[D];
@@ -402,7 +418,7 @@ __device__ __forceinline__ void tile_body(const JobIn& Jn, const LinDev& L, cons
                     match, e, gamma, J);
     if (dbg_match) { dbg_match[i] = match; dbg_status[i] = status; }
   }
-  tile_reduce<KIND>(status, e, gamma, J, wpart, fac);
+  tile_reduce<KIND, STRIDE, STATS>(status, e, gamma, J, wpart, fac);
 }
 
 // Two tiles of one (job, fixed entry) per block: thread t takes leaf t of both, runs the
@@ -670,49 +686,48 @@ static_assert(sizeof(JobIn) % 8 == 0 && sizeof(JobState) % 8 == 0, "staged as 8 
 static_assert(kTailDoubles <= kWarps * kPStride, "the step's scratch reuses the warps' partials");
 static_assert(sizeof(JobIn) / 8 + sizeof(JobState) / 8 + 18 <= kBlock, "one staged word per thread");
 
-// Sums entry by entry over the nt partials at `partials`, in tile order over four interleaved
-// accumulators; H and b go to scr, the dual blocks to O.  Threads 0..kBlock-1 (tid).
-template <int KIND, bool SMEM>
-__device__ __forceinline__ void tail_sums(const double* partials, int stride, int nt, double* scr, JobOut& O, int tid) {
+// Sum of v(t) over the nt tiles in tile order over four interleaved accumulators; sixteen
+// loads in flight.
+template <class Load>
+__device__ __forceinline__ double sum_tiles(int nt, Load v) {
+  double a4[4] = {0.0, 0.0, 0.0, 0.0};
+  int t = 0;
+  for (; t + 16 <= nt; t += 16) {
+    double x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = v(t + u);
+#pragma unroll
+    for (int u = 0; u < 16; ++u) a4[u & 3] += x[u];
+  }
+  for (; t + 4 <= nt; t += 4) {
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = v(t + u);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a4[u] += x[u];
+  }
+  for (; t < nt; ++t) a4[0] += v(t);
+  return (a4[0] + a4[1]) + (a4[2] + a4[3]);
+}
+// Entry e of the sums (e >= M: stats value e - M) to its place: H, b and stats in scr, the
+// dual blocks in O.  (r, c): entry_rc of e.
+template <int KIND>
+__device__ __forceinline__ void tail_place(int e, int r, int c, double v, double* scr, JobOut& O) {
   constexpr int DK = KindDim<KIND>::D;
   constexpr int M = DK * (DK + 1) / 2 + DK;
   constexpr int D = KIND == 0 ? 6 : 12;
-  auto load = [&](const double* p) { return SMEM ? *p : __ldcg(p); };
-  for (int e = tid; e < M + 7; e += kBlock) {
-    int r = 0, c = 0;
-    if (e < M) entry_rc(DK, e, r, c);
-    const double* src = partials + (SMEM || e < M ? e : kPStats + (e - M));
-    double a4[4] = {0.0, 0.0, 0.0, 0.0};
-    int t = 0;
-    for (; t + 16 <= nt; t += 16) {  // sixteen loads in flight
-      double v[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) v[u] = load(src + (size_t)(t + u) * stride);
-#pragma unroll
-      for (int u = 0; u < 16; ++u) a4[u & 3] += v[u];
-    }
-    for (; t + 4 <= nt; t += 4) {
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = load(src + (size_t)(t + u) * stride);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a4[u] += v[u];
-    }
-    for (; t < nt; ++t) a4[0] += load(src + (size_t)t * stride);
-    const double v = (a4[0] + a4[1]) + (a4[2] + a4[3]);
-    if (e >= M) {
-      scr[kTailStats + e - M] = v;
-    } else if (c == DK) {
-      if (r < D) scr[kTailB + r] = v;
-      else O.b_vel_B[r - 12] = v;
-    } else if (c < D) {
-      scr[kTailH + r * D + c] = v;
-      scr[kTailH + c * D + r] = v;
-    } else {  // dual blocks, c >= 12
-      if (r < 6) O.H_cross_pose_vel_B[r * 6 + (c - 12)] = v;
-      else if (r < 12) O.H_cross_vel_AB[(r - 6) * 6 + (c - 12)] = v;
-      else { O.H_vel_B[(r - 12) * 6 + (c - 12)] = v; O.H_vel_B[(c - 12) * 6 + (r - 12)] = v; }
-    }
+  if (e >= M) {
+    scr[kTailStats + e - M] = v;
+  } else if (c == DK) {
+    if (r < D) scr[kTailB + r] = v;
+    else O.b_vel_B[r - 12] = v;
+  } else if (c < D) {
+    scr[kTailH + r * D + c] = v;
+    scr[kTailH + c * D + r] = v;
+  } else {  // dual blocks, c >= 12
+    if (r < 6) O.H_cross_pose_vel_B[r * 6 + (c - 12)] = v;
+    else if (r < 12) O.H_cross_vel_AB[(r - 6) * 6 + (c - 12)] = v;
+    else { O.H_vel_B[(r - 12) * 6 + (c - 12)] = v; O.H_vel_B[(c - 12) * 6 + (r - 12)] = v; }
   }
 }
 
@@ -730,78 +745,70 @@ __device__ __forceinline__ kds_stats tail_stats(const double* scr) {
   return st;
 }
 
-// dx = -(H + damping)^-1 b by one warp: lane i holds row i of the lower triangle (Cholesky by
-// columns, right-looking), then L y = -b and L^T x = y by column sweeps.  0 where H + damping
-// is not positive definite.  The rows in registers make a pivot a chain of one shuffle,
-// square root and division (350 cycles; 1,000 with the matrix in shared memory).
+// dx = -(H + damping)^-1 b by one warp: Cholesky by columns (right-looking), lane i with row i
+// of the lower triangle and y_i of L y = -b, then L^T x = y by column sweeps.  0 where
+// H + damping is not positive definite.  One warp's instructions are what it costs, beside the
+// chain of a square root, a division and two shared-memory round trips per pivot: a new
+// column is read by broadcast (two shuffles per value otherwise), a row shifts down one
+// register per pivot so that the pivots are one short loop (unrolled, the code is fetched
+// anew every iteration, at twice the time), and entries above the diagonal are worked on
+// unmasked and never read.  5,300 cycles for D = 12, 2,500 for D = 6; with the matrix in
+// shared memory, element by element, 11,900 and 4,000.
 template <int D>
 __device__ __forceinline__ void tail_solve(double* scr, float damping, float velocity_damping, int lane) {
-  double a[D];
+  double a[D];  // columns k, k + 1, ... of row `lane` at pivot k
 #pragma unroll
   for (int j = 0; j < D; ++j) {
     a[j] = lane < D ? scr[kTailH + lane * D + j] : 0.0;
     if (lane == j) a[j] += j < 6 ? (double)damping : (double)velocity_damping;
   }
+  double y = lane < D ? -scr[kTailB + lane] : 0.0;
   double myinv = 0.0;  // 1 / L(lane, lane)
   bool ok = true;
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    const double d = __shfl_sync(0xffffffffu, a[k], k);
+  double* col = scr + kTailA;  // column k of L, below the diagonal
+#pragma unroll 1
+  for (int k = 0; k < D; ++k, col += D) {
+    const double d = __shfl_sync(0xffffffffu, a[0], k);
     ok = ok && (d > 0.0);
     const double lkk = sqrt(fmax(d, 1e-300));
     const double inv = 1.0 / lkk;
-    if (lane == k) {
-      a[k] = lkk;
-      myinv = inv;
-    } else if (lane > k) {
-      a[k] *= inv;
-    }
+    const double l = a[0] * inv;
+    if (lane < D) col[lane] = l;
+    const double yk = __shfl_sync(0xffffffffu, y * inv, k);
+    myinv = lane == k ? inv : myinv;
+    y = lane == k ? yk : (lane > k ? y - l * yk : y);
+    __syncwarp();
 #pragma unroll
-    for (int j = k + 1; j < D; ++j) {
-      const double ljk = __shfl_sync(0xffffffffu, a[k], j);
-      if (lane >= j) a[j] -= a[k] * ljk;
-    }
+    for (int j = 1; j < D; ++j) a[j - 1] = a[j] - l * col[k + j];
   }
-  if (lane < D) {
-#pragma unroll
-    for (int j = 0; j < D; ++j) scr[kTailA + lane * D + j] = a[j];
-  }
-  double y = lane < D ? -scr[kTailB + lane] : 0.0;
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    const double yk = __shfl_sync(0xffffffffu, y * myinv, k);
-    if (lane == k) y = yk;
-    if (lane > k) y -= a[k] * yk;
-  }
-  __syncwarp();
-  double lt[D];  // column `lane` of L
-#pragma unroll
-  for (int k = 0; k < D; ++k) lt[k] = lane < D && k > lane ? scr[kTailA + k * D + lane] : 0.0;
-#pragma unroll
+#pragma unroll 1
   for (int k = D - 1; k >= 0; --k) {
+    const double lt = lane < k ? scr[kTailA + lane * D + k] : 0.0;
     const double xk = __shfl_sync(0xffffffffu, y * myinv, k);
-    if (lane == k) y = xk;
-    if (lane < k) y -= lt[k] * xk;
+    y = lane == k ? xk : (lane < k ? y - lt * xk : y);
   }
   if (lane < D) scr[kTailX + lane] = ok ? y : 0.0;
   __syncwarp();
 }
+static_assert(kTailA + 11 * 12 + 22 < kTailDoubles, "a column is read past its end (values never used)");
 
-// The float caches of one (job, fixed entry) pair at pose X and velocities v (shared memory)
-// by one warp: element e of the caches through put(e, value).  Xf, fv: the entry's (shared);
-// tmp: 12 doubles.
-template <class Put>
-__device__ __forceinline__ void tail_caches(const double* X, const double* v, const double* Xf, const double* fv,
-                                            double* tmp, int lane, Put put) {
-  if (lane < 12) {  // inverse of Xf
-    const int i = lane >> 2, j = lane & 3;
-    tmp[lane] = j < 3 ? Xf[j * 4 + i] : -ddot3(Xf[i], Xf[4 + i], Xf[8 + i], Xf[3], Xf[7], Xf[11]);
-  }
-  __syncwarp();
+// Inverse of the pose Xf (shared memory), an element per lane, into iXf.
+__device__ __forceinline__ void tail_inverse(const double* Xf, double* iXf, int lane) {
   if (lane < 12) {
     const int i = lane >> 2, j = lane & 3;
-    double m = ddot3(tmp[i * 4], tmp[i * 4 + 1], tmp[i * 4 + 2], X[j], X[4 + j], X[8 + j]);
-    if (j == 3) m = da(m, tmp[i * 4 + 3]);
+    iXf[lane] = j < 3 ? Xf[j * 4 + i] : -ddot3(Xf[i], Xf[4 + i], Xf[8 + i], Xf[3], Xf[7], Xf[11]);
+  }
+  __syncwarp();
+}
+// The float caches of one (job, fixed entry) pair at pose X and velocities v (shared memory)
+// by one warp: element e of the caches through put(e, value).  Xf, fv, iXf: the entry's.
+template <class Put>
+__device__ __forceinline__ void tail_caches(const double* X, const double* v, const double* Xf, const double* fv,
+                                            const double* iXf, int lane, Put put) {
+  if (lane < 12) {
+    const int i = lane >> 2, j = lane & 3;
+    double m = ddot3(iXf[i * 4], iXf[i * 4 + 1], iXf[i * 4 + 2], X[j], X[4 + j], X[8 + j]);
+    if (j == 3) m = da(m, iXf[i * 4 + 3]);
     put(lane, (float)X[lane]);
     put(12 + lane, (float)Xf[lane]);
     put(24 + lane, (float)m);
@@ -813,10 +820,11 @@ __device__ __forceinline__ void tail_caches(const double* X, const double* v, co
 }
 
 // A COMPUTE job's step by one warp, from H, b and the stats in scr: solve, update, test, then
-// caches() (unless the job is done), then the outputs.  Jn and S are in shared memory.
-template <int KIND, class Caches>
+// caches() (unless the job is done) and publish() (the state is final), then the outputs.  Jn
+// and S are in shared memory.
+template <int KIND, class Caches, class Publish>
 __device__ __forceinline__ void tail_step(const JobIn& Jn, JobState& S, JobOut& O, kds_stats* log, double* scr,
-                                          int lane, Caches caches) {
+                                          int lane, Caches caches, Publish publish) {
   constexpr int D = KIND == 0 ? 6 : 12;
   kds_stats st = tail_stats(scr);
   const int it = S.iter;
@@ -832,6 +840,7 @@ __device__ __forceinline__ void tail_step(const JobIn& Jn, JobState& S, JobOut& 
       S.arrive = 0u;
     }
     __syncwarp();
+    publish();
     return;
   }
   if (g_phase_on && lane == 0) g_phase[11] = clock64();
@@ -856,17 +865,20 @@ __device__ __forceinline__ void tail_step(const JobIn& Jn, JobState& S, JobOut& 
     }
   }
   bool stop = false;
-  double pp = 0.0, pv = 0.0;
+  auto norms = [&]() {
+    double pp = 0.0, pv = 0.0;
 #pragma unroll
-  for (int i = 0; i < 6; ++i) pp += dx[i] * dx[i];
-  st.pert_pose_norm = (float)sqrt(pp);
-  if (D == 12) {
+    for (int i = 0; i < 6; ++i) pp += dx[i] * dx[i];
+    st.pert_pose_norm = (float)sqrt(pp);
+    if (D == 12) {
 #pragma unroll
-    for (int i = 6; i < D; ++i) pv += dx[i] * dx[i];
-    st.pert_vel_norm = (float)sqrt(pv);
-  }
+      for (int i = 6; i < D; ++i) pv += dx[i] * dx[i];
+      st.pert_vel_norm = (float)sqrt(pv);
+    }
+  };
   float score = 0.f;
   if (Jn.P.term_crit) {
+    norms();
     // ICPTerminationCriteriaScore_::hasToStop (kd/icp/icp_stats_.h:91-101)
     int nl = st.num_inliers + st.num_outliers + st.num_bad + st.num_err_normal + st.num_err_fn;
     float ratio = nl ? (float)st.num_inliers / (float)nl : 0.f;
@@ -892,6 +904,8 @@ __device__ __forceinline__ void tail_step(const JobIn& Jn, JobState& S, JobOut& 
   }
   __syncwarp();
   if (!stop && !last) caches();
+  publish();
+  if (!Jn.P.term_crit) norms();
   if (lane < D) O.dx[lane] = dx[lane];
   if (lane < 12) O.X[lane] = S.X[lane];
   else if (lane < 18) O.v[lane - 12] = S.v[lane - 12];
@@ -921,7 +935,18 @@ __device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O,
   else if (tid < NJ + NS) word = reinterpret_cast<const u64*>(&SG)[tid - NJ];
   else if (tid < NJ + NS + 12) word = __double_as_longlong(lins[JnG.lin_begin].Xf[tid - NJ - NS]);
   else if (tid < NJ + NS + 18) word = __double_as_longlong(lins[JnG.lin_begin].fv[tid - NJ - NS - 12]);
-  tail_sums<KIND, false>(partials + (size_t)JnG.tile_begin * kPStride, kPStride, JnG.tile_count, scr, O, tid);
+  {
+    constexpr int DK = KindDim<KIND>::D;
+    constexpr int M = DK * (DK + 1) / 2 + DK;
+    const double* base = partials + (size_t)JnG.tile_begin * kPStride;
+    const int nt = JnG.tile_count;
+    for (int e = tid; e < M + 7; e += kBlock) {
+      int r = 0, c = 0;
+      if (e < M) entry_rc(DK, e, r, c);
+      const double* src = base + (e < M ? e : kPStats + (e - M));
+      tail_place<KIND>(e, r, c, sum_tiles(nt, [&](int t) { return __ldcg(src + (size_t)t * kPStride); }), scr, O);
+    }
+  }
   u64* dst = reinterpret_cast<u64*>(scr);
   if (tid < NJ + NS) dst[kTailJob + tid] = word;
   else if (tid < NJ + NS + 18) dst[kTailLin + tid - NJ - NS] = word;
@@ -959,10 +984,11 @@ __device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O,
         __syncwarp();
       }
       float* c = reinterpret_cast<float*>(&L.cache);
+      tail_inverse(scr + kTailLin, scr + kTailP, lane);
       tail_caches(S.X, S.v, scr + kTailLin, scr + kTailLin + 12, scr + kTailP, lane,
                   [&](int e, float x) { c[e] = x; });
     }
-  });
+  }, []() {});
   __syncwarp();
   if (lane < NS) reinterpret_cast<u64*>(&SG)[lane] = reinterpret_cast<const u64*>(&S)[lane];
   if (stamp) g_phase[15] = clock64();
@@ -979,7 +1005,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize(const JobIn* __restrict
   constexpr int D = KindDim<KIND>::D;
   constexpr int M = D * (D + 1) / 2 + D;
   __shared__ CacheF sC;
-  __shared__ float sfac[kWarps * 32 * kMaxFS];
+  __shared__ __align__(16) float sfac[kWarps * kMaxFac];
   __shared__ double swp[kWarps * kPStride];
   __shared__ int s_last;
   __shared__ __align__(8) unsigned long long s_mbar;
@@ -1064,7 +1090,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_pair(const JobIn* __res
   constexpr int D = KindDim<KIND>::D;
   constexpr int M = D * (D + 1) / 2 + D;
   __shared__ CacheF sC;
-  __shared__ float sfac[kWarps * 32 * kMaxFS];
+  __shared__ __align__(16) float sfac[kWarps * kMaxFac];
   __shared__ double swp[2][kWarps * kPStride];
   __shared__ int s_last;
   __shared__ __align__(8) unsigned long long s_mbar;
@@ -1165,7 +1191,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_persistent(const JobIn*
                                                                  int max_iter, int stage, double* partials,
                                                                  int32_t* ready, unsigned int* queue, int32_t* err) {
   __shared__ CacheF sC;
-  __shared__ float sfac[kWarps * 32 * kMaxFS];
+  __shared__ __align__(16) float sfac[kWarps * kMaxFac];
   __shared__ double swp[kWarps * kPStride];
   __shared__ int s_item, s_skip, s_last, s_fail;
   __shared__ __align__(8) unsigned long long s_mbar;
@@ -1280,6 +1306,188 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_persistent(const JobIn*
   }
 }
 
+// ---------------------------------------------------------------------------
+// One alignment in one launch: a thread-block cluster runs every iteration of a single
+// COMPUTE job.  A launch per iteration spends as long around the work as on it: the grid's
+// start and end, the tree top staged anew, the partials through global memory with a fence
+// and a counter (rigid 16 x 1024 scan, 5 tiles: 11.7 us an iteration, of which the tile takes
+// 2.3 and the step 2.8).  Here the tree top is staged once per block, a tile's partial goes
+// straight into the first block's shared memory, that block's first warp runs the step, and
+// the new caches go back into every block's shared memory; two cluster barriers per
+// iteration.  Tiles, partials and the step are those of k_linearize, in the same order, so the
+// results are bit-identical.  The inputs are the kernel's parameters and the results go to
+// page-locked host memory: no copies around the launch.
+// Bound by the chain of one iteration (64 x 1024 CT scan on a 1.45M-node map, 23 tiles in 16
+// blocks: 29,000 cycles, of which the tile 12,300 and the step's FP64 chain 13,000).
+constexpr int kClusterThreads = 512;
+constexpr int kClusterGroups = kClusterThreads / kBlock;  // tiles at a time per block, at most
+constexpr int kClusterMax = 16;                           // blocks per cluster (8 is the portable size)
+constexpr int kClusterTiles = 64;
+
+// Shared memory of a block: this, then the warps' partials, the tiles' partials (used in the
+// first block) and the factor rows.
+struct __align__(16) ClusterSmem {
+  double scr[kTailDoubles];  // the first block's
+  JobOut out;
+  alignas(16) float cache[56];  // a CacheF, in whole 16 B words
+  kds_stats log[kMaxLog];
+  int32_t done, err;
+  unsigned long long mbar;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_align_cluster(const __grid_constant__ JobIn job, const __grid_constant__ LinDev lin, int stage, ClusterOut* res) {
+  constexpr int DK = KindDim<KIND>::D;
+  constexpr int D = DK;
+  constexpr int M = D * (D + 1) / 2 + D;
+  constexpr int kStride = M + 7;
+  extern __shared__ float4 sDyn[];
+  const DNode* sN = reinterpret_cast<const DNode*>(sDyn);
+  ClusterSmem& sm = *reinterpret_cast<ClusterSmem*>(reinterpret_cast<char*>(sDyn) + (size_t)stage * sizeof(DNode));
+  double* wpart = reinterpret_cast<double*>(&sm + 1);
+  double* part = wpart + (size_t)(blockDim.x / 32) * kStride;  // the first block's: the tiles' partials
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int rank = (int)cluster.block_rank(), nblk = (int)cluster.num_blocks();
+  const int tid = threadIdx.x, lane = tid & 31, group = tid / kBlock, groups = blockDim.x / kBlock;
+  const int nt = job.tile_count;
+  float* fac = reinterpret_cast<float*>(part + (size_t)((nt + 1) & ~1) * kStride);
+  double* lead_part = cluster.map_shared_rank(part, 0);
+  ClusterSmem* lead = cluster.map_shared_rank(&sm, 0);
+  // the tree top: one bulk copy per block (this GPU's memory, no multicast)
+  int nst = min(stage, lin.f_num_nodes);
+  const uint32_t bytes = (uint32_t)nst * (uint32_t)sizeof(DNode);
+  const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(&sm.mbar);
+  if (tid == 0) {
+    sm.done = 0;
+    sm.err = 0;
+    if (bytes > 0) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(sDyn)),
+                   "l"(lin.fnodes), "r"(bytes), "r"(mbar)
+                   : "memory");
+    }
+  }
+  // The first block keeps the job's inputs, state, outputs and log in shared memory.  Every
+  // block must have started before another writes its shared memory.
+  JobIn& Jn = *reinterpret_cast<JobIn*>(sm.scr + kTailJob);
+  JobState& S = *reinterpret_cast<JobState*>(sm.scr + kTailState);
+  if (rank == 0) {
+    typedef unsigned long long u64;
+    for (int k = tid; k < (int)(sizeof(JobIn) / 8); k += blockDim.x)
+      reinterpret_cast<u64*>(&Jn)[k] = reinterpret_cast<const u64*>(&job)[k];
+    for (int k = tid; k < (int)(sizeof(JobOut) / 8); k += blockDim.x) reinterpret_cast<u64*>(&sm.out)[k] = 0ull;
+    __syncthreads();
+    if (tid < 12) {
+      S.X[tid] = sm.out.X[tid] = job.X0[tid];
+      sm.scr[kTailLin + tid] = lin.Xf[tid];
+    } else if (tid < 18) {
+      S.v[tid - 12] = sm.out.v[tid - 12] = job.v0[tid - 12];
+      sm.scr[kTailLin + tid] = lin.fv[tid - 12];
+    } else if (tid == 18) {
+      S.iter = S.done = S.result = 0;
+      S.arrive = 0u;
+      S.prev_score = 0.f;
+      S.max_iter = job.stats_mode ? 1 : job.P.max_iterations;
+      sm.out.result = job.P.max_iterations;
+    }
+  }
+  cluster.sync();
+  constexpr int kCacheQuads = (int)(sizeof(ClusterSmem::cache) / 16);
+  auto caches = [&]() {  // the first block's first warp: the caches into every block
+    float* c = sm.cache;
+    tail_caches(S.X, S.v, sm.scr + kTailLin, sm.scr + kTailLin + 12, sm.scr + kTailP, lane,
+                [&](int e, float x) { c[e] = x; });
+    // two blocks at a time, 16 B a lane
+    if (lane < 2 * kCacheQuads) {
+      float4* q = reinterpret_cast<float4*>(c) + (lane < kCacheQuads ? lane : lane - kCacheQuads);
+      const float4 x = *q;
+      for (int b = 1 + (lane >= kCacheQuads ? 1 : 0); b < nblk; b += 2) *cluster.map_shared_rank(q, b) = x;
+    }
+  };
+  const CacheF& C = *reinterpret_cast<const CacheF*>(sm.cache);
+  static_assert(sizeof(CacheF) <= sizeof(sm.cache), "cache words");
+  // the entry of the sums that this thread of the first block adds up
+  int er = 0, ec = 0;
+  if (tid < M) entry_rc(DK, tid, er, ec);
+  if (rank == 0 && tid < 32) {
+    tail_inverse(sm.scr + kTailLin, sm.scr + kTailP, lane);
+    caches();
+  }
+  if (bytes > 0 && !mbar_wait(mbar, 0u, g_wait_spins)) {
+    // copy not observed complete: record it and read the whole tree from global memory
+    atomicOr(&sm.err, 1);
+    nst = 0;
+  }
+  cluster.sync();
+  for (;;) {
+    for (int t0 = 0; t0 < nt; t0 += nblk * groups) {
+      const int t = t0 + group * nblk + rank;
+      if (t < nt) {  // uniform per group
+        TileDev T;
+        T.job = 0;
+        T.lin = 0;
+        T.leaf_begin = t * kBlock;
+        T.leaf_end = min(T.leaf_begin + kBlock, job.m_num_leaves);
+        tile_body<KIND, kStride, M>(job, lin, C, T, sN, nst, wpart, fac, nullptr, nullptr);
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(kBlock) : "memory");
+        const int e = tid & (kBlock - 1);
+        if (e < kStride) {
+          double acc = 0.0;
+#pragma unroll
+          for (int w = 0; w < kWarps; ++w) acc += wpart[(group * kWarps + w) * kStride + e];
+          lead_part[t * kStride + e] = acc;
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(kBlock) : "memory");
+      }
+    }
+    cluster.sync();
+    if (rank == 0 && tid < kBlock) {
+      if (tid < kStride) {
+        const double* src = part + tid;
+        const double v = sum_tiles(nt, [&](int t) { return src[t * kStride]; });
+        tail_place<KIND>(tid, er, ec, v, sm.scr, sm.out);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1), "r"(kBlock) : "memory");
+      if (tid < 32) {
+        if (job.prior_enabled) {
+          if (tid == 0) add_pose_prior(Jn, S.X, sm.scr + kTailH, sm.scr + kTailB, D);
+          __syncwarp();
+        }
+        tail_step<KIND>(Jn, S, sm.out, sm.log, sm.scr, lane, caches, [&]() {
+          if (S.done && lane < nblk) *cluster.map_shared_rank(&sm.done, lane) = 1;
+          __syncwarp();
+          cluster.barrier_arrive();  // the others go on while this warp writes the outputs
+        });
+      }
+    }
+    if (rank != 0 || tid >= 32) cluster.barrier_arrive();
+    cluster.barrier_wait();
+    if (sm.done) break;
+  }
+  // before the blocks exit: the copy has landed, the errors are collected
+  if (tid == 0) {
+    if (bytes > 0 && !mbar_wait(mbar, 0u)) atomicOr(&sm.err, 2);
+    if (rank > 0 && sm.err) atomicOr(&lead->err, sm.err);
+  }
+  cluster.sync();
+  if (rank != 0) return;
+  for (int i = tid; i < D * D; i += blockDim.x) sm.out.H[i] = sm.scr[kTailH + i];
+  if (tid < D) sm.out.b[tid] = sm.scr[kTailB + tid];
+  __syncthreads();
+  typedef unsigned long long u64;
+  static_assert(sizeof(JobOut) % 8 == 0 && sizeof(kds_stats) % 4 == 0, "copied as words");
+  for (int k = tid; k < (int)(sizeof(JobOut) / 8); k += blockDim.x)
+    reinterpret_cast<u64*>(&res->out)[k] = reinterpret_cast<const u64*>(&sm.out)[k];
+  const int nlog = min(sm.out.iterations, kMaxLog) * (int)(sizeof(kds_stats) / 4);
+  for (int k = tid; k < nlog; k += blockDim.x)
+    reinterpret_cast<int32_t*>(res->log)[k] = reinterpret_cast<const int32_t*>(sm.log)[k];
+  if (tid == 0) res->err = sm.err;
+}
+
 // Resets control state, seeds state from the job inputs and writes the first caches: a warp
 // per job (a thread per job took 7 us for one job, 20 us for 250: every store a sector of its
 // own, the pose algebra one element after the other).
@@ -1330,6 +1538,7 @@ __device__ __forceinline__ void init_job(int j, const JobIn* jobs, JobState* sta
     else if (lane < 18) C.fv[lane - 12] = L.fv[lane - 12];
     __syncwarp();
     float* c = reinterpret_cast<float*>(&L.cache);
+    tail_inverse(C.Xf, C.tmp, lane);
     tail_caches(C.X, C.v, C.Xf, C.fv, C.tmp, lane, [&](int e, float x) { c[e] = x; });
   }
 }
@@ -1458,6 +1667,11 @@ void Runner::release() {
   if (block) cudaFree(block);
   block = nullptr;
   cap_jobs = cap_lins = cap_tiles = 0;
+}
+
+Runner::~Runner() {
+  release();
+  if (h_cluster) cudaFreeHost(h_cluster);
 }
 
 void Runner::drop_graph() {
@@ -1681,6 +1895,94 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   }
   KDS_CK(cudaGetLastError());
   return KDS_OK;
+}
+
+// Whether a job runs as one cluster launch: a COMPUTE job of one fixed entry whose tiles fit
+// the first block's partials, and no per-launch events asked for.  Against a 1.45M-node map,
+// rigid / CT: 154 / 246 us at 1,024 surfels (a launch per iteration: 179 / 295), 167 / 297 at
+// 8,192 (195 / 319).  There the partials end and the blocks begin a second round of tiles,
+// while a launch per iteration still has SMs to spare.
+bool cluster_fits(const JobIn& J, bool profiling) {
+  return !profiling && J.mode == KDS_JOB_COMPUTE && (J.kind == 0 || J.kind == 1) && J.lin_count == 1 &&
+         !J.keep_cache && J.m_num_leaves > 0 && J.m_num_leaves <= kClusterTiles * kBlock &&
+         (J.stats_mode || J.P.max_iterations > 0);
+}
+
+template <int KIND>
+static int launch_cluster(const JobIn& J, const LinDev& L, int stage, int max_blocks, ClusterOut* res,
+                          cudaStream_t s) {
+  // as many blocks as tiles, up to the largest cluster that the device schedules: fewer warps
+  // per SM to share its issue slots, and more of its L1 per tile for the lower tree levels
+  int nblk = 1;
+  while (nblk < max_blocks && nblk < J.tile_count) nblk *= 2;
+  const int groups = std::min(kClusterGroups, (J.tile_count + nblk - 1) / nblk);
+  const int kStride = KIND == 0 ? 34 : 97;
+  const size_t smem = (size_t)stage * sizeof(DNode) + sizeof(ClusterSmem) +
+                      sizeof(double) * kStride * ((size_t)groups * kWarps + ((J.tile_count + 1) & ~1)) +
+                      sizeof(float) * ((KIND == 0 ? 6 : 12) + 2) * kFacStride * groups * kWarps;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nblk);
+  cfg.blockDim = dim3((unsigned)(groups * kBlock));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)nblk;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  KDS_CK(cudaLaunchKernelEx(&cfg, k_align_cluster<KIND>, J, L, stage, res));
+  count_launch();
+  return KDS_OK;
+}
+
+// Sets the cluster kernels' limits (always to the same values: they belong to the process) and
+// asks for the largest cluster that this device schedules: 16 need its leave, 8 always fit.
+constexpr int kClusterSmemMax = 200 * 1024;  // 172 KB at 64 CT tiles and 2,047 staged nodes
+static int cluster_setup(int* max_blocks) {
+  const void* fs[2] = {(const void*)k_align_cluster<0>, (const void*)k_align_cluster<1>};
+  for (const void* f : fs) {
+    KDS_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax));
+    KDS_CK(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterMax);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = kClusterSmemMax;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterMax;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  *max_blocks = 8;
+  if (cudaOccupancyMaxActiveClusters(&n, k_align_cluster<1>, &cfg) == cudaSuccess && n > 0) *max_blocks = kClusterMax;
+  else cudaGetLastError();
+  return KDS_OK;
+}
+
+int Runner::run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log) {
+  if (!h_cluster) {
+    KDS_CK(cudaHostAlloc((void**)&h_cluster, sizeof(ClusterOut), cudaHostAllocMapped));
+    memset(h_cluster, 0, sizeof(ClusterOut));
+  }
+  ClusterOut* d = nullptr;
+  KDS_CK(cudaHostGetDevicePointer((void**)&d, h_cluster, 0));
+  J.tile_begin = 0;
+  J.tile_count = (J.m_num_leaves + kBlock - 1) / kBlock;
+  J.lin_begin = 0;
+  if (!cluster_blocks) {
+    const int rc = cluster_setup(&cluster_blocks);
+    if (rc) { cluster_blocks = 0; return rc; }
+  }
+  int rc = J.kind == 0 ? launch_cluster<0>(J, L, stage_nodes, cluster_blocks, d, s)
+                       : launch_cluster<1>(J, L, stage_nodes, cluster_blocks, d, s);
+  if (rc) return rc;
+  KDS_CK(cudaStreamSynchronize(s));
+  *out = h_cluster->out;
+  if (log) log->assign(h_cluster->log, h_cluster->log + kMaxLog);
+  return timeout_status(h_cluster->err);
 }
 
 int Runner::run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg_status) {

@@ -92,6 +92,15 @@ struct TileDev {
   int32_t leaf_end;
 };
 
+// What a cluster launch writes back (page-locked host memory).
+struct ClusterOut {
+  JobOut out;
+  kds_stats log[kMaxLog];
+  int32_t err;
+  int32_t pad_;
+};
+bool cluster_fits(const JobIn& J, bool profiling);
+
 // Owns the device buffers of a batch of jobs and (optionally) a CUDA graph of its
 // launches: k_init_jobs followed by one k_linearize per Gauss-Newton iteration.
 struct Runner {
@@ -129,6 +138,8 @@ struct Runner {
   // 1: two tiles of one (job, fixed entry) per block, two descents in flight per thread
   // (k_linearize_pair); ignored by the persistent form
   int pair_tiles = 0;
+  ClusterOut* h_cluster = nullptr;  // results of run_cluster
+  int cluster_blocks = 0;           // largest cluster (0: not asked yet)
   bool smem_attr_set = false;
   bool persistent_attr_set = false;
   // optional event pair per linearization launch (measurement only)
@@ -146,7 +157,9 @@ struct Runner {
   int enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status);
   int run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg_status);
   int fetch(cudaStream_t s, std::vector<JobOut>& outs, std::vector<kds_stats>* logs);
-  ~Runner() { release(); }
+  // one job in one cluster launch (cluster_fits); waits for it
+  int run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log);
+  ~Runner();
 };
 
 int count_touched(Runner& R, int kind, int64_t fixed_nodes, int64_t* out, cudaStream_t s);

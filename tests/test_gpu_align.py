@@ -280,3 +280,76 @@ def test_tree_top_wait_fallback(trees):
     b = run()
     b.compute()
     assert np.array_equal(b.get_x(), ref.get_x())
+
+
+@pytest.mark.parametrize("leaves", [1, 127, 128, 129, 2048, 2049, 4097, 8192, 8193])
+@pytest.mark.parametrize("kind", ["icp", "ct"])
+def test_single_alignment_forms_agree(scene, leaves, kind):
+    """One alignment in one launch (up to 64 tiles of 128 surfels) against the launch per
+    iteration of the same job in a batch, at the edges of tiles, of blocks per cluster, of tiles
+    per block and of the rule itself: pose, velocities, H, b, statistics and result equal bit
+    for bit."""
+    import kd_slam2_b200 as kds
+    from kd_slam2_b200 import synth
+    rng = np.random.default_rng(leaves)
+    fx, fs = make_scan(scene, 2500, beams=64, elev=(-22.5, 22.5))
+    fixed = kds.TreeGeneratorB2003D(leaf_max_points=16).make_tree(fx, fs)
+    e = fixed.export()
+    k = rng.integers(0, len(e["leaves"]), leaves)
+    mean, nrm = e["mean"][e["leaves"]][k], e["dir"][e["leaves"]][k]
+    mean = (mean + rng.normal(scale=0.02, size=mean.shape)).astype(np.float32)
+    n = 2 * leaves - 1  # a left-deep chain: inner node i has leaf 2i + 1 and the next inner node 2i + 2
+    left, right = np.full(n, -1, np.int32), np.full(n, -1, np.int32)
+    inner = np.arange(0, n - 1, 2)
+    left[inner], right[inner] = inner + 1, inner + 2
+    isleaf = left < 0
+    m, d = np.zeros((n, 3), np.float32), np.tile(np.float32([0, 0, 1]), (n, 1))
+    m[isleaf], d[isleaf] = mean, nrm
+    moving = kds.Tree.import_nodes(m, d, left, right, dts_mean=np.where(isleaf, rng.uniform(0, 0.1, n), 0.0))
+    X0 = synth.pose((0.05, -0.04, 0.02), (0.003, -0.004, 0.01))
+    prm = dict(max_error=0.5, max_iterations=4, min_good_measurements=1)
+    if kind == "ct":
+        prm["velocity_damping"] = 10.0
+    a = (kds.ICPB2003D if kind == "icp" else kds.CTICPB2003D)(**prm)
+    a.set_fixed(fixed)
+    a.set_moving(moving)
+    a.set_x(X0)
+    ret = a.compute()
+    job = kds.make_job(kds.abi.KDS_ICP if kind == "icp" else kds.abi.KDS_CTICP, fixed, moving, a.params, X=X0)
+    r = kds.Batch().run([job], use_graph=False)[0]
+    D = 6 if kind == "icp" else 12
+    assert ret == r.result and len(a.stats_log) == r.iterations
+    assert np.array_equal(a.get_x().reshape(12), np.array(r.X[:]))
+    assert np.array_equal(a.velocities(), np.array(r.v[:]))
+    assert np.array_equal(a.H.reshape(-1), np.array(r.H[:D * D])) and np.array_equal(a.b, np.array(r.b[:D]))
+    assert a.stats == r.stats.as_dict()
+
+
+def test_single_alignment_options(scene):
+    """Statistics only, the termination criterion, a pose prior, too few measurements and one
+    round: the one-launch form against the oracle."""
+    import kd_slam2_b200 as kds
+    from kd_slam2_b200 import synth
+    fx, fs = make_scan(scene, 2510)
+    mx, ms = make_scan(scene, 2511, vel=[6.0, 0, 0, 0, 0, 0.2])
+    G = kds.TreeGeneratorB2003D(leaf_max_points=16)
+    F, M = G.make_tree(fx, fs), G.make_tree(mx, ms)
+    OF, OM = (orc.OTree.build(x, s, orc.tree_params(leaf_max_points=16)) for x, s in ((fx, fs), (mx, ms)))
+    X0 = synth.pose((0.1, -0.05, 0.0), (0.0, 0.0, 0.02))
+    base = dict(max_error=0.5, max_iterations=8)
+    for kw in (dict(term_crit=1, d_pert=1e-3, d_score=1e-2), dict(min_good_measurements=10**6), dict(max_iterations=1)):
+        for cls, kind in ((kds.ICPB2003D, orc.KIND_ICP), (kds.CTICPB2003D, orc.KIND_CT)):
+            prm = dict(base, **kw)
+            if kind == orc.KIND_CT:
+                prm["velocity_damping"] = 10.0
+            a = cls(**prm)
+            a.set_fixed(F)
+            a.set_moving(M)
+            a.set_x(X0)
+            ret = a.compute()
+            r = orc.align(kind, orc.MODE_MIXED, OF, OM, orc.align_params(**prm), X0,
+                          v0=np.zeros(6) if kind == orc.KIND_CT else None)
+            assert ret == r["ret"] and np.array_equal(a.get_x(), np.asarray(r["X"]).reshape(3, 4))
+            X = a.get_x()
+            a.compute(stats_mode=True)  # leaves the pose alone
+            assert np.array_equal(a.get_x(), X)
