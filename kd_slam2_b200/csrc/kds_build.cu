@@ -395,9 +395,12 @@ struct BNode {
   int32_t has_prop;   // propagated normal handed to the children
   int32_t parent;     // parent node, -1 for a root
   float mean[3], dir[3];
+  int32_t big;        // large nodes: ordinal among the level's
+  int32_t pad_;
   double prop[3];
   double par_prop[3];
 };
+static_assert(sizeof(BNode) == 128, "one L1 line");
 
 struct BuildParams {
   int32_t propagate_normal;
@@ -638,12 +641,13 @@ __device__ __forceinline__ int block_scan(int v, int* sm, int* total) {
   return wprefix + x - v;
 }
 
-// The node range [b, e) of this block when gridDim.x blocks split the current level.
-__device__ __forceinline__ void level_range(const LevelState* ls, int& b, int& e) {
+// The node range [b, e) of this block when gridDim.x / parts ranges split the current level.
+__device__ __forceinline__ void level_range(const LevelState* ls, int& b, int& e, int parts = 1) {
   const int lb = ls->lb, le = ls->le;
   const int nl = le - lb;
-  const int per = (nl + gridDim.x - 1) / gridDim.x;
-  b = lb + blockIdx.x * per;
+  const int ranges = gridDim.x / parts;
+  const int per = (nl + ranges - 1) / ranges;
+  b = lb + (blockIdx.x / parts) * per;
   e = min(b + per, le);
 }
 
@@ -757,20 +761,62 @@ __global__ void __launch_bounds__(kThreads) k_root_moments(const BNode* nodes, i
   }
 }
 
+// Accumulators of the large nodes' smaller children: two sets by level parity, so that a
+// level's may be read while the next one's are cleared.
+struct ChildSums {
+  U128* acc[2];
+};
+// A node whose parent is large has no sums yet: the parent's scatter left the smaller child's
+// in the accumulators of its level, the other child's are the parent's minus them.
+struct PendingSums {
+  const U128* q;    // nullptr: the sums are in mom[i]
+  const U128* par;
+  bool small;
+};
+__device__ __forceinline__ PendingSums pending_sums(const BNode* nodes, const U128* mom, const ChildSums& C, int depth,
+                                                    int i, int parent) {
+  PendingSums r;
+  r.q = nullptr;
+  r.par = nullptr;
+  r.small = false;
+  if (parent < 0) return r;
+  const BNode& p = nodes[parent];
+  const int s = p.start, e = p.end;
+  if (e - s <= kBig) return r;
+  r.q = C.acc[(depth & 1) ^ 1] + (size_t)p.big * kSums;
+  r.par = mom + (size_t)parent * kSums;
+  r.small = (p.left == i) == (p.mid - s <= e - p.mid);
+  return r;
+}
+__device__ __forceinline__ U128 pending_value(const PendingSums& r, int k) {
+  const U128 q = r.q[k];
+  return r.small ? q : u128_sub(r.par[k], q);
+}
+
 // Thread per node of the level: the leaf/split decision from its sums.  Block b takes
 // the b-th contiguous range of the level's nodes and writes its count of split nodes
 // (the children's numbering scans these counts).
-__global__ void k_decide(BNode* nodes, const LevelState* ls, const U128* mom, BuildParams P, int32_t* bsum,
-                         int32_t* bbig, double* root_frame) {
-  __shared__ int sm[32];
+__device__ __forceinline__ void level_decide(BNode* nodes, const LevelState* ls, U128* mom, const ChildSums& C,
+                                             const BuildParams& P, int32_t* bsum, int32_t* bbig, double* root_frame,
+                                             int* sm) {
   int b, e;
   level_range(ls, b, e);
+  const int depth = ls->depth;
   int v = 0, nc = 0, nb = 0;
   for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
     BNode nd = nodes[i];
     const int n = nd.end - nd.start;
     double Sd[kSums];
-    for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(mom[(size_t)i * kSums + k]);
+    const PendingSums r = pending_sums(nodes, mom, C, depth, i, nd.parent);
+    if (r.q) {
+      for (int k = 0; k < kSums; ++k) {
+        const U128 q = pending_value(r, k);
+        mom[(size_t)i * kSums + k] = q;
+        Sd[k] = fx_to_d(q);
+      }
+    } else {
+      for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(mom[(size_t)i * kSums + k]);
+    }
     decide(Sd, n, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
     nodes[i] = nd;
     v += nd.split ? 1 : 0;
@@ -788,6 +834,11 @@ __global__ void k_decide(BNode* nodes, const LevelState* ls, const U128* mom, Bu
     bbig[2 * blockIdx.x] = tc;  // as k_big_sums
     bbig[2 * blockIdx.x + 1] = tb;
   }
+}
+__global__ void k_decide(BNode* nodes, const LevelState* ls, U128* mom, ChildSums C, BuildParams P, int32_t* bsum,
+                         int32_t* bbig, double* root_frame) {
+  __shared__ int sm[32];
+  level_decide(nodes, ls, mom, C, P, bsum, bbig, root_frame, sm);
 }
 
 // The level's split count from k_decide's per-block counts, then the next level (one
@@ -990,9 +1041,11 @@ __global__ void k_big_sums(const BNode* nodes, const LevelState* ls, int32_t* bb
   }
 }
 
-__global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bbig, Chunk* chunks, int32_t chunk_cap,
-                           int32_t* big_list, int32_t* node_chunk0, U128* acc, U128* accl) {
-  __shared__ int sm[32];
+// acc: the sums to clear for the large nodes listed.  parts: blocks that share one node range
+// and write its chunks in turn.
+__device__ __forceinline__ void level_plan(BNode* nodes, LevelState* ls, const int32_t* bbig, Chunk* chunks,
+                                           int32_t chunk_cap, int32_t* big_list, int32_t* node_chunk0, U128* acc,
+                                           int* sm, int part, int parts) {
   if (ls->max_size <= kBig) {  // no large node on this level
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       ls->num_chunks = 0;
@@ -1001,12 +1054,12 @@ __global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bb
     return;
   }
   int b, e;
-  level_range(ls, b, e);
+  level_range(ls, b, e, parts);
   int carry_c, carry_b, all_c, all_b;  // chunks / large nodes of the blocks before this one, of all
   {
     int vc = 0, vb = 0, ac = 0, ab = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-      if (k < (int)blockIdx.x) {
+    for (int k = threadIdx.x; k < (int)(gridDim.x / parts); k += blockDim.x) {
+      if (k < (int)(blockIdx.x / parts)) {
         vc += bbig[2 * k];
         vb += bbig[2 * k + 1];
       }
@@ -1043,13 +1096,11 @@ __global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bb
       s_end[ob] = en;
       big_list[carry_b + ob] = i;
       node_chunk0[carry_b + ob] = carry_c + oc;
+      nodes[i].big = carry_b + ob;
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < tb * kSums; k += blockDim.x) {
-      acc[(size_t)carry_b * kSums + k] = u128_zero();
-      accl[(size_t)carry_b * kSums + k] = u128_zero();
-    }
-    for (int c = threadIdx.x; c < tc; c += blockDim.x) {
+    for (int k = threadIdx.x; k < tb * kSums; k += blockDim.x) acc[(size_t)carry_b * kSums + k] = u128_zero();
+    for (int c = part * blockDim.x + threadIdx.x; c < tc; c += parts * blockDim.x) {
       int lo = 0, hi = tb;  // the last listed node whose first chunk is at or before c
       while (hi - lo > 1) {
         const int m = (lo + hi) >> 1;
@@ -1075,6 +1126,14 @@ __global__ void k_big_plan(const BNode* nodes, LevelState* ls, const int32_t* bb
     ls->num_big = all_b;
     if (all_c > chunk_cap) ls->error = 1;
   }
+}
+
+// root: clear the roots' own sums, else the smaller children's of this level.
+__global__ void k_big_plan(BNode* nodes, LevelState* ls, const int32_t* bbig, Chunk* chunks, int32_t chunk_cap,
+                           int32_t* big_list, int32_t* node_chunk0, U128* root_acc, ChildSums C, int parts) {
+  __shared__ int sm[32];
+  level_plan(nodes, ls, bbig, chunks, chunk_cap, big_list, node_chunk0, root_acc ? root_acc : C.acc[ls->depth & 1], sm,
+             (int)blockIdx.x % parts, parts);
 }
 
 // Block sum of the warps' sums into one 128-bit accumulator set (any order: exact).
@@ -1184,38 +1243,6 @@ __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
   return n;
 }
 
-// Block per large node: the exclusive scan of its chunks' left counts (each chunk's left
-// offset inside the node), then the node's split point and its children's ranges.
-__global__ void k_big_offsets(BNode* nodes, LevelState* ls, const int32_t* big_list,
-                              const int32_t* node_chunk0, const SegCounts* seg, int32_t* chunk_loff) {
-  __shared__ int sm[32];
-  const int nb = ls->num_big, nc = ls->num_chunks;
-  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    const int c0 = node_chunk0[b];
-    const int c1 = (b + 1 < nb) ? node_chunk0[b + 1] : nc;
-    int carry = 0;
-    for (int base = c0; base < c1; base += blockDim.x) {
-      const int c = base + threadIdx.x;
-      const int v = c < c1 ? seg_before(seg[c], kSegs) : 0;
-      int tot;
-      const int ex = block_scan(v, sm, &tot);
-      if (c < c1) chunk_loff[c] = carry + ex;
-      carry += tot;
-    }
-    if (threadIdx.x == 0) {
-      BNode& nd = nodes[big_list[b]];
-      nd.mid = nd.split ? nd.start + carry : nd.end;
-      if (nd.split) {
-        nodes[nd.left].start = nd.start;
-        nodes[nd.left].end = nd.mid;
-        nodes[nd.right].start = nd.mid;
-        nodes[nd.right].end = nd.end;
-        atomicMax(&ls->max_next, max(nd.mid - nd.start, nd.end - nd.mid));
-      }
-    }
-  }
-}
-
 // Stable scatter by warp ballots: warp w of a block moves segment w of each of its chunks, in
 // four rounds of 32 points, so left and right runs are written contiguously.  The points
 // that go to the node's smaller child are summed on the way (the sums of the large node's
@@ -1226,12 +1253,15 @@ __global__ void k_big_offsets(BNode* nodes, LevelState* ls, const int32_t* big_l
 // chunk and added with 22 atomics each, it took 235-310 us, and 691 us on the root, where
 // every warp hits the same words; three blocks per SM spill and take 118 us.
 __global__ void __launch_bounds__(kThreads, kScatterPerSM)
-    k_big_scatter(const Chunk* chunks, const LevelState* ls, const BNode* nodes, PointBufs B, const SegCounts* seg,
-                  const int32_t* chunk_loff, U128* accl) {
+    k_big_scatter(const Chunk* chunks, LevelState* ls, BNode* nodes, PointBufs B, const SegCounts* seg,
+                  const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t* level_begin,
+                  unsigned* done) {
   __shared__ U128 smm[kSegs][kSums];
-  const int nc = ls->num_chunks, cur = ls->cur;
+  __shared__ int s_pre[kSegs], s_tot[kSegs];
+  const int nc = ls->num_chunks, nbig = ls->num_big, cur = ls->cur;
   const float4* pin = B.p[cur];
   float4* pout = B.p[cur ^ 1];
+  U128* accl = C.acc[ls->depth & 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   LaneSums S;
@@ -1243,6 +1273,7 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
   int big = -1, held = 0;
   float mean[3], dir[3];
   int nstart = 0, nmid = 0;
+  int before = 0;  // left points of the node's chunks before this one
   bool split = false, small_left = false;
   for (int ci = c0; ci < c1; ++ci) {
     const Chunk c = chunks[ci];
@@ -1251,12 +1282,12 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
       if (wb + u * 32 + lane < c.end) pv[u] = pin[wb + u * 32 + lane];
-    const int loff = chunk_loff[ci] + seg_before(seg[ci], w);  // left points of the node before this segment
+    const SegCounts sc = seg[ci];
     if (c.big != big) {
       if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, false);
       big = c.big;
       held = 0;
-      const BNode& nd = nodes[c.node];
+      BNode& nd = nodes[c.node];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         mean[k] = nd.mean[k];
@@ -1264,8 +1295,46 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
       }
       split = nd.split != 0;
       nstart = nd.start;
-      nmid = nd.mid;
-      small_left = nd.mid - nd.start <= nd.end - nd.mid;
+      // the node's left points, and those before this chunk, from its chunks' counts (every
+      // block of the node adds them up itself: no pass of its own over the counts)
+      const int n0 = node_chunk0[big], n1 = big + 1 < nbig ? min(node_chunk0[big + 1], nc) : nc;
+      const bool few = n1 - n0 <= 64;  // each warp for itself, no barrier
+      int pre = 0, tot = 0;
+      for (int k = n0 + (few ? lane : (int)threadIdx.x); k < n1; k += few ? 32 : kThreads) {
+        const int n = seg_before(seg[k], kSegs);
+        tot += n;
+        if (k < ci) pre += n;
+      }
+      pre = __reduce_add_sync(0xffffffffu, pre);
+      tot = __reduce_add_sync(0xffffffffu, tot);
+      if (!few) {
+        if (lane == 0) {
+          s_pre[w] = pre;
+          s_tot[w] = tot;
+        }
+        __syncthreads();
+        pre = tot = 0;
+#pragma unroll
+        for (int k = 0; k < kSegs; ++k) {
+          pre += s_pre[k];
+          tot += s_tot[k];
+        }
+        __syncthreads();  // they may be rewritten after this
+      }
+      before = pre;
+      nmid = nstart + tot;
+      const int nend = nd.end;
+      small_left = nmid - nstart <= nend - nmid;
+      if (ci == n0 && threadIdx.x == 0) {  // the node's first block: its children's ranges
+        nd.mid = split ? nmid : nend;
+        if (split) {
+          nodes[nd.left].start = nstart;
+          nodes[nd.left].end = nmid;
+          nodes[nd.right].start = nmid;
+          nodes[nd.right].end = nend;
+          atomicMax(&ls->max_next, max(nmid - nstart, nend - nmid));
+        }
+      }
     } else if (++held == kFoldChunks) {
       lane_fold(S, lane);
       held = 0;
@@ -1276,6 +1345,8 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
         if (wb + u * 32 + lane < c.end) B.perm[wb + u * 32 + lane] = __float_as_int(pv[u].w);
       continue;
     }
+    const int loff = before + seg_before(sc, w);  // left points of the node before this segment
+    before += seg_before(sc, kSegs);
     int lo = nstart + loff;
     int ro = nmid + min(wb, c.end) - nstart - loff;  // the node's points before this segment, less the left ones
 #pragma unroll
@@ -1290,29 +1361,12 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     }
   }
   if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, per == 1);
-}
-
-// Children's sums of the large split nodes: the smaller from accl, the other = parent - it.
-__global__ void k_big_childmom(const BNode* nodes, LevelState* ls, const int32_t* big_list, const U128* accl,
-                               U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin, unsigned* done) {
-  const int nb = ls->num_big;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * kSums; t += gridDim.x * blockDim.x) {
-    const int b = t / kSums, k = t % kSums;
-    const int i = big_list[b];
-    if (!nodes[i].split) continue;
-    const U128 q = accl[t];  // the smaller child's sums
-    const U128 other = u128_sub(mom[(size_t)i * kSums + k], q);
-    const bool small_left = nodes[i].mid - nodes[i].start <= nodes[i].end - nodes[i].mid;
-    mom[(size_t)nodes[i].left * kSums + k] = small_left ? q : other;
-    mom[(size_t)nodes[i].right * kSums + k] = small_left ? other : q;
-  }
   advance_if_last(ls, bsum, nblocks, level_begin, done);
 }
 
 // ---- children ------------------------------------------------------------------------
 
-__global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap) {
-  __shared__ int sm[32];
+__device__ __forceinline__ void level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap, int* sm) {
   int b, e;
   level_range(ls, b, e);
   const int le = ls->le;
@@ -1359,6 +1413,28 @@ __global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bs
       }
     }
   }
+}
+
+__global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap) {
+  __shared__ int sm[32];
+  level_children(nodes, ls, bsum, cap, sm);
+}
+
+// A level of at most kThreads nodes: decisions, children and the large nodes' chunks by one
+// block in one launch (8 + 2.5 + 3.5 us and two gaps as three kernels, whose later two read
+// back what the first wrote).
+__global__ void __launch_bounds__(kThreads) k_level_small(BNode* nodes, LevelState* ls, U128* mom, ChildSums C,
+                                                          BuildParams P, int32_t* bsum, int32_t* bbig,
+                                                          double* root_frame, int32_t cap, Chunk* chunks,
+                                                          int32_t chunk_cap, int32_t* big_list, int32_t* node_chunk0,
+                                                          int plan) {
+  __shared__ int sm[32];
+  level_decide(nodes, ls, mom, C, P, bsum, bbig, root_frame, sm);
+  __syncthreads();
+  level_children(nodes, ls, bsum, cap, sm);
+  if (!plan) return;
+  __syncthreads();
+  level_plan(nodes, ls, bbig, chunks, chunk_cap, big_list, node_chunk0, C.acc[ls->depth & 1], sm, 0, 1);
 }
 
 // ---- deep levels: whole subtrees in shared memory --------------------------------------
@@ -1412,13 +1488,13 @@ struct DeepWarpSmem {                // one warp's slice
 };
 
 __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
-    k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, BuildParams P,
+    k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, ChildSums C, BuildParams P,
                  double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* ring, int32_t* counts,
                  int32_t dcap) {
   extern __shared__ __align__(16) unsigned char deep_smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   DeepWarpSmem& S = reinterpret_cast<DeepWarpSmem*>(deep_smem_raw)[wib];
-  const int lb = ls->lb, le = ls->le, cur0 = ls->cur;
+  const int lb = ls->lb, le = ls->le, cur0 = ls->cur, depth0 = ls->depth;
   const int nroots = le - lb;
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
   const int gw = blockIdx.x * kDeepWarpsPerBlock + wib, nw = gridDim.x * kDeepWarpsPerBlock;
@@ -1451,7 +1527,12 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
           break;
         }
       }
-      const U128* psums = d == 0 ? mom + (size_t)R * kSums : myring + (size_t)(d & 1) * kDeepNodes * kSums;
+      const U128* psums = myring + (size_t)(d & 1) * kDeepNodes * kSums;
+      if (d == 0) {  // the root's sums into the ring
+        const PendingSums ps = pending_sums(nodes, mom, C, depth0, R, root.parent);
+        if (lane < kSums) myring[lane] = ps.q ? pending_value(ps, lane) : mom[(size_t)R * kSums + lane];
+        __syncwarp();
+      }
       for (int r = lane; r < cnt; r += 32) {
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
@@ -1473,7 +1554,7 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
           }
         }
         double Sd[kSums];
-        const U128* ms = d == 0 ? psums : psums + (size_t)r * kSums;
+        const U128* ms = psums + (size_t)r * kSums;
         for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(ms[k]);
         decide(Sd, en - st, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
         S.split[r] = nd.split ? 1 : 0;
@@ -1568,7 +1649,7 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
         const U128 qs = sums_total(W, S.stage, lane);
         if (lane < kSums) {
           const int k = lane;
-          const U128 ps = d == 0 ? psums[k] : psums[(size_t)r * kSums + k];
+          const U128 ps = psums[(size_t)r * kSums + k];
           const U128 other = u128_sub(ps, qs);
           U128* nxt = myring + (size_t)((d + 1) & 1) * kDeepNodes * kSums;
           nxt[(size_t)(2 * q) * kSums + k] = small_left ? qs : other;
@@ -1940,9 +2021,9 @@ struct BuildWs {
   int32_t *alive, *rank, *leaf_flag, *lrank, *tile_sums;
   Chunk* chunks;
   SegCounts* seg;
-  int32_t *chunk_loff, *big_list, *node_chunk0;
-  U128* acc;
-  U128* accl;  // left-child sums of the level's large nodes
+  int32_t *big_list, *node_chunk0;
+  U128* acc;       // the large roots' sums
+  ChildSums accl;  // the smaller children's sums of large nodes, by level parity
   U128* mom;   // exact sums of every node
   double* ts0;   // per cloud
   double* dt;    // stamps less ts0, input order
@@ -1969,8 +2050,8 @@ size_t ws_bytes(int64_t n, int R) {
   const int64_t G = (int64_t)(kMaxDepth + 2) * R;
   return carve_size<float4>(2 * n + 2) + carve_size<int32_t>(n) +
          carve_size<BNode>(cn) + 4 * carve_size<int32_t>(cn) + carve_size<int32_t>(ntiles) +
-         carve_size<Chunk>(chunk_cap) + carve_size<SegCounts>(chunk_cap) + 3 * carve_size<int32_t>(chunk_cap) +
-         2 * carve_size<U128>((size_t)kSums * (n / kBig + 2)) + carve_size<U128>((size_t)kSums * cn) + carve_size<unsigned long long>(R) + carve_size<double>(R) + carve_size<double>(n) +
+         carve_size<Chunk>(chunk_cap) + carve_size<SegCounts>(chunk_cap) + 2 * carve_size<int32_t>(chunk_cap) +
+         3 * carve_size<U128>((size_t)kSums * (n / kBig + 2)) + carve_size<U128>((size_t)kSums * cn) + carve_size<unsigned long long>(R) + carve_size<double>(R) + carve_size<double>(n) +
          carve_size<DtSum>(n / kDtTile + 1) +
          carve_size<double>((size_t)kRootFrame * R) + carve_size<int64_t>(R + 1) +
          carve_size<LevelState>(1) + carve_size<int32_t>(kMaxDepth + 2) + carve_size<unsigned>(1) +
@@ -2006,11 +2087,10 @@ int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
   w.tile_sums = carve<int32_t>(p, ntiles);
   w.chunks = carve<Chunk>(p, w.chunk_cap);
   w.seg = carve<SegCounts>(p, w.chunk_cap);
-  w.chunk_loff = carve<int32_t>(p, w.chunk_cap);
   w.big_list = carve<int32_t>(p, w.chunk_cap);
   w.node_chunk0 = carve<int32_t>(p, w.chunk_cap);
   w.acc = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
-  w.accl = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
+  for (int k = 0; k < 2; ++k) w.accl.acc[k] = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
   w.mom = carve<U128>(p, (size_t)kSums * cn);
   w.ts0 = carve<double>(p, R);
   w.dt = carve<double>(p, n);
@@ -2085,7 +2165,7 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * ncount, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(dn_count, 0, sizeof(int32_t), s);
   if (e == cudaSuccess) {
-    k_deep_build<<<grid, kDeepThreads, sizeof(DeepWarpSmem) * kDeepWarpsPerBlock, s>>>(w.nodes, w.ls, w.B, w.mom, P, w.root_frame, dn,
+    k_deep_build<<<grid, kDeepThreads, sizeof(DeepWarpSmem) * kDeepWarpsPerBlock, s>>>(w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame, dn,
                                                               dn_cap, dn_count, ring, counts, dcap);
     count_launch();
     rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
@@ -2259,38 +2339,48 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       const int lvl_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(kLevelBlocks, (nodes_bound + kThreads - 1) / kThreads));
       const int small_blocks =
           (int)std::max<int64_t>(1, std::min<int64_t>(kSmallBlocks, (nodes_bound + kThreads / 32 - 1) / (kThreads / 32)));
+      // blocks per node range that write its chunks: a thread each for a few thousand chunks
+      // (one block takes 25 us for 11,000), none but the level's own where those do
+      const int plan_parts = lvl_blocks == 1 ? (int)std::max<int64_t>(1, std::min<int64_t>(64, N / (4096 * kChunk / 4)))
+                                             : 1;
       if (level0) {  // the roots' sums
         k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
         count_launch();
         if (host_max > kBig) {
           k_big_sums<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig);
-          k_big_plan<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list,
-                                                     w.node_chunk0, w.acc, w.accl);
+          k_big_plan<<<lvl_blocks * plan_parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
+                                                                  w.big_list, w.node_chunk0, w.acc, w.accl, plan_parts);
           k_big_moments<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.acc);
           k_big_to_mom<<<64, 256, 0, s>>>(w.ls, w.big_list, w.acc, w.mom);
           for (int c = 0; c < 4; ++c) count_launch();
         }
       }
-      k_decide<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, P, w.bsum, w.bbig, w.root_frame);
-      k_level_children<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
       const bool big = host_max > kBig;  // the large-node kernels run after the partition
-      k_small_part<<<small_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks,
-                                                     w.level_begin, big ? nullptr : w.done);
-      for (int c = 0; c < 3; ++c) count_launch();
+      if (lvl_blocks == 1) {
+        k_level_small<<<1, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame,
+                                             (int32_t)w.cap_nodes, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0,
+                                             plan_parts == 1 ? 1 : 0);
+        count_launch();
+      } else {
+        k_decide<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame);
+        k_level_children<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
+        count_launch();
+        count_launch();
+      }
+      if (big && (lvl_blocks > 1 || plan_parts > 1)) {  // the decisions counted the large nodes per block
+        k_big_plan<<<lvl_blocks * plan_parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
+                                                                w.big_list, w.node_chunk0, nullptr, w.accl, plan_parts);
+        count_launch();
+      }
+      k_small_part<<<small_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks, w.level_begin,
+                                                     big ? nullptr : w.done);
+      count_launch();
       if (big) {
-        if (!level0) {  // k_decide counted the large nodes per block
-          k_big_plan<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list,
-                                                     w.node_chunk0, w.acc, w.accl);
-          count_launch();
-        }
         k_big_count<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg);
-        k_big_offsets<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, w.ls, w.big_list, w.node_chunk0, w.seg,
-                                                       w.chunk_loff);
-        k_big_scatter<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg, w.chunk_loff,
-                                                  w.accl);
-        k_big_childmom<<<64, 256, 0, s>>>(w.nodes, w.ls, w.big_list, w.accl, w.mom, w.bsum, lvl_blocks,
-                                          w.level_begin, w.done);
-        for (int c = 0; c < 5; ++c) count_launch();
+        k_big_scatter<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
+                                              lvl_blocks, w.level_begin, w.done);
+        count_launch();
+        count_launch();
       }
     }
     KDS_CK(cudaGetLastError());
