@@ -1438,31 +1438,43 @@ __global__ void __launch_bounds__(kThreads) k_level_small(BNode* nodes, LevelSta
 }
 
 // ---- deep levels: whole subtrees in shared memory --------------------------------------
-// Once every node of a level has at most kDeepMax points, each of them is the root of a
-// subtree that one warp builds to the end in its own slice of shared memory: the points
-// are loaded once, and every depth below runs the same steps as the level kernels --
-// decide (lane per node, from the node's exact sums), children numbered by a warp scan,
-// stable ballot partition by whichSide (the warp per node) with the smaller child summed
-// on the way (the other = parent - smaller).  The arithmetic and the partition order are
-// those of k_decide / k_small_part, so the nodes are bit-identical to a level-by-level
-// build.  The warps of a block share nothing and never wait for each other.  Nodes below
-// the roots are written as DeepNode records tagged (subtree, depth, rank); k_deep_place
-// then puts them at their breadth-first positions: depth by depth, subtree by subtree in
-// the roots' order, by rank inside a subtree -- the order in which the level kernels
-// would have numbered them.
-constexpr int kDeepMax = 256;      // largest subtree root (points)
-// The subtree pass runs only while the level has at most this many nodes: it finishes a
-// few thousand subtrees in about one subtree's latency, which beats the level kernels'
-// launches for single trees and small batches; for large forests (hundreds of thousands
-// of tiny subtrees, where a warp's decide runs on a few lanes) the level kernels, with a
-// thread per node of the whole level, are faster.
-constexpr int kDeepMaxRoots = 8192;
-constexpr int kDeepNodes = 192;    // nodes of one depth: at most 2 x (kDeepMax / 3) split children
-constexpr int kDeepWarpsPerBlock = 4;
-constexpr int kDeepThreads = 32 * kDeepWarpsPerBlock;
-constexpr int kDeepBlocksPerSM = 4;
-static_assert(kDeepMax <= kBig, "deep subtree roots are summed by k_root_moments");
-static_assert(2 * (kDeepMax / 3) <= kDeepNodes, "node capacity of one depth");
+// Once every node of a level is small enough, each of them is the root of a subtree that one
+// group of threads builds to the end in shared memory: the points are loaded once, and every
+// depth below runs the same steps as the level kernels -- decide (thread per node, from the
+// node's exact sums), children numbered by a scan, stable ballot partition by whichSide (a
+// warp per node) with the smaller child summed on the way (the other = parent - smaller).  The
+// arithmetic and the partition order are those of k_decide / k_small_part, so the nodes are
+// bit-identical to a level-by-level build.  Nodes below the roots are written as DeepNode
+// records tagged (subtree, depth, rank); k_deep_place then puts them at their breadth-first
+// positions: depth by depth, subtree by subtree in the roots' order, by rank inside a subtree
+// -- the order in which the level kernels would have numbered them.
+//
+// Two forms, both for levels that leave most of the machine idle, where a level costs its
+// launches and the chain of one decision however few nodes it has:
+//  * a block of 16 warps per subtree of at most 2,048 points, while the level has at most
+//    kBlockRoots of them: a 12,000-point scan leaves the level kernels after 3 levels, a
+//    180,000-point one after 8 (DEEPNOTE);
+//  * a warp per subtree of at most 256 points, up to 8,192 of them.
+// For large forests (hundreds of thousands of tiny subtrees, where a decision runs on a few
+// lanes) the level kernels, with a thread per node of the whole level, are faster: the warp
+// form on all deep levels of 80 scans took 7.1 ms in place of 4.8.
+template <int WARPS>
+struct DeepForm;
+template <>
+struct DeepForm<1> {
+  static constexpr int kPoints = 256, kGroups = 4, kPerSM = 4, kRoots = 8192;
+};
+template <>
+struct DeepForm<16> {
+  static constexpr int kPoints = 2048, kGroups = 1, kPerSM = 1, kRoots = 296;
+};
+constexpr int kDeepMax = DeepForm<1>::kPoints;
+constexpr int kDeepMaxRoots = DeepForm<1>::kRoots;
+constexpr int kBlockMax = DeepForm<16>::kPoints;
+constexpr int kBlockRoots = DeepForm<16>::kRoots;
+// nodes of one depth: at most two children per split node, which holds at least three points
+template <int WARPS>
+constexpr int deep_nodes() { return (2 * (DeepForm<WARPS>::kPoints / 3) + 31) / 32 * 32; }
 
 struct DeepNode {
   float mean[3], dir[3];
@@ -1478,62 +1490,73 @@ struct DeepNode {
 static_assert(sizeof(DeepNode) == 80, "DeepNode layout");
 static_assert(sizeof(DeepNode) <= kSums * sizeof(U128), "a DeepNode fits the sums slot of one node");
 
-struct DeepWarpSmem {                // one warp's slice
-  float4 pts[2][kDeepMax];           // the 16 B point records (w = input index)
-  uint32_t range[2][kDeepNodes];     // node start | end << 16 (subtree offsets), by depth parity
-  int32_t prank[2][kDeepNodes];      // parent's rank, by depth parity
-  int32_t list[kDeepNodes];          // q -> rank of the q-th split node of the depth
-  uint8_t split[kDeepNodes];
-  SumStage stage;
+template <int WARPS>
+struct DeepSmem {                             // one group's
+  float4 pts[2][DeepForm<WARPS>::kPoints];    // the 16 B point records (w = input index)
+  SumStage stage[WARPS];
+  uint32_t range[2][deep_nodes<WARPS>()];     // node start | end << 16 (subtree offsets), by depth parity
+  int32_t prank[2][deep_nodes<WARPS>()];      // parent's rank, by depth parity
+  int32_t list[deep_nodes<WARPS>()];          // q -> rank of the q-th split node of the depth
+  int32_t scan[32];
+  int32_t base, pad_[3];
+  uint8_t split[deep_nodes<WARPS>()];
 };
 
-__global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepForm<WARPS>::kPerSM)
     k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, ChildSums C, BuildParams P,
                  double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* ring, int32_t* counts,
                  int32_t dcap) {
+  constexpr int kNodes = deep_nodes<WARPS>();
+  constexpr int kThreadsG = 32 * WARPS;
   extern __shared__ __align__(16) unsigned char deep_smem_raw[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  DeepWarpSmem& S = reinterpret_cast<DeepWarpSmem*>(deep_smem_raw)[wib];
+  const int lane = threadIdx.x & 31, group = WARPS == 1 ? (int)threadIdx.x >> 5 : 0;
+  const int tid = WARPS == 1 ? lane : (int)threadIdx.x, warp = WARPS == 1 ? 0 : (int)threadIdx.x >> 5;
+  auto sync = []() {  // the group's threads
+    if (WARPS == 1) __syncwarp();
+    else __syncthreads();
+  };
+  DeepSmem<WARPS>& S = reinterpret_cast<DeepSmem<WARPS>*>(deep_smem_raw)[group];
+  SumStage& sg = S.stage[warp];
   const int lb = ls->lb, le = ls->le, cur0 = ls->cur, depth0 = ls->depth;
   const int nroots = le - lb;
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
-  const int gw = blockIdx.x * kDeepWarpsPerBlock + wib, nw = gridDim.x * kDeepWarpsPerBlock;
-  stage_init(S.stage, lane);
+  const int gw = blockIdx.x * DeepForm<WARPS>::kGroups + group, nw = gridDim.x * DeepForm<WARPS>::kGroups;
+  stage_init(sg, lane);
   WarpSums W;
   sums_zero(W);
-  U128* myring = ring + (size_t)gw * 2 * kDeepNodes * kSums;
+  U128* myring = ring + (size_t)gw * 2 * kNodes * kSums;
   const float4* pin = B.p[cur0];
   for (int sub = gw; sub < nroots; sub += nw) {
     const int R = lb + sub;
     const BNode root = nodes[R];
     const int n = root.end - root.start;
     const int pbase = root.start;
-    for (int i = lane; i < n; i += 32) S.pts[0][i] = pin[pbase + i];
-    if (lane == 0) {
+    for (int i = tid; i < n; i += kThreadsG) S.pts[0][i] = pin[pbase + i];
+    if (tid == 0) {
       S.range[0][0] = (uint32_t)n << 16;
       S.prank[0][0] = -1;
     }
-    __syncwarp();
+    if (tid < kSums) {  // the root's sums into the ring
+      const PendingSums ps = pending_sums(nodes, mom, C, depth0, R, root.parent);
+      myring[tid] = ps.q ? pending_value(ps, tid) : mom[(size_t)R * kSums + tid];
+    }
+    sync();
     int cnt = 1, c = 0, base = 0, base_prev = 0;
     for (int d = 0; cnt > 0; ++d, c ^= 1) {
-      // ---- decide: lane per node of this depth; record slots for the depth's nodes
+      // ---- decide: thread per node of this depth; record slots for the depth's nodes
       if (d > 0) {
         base_prev = base;
-        int b = 0;
-        if (lane == 0) b = atomicAdd(dn_count, cnt);
-        base = __shfl_sync(full, b, 0);
+        if (tid == 0) S.base = atomicAdd(dn_count, cnt);
+        sync();
+        base = S.base;
         if (base + cnt > dn_cap) {
-          if (lane == 0) ls->error = 1;  // out of record slots: the build reports KDS_ERR_CAPACITY
+          if (tid == 0) ls->error = 1;  // out of record slots: the build reports KDS_ERR_CAPACITY
           break;
         }
       }
-      const U128* psums = myring + (size_t)(d & 1) * kDeepNodes * kSums;
-      if (d == 0) {  // the root's sums into the ring
-        const PendingSums ps = pending_sums(nodes, mom, C, depth0, R, root.parent);
-        if (lane < kSums) myring[lane] = ps.q ? pending_value(ps, lane) : mom[(size_t)R * kSums + lane];
-        __syncwarp();
-      }
-      for (int r = lane; r < cnt; r += 32) {
+      const U128* psums = myring + (size_t)(d & 1) * kNodes * kSums;
+      for (int r = tid; r < cnt; r += kThreadsG) {
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
         BNode nd;
@@ -1578,38 +1601,44 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
           dn[base + r] = x;
         }
       }
-      __syncwarp();
-      // ---- children numbering: split ranks by a warp scan in rank order
+      sync();
+      // ---- children numbering: split ranks by a scan in rank order
       int nsplit = 0;
-      for (int r0 = 0; r0 < cnt; r0 += 32) {
-        const int r = r0 + lane;
+      for (int r0 = 0; r0 < cnt; r0 += kThreadsG) {
+        const int r = r0 + tid;
         const bool f = r < cnt && S.split[r];
-        const unsigned bf = __ballot_sync(full, f);
-        if (f) {
-          const int q = nsplit + __popc(bf & lt);
-          S.list[q] = r;
-          if (d > 0) dn[base + r].q = q;
+        int q, total;
+        if (WARPS == 1) {
+          const unsigned bf = __ballot_sync(full, f);
+          q = __popc(bf & lt);
+          total = __popc(bf);
+        } else {
+          q = block_scan(f ? 1 : 0, S.scan, &total);
         }
-        nsplit += __popc(bf);
+        if (f) {
+          S.list[nsplit + q] = r;
+          if (d > 0) dn[base + r].q = nsplit + q;
+        }
+        nsplit += total;
       }
-      if (2 * nsplit > kDeepNodes) {  // cannot happen (split nodes hold >= 3 points); refuse rather than overrun
-        if (lane == 0) ls->error = 1;
+      if (2 * nsplit > kNodes) {  // cannot happen (split nodes hold >= 3 points); refuse rather than overrun
+        if (tid == 0) ls->error = 1;
         break;
       }
-      if (nsplit > 0 && lane == 0) {
+      if (nsplit > 0 && tid == 0) {
         if (d + 1 < dcap) counts[(size_t)(d + 1) * nroots + sub] = 2 * nsplit;
         else ls->error = 1;
       }
-      __syncwarp();
-      // ---- the leaves' point order (lane per leaf)
-      for (int r = lane; r < cnt; r += 32) {
+      sync();
+      // ---- the leaves' point order (thread per leaf)
+      for (int r = tid; r < cnt; r += kThreadsG) {
         if (S.split[r]) continue;
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
         for (int i = st; i < en; ++i) B.perm[pbase + i] = __float_as_int(S.pts[c][i].w);
       }
-      // ---- partition of the split nodes, the warp per node
-      for (int q = 0; q < nsplit; ++q) {
+      // ---- partition of the split nodes, a warp per node
+      for (int q = warp; q < nsplit; q += WARPS) {
         const int r = S.list[q];
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
@@ -1641,17 +1670,17 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
             const int dst = left ? (st + cl + __popc(bl & lt)) : (mid + cr + __popc(br & lt));
             S.pts[c ^ 1][dst] = p;
           }
-          sums_add(W, S.stage, valid && left == small_left, p, lane);
-          sums_room(W, S.stage, kStage - 32, lane);
+          sums_add(W, sg, valid && left == small_left, p, lane);
+          sums_room(W, sg, kStage - 32, lane);
           cl += __popc(bl);
           cr += __popc(br);
         }
-        const U128 qs = sums_total(W, S.stage, lane);
+        const U128 qs = sums_total(W, sg, lane);
         if (lane < kSums) {
           const int k = lane;
           const U128 ps = psums[(size_t)r * kSums + k];
           const U128 other = u128_sub(ps, qs);
-          U128* nxt = myring + (size_t)((d + 1) & 1) * kDeepNodes * kSums;
+          U128* nxt = myring + (size_t)((d + 1) & 1) * kNodes * kSums;
           nxt[(size_t)(2 * q) * kSums + k] = small_left ? qs : other;
           nxt[(size_t)(2 * q + 1) * kSums + k] = small_left ? other : qs;
         }
@@ -1664,19 +1693,19 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocksPerSM)
       }
       cnt = 2 * nsplit;
       if (d + 1 >= dcap) cnt = 0;
-      __syncwarp();
+      sync();
     }
-    __syncwarp();
+    sync();
   }
 }
 
 // Deep nodes to their breadth-first positions: node (subtree s, depth d, rank r) goes to
 // le + off[d * nroots + s] + r, where off is the exclusive scan of the per-(depth,
 // subtree) node counts in depth-major order.  The roots get their children's indices.
-__global__ void k_deep_place(BNode* nodes, LevelState* ls, const DeepNode* dn, const int32_t* dn_count,
-                             int32_t dn_cap, const int32_t* off, int32_t dcap, int32_t cap_nodes) {
+__global__ void k_deep_place(BNode* nodes, LevelState* ls, int32_t lb, int32_t le, const DeepNode* dn,
+                             const int32_t* dn_count, int32_t dn_cap, const int32_t* off, int32_t dcap,
+                             int32_t cap_nodes) {
   if (ls->error) return;  // the build fails; records may be missing
-  const int lb = ls->lb, le = ls->le;
   const int nroots = le - lb;
   const int nd_total = min(*dn_count, dn_cap);
   const int stride = gridDim.x * blockDim.x;
@@ -1723,27 +1752,56 @@ __global__ void k_deep_place(BNode* nodes, LevelState* ls, const DeepNode* dn, c
   }
 }
 
-// One thread: the level state after the deep levels (every level done), the begin of
-// each deep level, the depth, and the node capacity check.
-__global__ void k_deep_finish(LevelState* ls, const int32_t* off, const int32_t* total, int32_t dcap,
-                              int32_t cap_nodes, int32_t* level_begin) {
-  if (blockIdx.x != 0 || threadIdx.x != 0 || ls->error) return;
-  const int lb = ls->lb, le = ls->le;
+// One block: the level state after the deep levels (every level done), the begin of each deep
+// level, the depth, and the node capacity check (a thread per depth; one thread for all took
+// 11 us of dependent loads).
+__device__ __forceinline__ void deep_finish(LevelState* ls, int32_t lb, int32_t le, const int32_t* off, int32_t tot,
+                                            int32_t dcap, int32_t cap_nodes, int32_t* level_begin) {
+  __shared__ int s_dmax;  // deepest local depth holding nodes
+  const int depth0 = ls->depth;
+  const bool failed = ls->error != 0;
+  if (threadIdx.x == 0) s_dmax = 0;
+  __syncthreads();
+  if (failed) return;
   const int nroots = le - lb;
-  const int tot = *total;
-  int dmax = 0;  // deepest local depth holding nodes
-  for (int d = 1; d < dcap; ++d) {
+  for (int d = 1 + threadIdx.x; d < dcap; d += blockDim.x) {
     const int b = off[(size_t)d * nroots];
     const int e = d + 1 < dcap ? off[(size_t)(d + 1) * nroots] : tot;
     if (e > b) {
-      dmax = d;
-      if (ls->depth + d < kMaxDepth + 1) level_begin[ls->depth + d] = le + b;
+      atomicMax(&s_dmax, d);
+      if (depth0 + d < kMaxDepth + 1) level_begin[depth0 + d] = le + b;
     }
   }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   if (le + tot > cap_nodes) ls->error = 1;
-  ls->depth += dmax + 1;
+  ls->depth = depth0 + s_dmax + 1;
   ls->lb = ls->le = le + tot;
   if (ls->depth < kMaxDepth + 1) level_begin[ls->depth] = ls->lb;
+}
+__global__ void k_deep_finish(LevelState* ls, int32_t lb, int32_t le, const int32_t* off, const int32_t* total,
+                              int32_t dcap, int32_t cap_nodes, int32_t* level_begin) {
+  deep_finish(ls, lb, le, off, *total, dcap, cap_nodes, level_begin);
+}
+// The same with the scan of the counts by the one block: up to kDeepScan counts, a run per
+// thread (three scan launches and this otherwise).
+constexpr int kDeepScan = 16384;
+__global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, int32_t le, const int32_t* counts,
+                                                    int32_t ncount, int32_t* off, int32_t dcap, int32_t cap_nodes,
+                                                    int32_t* level_begin) {
+  __shared__ int sm[32];
+  const int per = (ncount + 1023) / 1024;
+  const int b = min((int)threadIdx.x * per, ncount), e = min(b + per, ncount);
+  int v = 0;
+  for (int i = b; i < e; ++i) v += counts[i];
+  int tot;
+  int x = block_scan(v, sm, &tot);
+  for (int i = b; i < e; ++i) {
+    off[i] = x;
+    x += counts[i];
+  }
+  __syncthreads();
+  deep_finish(ls, lb, le, off, tot, dcap, cap_nodes, level_begin);
 }
 
 // ---- prune and per-tree compaction -----------------------------------------------------
@@ -2121,11 +2179,13 @@ int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
 
 namespace {
 
-// The deep levels of a build whose current level (h, read at the last sync) has no node
-// above kDeepMax points: k_deep_build, the depth-major scan of the per-(depth, subtree)
-// node counts, k_deep_place, k_deep_finish.  The node records of the deep levels are
-// staged in the unused part of the sums array (slots from le on).
+// The deep levels of a build whose current level (h, read at the last sync) fits the form:
+// k_deep_build, the depth-major scan of the per-(depth, subtree) node counts, k_deep_place and
+// k_deep_finish.  The node records of the deep levels are staged in the unused part of the
+// sums array (slots from le on).
+template <int WARPS>
 int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_t s) {
+  using Form = DeepForm<WARPS>;
   const int lb = h.lb, le = h.le;
   const int nroots = le - lb;
   if (nroots <= 0) return KDS_OK;
@@ -2133,52 +2193,87 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   DeepNode* dn = reinterpret_cast<DeepNode*>(w.mom + (size_t)le * kSums);
   const int64_t dn_cap64 = ((w.cap_nodes - le) * (int64_t)(kSums * sizeof(U128))) / (int64_t)sizeof(DeepNode);
   const int32_t dn_cap = (int32_t)std::min<int64_t>(dn_cap64, INT32_MAX);
-  const int grid = (int)std::min<int64_t>((nroots + kDeepWarpsPerBlock - 1) / kDeepWarpsPerBlock,
-                                          148 * kDeepBlocksPerSM);
-  const int64_t nwarps = (int64_t)grid * kDeepWarpsPerBlock;
+  const int grid = (int)std::min<int64_t>((nroots + Form::kGroups - 1) / Form::kGroups, 148 * Form::kPerSM);
+  const size_t ring_n = (size_t)grid * Form::kGroups * 2 * deep_nodes<WARPS>() * kSums;
   const int64_t ncount = (int64_t)dcap * nroots;
   if (ncount > INT32_MAX / 2) { set_error("kds_tree_build: too many deep subtrees"); return KDS_ERR_CAPACITY; }
-  const size_t bc = carve_size<int32_t>(ncount), bt = carve_size<int32_t>(ncount / 4096 + 2),
-               br = carve_size<U128>((size_t)nwarps * 2 * kDeepNodes * kSums);
+  const size_t bc = carve_size<int32_t>(ncount + 64), bt = carve_size<int32_t>(ncount / 4096 + 2),
+               br = carve_size<U128>(ring_n);
   void* blk = nullptr;
-  cudaError_t e = cudaMallocAsync(&blk, 2 * bc + bt + 3 * 256 + br, s);
+  cudaError_t e = cudaMallocAsync(&blk, 2 * bc + bt + 256 + br, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_error("cudaMallocAsync for the deep tree levels failed: %s", cudaGetErrorString(e));
     return KDS_ERR_OOM;
   }
   char* p = (char*)blk;
-  int32_t* counts = carve<int32_t>(p, ncount);
-  int32_t* off = carve<int32_t>(p, ncount);
+  int32_t* counts = carve<int32_t>(p, ncount + 64);  // and dn_count behind them: cleared together
+  int32_t* dn_count = counts + ncount;
+  int32_t* off = carve<int32_t>(p, ncount + 64);
   int32_t* tiles = carve<int32_t>(p, ncount / 4096 + 2);
   int32_t* total = carve<int32_t>(p, 1);
-  int32_t* dn_count = carve<int32_t>(p, 1);
-  carve<int32_t>(p, 1);
-  U128* ring = carve<U128>(p, (size_t)nwarps * 2 * kDeepNodes * kSums);
+  U128* ring = carve<U128>(p, ring_n);
   int rc = KDS_OK;
+  const size_t smem = sizeof(DeepSmem<WARPS>) * Form::kGroups;
   static std::atomic<bool> attr_set{false};  // a property of the kernel, per process (builds may run on two threads)
   if (!attr_set.load()) {
-    e = cudaFuncSetAttribute((const void*)k_deep_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(DeepWarpSmem) * kDeepWarpsPerBlock));
+    e = cudaFuncSetAttribute((const void*)k_deep_build<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) attr_set.store(true);
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * ncount, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dn_count, 0, sizeof(int32_t), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * (ncount + 1), s);
   if (e == cudaSuccess) {
-    k_deep_build<<<grid, kDeepThreads, sizeof(DeepWarpSmem) * kDeepWarpsPerBlock, s>>>(w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame, dn,
-                                                              dn_cap, dn_count, ring, counts, dcap);
+    k_deep_build<WARPS><<<grid, 32 * WARPS * Form::kGroups, smem, s>>>(w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame,
+                                                                       dn, dn_cap, dn_count, ring, counts, dcap);
     count_launch();
-    rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
+    if (ncount <= kDeepScan) {
+      k_deep_scan<<<1, 1024, 0, s>>>(w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes,
+                                     w.level_begin);
+    } else {
+      rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
+      k_deep_finish<<<1, 64, 0, s>>>(w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
+    }
+    count_launch();
     const int pg = (int)std::min<int64_t>(nblk(std::max<int64_t>(w.cap_nodes - le, nroots), kThreads), kGridBlocks * 4);
-    k_deep_place<<<pg, kThreads, 0, s>>>(w.nodes, w.ls, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes);
-    k_deep_finish<<<1, 32, 0, s>>>(w.ls, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
-    count_launch();
+    k_deep_place<<<pg, kThreads, 0, s>>>(w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes);
     count_launch();
     e = cudaGetLastError();
   }
   cudaFreeAsync(blk, s);
   if (e != cudaSuccess) return cuda_status(e, "deep tree levels", __FILE__, __LINE__);
   return rc;
+}
+
+}  // namespace
+
+namespace {
+
+// Blocks that write the chunks of one node range: a thread each for a few thousand chunks (one
+// block takes 25 us for 11,000), none but the level's own below.
+int chunk_parts(int64_t N) { return (int)std::max<int64_t>(1, std::min<int64_t>(64, N / (1 << 20))); }
+
+int level_blocks(int64_t nodes) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kLevelBlocks, (nodes + kThreads - 1) / kThreads));
+}
+
+// Blocks that take a contiguous range of chunks each: one resident wave, so that no block
+// starts when the others are done.
+int scatter_blocks(const BuildWs& w) { return std::min<int>(w.chunk_cap, 148 * kScatterPerSM); }
+
+// Level 0: the roots' sums, from their points.
+int root_sums(BuildWs& w, int R, int32_t max_size, int64_t N, cudaStream_t s) {
+  k_root_moments<<<(int)std::min<int64_t>(kGridBlocks, (R + 7) / 8), kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
+  count_launch();
+  if (max_size > kBig) {
+    const int nb = level_blocks(R), parts = nb == 1 ? chunk_parts(N) : 1;
+    k_big_sums<<<nb, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig);
+    k_big_plan<<<nb * parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0,
+                                               w.acc, w.accl, parts);
+    k_big_moments<<<scatter_blocks(w), kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.acc);
+    k_big_to_mom<<<64, 256, 0, s>>>(w.ls, w.big_list, w.acc, w.mom);
+    for (int c = 0; c < 4; ++c) count_launch();
+  }
+  KDS_CK(cudaGetLastError());
+  return KDS_OK;
 }
 
 }  // namespace
@@ -2301,9 +2396,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   double* h_dbl = reinterpret_cast<double*>(stage + st_ls + st_cnt);
   int32_t host_max = max_size;
   const int cb = std::min<int>(w.chunk_cap, kGridBlocks * 2);
-  // blocks that take a contiguous range of chunks each: one resident wave, so that no block
-  // starts when the others are done
-  const int sb = std::min<int>(w.chunk_cap, 148 * kScatterPerSM);
+  const int sb = scatter_blocks(w);
   // Grids of the level kernels sized to the level: a level has at most twice the nodes
   // of the one before, and the host learns the current level's size at each sync.  The
   // node-range kernels (k_decide, k_level_children, k_big_plan) share
@@ -2314,15 +2407,16 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   hls.le = R;
   hls.depth = 0;
   for (int round = 0; round < kMaxDepth; ++round) {
-    if (host_max <= kDeepMax && level_nodes <= kDeepMaxRoots) {
-      // every node of the current level fits one block: the rest of every subtree is
-      // built in shared memory, then the host reads the final level state
+    const bool by_block = host_max <= kBlockMax && level_nodes <= kBlockRoots;
+    if (by_block || (host_max <= kDeepMax && level_nodes <= kDeepMaxRoots)) {
+      // every node of the current level fits one group's shared memory: the rest of every
+      // subtree is built there, then the host reads the final level state
       if (round == 0) {  // the roots' sums (every root has at most kBig points)
-        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
-        count_launch();
+        rc = root_sums(w, R, host_max, N, s);
+        if (rc) return rc;
       }
       global_levels = hls.depth;
-      rc = deep_pass(w, P, hls, s);
+      rc = by_block ? deep_pass<16>(w, P, hls, s) : deep_pass<1>(w, P, hls, s);
       if (rc) return rc;
       KDS_CK(cudaMemcpyAsync(&hls, w.ls, sizeof(LevelState), cudaMemcpyDeviceToHost, s));
       KDS_CK(cudaStreamSynchronize(s));
@@ -2330,30 +2424,28 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       if (hls.error == 1) { set_error("kds_tree_build: node capacity exceeded"); return KDS_ERR_CAPACITY; }
       break;
     }
-    // sync after every level once the subtree pass is within reach: the largest node within
-    // a few halvings of kDeepMax and the level small enough (nodes at most double per level)
-    const int nlev = (host_max <= 4 * kDeepMax && level_nodes * 4 <= kDeepMaxRoots) ? 1 : kLevelsPerSync;
+    // as many levels to the next look at the level state as halvings still separate the
+    // largest node from a subtree pass that the level is small enough for (nodes at most
+    // double per level), one at a time once it is near
+    int nlev = kLevelsPerSync;
+    for (int k = 1; k <= kLevelsPerSync; ++k) {
+      const bool block_near = (host_max >> k) <= kBlockMax && (level_nodes << k) <= kBlockRoots;
+      const bool warp_near = (host_max >> k) <= 2 * kDeepMax && (level_nodes << (k + 1)) <= kDeepMaxRoots;
+      if (block_near || warp_near) {
+        nlev = k;
+        break;
+      }
+    }
     for (int k = 0; k < nlev; ++k) {
       const bool level0 = round == 0 && k == 0;
       const int64_t nodes_bound = level_nodes << k;
-      const int lvl_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(kLevelBlocks, (nodes_bound + kThreads - 1) / kThreads));
+      const int lvl_blocks = level_blocks(nodes_bound);
       const int small_blocks =
           (int)std::max<int64_t>(1, std::min<int64_t>(kSmallBlocks, (nodes_bound + kThreads / 32 - 1) / (kThreads / 32)));
-      // blocks per node range that write its chunks: a thread each for a few thousand chunks
-      // (one block takes 25 us for 11,000), none but the level's own where those do
-      const int plan_parts = lvl_blocks == 1 ? (int)std::max<int64_t>(1, std::min<int64_t>(64, N / (4096 * kChunk / 4)))
-                                             : 1;
-      if (level0) {  // the roots' sums
-        k_root_moments<<<kGridBlocks, kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
-        count_launch();
-        if (host_max > kBig) {
-          k_big_sums<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig);
-          k_big_plan<<<lvl_blocks * plan_parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
-                                                                  w.big_list, w.node_chunk0, w.acc, w.accl, plan_parts);
-          k_big_moments<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.acc);
-          k_big_to_mom<<<64, 256, 0, s>>>(w.ls, w.big_list, w.acc, w.mom);
-          for (int c = 0; c < 4; ++c) count_launch();
-        }
+      const int plan_parts = lvl_blocks == 1 ? chunk_parts(N) : 1;
+      if (level0) {
+        rc = root_sums(w, R, host_max, N, s);
+        if (rc) return rc;
       }
       const bool big = host_max > kBig;  // the large-node kernels run after the partition
       if (lvl_blocks == 1) {

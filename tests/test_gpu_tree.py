@@ -257,3 +257,33 @@ def test_stamp_prefix_tiles(scene, n):
     for (x, s), T in zip(clouds, kds.TreeGeneratorB2003D(leaf_max_points=16).make_trees(clouds)):
         assert_same_tree(orc.OTree.build(x, s, orc.tree_params(leaf_max_points=16)), T)
     assert_same_tree(*build_both(xyz[:n], st[:n], leaf_max_points=16))
+
+
+@pytest.mark.parametrize("n,params", [
+    (255, {}), (256, {}), (257, {}), (1024, {}), (2047, {}), (2048, {}), (2049, {}), (4097, {}),
+    (2048, dict(leaf_max_points=3, leaf_min_points=3, leaf_density=1e9, tree_min_good_leaves=1)),
+    (2048, dict(leaf_max_points=16, propagate_normal=1, max_level=5, tree_min_good_leaves=1)),
+])
+def test_subtree_pass_sizes(scene, n, params):
+    """Clouds at the edges of the shared-memory subtree passes (256 and 2,048 points), down to
+    leaves of three points (the most nodes per depth) and with a level limit inside the pass."""
+    xyz, st = make_scan(scene, 2470, beams=64, elev=(-22.5, 22.5), vel=[5.0, 0, 0, 0, 0, 0.1])
+    k = np.sort(np.random.default_rng(n).choice(len(xyz), n, replace=False))
+    prm = dict(dict(leaf_max_points=16, tree_min_good_leaves=1), **params)
+    O, G = build_both(np.ascontiguousarray(xyz[k]), np.ascontiguousarray(st[k]), **prm)
+    assert_same_tree(O, G)
+
+
+@pytest.mark.parametrize("clouds", [295, 296, 297, 330])
+def test_subtree_pass_roots(scene, clouds):
+    """Forests at the edge of the block form's number of subtrees (296)."""
+    import kd_slam2_b200 as kds
+    xyz, st = make_scan(scene, 2471, beams=32)
+    rng = np.random.default_rng(clouds)
+    cs = []
+    for i in range(clouds):
+        k = np.sort(rng.choice(len(xyz), int(rng.integers(300, 1200)), replace=False))
+        cs.append((np.ascontiguousarray(xyz[k]), np.ascontiguousarray(st[k])))
+    prm = dict(leaf_max_points=16, tree_min_good_leaves=1)
+    for (x, s), T in zip(cs, kds.TreeGeneratorB2003D(**prm).make_trees(cs)):
+        assert_same_tree(orc.OTree.build(x, s, orc.tree_params(**prm)), T)
