@@ -430,17 +430,23 @@ __device__ __forceinline__ double ddot3(const double* a, const double* b) {
 }
 
 // Cyclic Jacobi eigensolver for a symmetric 3x3 (Golub & Van Loan, sec. 8.5), fixed
-// 8 sweeps; eigenvalues ascending, eigenvectors as columns of V.
-__device__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
+// 8 sweeps; eigenvalues ascending, eigenvectors as columns of V.  Every index is a constant
+// once the loops are unrolled, so the matrices stay in registers: with them in local memory a
+// decision took 7 us at the least, DECIDENOTE.
+__device__ __forceinline__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
   double a[3][3];
+#pragma unroll
   for (int i = 0; i < 3; ++i)
+#pragma unroll
     for (int j = 0; j < 3; ++j) { a[i][j] = Ain[i][j]; V[i][j] = (i == j) ? 1.0 : 0.0; }
+#pragma unroll 1
   for (int sweep = 0; sweep < 8; ++sweep) {
     if (a[0][1] == 0.0 && a[0][2] == 0.0 && a[1][2] == 0.0) break;
+#pragma unroll
     for (int pq = 0; pq < 3; ++pq) {
-      int p = (pq == 2) ? 1 : 0;
-      int q = (pq == 0) ? 1 : 2;
-      int r = 3 - p - q;
+      const int p = (pq == 2) ? 1 : 0;
+      const int q = (pq == 0) ? 1 : 2;
+      const int r = 3 - p - q;
       double apq = a[p][q];
       // negligible off-diagonal: set to zero (same rule in the CPU oracle)
       if (fabs(apq) <= 1e-18 * (fabs(a[p][p]) + fabs(a[q][q]))) {
@@ -462,6 +468,7 @@ __device__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
       double nrq = s * arp + c * arq;
       a[r][p] = nrp; a[p][r] = nrp;
       a[r][q] = nrq; a[q][r] = nrq;
+#pragma unroll
       for (int k = 0; k < 3; ++k) {
         double vkp = V[k][p], vkq = V[k][q];
         V[k][p] = c * vkp - s * vkq;
@@ -469,21 +476,23 @@ __device__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
       }
     }
   }
-  double d[3] = {a[0][0], a[1][1], a[2][2]};
-  int idx[3] = {0, 1, 2};
-  for (int i = 1; i < 3; ++i) {
-    int k = idx[i];
-    int j = i - 1;
-    while (j >= 0 && d[k] < d[idx[j]]) { idx[j + 1] = idx[j]; --j; }
-    idx[j + 1] = k;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) ev[i] = a[i][i];
+  // stable: neighbours change places only where the right one is strictly smaller
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int i = k & 1;
+    const bool sw = ev[i + 1] < ev[i];
+    const double lo = sw ? ev[i + 1] : ev[i], hi = sw ? ev[i] : ev[i + 1];
+    ev[i] = lo;
+    ev[i + 1] = hi;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double vl = sw ? V[j][i + 1] : V[j][i], vh = sw ? V[j][i] : V[j][i + 1];
+      V[j][i] = vl;
+      V[j][i + 1] = vh;
+    }
   }
-  double Vs[3][3];
-  for (int c2 = 0; c2 < 3; ++c2) {
-    ev[c2] = d[idx[c2]];
-    for (int r2 = 0; r2 < 3; ++r2) Vs[r2][c2] = V[r2][idx[c2]];
-  }
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) V[i][j] = Vs[i][j];
 }
 
 // FlatLeafPolicy_::fillMetadata over CountLeafPolicy_ and LabelPolicyBase_
@@ -494,16 +503,35 @@ __device__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
 // (kd/tree/tree_cpu_.h:72-86): [0..2] eigenvalues ascending, [3..11] eigenvectors
 // column-major (columns 0 and 2 reoriented as in fillMetadata, then column 0 negated if
 // the determinant is negative), [12..14] mean; zero where the node has < 3 points.
-__device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, const BuildParams& P, double* root) {
-  for (int i = 0; i < 3; ++i) { nd.mean[i] = 0.f; nd.dir[i] = 0.f; }
+struct Decision {
+  float mean[3], dir[3];
+  double prop[3];  // normal handed to the children
+  bool has_prop;
+  bool split;
+};
+__device__ __forceinline__ void flip_to_origin(const double* mean, double* e) {
+  if (ddot3(mean, e) > 0.0) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) e[i] = -e[i];
+  }
+}
+// par_has, par_prop: the normal that the parent handed down, if any (never for a root).
+__device__ __forceinline__ Decision decide(const double* Sd, int64_t n, bool par_has, const double* par_prop, int level,
+                                           const BuildParams& P, double* root) {
+  Decision nd;
   double mean_d[3] = {0, 0, 0};
   double e0[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
   double lam[3] = {0, 0, 0};
   bool is_bad = true;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) { nd.mean[i] = 0.f; nd.dir[i] = 0.f; nd.prop[i] = 0.0; }
   if (n > 0) {
     double dn = (double)n;
-    for (int i = 0; i < 3; ++i) mean_d[i] = Sd[6 + i] / dn;
-    for (int i = 0; i < 3; ++i) nd.mean[i] = (float)mean_d[i];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      mean_d[i] = Sd[6 + i] / dn;
+      nd.mean[i] = (float)mean_d[i];
+    }
     if (n >= 3) {
       double C[3][3];
       C[0][0] = Sd[0] / dn - mean_d[0] * mean_d[0];
@@ -517,9 +545,10 @@ __device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, cons
       C[2][1] = C[1][2];
       double V[3][3];
       jacobi3(C, lam, V);
+#pragma unroll
       for (int i = 0; i < 3; ++i) { e0[i] = V[i][0]; e2[i] = V[i][2]; }
-      if (ddot3(mean_d, e0) > 0.0) for (int i = 0; i < 3; ++i) e0[i] = -e0[i];
-      if (ddot3(mean_d, e2) > 0.0) for (int i = 0; i < 3; ++i) e2[i] = -e2[i];
+      flip_to_origin(mean_d, e0);
+      flip_to_origin(mean_d, e2);
       is_bad = false;
       if (root) {
         const double e1[3] = {V[0][1], V[1][1], V[2][1]};
@@ -529,6 +558,7 @@ __device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, cons
         const double cz = e1[0] * e2[1] - e1[1] * e2[0];
         const double det = e0[0] * cx + (e0[1] * cy + e0[2] * cz);
         const double sg = det < 0.0 ? -1.0 : 1.0;
+#pragma unroll
         for (int i = 0; i < 3; ++i) {
           root[i] = lam[i];
           root[3 + i] = sg * e0[i];
@@ -541,23 +571,17 @@ __device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, cons
   if (root) {
     if (is_bad)
       for (int i = 0; i < 12; ++i) root[i] = 0.0;
+#pragma unroll
     for (int i = 0; i < 3; ++i) root[12 + i] = mean_d[i];
   }
-  bool is_node = false, is_leaf = false;
-  if (is_bad) {
-    is_leaf = true;
-  } else if ((float)n > (float)P.leaf_max_points) {
-    is_node = true;
-    for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e2[i];
-  } else {
-    is_leaf = true;
-    for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e0[i];
-  }
-  bool has_prop = false;
+  // 0: no direction, 1: e0, 2: e2, 3: the normal handed down
+  bool is_node = !is_bad && (float)n > (float)P.leaf_max_points;
+  int dir = is_bad ? 0 : (is_node ? 2 : 1);
+  bool has_prop = P.propagate_normal && par_has;
   double prop[3] = {0, 0, 0};
-  if (nd.has_parent && P.propagate_normal) {
-    has_prop = nd.par_has != 0;
-    for (int i = 0; i < 3; ++i) prop[i] = nd.par_prop[i];
+  if (P.propagate_normal) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) prop[i] = par_prop[i];
   }
   bool is_flat = false;
   bool do_prop = false;
@@ -569,45 +593,39 @@ __device__ __noinline__ void decide(const double* Sd, int64_t n, BNode& nd, cons
               fabs(ddot3(mean_d, e0)) > (double)P.leaf_min_normal_incidence;
     if (is_flat) {
       has_prop = true;
+#pragma unroll
       for (int i = 0; i < 3; ++i) prop[i] = e0[i];
     }
     if (!is_node) {
       double volume = lam[1] * lam[2];
       double density = (double)n / volume;
       if (density < (double)P.leaf_density) {
-        is_leaf = false;
         is_node = true;
-        for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e2[i];
-      } else if (is_leaf && is_flat) {
-        for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e0[i];
+        dir = 2;
+      } else if (is_flat) {
+        dir = 1;
       } else {
         do_prop = true;
       }
     }
   }
-  if (do_prop) {
-    is_leaf = true;
-    if (has_prop) {
-      double d[3] = {prop[0], prop[1], prop[2]};
-      if (ddot3(mean_d, d) > 0.0) for (int i = 0; i < 3; ++i) d[i] = -d[i];
-      for (int i = 0; i < 3; ++i) nd.dir[i] = (float)d[i];
-    }
-  }
-  if (is_node && nd.level >= P.max_level - 1) {
+  if (do_prop && has_prop) dir = 3;
+  if (is_node && level >= P.max_level - 1) {
     is_node = false;
-    if (is_flat) {
-      for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e0[i];
-    } else if (has_prop) {
-      double d[3] = {prop[0], prop[1], prop[2]};
-      if (ddot3(mean_d, d) > 0.0) for (int i = 0; i < 3; ++i) d[i] = -d[i];
-      for (int i = 0; i < 3; ++i) nd.dir[i] = (float)d[i];
-    } else {
-      for (int i = 0; i < 3; ++i) nd.dir[i] = (float)e0[i];
-    }
+    dir = is_flat ? 1 : (has_prop ? 3 : 1);
   }
-  nd.split = is_node ? 1 : 0;
-  nd.has_prop = has_prop ? 1 : 0;
-  for (int i = 0; i < 3; ++i) nd.prop[i] = prop[i];
+  double d[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) d[i] = dir == 3 ? prop[i] : (dir == 2 ? e2[i] : (dir == 1 ? e0[i] : 0.0));
+  if (dir == 3) flip_to_origin(mean_d, d);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    nd.dir[i] = (float)d[i];
+    nd.prop[i] = prop[i];
+  }
+  nd.split = is_node;
+  nd.has_prop = has_prop;
+  return nd;
 }
 
 __device__ __forceinline__ bool which_side_f(const float* mean, const float* dir, float4 q) {
@@ -804,22 +822,33 @@ __device__ __forceinline__ void level_decide(BNode* nodes, const LevelState* ls,
   const int depth = ls->depth;
   int v = 0, nc = 0, nb = 0;
   for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
-    BNode nd = nodes[i];
+    BNode& nd = nodes[i];
     const int n = nd.end - nd.start;
     double Sd[kSums];
     const PendingSums r = pending_sums(nodes, mom, C, depth, i, nd.parent);
     if (r.q) {
+#pragma unroll
       for (int k = 0; k < kSums; ++k) {
         const U128 q = pending_value(r, k);
         mom[(size_t)i * kSums + k] = q;
         Sd[k] = fx_to_d(q);
       }
     } else {
+#pragma unroll
       for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(mom[(size_t)i * kSums + k]);
     }
-    decide(Sd, n, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
-    nodes[i] = nd;
-    v += nd.split ? 1 : 0;
+    const double pp[3] = {nd.par_prop[0], nd.par_prop[1], nd.par_prop[2]};
+    const Decision q = decide(Sd, n, nd.has_parent && nd.par_has, pp, nd.level, P,
+                              depth == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      nd.mean[k] = q.mean[k];
+      nd.dir[k] = q.dir[k];
+      nd.prop[k] = q.prop[k];
+    }
+    nd.split = q.split ? 1 : 0;
+    nd.has_prop = q.has_prop ? 1 : 0;
+    v += q.split ? 1 : 0;
     if (n > kBig) {
       nc += (n + kChunk - 1) / kChunk;
       nb += 1;
@@ -1559,46 +1588,52 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
       for (int r = tid; r < cnt; r += kThreadsG) {
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
-        BNode nd;
+        double pp[3];
+        bool ph;
         if (d == 0) {
-          nd = root;
+          ph = root.has_parent && root.par_has;
+          for (int k = 0; k < 3; ++k) pp[k] = root.par_prop[k];
+        } else if (d == 1) {  // the root's decision, written at depth 0
+          ph = nodes[R].has_prop != 0;
+          for (int k = 0; k < 3; ++k) pp[k] = nodes[R].prop[k];
         } else {
-          memset(&nd, 0, sizeof(nd));
-          nd.level = root.level + d;
-          nd.tree = root.tree;
-          nd.has_parent = 1;
-          if (d == 1) {  // the root's decision, written at depth 0
-            for (int k = 0; k < 3; ++k) nd.par_prop[k] = nodes[R].prop[k];
-            nd.par_has = nodes[R].has_prop;
-          } else {
-            const DeepNode& pn = dn[base_prev + S.prank[c][r]];
-            nd.par_has = pn.has_prop;
-            for (int k = 0; k < 3; ++k) nd.par_prop[k] = pn.prop[k];
-          }
+          const DeepNode& pn = dn[base_prev + S.prank[c][r]];
+          ph = pn.has_prop != 0;
+          for (int k = 0; k < 3; ++k) pp[k] = pn.prop[k];
         }
         double Sd[kSums];
         const U128* ms = psums + (size_t)r * kSums;
+#pragma unroll
         for (int k = 0; k < kSums; ++k) Sd[k] = fx_to_d(ms[k]);
-        decide(Sd, en - st, nd, P, nd.level == 0 ? root_frame + (size_t)nd.tree * kRootFrame : nullptr);
-        S.split[r] = nd.split ? 1 : 0;
-        if (d == 0) {
-          nodes[R] = nd;  // left / right follow in k_deep_place
-        } else {
-          DeepNode x;
+        const Decision x = decide(Sd, en - st, ph, pp, root.level + d, P,
+                                  root.level + d == 0 ? root_frame + (size_t)root.tree * kRootFrame : nullptr);
+        S.split[r] = x.split ? 1 : 0;
+        if (d == 0) {  // left / right follow in k_deep_place
+          BNode& o = nodes[R];
+#pragma unroll
           for (int k = 0; k < 3; ++k) {
-            x.mean[k] = nd.mean[k];
-            x.dir[k] = nd.dir[k];
-            x.prop[k] = nd.prop[k];
+            o.mean[k] = x.mean[k];
+            o.dir[k] = x.dir[k];
+            o.prop[k] = x.prop[k];
           }
-          x.start = st;
-          x.end = en;
-          x.sub = sub;
-          x.depth = d;
-          x.rank = r;
-          x.q = -1;
-          x.parent_rank = S.prank[c][r];
-          x.has_prop = nd.has_prop;
-          dn[base + r] = x;
+          o.split = x.split ? 1 : 0;
+          o.has_prop = x.has_prop ? 1 : 0;
+        } else {
+          DeepNode& o = dn[base + r];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            o.mean[k] = x.mean[k];
+            o.dir[k] = x.dir[k];
+            o.prop[k] = x.prop[k];
+          }
+          o.start = st;
+          o.end = en;
+          o.sub = sub;
+          o.depth = d;
+          o.rank = r;
+          o.q = -1;
+          o.parent_rank = S.prank[c][r];
+          o.has_prop = x.has_prop ? 1 : 0;
         }
       }
       sync();
