@@ -383,7 +383,7 @@ __device__ __forceinline__ void lane_fold(LaneSums& S, int lane) {
 }
 
 // ---------------------------------------------------------------------------
-struct BNode {
+struct __align__(16) BNode {
   int32_t start, end;
   int32_t level;
   int32_t tree;
@@ -431,8 +431,8 @@ __device__ __forceinline__ double ddot3(const double* a, const double* b) {
 
 // Cyclic Jacobi eigensolver for a symmetric 3x3 (Golub & Van Loan, sec. 8.5), fixed
 // 8 sweeps; eigenvalues ascending, eigenvectors as columns of V.  Every index is a constant
-// once the loops are unrolled, so the matrices stay in registers: with them in local memory a
-// decision took 7 us at the least, DECIDENOTE.
+// once the loops are unrolled, so the matrices stay in registers: with them in local memory
+// the decisions of a level of 500,000 nodes took 200 us, now 132.
 __device__ __forceinline__ void jacobi3(const double Ain[3][3], double ev[3], double V[3][3]) {
   double a[3][3];
 #pragma unroll
@@ -1395,7 +1395,11 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
 
 // ---- children ------------------------------------------------------------------------
 
+// Numbers the level's children and writes their records, eight lanes a record (16 B each), so
+// that a warp's store is 512 B in a row (a thread per parent writing both of its children's
+// records took 100 us for a level of 500,000 nodes, now 63).
 __device__ __forceinline__ void level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap, int* sm) {
+  __shared__ int s_list[kThreads];  // split nodes of the batch, in order
   int b, e;
   level_range(ls, b, e);
   const int le = ls->le;
@@ -1405,45 +1409,56 @@ __device__ __forceinline__ void level_children(BNode* nodes, LevelState* ls, con
     for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) v += bsum[k];
     block_scan(v, sm, &pre);
   }
-  int carry = 0;
+  int first = le + 2 * pre;  // index of the batch's first child
   for (int base = b; base < e; base += blockDim.x) {
-    int i = base + threadIdx.x;
+    const int i = base + threadIdx.x;
     bool sp = (i < e) && nodes[i].split;
     int tot;
-    int r = block_scan(sp ? 1 : 0, sm, &tot) + carry + pre;
-    carry += tot;
+    const int r = block_scan(sp ? 1 : 0, sm, &tot);
     if (i < e) {
       BNode& nd = nodes[i];
-      if (!sp) {
-        nd.left = -1;
-        nd.right = -1;
-      } else {
-        int li = le + 2 * r;
-        if (li + 1 >= cap) {
-          ls->error = 1;
-          nd.split = 0;
-          nd.left = nd.right = -1;
-        } else {
-          nd.left = li;
-          nd.right = li + 1;
-          for (int k = 0; k < 2; ++k) {
-            BNode c;
-            memset(&c, 0, sizeof(c));  // start/end: set by the partition
-            c.level = nd.level + 1;
-            c.tree = nd.tree;
-            c.left = c.right = -1;
-            c.parent = i;
-            c.has_parent = 1;
-            c.par_has = nd.has_prop;
-            for (int j = 0; j < 3; ++j) c.par_prop[j] = nd.prop[j];
-            nodes[li + k] = c;
-          }
-        }
+      const int li = first + 2 * r;
+      if (sp && li + 1 >= cap) {
+        ls->error = 1;
+        nd.split = 0;
+        sp = false;
       }
+      nd.left = sp ? li : -1;
+      nd.right = sp ? li + 1 : -1;
+      if (sp) s_list[r] = i;
     }
+    __syncthreads();
+    const int room = min(2 * tot, max(0, (cap - first) & ~1));  // children that fit (all, or the build fails)
+    for (int k = threadIdx.x; k < room * 8; k += blockDim.x) {
+      const int child = k >> 3, word = k & 7;
+      const int par = s_list[child >> 1];
+      const BNode& nd = nodes[par];
+      int4 w = make_int4(0, 0, 0, 0);  // start and end: set by the partition
+      if (word == 0) {
+        w.z = nd.level + 1;
+        w.w = nd.tree;
+      } else if (word == 1) {
+        w.z = w.w = -1;  // left, right
+      } else if (word == 2) {
+        w = make_int4(1, nd.has_prop, 0, par);  // has_parent, par_has, has_prop, parent
+      } else if (word == 6) {
+        const long long p0 = __double_as_longlong(nd.prop[0]);
+        w.z = (int)p0;
+        w.w = (int)(p0 >> 32);
+      } else if (word == 7) {
+        const long long p1 = __double_as_longlong(nd.prop[1]), p2 = __double_as_longlong(nd.prop[2]);
+        w = make_int4((int)p1, (int)(p1 >> 32), (int)p2, (int)(p2 >> 32));
+      }
+      reinterpret_cast<int4*>(nodes + first + child)[word] = w;
+    }
+    first += 2 * tot;
+    __syncthreads();  // the list may be rewritten after this
   }
 }
-
+static_assert(offsetof(BNode, level) == 8 && offsetof(BNode, tree) == 12 && offsetof(BNode, left) == 24 &&
+                  offsetof(BNode, right) == 28 && offsetof(BNode, has_parent) == 32 && offsetof(BNode, par_has) == 36 &&
+                  offsetof(BNode, has_prop) == 40 && offsetof(BNode, parent) == 44 && offsetof(BNode, par_prop) == 104,
+              "BNode words as level_children writes them");
 __global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap) {
   __shared__ int sm[32];
   level_children(nodes, ls, bsum, cap, sm);
@@ -1481,8 +1496,8 @@ __global__ void __launch_bounds__(kThreads) k_level_small(BNode* nodes, LevelSta
 // Two forms, both for levels that leave most of the machine idle, where a level costs its
 // launches and the chain of one decision however few nodes it has:
 //  * a block of 16 warps per subtree of at most 2,048 points, while the level has at most
-//    kBlockRoots of them: a 12,000-point scan leaves the level kernels after 3 levels, a
-//    180,000-point one after 8 (DEEPNOTE);
+//    kBlockRoots of them: a 12,000-point scan leaves the level kernels after 4 levels (of
+//    45 us each) for 91 us here, a 180,000-point one after 8 for 149;
 //  * a warp per subtree of at most 256 points, up to 8,192 of them.
 // For large forests (hundreds of thousands of tiny subtrees, where a decision runs on a few
 // lanes) the level kernels, with a thread per node of the whole level, are faster: the warp
@@ -1528,6 +1543,7 @@ struct DeepSmem {                             // one group's
   int32_t list[deep_nodes<WARPS>()];          // q -> rank of the q-th split node of the depth
   int32_t scan[32];
   int32_t base, pad_[3];
+  U128 part[WARPS][kSums + 1];                // a node's warps: their sums; [kSums].lo: left points
   uint8_t split[deep_nodes<WARPS>()];
 };
 
@@ -1672,8 +1688,81 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
         for (int i = st; i < en; ++i) B.perm[pbase + i] = __float_as_int(S.pts[c][i].w);
       }
-      // ---- partition of the split nodes, a warp per node
-      for (int q = warp; q < nsplit; q += WARPS) {
+      // ---- partition of the split nodes: several warps per node while there are fewer nodes
+      // than warps (one warp takes 20 us for a node of 2,000 points) ...
+      int team = 1;  // warps per node
+      for (int k = WARPS; k > 1 && nsplit > 0; k /= 2)
+        if (2 * team * nsplit <= WARPS) team *= 2;
+      if (team > 1) {
+        const int q = warp / team, m = warp % team;
+        const bool on = q < nsplit;
+        int st = 0, en = 0, b = 0, e = 0, r = 0;
+        float mean[3], dir[3];
+        if (on) {
+          r = S.list[q];
+          const uint32_t rg = S.range[c][r];
+          st = (int)(rg & 0xffffu);
+          en = (int)(rg >> 16);
+          const int per = (en - st + 32 * team - 1) / (32 * team) * 32;
+          b = min(st + m * per, en);
+          e = min(b + per, en);
+          const float* pm = d == 0 ? nodes[R].mean : dn[base + r].mean;
+          const float* pd = d == 0 ? nodes[R].dir : dn[base + r].dir;
+          for (int k = 0; k < 3; ++k) { mean[k] = pm[k]; dir[k] = pd[k]; }
+          int nl = 0;
+          for (int k0 = b; k0 < e; k0 += 32) {
+            const int i = k0 + lane;
+            nl += __popc(__ballot_sync(full, i < e && which_side_f(mean, dir, S.pts[c][i])));
+          }
+          if (lane == 0) S.part[warp][kSums].lo = (unsigned long long)nl;
+        }
+        sync();
+        int mid = st, lo = st;
+        if (on) {
+          for (int k = 0; k < team; ++k) {
+            const int nl = (int)S.part[q * team + k][kSums].lo;
+            mid += nl;
+            if (k < m) lo += nl;
+          }
+          int ro = mid + (b - st) - (lo - st);
+          const bool small_left = mid - st <= en - mid;
+          for (int k0 = b; k0 < e; k0 += 32) {
+            const int i = k0 + lane;
+            const bool valid = i < e;
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (valid) p = S.pts[c][i];
+            const bool left = valid && which_side_f(mean, dir, p);
+            const unsigned bl = __ballot_sync(full, left), br = __ballot_sync(full, valid && !left);
+            if (valid) S.pts[c ^ 1][left ? lo + __popc(bl & lt) : ro + __popc(br & lt)] = p;
+            sums_add(W, sg, valid && left == small_left, p, lane);
+            sums_room(W, sg, kStage - 32, lane);
+            lo += __popc(bl);
+            ro += __popc(br);
+          }
+          const U128 qs = sums_total(W, sg, lane);
+          if (lane < kSums) S.part[warp][lane] = qs;
+        }
+        sync();
+        if (on && m == 0) {
+          const bool small_left = mid - st <= en - mid;
+          if (lane < kSums) {
+            U128 qs = u128_zero();
+            for (int k = 0; k < team; ++k) qs = u128_add(qs, S.part[warp + k][lane]);
+            const U128 other = u128_sub(psums[(size_t)r * kSums + lane], qs);
+            U128* nxt = myring + (size_t)((d + 1) & 1) * kNodes * kSums;
+            nxt[(size_t)(2 * q) * kSums + lane] = small_left ? qs : other;
+            nxt[(size_t)(2 * q + 1) * kSums + lane] = small_left ? other : qs;
+          }
+          if (lane == 0) {
+            S.range[c ^ 1][2 * q] = (uint32_t)st | ((uint32_t)mid << 16);
+            S.range[c ^ 1][2 * q + 1] = (uint32_t)mid | ((uint32_t)en << 16);
+            S.prank[c ^ 1][2 * q] = r;
+            S.prank[c ^ 1][2 * q + 1] = r;
+          }
+        }
+      }
+      // ... a warp per node then
+      for (int q = team > 1 ? nsplit : warp; q < nsplit; q += WARPS) {
         const int r = S.list[q];
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
