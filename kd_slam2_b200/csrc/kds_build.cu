@@ -690,15 +690,16 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k) {
   return __longlong_as_double((long long)b);
 }
 
-// ts_start of each tree = min stamp (label_policy_base_impl_.h:28-35); blockIdx.y = tree.
+// ts_start of each tree = min stamp (label_policy_base_impl_.h:28-35), as the largest
+// complement of its key (tsmin starts at 0); blockIdx.y = tree.
 __global__ void k_tree_min(const double* sts, const int64_t* off, unsigned long long* tsmin) {
   const int r = blockIdx.y;
   const int64_t b = off[r], e = off[r + 1];
-  unsigned long long m = ~0ull;
+  unsigned long long m = 0ull;
   for (int64_t i = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e; i += (int64_t)gridDim.x * blockDim.x)
-    m = min(m, dkey(sts[i]));
-  for (int off2 = 16; off2 > 0; off2 >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, off2));
-  if ((threadIdx.x & 31) == 0 && m != ~0ull) atomicMin(&tsmin[r], m);
+    m = max(m, ~dkey(sts[i]));
+  for (int off2 = 16; off2 > 0; off2 >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off2));
+  if ((threadIdx.x & 31) == 0 && m != 0ull) atomicMax(&tsmin[r], m);
 }
 
 // decodes ts_start, checks every point's stamp and writes its dt; blockIdx.y = tree.
@@ -706,7 +707,7 @@ __global__ void k_tree_check(const double* sts, const int64_t* off, const unsign
                              double* dt, LevelState* ls) {
   const int r = blockIdx.y;
   const int64_t b = off[r], e = off[r + 1];
-  const double t0 = (e > b) ? dkey_inv(tsmin[r]) : 0.0;
+  const double t0 = (e > b) ? dkey_inv(~tsmin[r]) : 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) ts0[r] = t0;
   for (int64_t i = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e; i += (int64_t)gridDim.x * blockDim.x) {
     const double s = sts[i];
@@ -1952,8 +1953,9 @@ __global__ void k_alive(const BNode* nodes, int32_t total, int32_t* alive, float
 // group = (level, tree); nodes of one group are contiguous in global order
 // Counts per (level, tree) group; lanes with the same group combine their counts
 // before one atomic per group and warp.
+// flags[i]: x = alive, y = alive leaf.
 __global__ void k_group_counts(const BNode* nodes, int32_t total, const int32_t* alive, int R, int32_t* cnt,
-                               int32_t* lcnt, int32_t* ucnt, int32_t* leaf_flag) {
+                               int32_t* lcnt, int32_t* ucnt, int2* flags) {
   const int lane = threadIdx.x & 31;
   for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
@@ -1966,7 +1968,7 @@ __global__ void k_group_counts(const BNode* nodes, int32_t total, const int32_t*
       g = nd.level * R + nd.tree;
       al = alive[i] != 0;
       leaf = al && nd.left < 0 && nd.right < 0;
-      leaf_flag[i] = leaf ? 1 : 0;
+      flags[i] = make_int2(al ? 1 : 0, leaf ? 1 : 0);
     }
     const unsigned pt = __match_any_sync(0xffffffffu, tree);
     if (valid && lane == __ffs(pt) - 1) atomicAdd(&ucnt[tree], __popc(pt));
@@ -1978,6 +1980,54 @@ __global__ void k_group_counts(const BNode* nodes, int32_t total, const int32_t*
       if (c) atomicAdd(&cnt[g], c);
       if (lc) atomicAdd(&lcnt[g], lc);
     }
+  }
+}
+
+// Exclusive scan of the flag pairs (both at once), in place: tiles of kFlagTile pairs, their
+// sums by one block, then the prefixes; a single block does it all for small trees.
+constexpr int kFlagItems = 4;
+constexpr int kFlagTile = 1024 * kFlagItems;
+constexpr int kFlagOne = 32768;  // pairs that one block scans by itself
+__device__ __forceinline__ int2 pair_add(int2 a, int2 b) { return make_int2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ int2 pair_block_scan(int2 v, int* sm, int2* total) {
+  int2 r;
+  r.x = block_scan(v.x, sm, &total->x);
+  r.y = block_scan(v.y, sm, &total->y);
+  return r;
+}
+__global__ void __launch_bounds__(1024) k_flag_tiles(const int2* flags, int32_t n, int2* tiles) {
+  __shared__ int sm[32];
+  const int base = blockIdx.x * kFlagTile + threadIdx.x * kFlagItems;
+  int2 v = make_int2(0, 0), tot;
+  for (int k = 0; k < kFlagItems; ++k)
+    if (base + k < n) v = pair_add(v, flags[base + k]);
+  pair_block_scan(v, sm, &tot);
+  if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
+}
+__global__ void __launch_bounds__(1024) k_flag_top(int2* tiles, int32_t nt) {
+  __shared__ int sm[32];
+  int2 carry = make_int2(0, 0);
+  for (int b = 0; b < nt; b += blockDim.x) {
+    const int i = b + threadIdx.x;
+    int2 tot;
+    const int2 ex = pair_block_scan(i < nt ? tiles[i] : make_int2(0, 0), sm, &tot);
+    if (i < nt) tiles[i] = pair_add(carry, ex);
+    carry = pair_add(carry, tot);
+  }
+}
+// tiles == nullptr: one block, a run of pairs per thread.
+__global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, int32_t n, const int2* tiles) {
+  __shared__ int sm[32];
+  const int items = tiles ? kFlagItems : (n + 1023) / 1024;
+  const int b = min((int)(blockIdx.x * 1024 + threadIdx.x) * items, n), e = min(b + items, n);
+  int2 v = make_int2(0, 0), tot;
+  for (int i = b; i < e; ++i) v = pair_add(v, flags[i]);
+  int2 x = pair_block_scan(v, sm, &tot);
+  if (tiles) x = pair_add(x, tiles[blockIdx.x]);
+  for (int i = b; i < e; ++i) {
+    const int2 f = flags[i];
+    flags[i] = x;
+    x = pair_add(x, f);
   }
 }
 
@@ -2127,20 +2177,21 @@ __global__ void __launch_bounds__(kThreads) k_dt_prefix(const double* dt, const 
 }
 
 // pre: prefix sums of the stamps over the point order (nullptr: every dt is 0)
-__global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_t* alive, const int32_t* rank,
-                                 const int32_t* leaf_flag, const int32_t* lrank, int R, const int32_t* gp,
-                                 const int32_t* lgp, const int32_t* to, const int32_t* lto, const DtSum* pre,
-                                 TreeDev* trees) {
+// rank[i]: alive nodes and alive leaves before node i.
+__global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_t* alive, const int2* rank, int R,
+                                 const int32_t* gp, const int32_t* lgp, const int32_t* to, const int32_t* lto,
+                                 const DtSum* pre, const int64_t* off, TreeDev* trees) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (!alive[i]) continue;
     const BNode& nd = nodes[i];
     TreeDev& T = trees[nd.tree];
     if (T.nodes == nullptr) continue;  // rejected tree
     int g = nd.level * R + nd.tree;
-    int o = to[g] + (rank[i] - gp[g]);
+    const int2 rk = rank[i];
+    int o = to[g] + (rk.x - gp[g]);
     int gc = (nd.level + 1) * R + nd.tree;
-    int l = (nd.left >= 0 && alive[nd.left]) ? to[gc] + (rank[nd.left] - gp[gc]) : -1;
-    int r = (nd.right >= 0 && alive[nd.right]) ? to[gc] + (rank[nd.right] - gp[gc]) : -1;
+    int l = (nd.left >= 0 && alive[nd.left]) ? to[gc] + (rank[nd.left].x - gp[gc]) : -1;
+    int r = (nd.right >= 0 && alive[nd.right]) ? to[gc] + (rank[nd.right].x - gp[gc]) : -1;
     DNode d;
     d.a = make_float4(nd.mean[0], nd.mean[1], nd.mean[2], nd.dir[0]);
     d.b = make_float4(nd.dir[1], nd.dir[2], __int_as_float(l), __int_as_float(r));
@@ -2155,35 +2206,28 @@ __global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_
     T.dts_f[o] = (float)dts_mean;
     T.dts_mean[o] = dts_mean;
     T.dts_cov[o] = dts_cov;
-    int64_t base = nd.start;  // ranges are global; made tree-relative below
-    T.range[2 * o] = base;
-    T.range[2 * o + 1] = nd.end;
+    const int64_t o0 = off[nd.tree];  // ranges are global here
+    T.range[2 * o] = nd.start - o0;
+    T.range[2 * o + 1] = nd.end - o0;
     T.level[o] = nd.level;
-    if (leaf_flag[i]) T.leaf_idx[lto[g] + (lrank[i] - lgp[g])] = o;
+    if (nd.left < 0 && nd.right < 0) {
+      const int lf = lto[g] + (rk.y - lgp[g]);
+      T.leaf_idx[lf] = o;
+      T.leaf_md[lf] = make_float4(nd.mean[0], nd.mean[1], nd.mean[2], (float)dts_mean);
+      T.leaf_nrm[lf] = make_float4(nd.dir[0], nd.dir[1], nd.dir[2], 0.f);
+    }
   }
 }
 
-// tree-relative point ranges and point order; blockIdx.y = tree
+// tree-relative point order; blockIdx.y = tree
 __global__ void k_finish_trees(TreeDev* trees, const int64_t* off, const int32_t* perm_final) {
   const int r = blockIdx.y;
   TreeDev& T = trees[r];
   if (T.nodes == nullptr) return;
   const int64_t o0 = off[r];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.num_nodes;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    T.range[2 * i] -= o0;
-    T.range[2 * i + 1] -= o0;
-  }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.num_points;
        i += (int64_t)gridDim.x * blockDim.x)
     T.perm[i] = perm_final[o0 + i] - (int32_t)o0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.num_leaves;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int o = T.leaf_idx[i];
-    DNode d = T.nodes[o];
-    T.leaf_md[i] = make_float4(d.a.x, d.a.y, d.a.z, T.dts_f[o]);
-    T.leaf_nrm[i] = make_float4(d.a.w, d.b.x, d.b.y, 0.f);
-  }
 }
 
 inline int nblk(int64_t n, int t) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + t - 1) / t, 1 << 20)); }
@@ -2200,7 +2244,8 @@ struct BuildWs {
   void* block = nullptr;
   PointBufs B;
   BNode* nodes;
-  int32_t *alive, *rank, *leaf_flag, *lrank, *tile_sums;
+  int32_t* alive;
+  int2 *flags, *flag_tiles;  // (alive, leaf) of every node, then the exclusive prefixes
   Chunk* chunks;
   SegCounts* seg;
   int32_t *big_list, *node_chunk0;
@@ -2213,42 +2258,74 @@ struct BuildWs {
   double* root_frame;  // kRootFrame per cloud (k_decide at level 0)
   unsigned long long* tsmin;
   int64_t* off;
+  // cleared together at the start: from ls to zero_end
   LevelState* ls;
-  int32_t* level_begin;
   unsigned* done;  // last-block counter of the level's last kernel
+  char* zero_end;
+  int32_t* level_begin;
   int32_t* bsum;
   int32_t* bbig;  // per-block (chunks, large nodes) of the level
-  int32_t *cnt, *lcnt, *ucnt, *gp, *lgp, *to, *lto, *tot_nodes, *tot_leaves, *scan_tot;
+  int32_t *cnt, *lcnt, *gp, *lgp, *to, *lto;
+  // read back together: tot_nodes, tot_leaves, ucnt (R each), then ts0 and root_frame
+  int32_t *tot_nodes, *tot_leaves, *ucnt;
   TreeDev* trees;
   int64_t cap_nodes;
   int32_t chunk_cap;
 };
 
-// Bytes of the build workspace for n points in R clouds.
-size_t ws_bytes(int64_t n, int R) {
-  const int64_t cn = 2 * n + 4096 + 4 * (int64_t)R;
-  const int64_t chunk_cap = n / kChunk + n / kBig + 16;
-  const int64_t ntiles = cn / 4096 + 2;
-  const int64_t G = (int64_t)(kMaxDepth + 2) * R;
-  return carve_size<float4>(2 * n + 2) + carve_size<int32_t>(n) +
-         carve_size<BNode>(cn) + 4 * carve_size<int32_t>(cn) + carve_size<int32_t>(ntiles) +
-         carve_size<Chunk>(chunk_cap) + carve_size<SegCounts>(chunk_cap) + 2 * carve_size<int32_t>(chunk_cap) +
-         3 * carve_size<U128>((size_t)kSums * (n / kBig + 2)) + carve_size<U128>((size_t)kSums * cn) + carve_size<unsigned long long>(R) + carve_size<double>(R) + carve_size<double>(n) +
-         carve_size<DtSum>(n / kDtTile + 1) +
-         carve_size<double>((size_t)kRootFrame * R) + carve_size<int64_t>(R + 1) +
-         carve_size<LevelState>(1) + carve_size<int32_t>(kMaxDepth + 2) + carve_size<unsigned>(1) +
-         carve_size<int32_t>(kLevelBlocks) +
-         carve_size<int32_t>(2 * kLevelBlocks) +
-         7 * carve_size<int32_t>(G) + 3 * carve_size<int32_t>(R) + carve_size<int32_t>(8) + carve_size<TreeDev>(R) +
-         256;
-}
-
-int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
+// Lays the workspace for n points in R clouds out from p (a null base: sizes only); returns its end.
+char* ws_layout(BuildWs& w, char* p, int64_t n, int R) {
   w.cap_nodes = 2 * n + 4096 + 4 * (int64_t)R;
   w.chunk_cap = (int32_t)(n / kChunk + n / kBig + 16);
   const int64_t cn = w.cap_nodes;
-  const int64_t ntiles = cn / 4096 + 2;
   const int64_t G = (int64_t)(kMaxDepth + 2) * R;
+  const size_t nbig = (size_t)kSums * (n / kBig + 2);
+  w.B.p[0] = carve<float4>(p, 2 * n + 2);  // later the n + 1 stamp prefixes of 32 B
+  w.B.p[1] = w.B.p[0] + n;
+  w.B.perm = carve<int32_t>(p, n);
+  w.nodes = carve<BNode>(p, cn);
+  w.alive = carve<int32_t>(p, cn);
+  w.flags = carve<int2>(p, cn);
+  w.flag_tiles = carve<int2>(p, cn / kFlagTile + 2);
+  w.chunks = carve<Chunk>(p, w.chunk_cap);
+  w.seg = carve<SegCounts>(p, w.chunk_cap);
+  w.big_list = carve<int32_t>(p, w.chunk_cap);
+  w.node_chunk0 = carve<int32_t>(p, w.chunk_cap);
+  w.acc = carve<U128>(p, nbig);
+  for (int k = 0; k < 2; ++k) w.accl.acc[k] = carve<U128>(p, nbig);
+  w.mom = carve<U128>(p, (size_t)kSums * cn);
+  w.dt = carve<double>(p, n);
+  w.dt_tiles = carve<DtSum>(p, n / kDtTile + 1);
+  w.off = carve<int64_t>(p, R + 1);
+  w.ls = carve<LevelState>(p, 1);
+  w.done = carve<unsigned>(p, 1);
+  w.cnt = carve<int32_t>(p, G);
+  w.lcnt = carve<int32_t>(p, G);
+  w.tsmin = carve<unsigned long long>(p, R);
+  w.tot_nodes = carve<int32_t>(p, (size_t)3 * R + 1);
+  w.tot_leaves = w.tot_nodes + R;
+  w.ucnt = w.tot_leaves + R;
+  w.ts0 = carve<double>(p, (size_t)(1 + kRootFrame) * R);
+  w.root_frame = w.ts0 + R;
+  w.zero_end = p;
+  w.level_begin = carve<int32_t>(p, kMaxDepth + 2);
+  w.bsum = carve<int32_t>(p, kLevelBlocks);
+  w.bbig = carve<int32_t>(p, 2 * kLevelBlocks);
+  w.gp = carve<int32_t>(p, G);
+  w.lgp = carve<int32_t>(p, G);
+  w.to = carve<int32_t>(p, G);
+  w.lto = carve<int32_t>(p, G);
+  w.trees = carve<TreeDev>(p, R);
+  return p;
+}
+
+// Bytes of the build workspace for n points in R clouds.
+size_t ws_bytes(int64_t n, int R) {
+  BuildWs w;
+  return (size_t)(ws_layout(w, nullptr, n, R) - (char*)nullptr) + 256;
+}
+
+int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
   const size_t bytes = ws_bytes(n, R);
   cudaError_t e = cudaMallocAsync(&w.block, bytes, s);
   if (e != cudaSuccess) {
@@ -2257,45 +2334,7 @@ int ws_alloc(BuildWs& w, int64_t n, int R, cudaStream_t s) {
     set_error("cudaMallocAsync of %zu bytes for the tree build workspace failed: %s", bytes, cudaGetErrorString(e));
     return KDS_ERR_OOM;
   }
-  char* p = (char*)w.block;
-  w.B.p[0] = carve<float4>(p, 2 * n + 2);  // later the n + 1 stamp prefixes of 32 B
-  w.B.p[1] = w.B.p[0] + n;
-  w.B.perm = carve<int32_t>(p, n);
-  w.nodes = carve<BNode>(p, cn);
-  w.alive = carve<int32_t>(p, cn);
-  w.rank = carve<int32_t>(p, cn);
-  w.leaf_flag = carve<int32_t>(p, cn);
-  w.lrank = carve<int32_t>(p, cn);
-  w.tile_sums = carve<int32_t>(p, ntiles);
-  w.chunks = carve<Chunk>(p, w.chunk_cap);
-  w.seg = carve<SegCounts>(p, w.chunk_cap);
-  w.big_list = carve<int32_t>(p, w.chunk_cap);
-  w.node_chunk0 = carve<int32_t>(p, w.chunk_cap);
-  w.acc = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
-  for (int k = 0; k < 2; ++k) w.accl.acc[k] = carve<U128>(p, (size_t)kSums * (n / kBig + 2));
-  w.mom = carve<U128>(p, (size_t)kSums * cn);
-  w.ts0 = carve<double>(p, R);
-  w.dt = carve<double>(p, n);
-  w.dt_tiles = carve<DtSum>(p, n / kDtTile + 1);
-  w.root_frame = carve<double>(p, (size_t)kRootFrame * R);
-  w.tsmin = carve<unsigned long long>(p, R);
-  w.off = carve<int64_t>(p, R + 1);
-  w.ls = carve<LevelState>(p, 1);
-  w.level_begin = carve<int32_t>(p, kMaxDepth + 2);
-  w.done = carve<unsigned>(p, 1);
-  w.bsum = carve<int32_t>(p, kLevelBlocks);
-  w.bbig = carve<int32_t>(p, 2 * kLevelBlocks);
-  w.cnt = carve<int32_t>(p, G);
-  w.lcnt = carve<int32_t>(p, G);
-  w.gp = carve<int32_t>(p, G);
-  w.lgp = carve<int32_t>(p, G);
-  w.to = carve<int32_t>(p, G);
-  w.lto = carve<int32_t>(p, G);
-  w.ucnt = carve<int32_t>(p, G);
-  w.tot_nodes = carve<int32_t>(p, R);
-  w.tot_leaves = carve<int32_t>(p, R);
-  w.scan_tot = carve<int32_t>(p, R);
-  w.trees = carve<TreeDev>(p, R);
+  ws_layout(w, (char*)w.block, n, R);
   return KDS_OK;
 }
 
@@ -2489,14 +2528,11 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       d_st = (const double*)guard.h_st;
     }
   }
-  KDS_CK(cudaMemsetAsync(w.ls, 0, sizeof(LevelState), s));
-  KDS_CK(cudaMemsetAsync(w.done, 0, sizeof(unsigned), s));
+  KDS_CK(cudaMemsetAsync(w.ls, 0, (size_t)(w.zero_end - (char*)w.ls), s));
   KDS_CK(cudaMemcpyAsync(w.off, off.data(), sizeof(int64_t) * (R + 1), cudaMemcpyHostToDevice, s));
   k_ingest<<<nblk(N, kThreads), kThreads, 0, s>>>(d_xyz, N, w.B.p[0], w.ls);
   count_launch();
-  if (!d_st) KDS_CK(cudaMemsetAsync(w.ts0, 0, sizeof(double) * R, s));
   if (d_st) {
-    KDS_CK(cudaMemsetAsync(w.tsmin, 0xff, sizeof(unsigned long long) * R, s));
     // enough blocks to fill the machine whatever the number of clouds (64 per cloud before:
     // 370 + 200 us over the 11.4M stamps of one map)
     const int64_t gx = std::max<int64_t>(64, (148 * 8 + R - 1) / R);
@@ -2512,7 +2548,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
 
   // pinned: [level state | per-tree nodes, leaves, unpruned nodes | ts0 | root frames]
   const size_t st_ls = (sizeof(LevelState) + 255) & ~(size_t)255;
-  const size_t st_cnt = ((size_t)12 * R + 255) & ~(size_t)255;
+  const size_t st_cnt = (size_t)((char*)w.ts0 - (char*)w.tot_nodes);
   char* stage = (char*)pinned_stage(st_ls + st_cnt + sizeof(double) * (size_t)(1 + kRootFrame) * R);
   if (!stage) { set_error("kds_tree_build: page-locked staging of the level state failed"); return KDS_ERR_OOM; }
   LevelState& hls = *reinterpret_cast<LevelState*>(stage);
@@ -2616,24 +2652,24 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   k_alive<<<(int)std::min<int64_t>(nblk(total, kThreads), kGridBlocks * 4), kThreads, 0, s>>>(w.nodes, total, w.alive,
                                                                                           P.prune_incidence);
   count_launch();
-  const int64_t G = (int64_t)(kMaxDepth + 2) * R;
-  KDS_CK(cudaMemsetAsync(w.cnt, 0, sizeof(int32_t) * G, s));
-  KDS_CK(cudaMemsetAsync(w.lcnt, 0, sizeof(int32_t) * G, s));
-  KDS_CK(cudaMemsetAsync(w.ucnt, 0, sizeof(int32_t) * G, s));
-  k_group_counts<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, R, w.cnt, w.lcnt, w.ucnt,
-                                                            w.leaf_flag);
+  k_group_counts<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, R, w.cnt, w.lcnt, w.ucnt, w.flags);
   count_launch();
-  rc = scan_exclusive(w.alive, w.rank, total, w.tile_sums, w.scan_tot, s);
-  if (rc) return rc;
-  rc = scan_exclusive(w.leaf_flag, w.lrank, total, w.tile_sums, w.scan_tot, s);
-  if (rc) return rc;
+  if (total <= kFlagOne) {
+    k_flag_scan<<<1, 1024, 0, s>>>(w.flags, total, nullptr);
+  } else {
+    const int nt = (total + kFlagTile - 1) / kFlagTile;
+    k_flag_tiles<<<nt, 1024, 0, s>>>(w.flags, total, w.flag_tiles);
+    k_flag_top<<<1, 1024, 0, s>>>(w.flag_tiles, nt);
+    k_flag_scan<<<nt, 1024, 0, s>>>(w.flags, total, w.flag_tiles);
+    count_launch();
+    count_launch();
+  }
+  count_launch();
   k_group_tables<<<1, 1024, 0, s>>>(depth, R, w.cnt, w.lcnt, w.gp, w.lgp, w.to, w.lto, w.tot_nodes, w.tot_leaves);
   count_launch();
-  KDS_CK(cudaMemcpyAsync(h_cnt, w.tot_nodes, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, s));
-  KDS_CK(cudaMemcpyAsync(h_cnt + R, w.tot_leaves, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, s));
-  KDS_CK(cudaMemcpyAsync(h_cnt + 2 * R, w.ucnt, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, s));
-  KDS_CK(cudaMemcpyAsync(h_dbl, w.ts0, sizeof(double) * R, cudaMemcpyDeviceToHost, s));
-  KDS_CK(cudaMemcpyAsync(h_dbl + R, w.root_frame, sizeof(double) * kRootFrame * R, cudaMemcpyDeviceToHost, s));
+  KDS_CK(cudaMemcpyAsync(h_cnt, w.tot_nodes,
+                         (size_t)((char*)(w.ts0 + (size_t)(1 + kRootFrame) * R) - (char*)w.tot_nodes),
+                         cudaMemcpyDeviceToHost, s));
   KDS_CK(cudaStreamSynchronize(s));
   const std::vector<int32_t> tn(h_cnt, h_cnt + R), tl(h_cnt + R, h_cnt + 2 * R), tu(h_cnt + 2 * R, h_cnt + 3 * R);
   const std::vector<double> ts0(h_dbl, h_dbl + R), rf(h_dbl + R, h_dbl + R + (size_t)kRootFrame * R);
@@ -2679,10 +2715,10 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     k_dt_prefix<<<nt, kThreads, 0, s>>>(w.dt, w.B.perm, N, w.dt_tiles, nt > kThreads ? 1 : 0, pre);
     count_launch();
   }
-  k_compact_forest<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, w.rank, w.leaf_flag, w.lrank,
-                                                              R, w.gp, w.lgp, w.to, w.lto, pre, w.trees);
+  k_compact_forest<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, w.flags, R, w.gp, w.lgp, w.to,
+                                                              w.lto, pre, w.off, w.trees);
   count_launch();
-  dim3 fg((unsigned)std::min<int64_t>(nblk(max_size, kThreads), 256), (unsigned)R);
+  dim3 fg((unsigned)std::min<int64_t>(nblk(max_size, kThreads), std::max<int64_t>(64, 148 * 16 / R)), (unsigned)R);
   k_finish_trees<<<fg, kThreads, 0, s>>>(w.trees, w.off, w.B.perm);
   count_launch();
   cudaError_t e = cudaStreamSynchronize(s);
