@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "kds_internal.cuh"
@@ -45,6 +46,32 @@ constexpr int kUnroll = 2;  // rounds of 32 points in flight per lane in the war
 constexpr int kScatterPerSM = 2;  // 122 registers: the lanes' 21 64-bit parts and four points in flight
 constexpr int kSmallPerSM = 3;
 constexpr int kSmallBlocks = 148 * kSmallPerSM * 2;  // two waves: other streams' kernels interleave at block boundaries
+
+// ---------------------------------------------------------------------------
+// The build is a chain of short launches on one stream, each reading what the one before
+// wrote.  Every kernel may start while its predecessor still runs (programmatic dependent
+// launch): it lets its own successor be set up at once and waits here, before it reads
+// anything, for its predecessor's end, which includes the predecessor's own wait.  A
+// launch then costs its kernel and not the gap before it (an 11,000-point scan, 35 launches: 404 us without, 349 with).
+__device__ __forceinline__ void grid_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // errors: cudaGetLastError by the callers
+  count_launch();
+}
 
 // ---------------------------------------------------------------------------
 // 128-bit two's complement fixed point (units of 2^-64)
@@ -673,6 +700,7 @@ __device__ __forceinline__ void level_range(const LevelState* ls, int& b, int& e
 // Kernels
 
 __global__ void k_ingest(const float* xyz, int64_t n, float4* pts, LevelState* ls) {
+  grid_begin();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
     if (!(fabsf(x) < 32768.f && fabsf(y) < 32768.f && fabsf(z) < 32768.f)) ls->error = 2;
@@ -693,6 +721,7 @@ __device__ __forceinline__ double dkey_inv(unsigned long long k) {
 // ts_start of each tree = min stamp (label_policy_base_impl_.h:28-35), as the largest
 // complement of its key (tsmin starts at 0); blockIdx.y = tree.
 __global__ void k_tree_min(const double* sts, const int64_t* off, unsigned long long* tsmin) {
+  grid_begin();
   const int r = blockIdx.y;
   const int64_t b = off[r], e = off[r + 1];
   unsigned long long m = 0ull;
@@ -705,6 +734,7 @@ __global__ void k_tree_min(const double* sts, const int64_t* off, unsigned long 
 // decodes ts_start, checks every point's stamp and writes its dt; blockIdx.y = tree.
 __global__ void k_tree_check(const double* sts, const int64_t* off, const unsigned long long* tsmin, double* ts0,
                              double* dt, LevelState* ls) {
+  grid_begin();
   const int r = blockIdx.y;
   const int64_t b = off[r], e = off[r + 1];
   const double t0 = (e > b) ? dkey_inv(~tsmin[r]) : 0.0;
@@ -718,6 +748,7 @@ __global__ void k_tree_check(const double* sts, const int64_t* off, const unsign
 }
 
 __global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState* ls, int32_t* level_begin) {
+  grid_begin();
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < R) {
     BNode nd;
@@ -760,6 +791,7 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 
 // Level 0: warp per root of at most kBig points.
 __global__ void __launch_bounds__(kThreads) k_root_moments(const BNode* nodes, int R, PointBufs B, U128* mom) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   static_assert(kBig <= 32 * kLanePoints, "a root's points fit the lanes' sums");
@@ -867,6 +899,7 @@ __device__ __forceinline__ void level_decide(BNode* nodes, const LevelState* ls,
 }
 __global__ void k_decide(BNode* nodes, const LevelState* ls, U128* mom, ChildSums C, BuildParams P, int32_t* bsum,
                          int32_t* bbig, double* root_frame) {
+  grid_begin();
   __shared__ int sm[32];
   level_decide(nodes, ls, mom, C, P, bsum, bbig, root_frame, sm);
 }
@@ -925,6 +958,7 @@ static_assert(offsetof(BNode, start) == 0 && offsetof(BNode, end) == 4 && offset
 __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
                                                          U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin,
                                                          unsigned* done) {
+  grid_begin();
   const int lb = ls->lb, le = ls->le, cur = ls->cur;
   const float4* pin = B.p[cur];
   float4* pout = B.p[cur ^ 1];
@@ -1050,6 +1084,7 @@ struct __align__(16) Chunk {
 // kLevelBlocks blocks over contiguous node ranges: per-block counts first, then each
 // block writes its list at the prefix of the blocks before it.
 __global__ void k_big_sums(const BNode* nodes, const LevelState* ls, int32_t* bbig) {
+  grid_begin();
   __shared__ int sm[32];
   if (ls->max_size <= kBig) return;  // no large node on this level
   int b, e;
@@ -1161,6 +1196,7 @@ __device__ __forceinline__ void level_plan(BNode* nodes, LevelState* ls, const i
 // root: clear the roots' own sums, else the smaller children's of this level.
 __global__ void k_big_plan(BNode* nodes, LevelState* ls, const int32_t* bbig, Chunk* chunks, int32_t chunk_cap,
                            int32_t* big_list, int32_t* node_chunk0, U128* root_acc, ChildSums C, int parts) {
+  grid_begin();
   __shared__ int sm[32];
   level_plan(nodes, ls, bbig, chunks, chunk_cap, big_list, node_chunk0, root_acc ? root_acc : C.acc[ls->depth & 1], sm,
              (int)blockIdx.x % parts, parts);
@@ -1195,6 +1231,7 @@ static_assert(kPer * kThreads == kChunk && kSegs == 8, "a chunk is eight segment
 // sums once per root.
 __global__ void __launch_bounds__(kThreads, 2) k_big_moments(const Chunk* chunks, const LevelState* ls,
                                                              const PointBufs B, U128* acc) {
+  grid_begin();
   __shared__ U128 sm[kSegs][kSums];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   LaneSums S;
@@ -1233,6 +1270,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_big_moments(const Chunk* chunks
 
 // Level 0: the sums of the large roots, from the chunk accumulators.
 __global__ void k_big_to_mom(const LevelState* ls, const int32_t* big_list, const U128* acc, U128* mom) {
+  grid_begin();
   const int nb = ls->num_big;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * kSums; t += gridDim.x * blockDim.x)
     mom[(size_t)big_list[t / kSums] * kSums + t % kSums] = acc[t];
@@ -1244,6 +1282,7 @@ struct __align__(16) SegCounts {
 };
 __global__ void __launch_bounds__(kThreads) k_big_count(const Chunk* chunks, const LevelState* ls, const BNode* nodes,
                                                         const PointBufs B, SegCounts* seg) {
+  grid_begin();
   const int nc = ls->num_chunks;
   const float4* pts = B.p[ls->cur];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1286,6 +1325,7 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     k_big_scatter(const Chunk* chunks, LevelState* ls, BNode* nodes, PointBufs B, const SegCounts* seg,
                   const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t* level_begin,
                   unsigned* done) {
+  grid_begin();
   __shared__ U128 smm[kSegs][kSums];
   __shared__ int s_pre[kSegs], s_tot[kSegs];
   const int nc = ls->num_chunks, nbig = ls->num_big, cur = ls->cur;
@@ -1461,6 +1501,7 @@ static_assert(offsetof(BNode, level) == 8 && offsetof(BNode, tree) == 12 && offs
                   offsetof(BNode, has_prop) == 40 && offsetof(BNode, parent) == 44 && offsetof(BNode, par_prop) == 104,
               "BNode words as level_children writes them");
 __global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap) {
+  grid_begin();
   __shared__ int sm[32];
   level_children(nodes, ls, bsum, cap, sm);
 }
@@ -1473,6 +1514,7 @@ __global__ void __launch_bounds__(kThreads) k_level_small(BNode* nodes, LevelSta
                                                           double* root_frame, int32_t cap, Chunk* chunks,
                                                           int32_t chunk_cap, int32_t* big_list, int32_t* node_chunk0,
                                                           int plan) {
+  grid_begin();
   __shared__ int sm[32];
   level_decide(nodes, ls, mom, C, P, bsum, bbig, root_frame, sm);
   __syncthreads();
@@ -1553,6 +1595,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
     k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, ChildSums C, BuildParams P,
                  double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* ring, int32_t* counts,
                  int32_t dcap) {
+  grid_begin();
   constexpr int kNodes = deep_nodes<WARPS>();
   constexpr int kThreadsG = 32 * WARPS;
   extern __shared__ __align__(16) unsigned char deep_smem_raw[];
@@ -1830,6 +1873,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
 __global__ void k_deep_place(BNode* nodes, LevelState* ls, int32_t lb, int32_t le, const DeepNode* dn,
                              const int32_t* dn_count, int32_t dn_cap, const int32_t* off, int32_t dcap,
                              int32_t cap_nodes) {
+  grid_begin();
   if (ls->error) return;  // the build fails; records may be missing
   const int nroots = le - lb;
   const int nd_total = min(*dn_count, dn_cap);
@@ -1906,6 +1950,7 @@ __device__ __forceinline__ void deep_finish(LevelState* ls, int32_t lb, int32_t 
 }
 __global__ void k_deep_finish(LevelState* ls, int32_t lb, int32_t le, const int32_t* off, const int32_t* total,
                               int32_t dcap, int32_t cap_nodes, int32_t* level_begin) {
+  grid_begin();
   deep_finish(ls, lb, le, off, *total, dcap, cap_nodes, level_begin);
 }
 // The same with the scan of the counts by the one block: up to kDeepScan counts, a run per
@@ -1914,6 +1959,7 @@ constexpr int kDeepScan = 16384;
 __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, int32_t le, const int32_t* counts,
                                                     int32_t ncount, int32_t* off, int32_t dcap, int32_t cap_nodes,
                                                     int32_t* level_begin) {
+  grid_begin();
   __shared__ int sm[32];
   const int per = (ncount + 1023) / 1024;
   const int b = min((int)threadIdx.x * per, ncount), e = min(b + per, ncount);
@@ -1936,6 +1982,7 @@ __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, 
 // good leaf marks its ancestors up to the first one already marked: whoever marks a node
 // first goes on to its parent, so every ancestor ends marked whatever the order.
 __global__ void k_alive(const BNode* nodes, int32_t total, int32_t* alive, float incidence) {
+  grid_begin();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const BNode& nd = nodes[i];
     if (nd.left >= 0 || nd.right >= 0) continue;
@@ -1956,6 +2003,7 @@ __global__ void k_alive(const BNode* nodes, int32_t total, int32_t* alive, float
 // flags[i]: x = alive, y = alive leaf.
 __global__ void k_group_counts(const BNode* nodes, int32_t total, const int32_t* alive, int R, int32_t* cnt,
                                int32_t* lcnt, int32_t* ucnt, int2* flags) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
@@ -1996,6 +2044,7 @@ __device__ __forceinline__ int2 pair_block_scan(int2 v, int* sm, int2* total) {
   return r;
 }
 __global__ void __launch_bounds__(1024) k_flag_tiles(const int2* flags, int32_t n, int2* tiles) {
+  grid_begin();
   __shared__ int sm[32];
   const int base = blockIdx.x * kFlagTile + threadIdx.x * kFlagItems;
   int2 v = make_int2(0, 0), tot;
@@ -2005,6 +2054,7 @@ __global__ void __launch_bounds__(1024) k_flag_tiles(const int2* flags, int32_t 
   if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
 }
 __global__ void __launch_bounds__(1024) k_flag_top(int2* tiles, int32_t nt) {
+  grid_begin();
   __shared__ int sm[32];
   int2 carry = make_int2(0, 0);
   for (int b = 0; b < nt; b += blockDim.x) {
@@ -2017,6 +2067,7 @@ __global__ void __launch_bounds__(1024) k_flag_top(int2* tiles, int32_t nt) {
 }
 // tiles == nullptr: one block, a run of pairs per thread.
 __global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, int32_t n, const int2* tiles) {
+  grid_begin();
   __shared__ int sm[32];
   const int items = tiles ? kFlagItems : (n + 1023) / 1024;
   const int b = min((int)(blockIdx.x * 1024 + threadIdx.x) * items, n), e = min(b + items, n);
@@ -2035,6 +2086,7 @@ __global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, int32_t n, cons
 // and per-tree level offsets (one thread per tree).
 __global__ void k_group_tables(int depth, int R, const int32_t* cnt, const int32_t* lcnt, int32_t* gp, int32_t* lgp,
                                int32_t* to, int32_t* lto, int32_t* tot_nodes, int32_t* tot_leaves) {
+  grid_begin();
   __shared__ int sm[32];
   const int G = depth * R;
   int carry = 0, lcarry = 0;
@@ -2127,6 +2179,7 @@ __device__ __forceinline__ void dt_load(const double* dt, const int32_t* perm, i
   }
 }
 __global__ void __launch_bounds__(kThreads) k_dt_tiles(const double* dt, const int32_t* perm, int64_t n, DtSum* tiles) {
+  grid_begin();
   __shared__ DtSum sm[kThreads / 32];
   DtSum t[kDtItems], tot;
   dt_load(dt, perm, (int64_t)blockIdx.x * kDtTile + threadIdx.x * kDtItems, n, t);
@@ -2137,6 +2190,7 @@ __global__ void __launch_bounds__(kThreads) k_dt_tiles(const double* dt, const i
   if (threadIdx.x == 0) tiles[blockIdx.x] = tot;
 }
 __global__ void __launch_bounds__(kThreads) k_dt_top(DtSum* tiles, int nt) {
+  grid_begin();
   __shared__ DtSum sm[kThreads / 32];
   DtSum carry = dt_zero();
   for (int b = 0; b < nt; b += kThreads) {
@@ -2151,6 +2205,7 @@ __global__ void __launch_bounds__(kThreads) k_dt_top(DtSum* tiles, int nt) {
 // them) not, then each block adds up those before it.
 __global__ void __launch_bounds__(kThreads) k_dt_prefix(const double* dt, const int32_t* perm, int64_t n,
                                                         const DtSum* tiles, int scanned, DtSum* pre) {
+  grid_begin();
   __shared__ DtSum sm[kThreads / 32];
   const int64_t b = (int64_t)blockIdx.x * kDtTile + threadIdx.x * kDtItems;
   DtSum t[kDtItems], tot;
@@ -2181,6 +2236,7 @@ __global__ void __launch_bounds__(kThreads) k_dt_prefix(const double* dt, const 
 __global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_t* alive, const int2* rank, int R,
                                  const int32_t* gp, const int32_t* lgp, const int32_t* to, const int32_t* lto,
                                  const DtSum* pre, const int64_t* off, TreeDev* trees) {
+  grid_begin();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     if (!alive[i]) continue;
     const BNode& nd = nodes[i];
@@ -2221,6 +2277,7 @@ __global__ void k_compact_forest(const BNode* nodes, int32_t total, const int32_
 
 // tree-relative point order; blockIdx.y = tree
 __global__ void k_finish_trees(TreeDev* trees, const int64_t* off, const int32_t* perm_final) {
+  grid_begin();
   const int r = blockIdx.y;
   TreeDev& T = trees[r];
   if (T.nodes == nullptr) return;
@@ -2385,20 +2442,17 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * (ncount + 1), s);
   if (e == cudaSuccess) {
-    k_deep_build<WARPS><<<grid, 32 * WARPS * Form::kGroups, smem, s>>>(w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame,
+    launch(k_deep_build<WARPS>, grid, 32 * WARPS * Form::kGroups, smem, s, w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame,
                                                                        dn, dn_cap, dn_count, ring, counts, dcap);
-    count_launch();
     if (ncount <= kDeepScan) {
-      k_deep_scan<<<1, 1024, 0, s>>>(w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes,
+      launch(k_deep_scan, 1, 1024, 0, s, w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes,
                                      w.level_begin);
     } else {
       rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
-      k_deep_finish<<<1, 64, 0, s>>>(w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
+      launch(k_deep_finish, 1, 64, 0, s, w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
     }
-    count_launch();
     const int pg = (int)std::min<int64_t>(nblk(std::max<int64_t>(w.cap_nodes - le, nroots), kThreads), kGridBlocks * 4);
-    k_deep_place<<<pg, kThreads, 0, s>>>(w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes);
-    count_launch();
+    launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes);
     e = cudaGetLastError();
   }
   cudaFreeAsync(blk, s);
@@ -2424,16 +2478,14 @@ int scatter_blocks(const BuildWs& w) { return std::min<int>(w.chunk_cap, 148 * k
 
 // Level 0: the roots' sums, from their points.
 int root_sums(BuildWs& w, int R, int32_t max_size, int64_t N, cudaStream_t s) {
-  k_root_moments<<<(int)std::min<int64_t>(kGridBlocks, (R + 7) / 8), kThreads, 0, s>>>(w.nodes, R, w.B, w.mom);
-  count_launch();
+  launch(k_root_moments, (int)std::min<int64_t>(kGridBlocks, (R + 7) / 8), kThreads, 0, s, w.nodes, R, w.B, w.mom);
   if (max_size > kBig) {
     const int nb = level_blocks(R), parts = nb == 1 ? chunk_parts(N) : 1;
-    k_big_sums<<<nb, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig);
-    k_big_plan<<<nb * parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0,
+    launch(k_big_sums, nb, kThreads, 0, s, w.nodes, w.ls, w.bbig);
+    launch(k_big_plan, nb * parts, kThreads, 0, s, w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0,
                                                w.acc, w.accl, parts);
-    k_big_moments<<<scatter_blocks(w), kThreads, 0, s>>>(w.chunks, w.ls, w.B, w.acc);
-    k_big_to_mom<<<64, 256, 0, s>>>(w.ls, w.big_list, w.acc, w.mom);
-    for (int c = 0; c < 4; ++c) count_launch();
+    launch(k_big_moments, scatter_blocks(w), kThreads, 0, s, w.chunks, w.ls, w.B, w.acc);
+    launch(k_big_to_mom, 64, 256, 0, s, w.ls, w.big_list, w.acc, w.mom);
   }
   KDS_CK(cudaGetLastError());
   return KDS_OK;
@@ -2530,20 +2582,16 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   }
   KDS_CK(cudaMemsetAsync(w.ls, 0, (size_t)(w.zero_end - (char*)w.ls), s));
   KDS_CK(cudaMemcpyAsync(w.off, off.data(), sizeof(int64_t) * (R + 1), cudaMemcpyHostToDevice, s));
-  k_ingest<<<nblk(N, kThreads), kThreads, 0, s>>>(d_xyz, N, w.B.p[0], w.ls);
-  count_launch();
+  launch(k_ingest, nblk(N, kThreads), kThreads, 0, s, d_xyz, N, w.B.p[0], w.ls);
   if (d_st) {
     // enough blocks to fill the machine whatever the number of clouds (64 per cloud before:
     // 370 + 200 us over the 11.4M stamps of one map)
     const int64_t gx = std::max<int64_t>(64, (148 * 8 + R - 1) / R);
     dim3 g((unsigned)std::min<int64_t>(std::max<int64_t>((max_size + kThreads - 1) / kThreads, 1), gx), (unsigned)R);
-    k_tree_min<<<g, kThreads, 0, s>>>(d_st, w.off, w.tsmin);
-    k_tree_check<<<g, kThreads, 0, s>>>(d_st, w.off, w.tsmin, w.ts0, w.dt, w.ls);
-    count_launch();
-    count_launch();
+    launch(k_tree_min, g, kThreads, 0, s, d_st, w.off, w.tsmin);
+    launch(k_tree_check, g, kThreads, 0, s, d_st, w.off, w.tsmin, w.ts0, w.dt, w.ls);
   }
-  k_init_roots<<<(R + 127) / 128, 128, 0, s>>>(w.nodes, w.off, R, w.ls, w.level_begin);
-  count_launch();
+  launch(k_init_roots, (R + 127) / 128, 128, 0, s, w.nodes, w.off, R, w.ls, w.level_begin);
   KDS_CK(cudaGetLastError());
 
   // pinned: [level state | per-tree nodes, leaves, unpruned nodes | ts0 | root frames]
@@ -2609,30 +2657,23 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       }
       const bool big = host_max > kBig;  // the large-node kernels run after the partition
       if (lvl_blocks == 1) {
-        k_level_small<<<1, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame,
+        launch(k_level_small, 1, kThreads, 0, s, w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame,
                                              (int32_t)w.cap_nodes, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0,
                                              plan_parts == 1 ? 1 : 0);
-        count_launch();
       } else {
-        k_decide<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame);
-        k_level_children<<<lvl_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
-        count_launch();
-        count_launch();
+        launch(k_decide, lvl_blocks, kThreads, 0, s, w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame);
+        launch(k_level_children, lvl_blocks, kThreads, 0, s, w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
       }
       if (big && (lvl_blocks > 1 || plan_parts > 1)) {  // the decisions counted the large nodes per block
-        k_big_plan<<<lvl_blocks * plan_parts, kThreads, 0, s>>>(w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
+        launch(k_big_plan, lvl_blocks * plan_parts, kThreads, 0, s, w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
                                                                 w.big_list, w.node_chunk0, nullptr, w.accl, plan_parts);
-        count_launch();
       }
-      k_small_part<<<small_blocks, kThreads, 0, s>>>(w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks, w.level_begin,
+      launch(k_small_part, small_blocks, kThreads, 0, s, w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks, w.level_begin,
                                                      big ? nullptr : w.done);
-      count_launch();
       if (big) {
-        k_big_count<<<cb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg);
-        k_big_scatter<<<sb, kThreads, 0, s>>>(w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
+        launch(k_big_count, cb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg);
+        launch(k_big_scatter, sb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
                                               lvl_blocks, w.level_begin, w.done);
-        count_launch();
-        count_launch();
       }
     }
     KDS_CK(cudaGetLastError());
@@ -2649,24 +2690,18 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
   const int32_t total = hls.le;
   // prune
   KDS_CK(cudaMemsetAsync(w.alive, 0, sizeof(int32_t) * total, s));
-  k_alive<<<(int)std::min<int64_t>(nblk(total, kThreads), kGridBlocks * 4), kThreads, 0, s>>>(w.nodes, total, w.alive,
+  launch(k_alive, (int)std::min<int64_t>(nblk(total, kThreads), kGridBlocks * 4), kThreads, 0, s, w.nodes, total, w.alive,
                                                                                           P.prune_incidence);
-  count_launch();
-  k_group_counts<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, R, w.cnt, w.lcnt, w.ucnt, w.flags);
-  count_launch();
+  launch(k_group_counts, nblk(total, kThreads), kThreads, 0, s, w.nodes, total, w.alive, R, w.cnt, w.lcnt, w.ucnt, w.flags);
   if (total <= kFlagOne) {
-    k_flag_scan<<<1, 1024, 0, s>>>(w.flags, total, nullptr);
+    launch(k_flag_scan, 1, 1024, 0, s, w.flags, total, nullptr);
   } else {
     const int nt = (total + kFlagTile - 1) / kFlagTile;
-    k_flag_tiles<<<nt, 1024, 0, s>>>(w.flags, total, w.flag_tiles);
-    k_flag_top<<<1, 1024, 0, s>>>(w.flag_tiles, nt);
-    k_flag_scan<<<nt, 1024, 0, s>>>(w.flags, total, w.flag_tiles);
-    count_launch();
-    count_launch();
+    launch(k_flag_tiles, nt, 1024, 0, s, w.flags, total, w.flag_tiles);
+    launch(k_flag_top, 1, 1024, 0, s, w.flag_tiles, nt);
+    launch(k_flag_scan, nt, 1024, 0, s, w.flags, total, w.flag_tiles);
   }
-  count_launch();
-  k_group_tables<<<1, 1024, 0, s>>>(depth, R, w.cnt, w.lcnt, w.gp, w.lgp, w.to, w.lto, w.tot_nodes, w.tot_leaves);
-  count_launch();
+  launch(k_group_tables, 1, 1024, 0, s, depth, R, w.cnt, w.lcnt, w.gp, w.lgp, w.to, w.lto, w.tot_nodes, w.tot_leaves);
   KDS_CK(cudaMemcpyAsync(h_cnt, w.tot_nodes,
                          (size_t)((char*)(w.ts0 + (size_t)(1 + kRootFrame) * R) - (char*)w.tot_nodes),
                          cudaMemcpyDeviceToHost, s));
@@ -2705,22 +2740,17 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     pre = reinterpret_cast<DtSum*>(w.B.p[0]);
     const int nt = (int)(N / kDtTile + 1);  // tiles of the N + 1 positions
     if (nt > 1) {
-      k_dt_tiles<<<nt, kThreads, 0, s>>>(w.dt, w.B.perm, N, w.dt_tiles);
-      count_launch();
+      launch(k_dt_tiles, nt, kThreads, 0, s, w.dt, w.B.perm, N, w.dt_tiles);
     }
     if (nt > kThreads) {
-      k_dt_top<<<1, kThreads, 0, s>>>(w.dt_tiles, nt);
-      count_launch();
+      launch(k_dt_top, 1, kThreads, 0, s, w.dt_tiles, nt);
     }
-    k_dt_prefix<<<nt, kThreads, 0, s>>>(w.dt, w.B.perm, N, w.dt_tiles, nt > kThreads ? 1 : 0, pre);
-    count_launch();
+    launch(k_dt_prefix, nt, kThreads, 0, s, w.dt, w.B.perm, N, w.dt_tiles, nt > kThreads ? 1 : 0, pre);
   }
-  k_compact_forest<<<nblk(total, kThreads), kThreads, 0, s>>>(w.nodes, total, w.alive, w.flags, R, w.gp, w.lgp, w.to,
+  launch(k_compact_forest, nblk(total, kThreads), kThreads, 0, s, w.nodes, total, w.alive, w.flags, R, w.gp, w.lgp, w.to,
                                                               w.lto, pre, w.off, w.trees);
-  count_launch();
   dim3 fg((unsigned)std::min<int64_t>(nblk(max_size, kThreads), std::max<int64_t>(64, 148 * 16 / R)), (unsigned)R);
-  k_finish_trees<<<fg, kThreads, 0, s>>>(w.trees, w.off, w.B.perm);
-  count_launch();
+  launch(k_finish_trees, fg, kThreads, 0, s, w.trees, w.off, w.B.perm);
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
