@@ -73,3 +73,30 @@ def test_voxelize_full_sweep():
     gx, gs = kds.voxelize(xyz, st, **prm)
     ox, os_ = OV.voxelize(xyz, st, **prm)
     assert len(xyz) > 150000 and same(gx, ox) and same(gs, os_)
+
+
+@pytest.mark.parametrize("params", [
+    dict(range_max=30.0, space_res=0.25),                    # 8 bits an axis, 32-bit key
+    dict(range_max=126.5, space_res=0.25, use_boundary=1),   # 30 bits, edge of the axis' bits
+    dict(range_max=60.0, space_res=0.05),                    # 36 bits, 64-bit key
+    dict(range_max=60.0, space_res=0.1, time_res=0.004),     # 64 bits with the time bin
+    dict(range_max=60.0, space_res=0.05, time_res=0.004),    # past 64 bits: two sorts
+    dict(range_max=1e9, space_res=0.5),                      # cells past 20 bits: two sorts
+    dict(range_max=-40.0, space_res=0.5),                    # the bounds are squares
+    dict(range_max=35.0, range_min=0.0, space_res=1e-4),
+])
+def test_voxelize_key_forms(scene, params):
+    """Every form of the sort key against the restatement: points on the range bound, out of it,
+    NaN, on cell edges and at the origin among them."""
+    import kd_slam2_b200 as kds
+    xyz, st = make_scan(scene, 4310, beams=16, cols=400, vel=[4.0, 0, 0, 0, 0, 0.3])
+    R = abs(params["range_max"]) if params["range_max"] < 1e6 else 1000.0
+    extra = np.array([[R, 0, 0], [-R, 0, 0], [0, R, 0], [0, 0, -R], [R * 1.01, 0, 0], [0, -R * 0.999999, 0],
+                      [0, 0, 0], [1e-30, -1e-30, 0], [0.5, -0.5, 1.0], [np.nan, 0, 0], [3e4, 3e4, 3e4]], np.float32)
+    xyz = np.concatenate([xyz, extra])
+    st = np.concatenate([st, np.linspace(st.min(), st.max(), len(extra))])
+    p = dict(dict(range_min=0.0), **params)
+    gx, gs = kds.voxelize(xyz, st, **p)
+    ok = np.isfinite(xyz).all(1)
+    ox, os_ = OV.voxelize(xyz[ok], st[ok], **p)
+    assert same(gx, ox) and same(gs, os_)
