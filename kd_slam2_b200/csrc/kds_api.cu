@@ -281,11 +281,13 @@ int kds_tree_to_msg(const kds_tree* t, kds_kdtree3f* msg) {
     return KDS_ERR_CAPACITY;
   }
   if (n == 0) return KDS_OK;
+  int rc = KDS_OK;
+  if (tree_export_msg(t, msg->nodes, &rc)) return rc;
   std::vector<float> mean(3 * n), dir(3 * n);
   std::vector<double> dm(n), dc(n);
   std::vector<int64_t> s0(n), e0(n);
   std::vector<int32_t> l(n), r(n);
-  int rc = tree_export(t, mean.data(), dir.data(), dm.data(), dc.data(), s0.data(), e0.data(), l.data(), r.data(),
+  rc = tree_export(t, mean.data(), dir.data(), dm.data(), dc.data(), s0.data(), e0.data(), l.data(), r.data(),
                        nullptr, nullptr, nullptr);
   if (rc) return rc;
   for (int64_t i = 0; i < n; ++i) {

@@ -232,6 +232,7 @@ int tree_clone(const kds_tree* src, cudaStream_t s, kds_tree** out);
 int points_voxelize(const float* xyz, const double* stamps, int64_t n, int32_t mem, double msg_t,
                     double scan_duration, const kds_voxel_params* prm, cudaStream_t s, float* out_xyz,
                     double* out_stamps, int64_t* out_n);
+bool tree_export_msg(const kds_tree* t, kds_kdnode3f* out, int* rc);
 int tree_export(const kds_tree* t, float* mean, float* dir, double* dts_mean, double* dts_cov, int64_t* s0,
                 int64_t* e0, int32_t* left, int32_t* right, int32_t* level, int64_t* leaves, int64_t* perm);
 }  // namespace kds

@@ -162,7 +162,7 @@ static_assert(sizeof(kds_kdnode3f) == 56 && offsetof(kds_kdnode3f, idx_start) ==
 
 // kd_slam2_msgs/msg/KDNode3f records -> device node arrays (the bag reader's per-node
 // copy, lib/kd_io/rosbag2_message_reader.cpp:180-188), with the same checks as k_import.
-__global__ void k_import_msg(TreeDev t, const kds_kdnode3f* rec, int32_t* bad) {
+__global__ void k_import_msg(TreeDev t, const kds_kdnode3f* rec, int32_t* flag, int32_t* bad) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= t.num_nodes) return;
   const kds_kdnode3f k = rec[i];
@@ -178,6 +178,31 @@ __global__ void k_import_msg(TreeDev t, const kds_kdnode3f* rec, int32_t* bad) {
   t.range[2 * i] = (int64_t)k.idx_start;
   t.range[2 * i + 1] = (int64_t)k.idx_end;
   t.level[i] = 0;
+  flag[i] = l < 0 && r < 0 ? 1 : 0;
+}
+
+// Device node arrays -> KDNode3f records.  One packed copy crosses to the host instead of four
+// arrays and a loop over the nodes there, whose 100 bytes a node of fresh vectors cost more in
+// page faults than the copies (64 x 1,024 returns,
+// both ways: 362 us to 238).
+__global__ void k_export_msg(TreeDev t, kds_kdnode3f* rec) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= t.num_nodes) return;
+  const DNode d = t.nodes[i];
+  kds_kdnode3f k;
+  k.mean[0] = d.a.x;
+  k.mean[1] = d.a.y;
+  k.mean[2] = d.a.z;
+  k.direction[0] = d.a.w;
+  k.direction[1] = d.b.x;
+  k.direction[2] = d.b.y;
+  k.idx_start = (uint32_t)t.range[2 * i];
+  k.idx_end = (uint32_t)t.range[2 * i + 1];
+  k.idx_left = node_left(d);
+  k.idx_right = node_right(d);
+  k.dts_mean = t.dts_mean[i];
+  k.dts_covariance = t.dts_cov[i];
+  rec[i] = k;
 }
 
 __global__ void k_leaf_flags_plain(const DNode* nodes, int32_t n, int32_t* flag) {
@@ -186,10 +211,15 @@ __global__ void k_leaf_flags_plain(const DNode* nodes, int32_t n, int32_t* flag)
   DNode d = nodes[i];
   flag[i] = (node_left(d) < 0 && node_right(d) < 0) ? 1 : 0;
 }
-__global__ void k_leaf_scatter_plain(const int32_t* flag, const int32_t* rank, int32_t n, int32_t* leaf_idx) {
+// Leaf list and leaf arrays of an imported tree.
+__global__ void k_import_leaves(TreeDev t, const int32_t* flag, const int32_t* rank) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (flag[i]) leaf_idx[rank[i]] = i;
+  if (i >= t.num_nodes || !flag[i]) return;
+  const int o = rank[i];
+  const DNode d = t.nodes[i];
+  t.leaf_idx[o] = i;
+  t.leaf_md[o] = make_float4(d.a.x, d.a.y, d.a.z, t.dts_f[i]);
+  t.leaf_nrm[o] = make_float4(d.a.w, d.b.x, d.b.y, 0.f);
 }
 
 inline int nblk(int64_t n, int t) { return (int)std::max<int64_t>(1, (n + t - 1) / t); }
@@ -317,20 +347,19 @@ int tree_import(const float* mean, const float* dir, const double* dts_mean, con
   // leaf list by scan over leaf flags, reusing the staging arrays (dl as flag, dr as rank)
   int32_t* flag = (int32_t*)ds;  // ds/de no longer needed after k_import on this stream
   int32_t* rank = (int32_t*)de;
+  k_leaf_flags_plain<<<nblk(num_nodes, 256), 256, 0, s>>>(t->d.nodes, (int32_t)num_nodes, flag); ::kds::count_launch();
   return import_finish(t, flag, rank, dl, dbad, stg, s, "kds_tree_import", out);
 }
 
-// Leaf list of an imported tree (scan over leaf flags), the leaf arrays, and the result
+// Leaf list of an imported tree (scan over its leaf flags), the leaf arrays, and the result
 // of the node checks; frees the staging block and hands the tree out (or releases it).
 // flag, rank, tiles: num_nodes int32 scratch each; dbad[0] the check flag, dbad[1] scratch.
 static int import_finish(kds_tree* t, int32_t* flag, int32_t* rank, int32_t* tiles, int32_t* dbad, void* stg,
                          cudaStream_t s, const char* who, kds_tree** out) {
   const int64_t num_nodes = t->d.num_nodes;
   int32_t* total = dbad + 1;
-  k_leaf_flags_plain<<<nblk(num_nodes, 256), 256, 0, s>>>(t->d.nodes, (int32_t)num_nodes, flag); ::kds::count_launch();
   int rc2 = scan_exclusive(flag, rank, (int32_t)num_nodes, tiles, total, s);
-  k_leaf_scatter_plain<<<nblk(num_nodes, 256), 256, 0, s>>>(flag, rank, (int32_t)num_nodes, t->d.leaf_idx); ::kds::count_launch();
-  tree_gather_leaves(t->d, s);
+  k_import_leaves<<<nblk(num_nodes, 256), 256, 0, s>>>(t->d, flag, rank); ::kds::count_launch();
   int32_t bad = 0;
   cudaMemcpyAsync(&bad, dbad, 4, cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(stg, s);
@@ -389,7 +418,7 @@ int tree_from_msg(const kds_kdtree3f* msg, kds_tree** out) {
   int32_t* dbad = tiles + n;
   cudaMemcpyAsync(drec, msg->nodes, (size_t)n * sizeof(kds_kdnode3f), cudaMemcpyHostToDevice, s);
   cudaMemsetAsync(dbad, 0, 4, s);
-  k_import_msg<<<nblk(n, 256), 256, 0, s>>>(t->d, drec, dbad); ::kds::count_launch();
+  k_import_msg<<<nblk(n, 256), 256, 0, s>>>(t->d, drec, flag, dbad); ::kds::count_launch();
   return import_finish(t, flag, rank, tiles, dbad, stg, s, "kds_tree_from_msg", out);
 }
 
@@ -429,6 +458,35 @@ int tree_extract_leaves(const kds_tree* t, const float* v6, float* out_host, flo
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e, "extract leaves", __FILE__, __LINE__);
   return KDS_OK;
+}
+
+// Node records of a tree into host memory.  On the legacy stream, like tree_export's copies: after
+// the work of every blocking stream.  Returns false, with nothing written, where the device has
+// no room for the packed records or the tree lives on another than the current one.
+bool tree_export_msg(const kds_tree* t, kds_kdnode3f* out, int* rc) {
+  const int64_t n = t->d.num_nodes;
+  const size_t bytes = (size_t)n * sizeof(kds_kdnode3f);
+  const cudaStream_t s = cudaStreamLegacy;
+  void* rec = nullptr;
+  int dev = 0;
+  cudaPointerAttributes at;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, t->d.nodes) != cudaSuccess ||
+      at.device != dev || at.type != cudaMemoryTypeDevice) {
+    cudaGetLastError();
+    return false;
+  }
+  if (cudaMallocAsync(&rec, bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  k_export_msg<<<nblk(n, 256), 256, 0, s>>>(t->d, (kds_kdnode3f*)rec); ::kds::count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, rec, bytes, cudaMemcpyDeviceToHost, s);
+  cudaFreeAsync(rec, s);
+  const cudaError_t w = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = w;
+  *rc = e == cudaSuccess ? KDS_OK : cuda_status(e, "kds_tree_to_msg", __FILE__, __LINE__);
+  return true;
 }
 
 int tree_export(const kds_tree* t, float* mean, float* dir, double* dts_mean, double* dts_cov, int64_t* s0,

@@ -76,3 +76,25 @@ def test_malformed_messages_are_refused():
     with pytest.raises(KdsError) as e:
         kds.Tree.from_msg({"nodes": bad})
     assert e.value.code == KDS_ERR_BAD_TREE
+
+
+@pytest.mark.parametrize("nodes", [1, 255, 257, 9001])
+def test_message_records_of_all_fields(nodes):
+    """One node, and node counts around the launch's blocks: every field of every record."""
+    import kd_slam2_b200 as kds
+    rng = np.random.default_rng(nodes)
+    i = np.arange(nodes)
+    left = np.where(2 * i + 2 < nodes, 2 * i + 1, -1).astype(np.int32)
+    right = np.where(left >= 0, left + 1, -1).astype(np.int32)
+    f = rng.standard_normal((2, nodes, 3)).astype(np.float32)
+    d = rng.standard_normal((2, nodes))
+    s = rng.integers(0, 1 << 32, (2, nodes))
+    T = kds.Tree.import_nodes(f[0], f[1], left, right, d[0], d[1], s[0], s[1], ts_start=3.5)
+    msg = T.to_msg()
+    n = msg["nodes"]
+    for name, v in (("mean", f[0]), ("direction", f[1]), ("idx_start", s[0]), ("idx_end", s[1]), ("idx_left", left),
+                    ("idx_right", right), ("dts_mean", d[0]), ("dts_covariance", d[1])):
+        assert np.array_equal(n[name], v.astype(n[name].dtype)), name
+    U = kds.Tree.from_msg(msg)
+    assert np.array_equal(U.export()["leaves"], np.flatnonzero(left < 0))
+    assert np.array_equal(U.extract_compressed_leaves(), T.extract_compressed_leaves())
