@@ -994,18 +994,25 @@ __device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O,
   if (stamp) g_phase[15] = clock64();
 }
 
-// One Gauss-Newton iteration over the tiles [tile0, tile0 + gridDim.x) of one kind.
+// One Gauss-Newton iteration over the tiles [tile0, tile0 + gridDim.x) of one kind.  A descent is
+// a chain of dependent node reads, so a launch with tiles for every SM is bound by the blocks
+// that an SM holds until it is bound by issue: 8 (64 registers; the 18-parameter kind spills
+// there and takes 6), with the tree top staged as far as shared memory leaves room
+// (stage_room).  4,800 tiles, continuous-time / rigid: 116 / 97 us with 2 blocks and 2,047
+// nodes, 74 / 59 with 4 and 1,023, 61 / 46 with 6 and 511, 58 / 42 with 8 and 255.
+template <int KIND>
+constexpr int kLinBlocks = KIND == 2 ? 6 : 8;
 __device__ __forceinline__ void report_error(int32_t* err, int bits) { atomicOr(err ? err : &g_kernel_error, bits); }
 
 template <int KIND>
-__global__ void __launch_bounds__(kBlock, 4) k_linearize(const JobIn* __restrict__ jobs, JobState* states, JobOut* outs,
+__global__ void __launch_bounds__(kBlock, kLinBlocks<KIND>) k_linearize(const JobIn* __restrict__ jobs, JobState* states, JobOut* outs,
                                                       kds_stats* logs, LinDev* lins, const TileDev* __restrict__ tiles,
                                                       int tile0, int stage, double* partials, int32_t* dbg_match,
                                                       int32_t* dbg_status, int32_t* err) {
   constexpr int D = KindDim<KIND>::D;
   constexpr int M = D * (D + 1) / 2 + D;
   __shared__ CacheF sC;
-  __shared__ __align__(16) float sfac[kWarps * kMaxFac];
+  __shared__ __align__(16) float sfac[kWarps * (D + 2) * kFacStride];
   __shared__ double swp[kWarps * kPStride];
   __shared__ int s_last;
   __shared__ __align__(8) unsigned long long s_mbar;
@@ -1662,6 +1669,14 @@ int Runner::reserve(int nj, int nl, int nt) {
 
 void Runner::release() {
   drop_graph();
+  if (side) {
+    for (cudaEvent_t& e : fork_ev) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+    cudaStreamDestroy(side);
+    side = nullptr;
+  }
   for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
   prof_ev.clear();
   if (block) cudaFree(block);
@@ -1737,9 +1752,10 @@ int Runner::setup(const std::vector<JobIn>& jobs_in, const std::vector<LinDev>& 
   return KDS_OK;
 }
 
-int Runner::max_launches() const {
+int Runner::max_launches(int kind) const {
   int m = 0;
   for (const JobIn& J : h_jobs) {
+    if (kind >= 0 && J.kind != kind) continue;
     int it = (J.mode == KDS_JOB_COMPUTE) ? (J.stats_mode ? 1 : J.P.max_iterations) : 1;
     m = std::max(m, it);
   }
@@ -1809,6 +1825,52 @@ static int persistent_grid(size_t smem, int64_t items) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)nsm * per));
 }
 
+// Tree-top nodes that each block of a launch stages, `limit` at most: as many complete levels as
+// fit the share of an SM's shared memory that is left to each of the blocks it will hold (of
+// fixed_bytes of their own).  One or two blocks per SM stage 2,047 nodes, 3 and 4 1,023; more
+// hide the reads of the lower levels better than a staged top saves them (figures at
+// k_linearize).
+static int stage_room(int limit, int blocks, int most_blocks, size_t fixed_bytes) {
+  int nsm = 0, dev = 0, smem = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0 ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess || smem <= 0) {
+    cudaGetLastError();
+    nsm = 148;
+    smem = 228 * 1024;
+  }
+  const int per = std::min(most_blocks, (blocks + nsm - 1) / nsm);
+  const size_t share = (size_t)smem / (size_t)std::max(1, per), own = fixed_bytes + 1024;  // 1 KB: the system's
+  int n = 2047;
+  while (n > 0 && n * sizeof(DNode) + own > share) n >>= 1;
+  return std::min(limit, n);
+}
+
+// Static shared memory of a block: the pose cache, the leaves' factors, the warps' partials.
+template <int KIND>
+static constexpr size_t lin_bytes() {
+  return sizeof(CacheF) + sizeof(float) * kWarps * (KindDim<KIND>::D + 2) * kFacStride +
+         sizeof(double) * kWarps * kPStride + 64;
+}
+constexpr size_t kPairBytes = sizeof(CacheF) + sizeof(float) * kWarps * kMaxFac + sizeof(double) * 2 * kWarps * kPStride + 64;
+
+// One iteration's launch of one kind.
+template <int KIND>
+void Runner::enqueue_kind(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
+  if (pair_tiles) {
+    const int nb = kind_pair_count[KIND], stage = stage_room(stage_nodes, nb, 4, kPairBytes);
+    k_linearize_pair<KIND><<<nb, kBlock, stage * sizeof(DNode), s>>>(d_jobs, d_states, d_outs, d_logs, d_lins, d_tiles,
+                                                                     d_pairs, kind_pair_begin[KIND], stage, d_partials,
+                                                                     dbg_match, dbg_status, d_err);
+  } else {
+    const int nb = kind_count[KIND], stage = stage_room(stage_nodes, nb, kLinBlocks<KIND>, lin_bytes<KIND>());
+    k_linearize<KIND><<<nb, kBlock, stage * sizeof(DNode), s>>>(d_jobs, d_states, d_outs, d_logs, d_lins, d_tiles,
+                                                                kind_begin[KIND], stage, d_partials, dbg_match,
+                                                                dbg_status, d_err);
+  }
+  ::kds::count_launch();
+}
+
 int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   if (num_jobs == 0) return KDS_OK;
   if (persistent && !dbg_match) {
@@ -1842,58 +1904,57 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   k_init_jobs<<<(num_jobs + kInitWarps - 1) / kInitWarps, 32 * kInitWarps, 0, s>>>(d_jobs, d_states, d_outs, d_lins,
                                                                                    num_jobs, d_err);
   ::kds::count_launch();
-  int L = max_launches();
-  int nk = (kind_count[0] ? 1 : 0) + (kind_count[1] ? 1 : 0) + (kind_count[2] ? 1 : 0);
-  prof_launches = profiling ? L * nk : 0;
+  // each kind for the iterations its own jobs can take
+  int L[3], nmax = 0, total = 0;
+  for (int kind = 0; kind < 3; ++kind) {
+    L[kind] = kind_count[kind] ? max_launches(kind) : 0;
+    nmax = std::max(nmax, L[kind]);
+    total += L[kind];
+  }
+  prof_launches = profiling ? total : 0;
   if (profiling) {
     int rc = ensure_events(2 * prof_launches);
     if (rc) return rc;
   }
   int ev = 0;
-  const int stage = stage_nodes;
-  const size_t stage_bytes = (size_t)stage * sizeof(DNode);
-  if (stage_bytes > 0 && !smem_attr_set) {  // static + dynamic shared memory can pass 48 KB
+  if (stage_nodes > 0 && !smem_attr_set) {  // static + dynamic shared memory can pass 48 KB
     const void* fs[6] = {(const void*)k_linearize<0>, (const void*)k_linearize<1>, (const void*)k_linearize<2>,
                          (const void*)k_linearize_pair<0>, (const void*)k_linearize_pair<1>,
                          (const void*)k_linearize_pair<2>};
     for (int k = 0; k < 6; ++k) KDS_CK(cudaFuncSetAttribute(fs[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     smem_attr_set = true;
   }
-  for (int i = 0; i < L; ++i) {
+  // The kinds' jobs don't depend on each other: the first kind's iterations run on s, the others'
+  // beside them, so that one kind's blocks fill the SMs where the other's last tiles and solves
+  // run (a batch of 125 pairs of each kind: 1,735 us
+  // one after the other, 1,455 side by side).  In order where each launch is timed.
+  const int first = L[0] ? 0 : (L[1] ? 1 : 2);
+  const bool fork = !profiling && total > L[first];
+  if (fork) {
+    if (!side) {
+      KDS_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+      for (cudaEvent_t& e : fork_ev) KDS_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    KDS_CK(cudaEventRecord(fork_ev[0], s));
+    KDS_CK(cudaStreamWaitEvent(side, fork_ev[0], 0));
+  }
+  for (int i = 0; i < nmax; ++i) {
     for (int kind = 0; kind < 3; ++kind) {
-      if (!kind_count[kind]) continue;
+      if (i >= L[kind]) continue;
       if (profiling) KDS_CK(record_profile_event(prof_ev[ev++], s));
-      if (pair_tiles) {
-        const int nb = kind_pair_count[kind], p0 = kind_pair_begin[kind];
-        if (kind == 0)
-          k_linearize_pair<0><<<nb, kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins, d_tiles,
-                                                              d_pairs, p0, stage, d_partials, dbg_match, dbg_status,
-                                                              d_err);
-        else if (kind == 1)
-          k_linearize_pair<1><<<nb, kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins, d_tiles,
-                                                              d_pairs, p0, stage, d_partials, dbg_match, dbg_status,
-                                                              d_err);
-        else
-          k_linearize_pair<2><<<nb, kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins, d_tiles,
-                                                              d_pairs, p0, stage, d_partials, dbg_match, dbg_status,
-                                                              d_err);
-      } else if (kind == 0)
-        k_linearize<0><<<kind_count[0], kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins,
-                                                                     d_tiles, kind_begin[0], stage, d_partials,
-                                                                     dbg_match, dbg_status, d_err);
-      else if (kind == 1)
-        k_linearize<1><<<kind_count[1], kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins,
-                                                                     d_tiles, kind_begin[1], stage, d_partials,
-                                                                     dbg_match, dbg_status, d_err);
-      else
-        k_linearize<2><<<kind_count[2], kBlock, stage_bytes, s>>>(d_jobs, d_states, d_outs, d_logs, d_lins,
-                                                                     d_tiles, kind_begin[2], stage, d_partials,
-                                                                     dbg_match, dbg_status, d_err);
-      ::kds::count_launch();
+      const cudaStream_t ks = fork && kind != first ? side : s;
+      if (kind == 0) enqueue_kind<0>(ks, dbg_match, dbg_status);
+      else if (kind == 1) enqueue_kind<1>(ks, dbg_match, dbg_status);
+      else enqueue_kind<2>(ks, dbg_match, dbg_status);
       if (profiling) KDS_CK(record_profile_event(prof_ev[ev++], s));
     }
   }
-  KDS_CK(cudaGetLastError());
+  const cudaError_t le = cudaGetLastError();
+  if (fork) {  // joined also after a failed launch: what did start still uses the batch's buffers
+    KDS_CK(cudaEventRecord(fork_ev[1], side));
+    KDS_CK(cudaStreamWaitEvent(s, fork_ev[1], 0));
+  }
+  KDS_CK(le);
   return KDS_OK;
 }
 
@@ -1992,8 +2053,7 @@ int Runner::run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg
   key.push_back((int64_t)(uintptr_t)block);
   key.push_back(num_jobs);
   key.push_back(num_tiles);
-  key.push_back(max_launches());
-  for (int k = 0; k < 3; ++k) { key.push_back(kind_begin[k]); key.push_back(kind_count[k]); }
+  for (int k = 0; k < 3; ++k) { key.push_back(kind_begin[k]); key.push_back(kind_count[k]); key.push_back(max_launches(k)); }
   key.push_back(profiling ? 1 : 0);
   key.push_back(stage_nodes);
   key.push_back(order_by_size);
@@ -2116,19 +2176,20 @@ int launch_admit_slots(const int32_t* d_slots, int n, const JobIn* new_jobs, con
   return KDS_OK;
 }
 
+template <int KIND>
+static void serve_kind(int ntiles, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
+                       const TileDev* tiles, double* partials, cudaStream_t s) {
+  const int stage = stage_room(kServeStage, ntiles, kLinBlocks<KIND>, lin_bytes<KIND>());
+  k_linearize<KIND><<<ntiles, kBlock, stage * sizeof(DNode), s>>>(jobs, states, outs, nullptr, lins, tiles, 0, stage,
+                                                                  partials, nullptr, nullptr, nullptr);
+}
+
 int launch_linearize(int kind, int ntiles, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
                      const TileDev* tiles, double* partials, cudaStream_t s) {
   if (ntiles <= 0) return KDS_OK;
-  const size_t stage_bytes = (size_t)kServeStage * sizeof(DNode);
-  if (kind == 0)
-    k_linearize<0><<<ntiles, kBlock, stage_bytes, s>>>(jobs, states, outs, nullptr, lins, tiles, 0, kServeStage,
-                                                       partials, nullptr, nullptr, nullptr);
-  else if (kind == 1)
-    k_linearize<1><<<ntiles, kBlock, stage_bytes, s>>>(jobs, states, outs, nullptr, lins, tiles, 0, kServeStage,
-                                                       partials, nullptr, nullptr, nullptr);
-  else
-    k_linearize<2><<<ntiles, kBlock, stage_bytes, s>>>(jobs, states, outs, nullptr, lins, tiles, 0, kServeStage,
-                                                       partials, nullptr, nullptr, nullptr);
+  if (kind == 0) serve_kind<0>(ntiles, jobs, states, outs, lins, tiles, partials, s);
+  else if (kind == 1) serve_kind<1>(ntiles, jobs, states, outs, lins, tiles, partials, s);
+  else serve_kind<2>(ntiles, jobs, states, outs, lins, tiles, partials, s);
   count_launch();
   KDS_CK(cudaGetLastError());
   return KDS_OK;

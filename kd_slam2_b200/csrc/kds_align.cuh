@@ -128,7 +128,8 @@ struct Runner {
   cudaGraphExec_t gexec = nullptr;
   std::vector<int64_t> graph_key;
   std::vector<int64_t> last_key;  // shape of the previous run
-  // number of top fixed-tree nodes each block stages in shared memory (32 B each)
+  // top fixed-tree nodes each block stages in shared memory (32 B each), at most: a launch with
+  // several blocks per SM stages fewer (stage_room)
   int stage_nodes = 2047;
   // tiles of larger jobs first (1) or in job order (0); tuned by kds_batch_autotune
   int order_by_size = 0;
@@ -140,6 +141,8 @@ struct Runner {
   int pair_tiles = 0;
   ClusterOut* h_cluster = nullptr;  // results of run_cluster
   int cluster_blocks = 0;           // largest cluster (0: not asked yet)
+  cudaStream_t side = nullptr;      // launches of a second kind of jobs
+  cudaEvent_t fork_ev[2] = {};
   bool smem_attr_set = false;
   bool persistent_attr_set = false;
   // optional event pair per linearization launch (measurement only)
@@ -153,8 +156,10 @@ struct Runner {
   void release();
   void drop_graph();
   int setup(const std::vector<JobIn>& jobs, const std::vector<LinDev>& lins, cudaStream_t s);
-  int max_launches() const;
+  int max_launches(int kind = -1) const;  // iterations of the longest job (of one kind)
   int enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status);
+  template <int KIND>
+  void enqueue_kind(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status);
   int run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg_status);
   int fetch(cudaStream_t s, std::vector<JobOut>& outs, std::vector<kds_stats>* logs);
   // one job in one cluster launch (cluster_fits); waits for it

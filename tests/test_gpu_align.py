@@ -248,6 +248,38 @@ def test_batch_equals_single_alignments(trees, ct_trees):
         assert s.stats.num_inliers == m.stats.num_inliers
 
 
+@pytest.mark.parametrize("blocks_per_sm", [1, 2, 2.01, 4, 4.01, 7, 9])
+def test_batch_sizes_equal_single_alignments(trees, ct_trees, blocks_per_sm):
+    """Batches around the sizes where blocks stage less of the tree: every job of both kinds, with
+    unlike iteration limits, is bit-identical to the job alone."""
+    import torch
+    import kd_slam2_b200 as kds
+    from kd_slam2_b200 import abi
+    Gf, Gm, _, _ = trees
+    Cf, Cm, _, _, vel = ct_trees
+    rng = np.random.default_rng(12)
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    proto = []
+    for k in range(3):
+        X0 = perturbation(rng, 0.1, 1.0)
+        proto.append(kds.make_job(abi.KDS_ICP, Gf, Gm, kds.aligner_params(max_error=0.5, max_iterations=2 + k), X=X0))
+        proto.append(kds.make_job(abi.KDS_CTICP, Cf, Cm, kds.aligner_params(max_error=0.5, max_iterations=3), X=X0,
+                                  v=np.zeros(6)))
+    single = [kds.Batch().run([j], use_graph=False)[0] for j in proto]
+    per_icp, per_ct = -(-Gm.info.num_leaves // 128), -(-Cm.info.num_leaves // 128)
+    n_icp, n_ct = -(-int(blocks_per_sm * nsm) // per_icp), -(-int(blocks_per_sm * nsm) // per_ct)
+    pick = [2 * (k % 3) for k in range(n_icp)] + [2 * (k % 3) + 1 for k in range(n_ct)]
+    B = kds.Batch()
+    for _ in range(3):  # launched directly, then captured, then replayed
+        out = B.run([proto[k] for k in pick], use_graph=True)
+        for k, m in zip(pick, out):
+            s = single[k]
+            assert s.result == m.result and s.iterations == m.iterations
+            assert list(s.X) == list(m.X) and list(s.v) == list(m.v)
+            assert s.stats.num_inliers == m.stats.num_inliers and s.stats.chi2 == m.stats.chi2
+            assert list(s.H) == list(m.H) and list(s.b) == list(m.b)
+
+
 def test_tree_top_wait_fallback(trees):
     """With the bounded wait for the tree-top TMA copy cut to zero polls, every block of
     compute() reads the fixed tree from global memory: the call reports KDS_ERR_TIMEOUT
