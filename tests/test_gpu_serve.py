@@ -140,3 +140,21 @@ def test_request_that_never_fits_is_refused(trace):
     res, st, _ = run(trace, hbm_cap=1 << 20)
     assert st["completed"] == len(trace.requests)
     assert all(r["status"] == abi.KDS_ERR_ADMISSION for r in res)
+
+
+@pytest.mark.parametrize("at", [0.0, 0.37, 1.0])
+@pytest.mark.parametrize("take", [4095, 4097, 1 << 30])
+def test_device_stamps_equal_host_stamps(trace, take, at):
+    """The first stamp of device arrays (at the start, inside, at the end of a request) is the one
+    of host arrays: the maps that later windows are aligned to depend on it."""
+    import torch
+    inputs = []
+    for r in trace.requests:
+        n = min(take, len(r.xyz))
+        xyz, st = r.xyz[:n].copy(), r.stamps[:n].copy()
+        st[[int(np.argmin(st)), int(at * (n - 1))]] = st[[int(at * (n - 1)), int(np.argmin(st))]]
+        st[int(at * (n - 1))] -= 0.01
+        inputs.append((xyz, st))
+    a, _, _ = run(trace, inputs=inputs)
+    b, _, _ = run(trace, inputs=[(torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()) for x, t in inputs])
+    same_results(a, b)
