@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+from array import array
 
 import numpy as np
 
@@ -612,10 +613,14 @@ class Batch:
         """MultiViewICPFactor_ / MultiViewCTICPFactor_ block updates of the last run, on the
         device (kds_batch_assemble).  factors: (job, [vars]) pairs.  Returns (block_rc (K,2),
         H_blocks (K,6,6), b (num_vars,6), enabled (num_factors,))."""
-        fa = (L.Factor * len(factors))()
-        for f, (job, vs) in enumerate(factors):
-            fa[f].job = job
-            fa[f].var[:] = list(vs) + [-1] * (4 - len(vs))
+        flat = array("i")  # one buffer of kds_factor records
+        for job, vs in factors:
+            if len(vs) > 4:
+                raise ValueError("a factor has at most four variables")
+            flat.append(job)
+            flat.extend(list(vs))
+            flat.extend((-1,) * (4 - len(vs)))
+        fa = (L.Factor * len(factors)).from_buffer(flat) if len(factors) else (L.Factor * 0)()
         nb = C.c_int32(0)
         _check(_lib.kds_batch_assemble(self._h, fa, len(factors), num_vars, disable_inlier_ratio, stream,
                                        C.byref(nb), None, None, None, None), "kds_batch_assemble")

@@ -99,12 +99,21 @@ __global__ void k_factor_b(const JobOut* outs, const Contrib* con, const int32_t
   b[t] = acc;
 }
 
-struct HEntry {
-  int32_t gr, gc;  // global block (row variable <= column variable)
+// One contribution: the global block (row variable <= column variable) as a key, its place in
+// factor order, what it adds.  Sorted by (key, place) through an index.
+struct Entry {
+  uint64_t key;
   int32_t factor;
-  int32_t seq;     // order inside the factor
   Contrib c;
 };
+std::vector<int32_t> entry_order(const std::vector<Entry>& e) {
+  std::vector<std::pair<uint64_t, int32_t>> k(e.size());
+  for (size_t i = 0; i < e.size(); ++i) k[i] = {e[i].key, (int32_t)i};
+  std::sort(k.begin(), k.end());
+  std::vector<int32_t> o(e.size());
+  for (size_t i = 0; i < e.size(); ++i) o[i] = k[i].second;
+  return o;
+}
 
 }  // namespace
 
@@ -114,10 +123,9 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
     set_error("kds_batch_assemble: bad arguments");
     return KDS_ERR_INVALID_ARG;
   }
-  std::vector<HEntry> hs;
-  std::vector<std::pair<int32_t, HEntry>> bs;  // (variable, contribution)
-  std::vector<int32_t> fjob(nf), jdim(R.num_jobs, 6);
-  for (int j = 0; j < R.num_jobs; ++j) jdim[j] = R.h_jobs[j].kind == 0 ? 6 : 12;
+  std::vector<Entry> hs, bs;  // of blocks, of variables
+  hs.reserve((size_t)nf * 10);
+  bs.reserve((size_t)nf * 4);
   for (int f = 0; f < nf; ++f) {
     const kds_factor& q = F[f];
     if (q.job < 0 || q.job >= R.num_jobs) {
@@ -135,16 +143,15 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
         set_error("kds_batch_assemble: factor %d: variable %d out of range", f, q.var[k]);
         return KDS_ERR_INVALID_ARG;
       }
-    fjob[f] = q.job;
-    int seq = 0;
     auto addH = [&](int r, int c, int src, int sign, int tr) {
       int gr = q.var[r], gc = q.var[c];
       if (gr > gc) { std::swap(gr, gc); tr ^= 1; }
-      hs.push_back({gr, gc, f, seq++, {q.job, src, sign, tr}});
+      const uint64_t key = (uint64_t)(uint32_t)gr << 32 | (uint32_t)gc;
+      hs.push_back({key, f, {q.job, src, sign, tr}});
       if (gr == gc && r != c)  // both variables of an off-diagonal block are one: its transpose lands here too
-        hs.push_back({gr, gc, f, seq++, {q.job, src, sign, tr ^ 1}});
+        hs.push_back({key, f, {q.job, src, sign, tr ^ 1}});
     };
-    auto addB = [&](int r, int src, int sign) { bs.push_back({q.var[r], {0, 0, f, seq++, {q.job, src, sign, 0}}}); };
+    auto addB = [&](int r, int src, int sign) { bs.push_back({(uint64_t)q.var[r], f, {q.job, src, sign, 0}}); };
     if (kind == 0) {  // ICP: x0 fixed pose, x1 moving pose (multiview_icp_factor_impl_.h:46-61)
       addH(0, 0, kH00, +1, 0);
       addH(0, 1, kH00, -1, 0);
@@ -168,29 +175,9 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
       addB(3, kB1, -1);
     }
   }
-  std::stable_sort(hs.begin(), hs.end(), [](const HEntry& a, const HEntry& b) {
-    return a.gr != b.gr ? a.gr < b.gr : a.gc < b.gc;  // factor order kept within a block
-  });
-  std::stable_sort(bs.begin(), bs.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-  std::vector<int32_t> hbeg, rc, hfac, bbeg(nvars + 1, 0), bfac;
-  std::vector<Contrib> hcon, bcon;
-  for (size_t k = 0; k < hs.size(); ++k) {
-    if (k == 0 || hs[k].gr != hs[k - 1].gr || hs[k].gc != hs[k - 1].gc) {
-      hbeg.push_back((int32_t)k);
-      rc.push_back(hs[k].gr);
-      rc.push_back(hs[k].gc);
-    }
-    hcon.push_back(hs[k].c);
-    hfac.push_back(hs[k].factor);
-  }
-  const int32_t nb = (int32_t)rc.size() / 2;
-  hbeg.push_back((int32_t)hs.size());
-  for (auto& e : bs) {
-    ++bbeg[e.first + 1];
-    bcon.push_back(e.second.c);
-    bfac.push_back(e.second.factor);
-  }
-  for (int v = 0; v < nvars; ++v) bbeg[v + 1] += bbeg[v];
+  const std::vector<int32_t> ho = entry_order(hs);
+  int32_t nb = 0;
+  for (size_t k = 0; k < ho.size(); ++k) nb += k == 0 || hs[ho[k]].key != hs[ho[k - 1]].key;
   const int32_t cap = *num_blocks;
   *num_blocks = nb;
   if (cap < nb || (nb > 0 && (!block_rc || !H_out))) {
@@ -198,17 +185,55 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
     set_error("kds_batch_assemble: %d blocks do not fit in %d", nb, cap);
     return KDS_ERR_CAPACITY;
   }
-  if (!rc.empty()) memcpy(block_rc, rc.data(), sizeof(int32_t) * rc.size());
-  // device buffers: one block from the stream-ordered pool
+  // One copy to the device and one back (twelve small ones took longer than the kernels):
+  // [job of each factor | dimension of each job | per block: contributions, begins, factors |
+  // the same per variable], then device only: [H | b | enabled].
+  const std::vector<int32_t> bo = entry_order(bs);
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t sz_fjob = al(sizeof(int32_t) * std::max(nf, 1)), sz_en = sz_fjob;
-  const size_t sz_jdim = al(sizeof(int32_t) * std::max(R.num_jobs, 1));
-  const size_t sz_hcon = al(sizeof(Contrib) * std::max<size_t>(hcon.size(), 1));
-  const size_t sz_hbeg = al(sizeof(int32_t) * hbeg.size()), sz_hfac = al(sizeof(int32_t) * std::max<size_t>(hfac.size(), 1));
-  const size_t sz_bcon = al(sizeof(Contrib) * std::max<size_t>(bcon.size(), 1));
-  const size_t sz_bbeg = al(sizeof(int32_t) * bbeg.size()), sz_bfac = al(sizeof(int32_t) * std::max<size_t>(bfac.size(), 1));
-  const size_t sz_H = al(sizeof(double) * 36 * std::max(nb, 1)), sz_b = al(sizeof(double) * 6 * nvars);
-  const size_t total = sz_fjob + sz_en + sz_jdim + sz_hcon + sz_hbeg + sz_hfac + sz_bcon + sz_bbeg + sz_bfac + sz_H + sz_b;
+  size_t total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t o = total;
+    total += al(std::max<size_t>(bytes, 1));
+    return o;
+  };
+  const size_t o_fjob = place(sizeof(int32_t) * nf), o_jdim = place(sizeof(int32_t) * R.num_jobs);
+  const size_t o_hcon = place(sizeof(Contrib) * hs.size()), o_hbeg = place(sizeof(int32_t) * ((size_t)nb + 1));
+  const size_t o_hfac = place(sizeof(int32_t) * hs.size());
+  const size_t o_bcon = place(sizeof(Contrib) * bs.size()), o_bbeg = place(sizeof(int32_t) * ((size_t)nvars + 1));
+  const size_t o_bfac = place(sizeof(int32_t) * bs.size());
+  const size_t up_bytes = total;
+  const size_t o_H = place(sizeof(double) * 36 * nb), o_b = place(sizeof(double) * 6 * nvars);
+  const size_t o_en = place(sizeof(int32_t) * nf);
+  std::vector<char> host(std::max(up_bytes, total - up_bytes));
+  {
+    char* u = host.data();
+    int32_t *fjob = (int32_t*)(u + o_fjob), *jdim = (int32_t*)(u + o_jdim);
+    int32_t *hbeg = (int32_t*)(u + o_hbeg), *hfac = (int32_t*)(u + o_hfac);
+    int32_t *bbeg = (int32_t*)(u + o_bbeg), *bfac = (int32_t*)(u + o_bfac);
+    Contrib *hcon = (Contrib*)(u + o_hcon), *bcon = (Contrib*)(u + o_bcon);
+    for (int f = 0; f < nf; ++f) fjob[f] = F[f].job;
+    for (int j = 0; j < R.num_jobs; ++j) jdim[j] = R.h_jobs[j].kind == 0 ? 6 : 12;
+    int32_t nblk = 0;
+    for (size_t k = 0; k < ho.size(); ++k) {
+      const Entry& q = hs[ho[k]];
+      if (k == 0 || q.key != hs[ho[k - 1]].key) {
+        block_rc[2 * nblk] = (int32_t)(q.key >> 32);
+        block_rc[2 * nblk + 1] = (int32_t)(uint32_t)q.key;
+        hbeg[nblk++] = (int32_t)k;
+      }
+      hcon[k] = q.c;
+      hfac[k] = q.factor;
+    }
+    hbeg[nb] = (int32_t)hs.size();
+    std::fill(bbeg, bbeg + nvars + 1, 0);
+    for (size_t k = 0; k < bo.size(); ++k) {
+      const Entry& q = bs[bo[k]];
+      ++bbeg[q.key + 1];
+      bcon[k] = q.c;
+      bfac[k] = q.factor;
+    }
+    for (int v = 0; v < nvars; ++v) bbeg[v + 1] += bbeg[v];
+  }
   void* blk = nullptr;
   cudaError_t e = cudaMallocAsync(&blk, total, s);
   if (e != cudaSuccess) {
@@ -217,32 +242,14 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
     return KDS_ERR_OOM;
   }
   char* p = (char*)blk;
-  auto take = [&](size_t n) { char* r = p; p += n; return (void*)r; };
-  int32_t* d_fjob = (int32_t*)take(sz_fjob);
-  int32_t* d_en = (int32_t*)take(sz_en);
-  int32_t* d_jdim = (int32_t*)take(sz_jdim);
-  Contrib* d_hcon = (Contrib*)take(sz_hcon);
-  int32_t* d_hbeg = (int32_t*)take(sz_hbeg);
-  int32_t* d_hfac = (int32_t*)take(sz_hfac);
-  Contrib* d_bcon = (Contrib*)take(sz_bcon);
-  int32_t* d_bbeg = (int32_t*)take(sz_bbeg);
-  int32_t* d_bfac = (int32_t*)take(sz_bfac);
-  double* d_H = (double*)take(sz_H);
-  double* d_b = (double*)take(sz_b);
-  std::vector<int32_t> en(std::max(nf, 1), 0);
+  const int32_t *d_fjob = (int32_t*)(p + o_fjob), *d_jdim = (int32_t*)(p + o_jdim);
+  const Contrib *d_hcon = (Contrib*)(p + o_hcon), *d_bcon = (Contrib*)(p + o_bcon);
+  const int32_t *d_hbeg = (int32_t*)(p + o_hbeg), *d_hfac = (int32_t*)(p + o_hfac);
+  const int32_t *d_bbeg = (int32_t*)(p + o_bbeg), *d_bfac = (int32_t*)(p + o_bfac);
+  double *d_H = (double*)(p + o_H), *d_b = (double*)(p + o_b);
+  int32_t* d_en = (int32_t*)(p + o_en);
   do {
-    if (nf > 0 && (e = cudaMemcpyAsync(d_fjob, fjob.data(), sizeof(int32_t) * nf, cudaMemcpyHostToDevice, s))) break;
-    if ((e = cudaMemcpyAsync(d_jdim, jdim.data(), sizeof(int32_t) * R.num_jobs, cudaMemcpyHostToDevice, s))) break;
-    if (!hcon.empty()) {
-      if ((e = cudaMemcpyAsync(d_hcon, hcon.data(), sizeof(Contrib) * hcon.size(), cudaMemcpyHostToDevice, s))) break;
-      if ((e = cudaMemcpyAsync(d_hfac, hfac.data(), sizeof(int32_t) * hfac.size(), cudaMemcpyHostToDevice, s))) break;
-    }
-    if ((e = cudaMemcpyAsync(d_hbeg, hbeg.data(), sizeof(int32_t) * hbeg.size(), cudaMemcpyHostToDevice, s))) break;
-    if (!bcon.empty()) {
-      if ((e = cudaMemcpyAsync(d_bcon, bcon.data(), sizeof(Contrib) * bcon.size(), cudaMemcpyHostToDevice, s))) break;
-      if ((e = cudaMemcpyAsync(d_bfac, bfac.data(), sizeof(int32_t) * bfac.size(), cudaMemcpyHostToDevice, s))) break;
-    }
-    if ((e = cudaMemcpyAsync(d_bbeg, bbeg.data(), sizeof(int32_t) * bbeg.size(), cudaMemcpyHostToDevice, s))) break;
+    if ((e = cudaMemcpyAsync(p, host.data(), up_bytes, cudaMemcpyHostToDevice, s))) break;
     if (nf > 0) {
       k_factor_enabled<<<(nf + 255) / 256, 256, 0, s>>>(R.d_outs, d_fjob, nf, ratio, d_en);
       count_launch();
@@ -254,9 +261,8 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
     k_factor_b<<<(nvars * 6 + 255) / 256, 256, 0, s>>>(R.d_outs, d_bcon, d_bbeg, d_bfac, d_en, nvars, d_b);
     count_launch();
     if ((e = cudaGetLastError())) break;
-    if (nb > 0 && (e = cudaMemcpyAsync(H_out, d_H, sizeof(double) * 36 * nb, cudaMemcpyDeviceToHost, s))) break;
-    if (b_out && (e = cudaMemcpyAsync(b_out, d_b, sizeof(double) * 6 * nvars, cudaMemcpyDeviceToHost, s))) break;
-    if (nf > 0 && (e = cudaMemcpyAsync(en.data(), d_en, sizeof(int32_t) * nf, cudaMemcpyDeviceToHost, s))) break;
+    // into the buffer of the copy up, which is before this one on the stream
+    if ((e = cudaMemcpyAsync(host.data(), p + up_bytes, total - up_bytes, cudaMemcpyDeviceToHost, s))) break;
     e = cudaStreamSynchronize(s);
   } while (false);
   cudaFreeAsync(blk, s);
@@ -265,7 +271,10 @@ int batch_assemble(Runner& R, const kds_factor* F, int32_t nf, int32_t nvars, fl
     cudaGetLastError();
     return rc2;
   }
-  if (enabled_out && nf > 0) memcpy(enabled_out, en.data(), sizeof(int32_t) * nf);
+  auto back = [&](size_t o) { return host.data() + (o - up_bytes); };
+  if (nb > 0) memcpy(H_out, back(o_H), sizeof(double) * 36 * nb);
+  if (b_out) memcpy(b_out, back(o_b), sizeof(double) * 6 * nvars);
+  if (enabled_out && nf > 0) memcpy(enabled_out, back(o_en), sizeof(int32_t) * nf);
   return KDS_OK;
 }
 

@@ -103,8 +103,9 @@ __global__ void __launch_bounds__(1024) k_first_stamp(const double* __restrict__
 }
 
 // The first stamp of n device stamps.  Reading the stamps back and searching them on the host took
-// 180 us a request (65,536 points); the kernel and 8 bytes take 40.  On the legacy stream, after the work of every blocking
-// stream, as the copy is.  The copy stays for stamps of another device and for pointers whose last element is no device memory.
+// 180 us a request (65,536 points); the kernel and 8 bytes take 40.  On the legacy stream, after
+// the work of every blocking stream, as the copy is.  The copy stays for stamps of another
+// device and for pointers whose last element is no device memory.
 int first_stamp(const double* st, int64_t n, double* scratch, double* out) {
   int dev = 0;
   cudaPointerAttributes a, z;
