@@ -1872,9 +1872,10 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
 // subtree) node counts in depth-major order.  The roots get their children's indices.
 __global__ void k_deep_place(BNode* nodes, LevelState* ls, int32_t lb, int32_t le, const DeepNode* dn,
                              const int32_t* dn_count, int32_t dn_cap, const int32_t* off, int32_t dcap,
-                             int32_t cap_nodes) {
+                             int32_t cap_nodes, int32_t* alive) {
   grid_begin();
   if (ls->error) return;  // the build fails; records may be missing
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ls->le; i += gridDim.x * blockDim.x) alive[i] = 0;
   const int nroots = le - lb;
   const int nd_total = min(*dn_count, dn_cap);
   const int stride = gridDim.x * blockDim.x;
@@ -1976,13 +1977,20 @@ __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, 
 }
 
 // ---- prune and per-tree compaction -----------------------------------------------------
+// Nodes of a finished build, on the device: the host sizes the launches below by what there can
+// be and does not wait for the subtree pass (a 180,000-point scan: 937 us with the wait, 866
+// without).  A build that failed has none: its records may be
+// incomplete.
+__device__ __forceinline__ int built_nodes(const LevelState* ls) { return ls->error ? 0 : ls->le; }
+
 // Prune in one launch (alive[] zeroed before): a leaf lives if it passes
 // IsGoodLeafPredicate_ (kd/tree/tree_predicates_.h:18-29, in float), an inner node if
 // any child lives, i.e. if a good leaf lies below it (kd/tree/tree_cpu_.h:172-196).  Each
 // good leaf marks its ancestors up to the first one already marked: whoever marks a node
 // first goes on to its parent, so every ancestor ends marked whatever the order.
-__global__ void k_alive(const BNode* nodes, int32_t total, int32_t* alive, float incidence) {
+__global__ void k_alive(const BNode* nodes, const LevelState* ls, int32_t* alive, float incidence) {
   grid_begin();
+  const int total = built_nodes(ls);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const BNode& nd = nodes[i];
     if (nd.left >= 0 || nd.right >= 0) continue;
@@ -2001,9 +2009,10 @@ __global__ void k_alive(const BNode* nodes, int32_t total, int32_t* alive, float
 // Counts per (level, tree) group; lanes with the same group combine their counts
 // before one atomic per group and warp.
 // flags[i]: x = alive, y = alive leaf.
-__global__ void k_group_counts(const BNode* nodes, int32_t total, const int32_t* alive, int R, int32_t* cnt,
+__global__ void k_group_counts(const BNode* nodes, const LevelState* ls, const int32_t* alive, int R, int32_t* cnt,
                                int32_t* lcnt, int32_t* ucnt, int2* flags) {
   grid_begin();
+  const int total = built_nodes(ls);
   const int lane = threadIdx.x & 31;
   for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
@@ -2043,8 +2052,9 @@ __device__ __forceinline__ int2 pair_block_scan(int2 v, int* sm, int2* total) {
   r.y = block_scan(v.y, sm, &total->y);
   return r;
 }
-__global__ void __launch_bounds__(1024) k_flag_tiles(const int2* flags, int32_t n, int2* tiles) {
+__global__ void __launch_bounds__(1024) k_flag_tiles(const int2* flags, const LevelState* ls, int2* tiles) {
   grid_begin();
+  const int n = built_nodes(ls);
   __shared__ int sm[32];
   const int base = blockIdx.x * kFlagTile + threadIdx.x * kFlagItems;
   int2 v = make_int2(0, 0), tot;
@@ -2066,8 +2076,9 @@ __global__ void __launch_bounds__(1024) k_flag_top(int2* tiles, int32_t nt) {
   }
 }
 // tiles == nullptr: one block, a run of pairs per thread.
-__global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, int32_t n, const int2* tiles) {
+__global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, const LevelState* ls, const int2* tiles) {
   grid_begin();
+  const int n = built_nodes(ls);
   __shared__ int sm[32];
   const int items = tiles ? kFlagItems : (n + 1023) / 1024;
   const int b = min((int)(blockIdx.x * 1024 + threadIdx.x) * items, n), e = min(b + items, n);
@@ -2084,10 +2095,11 @@ __global__ void __launch_bounds__(1024) k_flag_scan(int2* flags, int32_t n, cons
 
 // Exclusive prefix over groups in (level, tree) order (one block, scans with carry),
 // and per-tree level offsets (one thread per tree).
-__global__ void k_group_tables(int depth, int R, const int32_t* cnt, const int32_t* lcnt, int32_t* gp, int32_t* lgp,
+__global__ void k_group_tables(const LevelState* state, int R, const int32_t* cnt, const int32_t* lcnt, int32_t* gp, int32_t* lgp,
                                int32_t* to, int32_t* lto, int32_t* tot_nodes, int32_t* tot_leaves) {
   grid_begin();
   __shared__ int sm[32];
+  const int depth = state->error ? 0 : state->depth;
   const int G = depth * R;
   int carry = 0, lcarry = 0;
   for (int base = 0; base < G; base += blockDim.x) {
@@ -2452,7 +2464,8 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
       launch(k_deep_finish, 1, 64, 0, s, w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
     }
     const int pg = (int)std::min<int64_t>(nblk(std::max<int64_t>(w.cap_nodes - le, nroots), kThreads), kGridBlocks * 4);
-    launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes);
+    launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes,
+           w.alive);
     e = cudaGetLastError();
   }
   cudaFreeAsync(blk, s);
@@ -2463,6 +2476,13 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
 }  // namespace
 
 namespace {
+
+// What a finished or abandoned level reports.
+int build_error(const LevelState& h) {
+  if (h.error == 2) { set_error("kds_tree_build: coordinate >= 32768 m, non-finite stamp or dt >= 65536 s"); return KDS_ERR_RANGE; }
+  if (h.error == 1) { set_error("kds_tree_build: node capacity exceeded"); return KDS_ERR_CAPACITY; }
+  return KDS_OK;
+}
 
 // Blocks that write the chunks of one node range: a thread each for a few thousand chunks (one
 // block takes 25 us for 11,000), none but the level's own below.
@@ -2618,7 +2638,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     const bool by_block = host_max <= kBlockMax && level_nodes <= kBlockRoots;
     if (by_block || (host_max <= kDeepMax && level_nodes <= kDeepMaxRoots)) {
       // every node of the current level fits one group's shared memory: the rest of every
-      // subtree is built there, then the host reads the final level state
+      // subtree is built there; the host reads the final level state with the counts below
       if (round == 0) {  // the roots' sums (every root has at most kBig points)
         rc = root_sums(w, R, host_max, N, s);
         if (rc) return rc;
@@ -2626,10 +2646,6 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       global_levels = hls.depth;
       rc = by_block ? deep_pass<16>(w, P, hls, s) : deep_pass<1>(w, P, hls, s);
       if (rc) return rc;
-      KDS_CK(cudaMemcpyAsync(&hls, w.ls, sizeof(LevelState), cudaMemcpyDeviceToHost, s));
-      KDS_CK(cudaStreamSynchronize(s));
-      if (hls.error == 2) { set_error("kds_tree_build: coordinate >= 32768 m, non-finite stamp or dt >= 65536 s"); return KDS_ERR_RANGE; }
-      if (hls.error == 1) { set_error("kds_tree_build: node capacity exceeded"); return KDS_ERR_CAPACITY; }
       break;
     }
     // as many levels to the next look at the level state as halvings still separate the
@@ -2679,33 +2695,37 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     KDS_CK(cudaGetLastError());
     KDS_CK(cudaMemcpyAsync(&hls, w.ls, sizeof(LevelState), cudaMemcpyDeviceToHost, s));
     KDS_CK(cudaStreamSynchronize(s));
-    if (hls.error == 2) { set_error("kds_tree_build: coordinate >= 32768 m, non-finite stamp or dt >= 65536 s"); return KDS_ERR_RANGE; }
-    if (hls.error == 1) { set_error("kds_tree_build: node capacity exceeded"); return KDS_ERR_CAPACITY; }
+    if ((rc = build_error(hls))) return rc;
     if (hls.lb >= hls.le) break;
     host_max = hls.max_size;
     level_nodes = hls.le - hls.lb;
   }
-  if (hls.lb < hls.le) { set_error("kds_tree_build: depth limit"); return KDS_ERR_CAPACITY; }
-  const int depth = hls.depth;
-  const int32_t total = hls.le;
+  const bool deep = global_levels >= 0;
+  if (!deep && hls.lb < hls.le) { set_error("kds_tree_build: depth limit"); return KDS_ERR_CAPACITY; }
+  // most nodes there can be: the launches below take their number from the level state
+  const int64_t bound = deep ? w.cap_nodes : hls.le;
+  const int node_blocks = (int)std::min<int64_t>(nblk(bound, kThreads), kGridBlocks * 4);
   // prune
-  KDS_CK(cudaMemsetAsync(w.alive, 0, sizeof(int32_t) * total, s));
-  launch(k_alive, (int)std::min<int64_t>(nblk(total, kThreads), kGridBlocks * 4), kThreads, 0, s, w.nodes, total, w.alive,
-                                                                                          P.prune_incidence);
-  launch(k_group_counts, nblk(total, kThreads), kThreads, 0, s, w.nodes, total, w.alive, R, w.cnt, w.lcnt, w.ucnt, w.flags);
-  if (total <= kFlagOne) {
-    launch(k_flag_scan, 1, 1024, 0, s, w.flags, total, nullptr);
+  if (!deep) KDS_CK(cudaMemsetAsync(w.alive, 0, sizeof(int32_t) * bound, s));
+  launch(k_alive, node_blocks, kThreads, 0, s, w.nodes, w.ls, w.alive, P.prune_incidence);
+  launch(k_group_counts, node_blocks, kThreads, 0, s, w.nodes, w.ls, w.alive, R, w.cnt, w.lcnt, w.ucnt, w.flags);
+  if (bound <= kFlagOne) {
+    launch(k_flag_scan, 1, 1024, 0, s, w.flags, w.ls, nullptr);
   } else {
-    const int nt = (total + kFlagTile - 1) / kFlagTile;
-    launch(k_flag_tiles, nt, 1024, 0, s, w.flags, total, w.flag_tiles);
+    const int nt = (int)((bound + kFlagTile - 1) / kFlagTile);
+    launch(k_flag_tiles, nt, 1024, 0, s, w.flags, w.ls, w.flag_tiles);
     launch(k_flag_top, 1, 1024, 0, s, w.flag_tiles, nt);
-    launch(k_flag_scan, nt, 1024, 0, s, w.flags, total, w.flag_tiles);
+    launch(k_flag_scan, nt, 1024, 0, s, w.flags, w.ls, w.flag_tiles);
   }
-  launch(k_group_tables, 1, 1024, 0, s, depth, R, w.cnt, w.lcnt, w.gp, w.lgp, w.to, w.lto, w.tot_nodes, w.tot_leaves);
+  launch(k_group_tables, 1, 1024, 0, s, w.ls, R, w.cnt, w.lcnt, w.gp, w.lgp, w.to, w.lto, w.tot_nodes, w.tot_leaves);
+  if (deep) KDS_CK(cudaMemcpyAsync(&hls, w.ls, sizeof(LevelState), cudaMemcpyDeviceToHost, s));
   KDS_CK(cudaMemcpyAsync(h_cnt, w.tot_nodes,
                          (size_t)((char*)(w.ts0 + (size_t)(1 + kRootFrame) * R) - (char*)w.tot_nodes),
                          cudaMemcpyDeviceToHost, s));
   KDS_CK(cudaStreamSynchronize(s));
+  if (deep && (rc = build_error(hls))) return rc;
+  const int depth = hls.depth;
+  const int32_t total = hls.le;
   const std::vector<int32_t> tn(h_cnt, h_cnt + R), tl(h_cnt + R, h_cnt + 2 * R), tu(h_cnt + 2 * R, h_cnt + 3 * R);
   const std::vector<double> ts0(h_dbl, h_dbl + R), rf(h_dbl + R, h_dbl + R + (size_t)kRootFrame * R);
   std::vector<TreeDev> td(R);
