@@ -949,22 +949,69 @@ static_assert(offsetof(BNode, start) == 0 && offsetof(BNode, end) == 4 && offset
                   offsetof(BNode, mean) == 48,
               "BNode head layout");
 
+struct __align__(16) Chunk {
+  int32_t node;
+  int32_t begin;
+  int32_t end;
+  int32_t big;  // ordinal among the level's large nodes
+};
+
+constexpr int kSegs = kThreads / 32;     // 128-point segments per chunk, one per warp of a block
+constexpr int kPer = kChunk / kThreads;  // rounds of 32 points per segment
+static_assert(kPer * kThreads == kChunk && kSegs == 8, "a chunk is eight segments, its counts one 16 B word");
+// Left points of each chunk's eight 128-point segments; a warp per segment, no barrier.
+struct __align__(16) SegCounts {
+  uint16_t n[kSegs];
+};
+__device__ __forceinline__ void big_count(const Chunk* chunks, const LevelState* ls, const BNode* nodes,
+                                          const PointBufs& B, SegCounts* seg, int block, int blocks) {
+  const int nc = ls->num_chunks;
+  const float4* pts = B.p[ls->cur];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int ci = block; ci < nc; ci += blocks) {
+    const Chunk c = chunks[ci];
+    const BNode& nd = nodes[c.node];
+    int nl = 0;
+    if (nd.split) {
+      const int wb = c.begin + w * 32 * kPer;
+      float4 pv[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        if (wb + u * 32 + lane < c.end) pv[u] = pts[wb + u * 32 + lane];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        nl += __popc(__ballot_sync(0xffffffffu, wb + u * 32 + lane < c.end && which_side_f(nd.mean, nd.dir, pv[u])));
+    }
+    if (lane == 0) seg[ci].n[w] = (uint16_t)nl;
+  }
+}
+
 // Warp per node of at most kBig points, after its children are numbered: stable
 // partition by whichSide (or leaf point order), the children's ranges and sums.
 // Latency-bound at deep levels (many small nodes per warp), so each node's record
 // and sums are fetched in one round of loads, one node ahead.  The staged sums
 // (SumStage) leave room for 24 warps per SM: a level of 11.4M points in small nodes takes
 // 298 us at most; with eleven 128-bit terms per lane (124 registers, 16 warps) it took 510.
+// The first count_blocks blocks count the chunks of the large nodes instead (big_count): neither
+// needs the other's results, and a launch less per level takes an 11,000-point scan from 345
+// us to 329 and 32 keyframes from 2.46 ms to 2.34 (with the large nodes' lists written by
+// k_level_children).
 __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
                                                          U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin,
-                                                         unsigned* done) {
+                                                         unsigned* done, const Chunk* chunks, SegCounts* seg,
+                                                         int count_blocks) {
   grid_begin();
+  if ((int)blockIdx.x < count_blocks) {
+    big_count(chunks, ls, nodes, B, seg, blockIdx.x, count_blocks);
+    return;
+  }
+  const int blocks = gridDim.x - count_blocks, block = blockIdx.x - count_blocks;
   const int lb = ls->lb, le = ls->le, cur = ls->cur;
   const float4* pin = B.p[cur];
   float4* pout = B.p[cur ^ 1];
   const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int wslot = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // consecutive nodes on different SMs
+  const int nwarps = (blocks * blockDim.x) >> 5;
+  const int wslot = (threadIdx.x >> 5) * blocks + block;  // consecutive nodes on different SMs
   const bool sum_lane = lane < kSums;                              // holds sum lane
   __shared__ SumStage stage[kThreads / 32];
   SumStage& sg = stage[threadIdx.x >> 5];
@@ -1073,13 +1120,6 @@ __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nod
 }
 
 // ---- large nodes ------------------------------------------------------------------
-struct __align__(16) Chunk {
-  int32_t node;
-  int32_t begin;
-  int32_t end;
-  int32_t big;  // ordinal among the level's large nodes
-};
-
 // Large nodes of the level and their kChunk-point chunks, listed in node order by
 // kLevelBlocks blocks over contiguous node ranges: per-block counts first, then each
 // block writes its list at the prefix of the blocks before it.
@@ -1222,10 +1262,7 @@ __device__ __forceinline__ void block_add_sums(LaneSums& S, int lane, U128 (*sm)
   __syncthreads();
 }
 
-constexpr int kSegs = kThreads / 32;     // 128-point segments per chunk, one per warp of a block
-constexpr int kPer = kChunk / kThreads;  // rounds of 32 points per segment
 constexpr int kFoldChunks = kLanePoints / kPer;
-static_assert(kPer * kThreads == kChunk && kSegs == 8, "a chunk is eight segments, its counts one 16 B word");
 
 // Level 0: the large roots' sums; a block takes a contiguous range of chunks and adds its
 // sums once per root.
@@ -1276,33 +1313,6 @@ __global__ void k_big_to_mom(const LevelState* ls, const int32_t* big_list, cons
     mom[(size_t)big_list[t / kSums] * kSums + t % kSums] = acc[t];
 }
 
-// Left points of each chunk's eight 128-point segments; a warp per segment, no barrier.
-struct __align__(16) SegCounts {
-  uint16_t n[kSegs];
-};
-__global__ void __launch_bounds__(kThreads) k_big_count(const Chunk* chunks, const LevelState* ls, const BNode* nodes,
-                                                        const PointBufs B, SegCounts* seg) {
-  grid_begin();
-  const int nc = ls->num_chunks;
-  const float4* pts = B.p[ls->cur];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int ci = blockIdx.x; ci < nc; ci += gridDim.x) {
-    const Chunk c = chunks[ci];
-    const BNode& nd = nodes[c.node];
-    int nl = 0;
-    if (nd.split) {
-      const int wb = c.begin + w * 32 * kPer;
-      float4 pv[kPer];
-#pragma unroll
-      for (int u = 0; u < kPer; ++u)
-        if (wb + u * 32 + lane < c.end) pv[u] = pts[wb + u * 32 + lane];
-#pragma unroll
-      for (int u = 0; u < kPer; ++u)
-        nl += __popc(__ballot_sync(0xffffffffu, wb + u * 32 + lane < c.end && which_side_f(nd.mean, nd.dir, pv[u])));
-    }
-    if (lane == 0) seg[ci].n[w] = (uint16_t)nl;
-  }
-}
 // The eight counts of a chunk, and their sum before segment w (w = 8: of all).
 __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
   int n = 0;
@@ -1317,8 +1327,8 @@ __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
 // that go to the node's smaller child are summed on the way (the sums of the large node's
 // smaller child).  A block takes a contiguous range of chunks and its warps keep their sums
 // until the range reaches another node: only there do they meet, for one block total and 9
-// atomics.  Bound by issue and memory together: a level of 11.4M points takes 100 us (3.6 TB/s
-// of records read and written).  With eleven 128-bit terms per lane, reduced per warp and
+// atomics.  Bound by issue and memory together: a level of 11.4M points takes 110 us (3.3 TB/s
+// of records read and written; the node offsets included).  With eleven 128-bit terms per lane, reduced per warp and
 // chunk and added with 22 atomics each, it took 235-310 us, and 691 us on the root, where
 // every warp hits the same words; three blocks per SM spill and take 118 us.
 __global__ void __launch_bounds__(kThreads, kScatterPerSM)
@@ -1500,10 +1510,14 @@ static_assert(offsetof(BNode, level) == 8 && offsetof(BNode, tree) == 12 && offs
                   offsetof(BNode, right) == 28 && offsetof(BNode, has_parent) == 32 && offsetof(BNode, par_has) == 36 &&
                   offsetof(BNode, has_prop) == 40 && offsetof(BNode, parent) == 44 && offsetof(BNode, par_prop) == 104,
               "BNode words as level_children writes them");
-__global__ void k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum, int32_t cap) {
+__global__ void __launch_bounds__(kThreads) k_level_children(BNode* nodes, LevelState* ls, const int32_t* bsum,
+                                                             int32_t cap, int plan, const int32_t* bbig, Chunk* chunks,
+                                                             int32_t chunk_cap, int32_t* big_list,
+                                                             int32_t* node_chunk0, ChildSums C) {
   grid_begin();
   __shared__ int sm[32];
   level_children(nodes, ls, bsum, cap, sm);
+  if (plan) level_plan(nodes, ls, bbig, chunks, chunk_cap, big_list, node_chunk0, C.acc[ls->depth & 1], sm, 0, 1);
 }
 
 // A level of at most kThreads nodes: decisions, children and the large nodes' chunks by one
@@ -2678,16 +2692,17 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
                                              plan_parts == 1 ? 1 : 0);
       } else {
         launch(k_decide, lvl_blocks, kThreads, 0, s, w.nodes, w.ls, w.mom, w.accl, P, w.bsum, w.bbig, w.root_frame);
-        launch(k_level_children, lvl_blocks, kThreads, 0, s, w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes);
+        launch(k_level_children, lvl_blocks, kThreads, 0, s, w.nodes, w.ls, w.bsum, (int32_t)w.cap_nodes, big ? 1 : 0,
+               w.bbig, w.chunks, w.chunk_cap, w.big_list, w.node_chunk0, w.accl);
       }
-      if (big && (lvl_blocks > 1 || plan_parts > 1)) {  // the decisions counted the large nodes per block
-        launch(k_big_plan, lvl_blocks * plan_parts, kThreads, 0, s, w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap,
-                                                                w.big_list, w.node_chunk0, nullptr, w.accl, plan_parts);
+      if (big && plan_parts > 1) {  // the decisions counted the large nodes per block
+        launch(k_big_plan, plan_parts, kThreads, 0, s, w.nodes, w.ls, w.bbig, w.chunks, w.chunk_cap, w.big_list,
+               w.node_chunk0, nullptr, w.accl, plan_parts);
       }
-      launch(k_small_part, small_blocks, kThreads, 0, s, w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks, w.level_begin,
-                                                     big ? nullptr : w.done);
+      const int count_blocks = big ? cb : 0;
+      launch(k_small_part, count_blocks + small_blocks, kThreads, 0, s, w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks,
+             w.level_begin, big ? nullptr : w.done, w.chunks, w.seg, count_blocks);
       if (big) {
-        launch(k_big_count, cb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg);
         launch(k_big_scatter, sb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
                                               lvl_blocks, w.level_begin, w.done);
       }
