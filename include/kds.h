@@ -317,8 +317,8 @@ int kds_aligner_get_profile(const kds_aligner* a, double* mean_ms, int32_t* laun
 int kds_aligner_count_touched_nodes(kds_aligner* a, int64_t* count);
 /* SM-clock stamps of the last profiled linearization launch: [0..3] first block
  * (entry, fixed-tree top staged, tile done, partial published), [8..15] the block that
- * ran the Gauss-Newton step (entry, partials summed, state staged, factorization start,
- * factorized, solved, pose updated, done).  Measurement hook only. */
+ * ran the Gauss-Newton step (entry, partials summed, state staged, solve start, unused,
+ * solved, pose updated, done).  Measurement hook only. */
 int kds_phase_stamps(uint64_t out[16]);
 /* Diagnostics hook (no reference counterpart): the number of polls of the bounded wait
  * with which each linearization block waits for its TMA copy of the fixed tree's top

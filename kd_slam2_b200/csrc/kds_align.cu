@@ -1926,9 +1926,9 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   }
   // The kinds' jobs don't depend on each other: the first kind's iterations run on s, the others'
   // beside them, so that one kind's blocks fill the SMs where the other's last tiles and solves
-  // run (a batch of 125 pairs of each kind: 1,735 us
-  // one after the other, 1,455 side by side).  In order where each launch is
-  // timed, and for one launch a kind: 62 us of kernels give less than the stream costs to create.
+  // run (a batch of 125 pairs of each kind: 1,735 us one after the other, 1,455 side by side).
+  // In order where each launch is timed, and for one launch a kind: 62 us of kernels give less
+  // than the stream costs to create.
   const int first = L[0] ? 0 : (L[1] ? 1 : 2);
   const bool fork = !profiling && total > L[first] && nmax > 1;
   if (fork) {

@@ -1328,9 +1328,9 @@ __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
 // smaller child).  A block takes a contiguous range of chunks and its warps keep their sums
 // until the range reaches another node: only there do they meet, for one block total and 9
 // atomics.  Bound by issue and memory together: a level of 11.4M points takes 110 us (3.3 TB/s
-// of records read and written; the node offsets included).  With eleven 128-bit terms per lane, reduced per warp and
-// chunk and added with 22 atomics each, it took 235-310 us, and 691 us on the root, where
-// every warp hits the same words; three blocks per SM spill and take 118 us.
+// of records read and written; the node offsets included).  With eleven 128-bit terms per lane,
+// reduced per warp and chunk and added with 22 atomics each, it took 235-310 us, and 691 us on
+// the root, where every warp hits the same words; three blocks per SM spill and take 118 us.
 __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     k_big_scatter(const Chunk* chunks, LevelState* ls, BNode* nodes, PointBufs B, const SegCounts* seg,
                   const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t* level_begin,
@@ -1993,8 +1993,7 @@ __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, 
 // ---- prune and per-tree compaction -----------------------------------------------------
 // Nodes of a finished build, on the device: the host sizes the launches below by what there can
 // be and does not wait for the subtree pass (a 180,000-point scan: 937 us with the wait, 866
-// without).  A build that failed has none: its records may be
-// incomplete.
+// without).  A build that failed has none: its records may be incomplete.
 __device__ __forceinline__ int built_nodes(const LevelState* ls) { return ls->error ? 0 : ls->le; }
 
 // Prune in one launch (alive[] zeroed before): a leaf lives if it passes

@@ -183,8 +183,7 @@ __global__ void k_import_msg(TreeDev t, const kds_kdnode3f* rec, int32_t* flag, 
 
 // Device node arrays -> KDNode3f records.  One packed copy crosses to the host instead of four
 // arrays and a loop over the nodes there, whose 100 bytes a node of fresh vectors cost more in
-// page faults than the copies (64 x 1,024 returns,
-// both ways: 362 us to 238).
+// page faults than the copies (64 x 1,024 returns, both ways: 362 us to 238).
 __global__ void k_export_msg(TreeDev t, kds_kdnode3f* rec) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= t.num_nodes) return;
