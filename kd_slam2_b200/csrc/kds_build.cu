@@ -2019,16 +2019,29 @@ __global__ void k_alive(const BNode* nodes, const LevelState* ls, int32_t* alive
 }
 
 // group = (level, tree); nodes of one group are contiguous in global order
-// Counts per (level, tree) group; lanes with the same group combine their counts
-// before one atomic per group and warp.
+// Counts per (level, tree) group.  A block takes a contiguous range of nodes and keeps its
+// counts while they stay in one group (2.1M nodes of one tree: 71 us, 85 with the warps'
+// atomics meeting at the same three words); in rows of several groups, lanes with the
+// same group combine theirs before one atomic per group and warp.
 // flags[i]: x = alive, y = alive leaf.
-__global__ void k_group_counts(const BNode* nodes, const LevelState* ls, const int32_t* alive, int R, int32_t* cnt,
-                               int32_t* lcnt, int32_t* ucnt, int2* flags) {
+__global__ void __launch_bounds__(kThreads) k_group_counts(const BNode* nodes, const LevelState* ls,
+                                                           const int32_t* alive, int R, int32_t* cnt, int32_t* lcnt,
+                                                           int32_t* ucnt, int2* flags) {
   grid_begin();
   const int total = built_nodes(ls);
   const int lane = threadIdx.x & 31;
-  for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
-    const int i = base + threadIdx.x;
+  const int rows = (total + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int row0 = blockIdx.x * per, row1 = min(row0 + per, rows);
+  int hg = -1, ht = 0, hn = 0, hc = 0, hl = 0;  // the group held, its tree, nodes, alive nodes and leaves
+  auto put = [&]() {
+    if (hg < 0 || threadIdx.x != 0) return;
+    atomicAdd(&ucnt[ht], hn);
+    if (hc) atomicAdd(&cnt[hg], hc);
+    if (hl) atomicAdd(&lcnt[hg], hl);
+  };
+  for (int row = row0; row < row1; ++row) {
+    const int base = row * (int)blockDim.x, i = base + (int)threadIdx.x;
     const bool valid = i < total;
     int tree = -1, g = -1;
     bool al = false, leaf = false;
@@ -2039,6 +2052,20 @@ __global__ void k_group_counts(const BNode* nodes, const LevelState* ls, const i
       al = alive[i] != 0;
       leaf = al && nd.left < 0 && nd.right < 0;
       flags[i] = make_int2(al ? 1 : 0, leaf ? 1 : 0);
+    }
+    const int t0 = nodes[base].tree, g0 = nodes[base].level * R + t0;
+    if (__syncthreads_and(!valid || g == g0)) {
+      const int c = __syncthreads_count(al), l = __syncthreads_count(leaf);
+      if (g0 != hg) {
+        put();
+        hg = g0;
+        ht = t0;
+        hn = hc = hl = 0;
+      }
+      hn += min((int)blockDim.x, total - base);
+      hc += c;
+      hl += l;
+      continue;
     }
     const unsigned pt = __match_any_sync(0xffffffffu, tree);
     if (valid && lane == __ffs(pt) - 1) atomicAdd(&ucnt[tree], __popc(pt));
@@ -2051,6 +2078,7 @@ __global__ void k_group_counts(const BNode* nodes, const LevelState* ls, const i
       if (lc) atomicAdd(&lcnt[g], lc);
     }
   }
+  put();
 }
 
 // Exclusive scan of the flag pairs (both at once), in place: tiles of kFlagTile pairs, their
@@ -2306,10 +2334,19 @@ __global__ void k_finish_trees(TreeDev* trees, const int64_t* off, const int32_t
   const int r = blockIdx.y;
   TreeDev& T = trees[r];
   if (T.nodes == nullptr) return;
-  const int64_t o0 = off[r];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.num_points;
-       i += (int64_t)gridDim.x * blockDim.x)
-    T.perm[i] = perm_final[o0 + i] - (int32_t)o0;
+  const int64_t o0 = off[r], n = T.num_points;
+  int32_t* out = T.perm;  // read once: the writes could be to the record itself otherwise
+  const int32_t* in = perm_final + o0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    int32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = in[i + k * stride];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[i + k * stride] = v[k] - (int32_t)o0;
+  }
+  for (; i < n; i += stride) out[i] = in[i] - (int32_t)o0;
 }
 
 inline int nblk(int64_t n, int t) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + t - 1) / t, 1 << 20)); }
