@@ -1,0 +1,15 @@
+// Rules that choose between two forms of a call, as plain host functions (no CUDA), so that they
+// can be checked without a device.
+#pragma once
+
+namespace kds {
+
+// Whether a request's first stamp is found by a kernel on the calling thread's device: the
+// scratch that the kernel writes is the server's, so the caller, the server and both ends of
+// the stamps must be on one device.  Between two devices the pointers of one are not the
+// other's to read or write; the host copy works from any of them.
+inline bool first_stamp_on_device(int current, int server, int first, int last) {
+  return current == server && first == server && last == server;
+}
+
+}  // namespace kds

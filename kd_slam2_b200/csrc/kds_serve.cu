@@ -49,6 +49,7 @@
 
 #include "kds_align.cuh"
 #include "kds_internal.cuh"
+#include "kds_rules.h"
 
 namespace kds {
 
@@ -104,15 +105,16 @@ __global__ void __launch_bounds__(1024) k_first_stamp(const double* __restrict__
 
 // The first stamp of n device stamps.  Reading the stamps back and searching them on the host took
 // 180 us a request (65,536 points); the kernel and 8 bytes take 40.  On the legacy stream, after
-// the work of every blocking stream, as the copy is.  The copy stays for stamps of another
-// device and for pointers whose last element is no device memory.
-int first_stamp(const double* st, int64_t n, double* scratch, double* out) {
+// the work of every blocking stream, as the copy is.  The copy stays where the caller or the
+// stamps are on another device than the server's (device; scratch is there) and for pointers
+// whose last element is no device memory.
+int first_stamp(const double* st, int64_t n, int device, double* scratch, double* out) {
   int dev = 0;
   cudaPointerAttributes a, z;
   const bool here = scratch && ((uintptr_t)st & 7) == 0 && cudaGetDevice(&dev) == cudaSuccess &&
                     cudaPointerGetAttributes(&a, st) == cudaSuccess &&
-                    cudaPointerGetAttributes(&z, st + (n - 1)) == cudaSuccess && a.device == dev && z.device == dev &&
-                    z.type == cudaMemoryTypeDevice;
+                    cudaPointerGetAttributes(&z, st + (n - 1)) == cudaSuccess &&
+                    first_stamp_on_device(dev, device, a.device, z.device) && z.type == cudaMemoryTypeDevice;
   if (!here) {
     cudaGetLastError();
     std::vector<double> hs((size_t)n);
@@ -1280,7 +1282,7 @@ int kds_server_submit(kds_server* s, const kds_request* req, int64_t* ticket) {
     else
       cudaGetLastError();
     if (dev_stamps) {
-      const int rc = first_stamp(req->stamps, req->n, s->d_t0, &t0);
+      const int rc = first_stamp(req->stamps, req->n, s->device, s->d_t0, &t0);
       if (rc) return rc;
     } else {
       t0 = req->stamps[0];

@@ -1,0 +1,14 @@
+// Prints the decisions of kds_rules.h for the arguments given, one per line.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "kds_rules.h"
+
+int main(int argc, char** argv) {
+  if (argc == 6 && !strcmp(argv[1], "first_stamp")) {
+    std::printf("%d\n", kds::first_stamp_on_device(atoi(argv[2]), atoi(argv[3]), atoi(argv[4]), atoi(argv[5])) ? 1 : 0);
+    return 0;
+  }
+  return 2;
+}

@@ -1,0 +1,32 @@
+"""The host rules of kds_rules.h, without a device."""
+import itertools
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not available")
+    out = str(tmp_path_factory.mktemp("rules") / "rules_main")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wextra", "-Werror", "-I",
+                    os.path.join(ROOT, "kd_slam2_b200", "csrc"), os.path.join(ROOT, "tests", "cpp", "rules_main.cpp"),
+                    "-o", out], check=True, capture_output=True, text=True)
+
+    def call(*args):
+        r = subprocess.run([out, *map(str, args)], check=True, capture_output=True, text=True)
+        return [int(x) for x in r.stdout.split()]
+    return call
+
+
+def test_first_stamp_kernel_runs_on_the_servers_device_only(rules):
+    """The kernel's scratch is on the server's device: a caller whose current device and arrays
+    are on another one takes the copy (the kernel would write memory that it cannot reach)."""
+    for current, server, first, last in itertools.product((0, 1), repeat=4):
+        same = current == server == first == last
+        assert rules("first_stamp", current, server, first, last) == [1 if same else 0]
