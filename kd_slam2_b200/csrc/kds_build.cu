@@ -905,16 +905,25 @@ __global__ void k_decide(BNode* nodes, const LevelState* ls, U128* mom, ChildSum
 }
 
 // The level's split count from k_decide's per-block counts, then the next level (one
-// whole block).
-__device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nblocks, int32_t* level_begin) {
+// whole block).  Children that don't fit the node arrays have no records: the build has failed,
+// and the levels to come before the host looks are empty (every kernel takes its nodes from
+// [lb, le)).
+__device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nblocks, int32_t cap,
+                                    int32_t* level_begin) {
   __shared__ int sm[32];
   int v = 0;
   for (int k = threadIdx.x; k < nblocks; k += blockDim.x) v += bsum[k];
   int total;
   block_scan(v, sm, &total);
   if (threadIdx.x != 0 || ls->lb >= ls->le) return;
+  const bool fits = 2 * total <= cap - ls->le;
   ls->lb = ls->le;
-  ls->le = ls->le + 2 * total;
+  if (fits) {
+    ls->le += 2 * total;
+  } else {
+    ls->error = 1;
+    ls->max_next = 0;
+  }
   ls->cur ^= 1;
   ls->depth += 1;
   if (ls->depth < kMaxDepth + 1) level_begin[ls->depth] = ls->lb;
@@ -925,7 +934,7 @@ __device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nbl
 // The last block of the level's last kernel advances the level (done: a counter that
 // starts at 0 and is left at 0; nullptr: not the last kernel).  Every block of the
 // calling kernel must reach this.
-__device__ __forceinline__ void advance_if_last(LevelState* ls, const int32_t* bsum, int nblocks,
+__device__ __forceinline__ void advance_if_last(LevelState* ls, const int32_t* bsum, int nblocks, int32_t cap,
                                                 int32_t* level_begin, unsigned* done) {
   if (!done) return;
   __shared__ int s_last;
@@ -937,7 +946,7 @@ __device__ __forceinline__ void advance_if_last(LevelState* ls, const int32_t* b
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  level_advance_block(ls, bsum, nblocks, level_begin);
+  level_advance_block(ls, bsum, nblocks, cap, level_begin);
   if (threadIdx.x == 0) *done = 0u;
 }
 
@@ -997,7 +1006,7 @@ __device__ __forceinline__ void big_count(const Chunk* chunks, const LevelState*
 // us to 329 and 32 keyframes from 2.46 ms to 2.34 (with the large nodes' lists written by
 // k_level_children).
 __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
-                                                         U128* mom, const int32_t* bsum, int nblocks, int32_t* level_begin,
+                                                         U128* mom, const int32_t* bsum, int nblocks, int32_t cap, int32_t* level_begin,
                                                          unsigned* done, const Chunk* chunks, SegCounts* seg,
                                                          int count_blocks) {
   grid_begin();
@@ -1116,7 +1125,7 @@ __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nod
     }
   }
   if (lane == 0 && maxc > 0) atomicMax(&ls->max_next, maxc);
-  advance_if_last(ls, bsum, nblocks, level_begin, done);
+  advance_if_last(ls, bsum, nblocks, cap, level_begin, done);
 }
 
 // ---- large nodes ------------------------------------------------------------------
@@ -1333,7 +1342,7 @@ __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
 // the root, where every warp hits the same words; three blocks per SM spill and take 118 us.
 __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     k_big_scatter(const Chunk* chunks, LevelState* ls, BNode* nodes, PointBufs B, const SegCounts* seg,
-                  const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t* level_begin,
+                  const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t cap, int32_t* level_begin,
                   unsigned* done) {
   grid_begin();
   __shared__ U128 smm[kSegs][kSums];
@@ -1441,7 +1450,7 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     }
   }
   if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, per == 1);
-  advance_if_last(ls, bsum, nblocks, level_begin, done);
+  advance_if_last(ls, bsum, nblocks, cap, level_begin, done);
 }
 
 // ---- children ------------------------------------------------------------------------
@@ -2752,10 +2761,10 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       }
       const int count_blocks = big ? cb : 0;
       launch(k_small_part, count_blocks + small_blocks, kThreads, 0, s, w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks,
-             w.level_begin, big ? nullptr : w.done, w.chunks, w.seg, count_blocks);
+             (int32_t)w.cap_nodes, w.level_begin, big ? nullptr : w.done, w.chunks, w.seg, count_blocks);
       if (big) {
         launch(k_big_scatter, sb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
-                                              lvl_blocks, w.level_begin, w.done);
+                                              lvl_blocks, (int32_t)w.cap_nodes, w.level_begin, w.done);
       }
     }
     KDS_CK(cudaGetLastError());

@@ -108,6 +108,37 @@ def test_degenerate_inputs(scene):
     assert_same_tree(O, G)
 
 
+@pytest.mark.parametrize("clusters,pile,fits", [
+    (60, 0, True),        # a subtree pass from the first level
+    (60, 3000, True),     # the pile of equal points keeps the level kernels running to the last level
+    (200, 0, False),      # too many nodes: in the subtree pass by blocks
+    (30000, 0, False),    # ... by warps
+    (40000, 600, False),  # in the level kernels of small nodes, some levels before the host looks
+    (2000, 3000, False),  # ... with a large node beside them
+    (5000, 70000, False),
+])
+def test_clouds_of_equal_points(clusters, pile, fits):
+    """More than leaf_max_points equal points split at every level down to max_level, with one
+    empty child each: the trees equal the oracle's while their nodes fit the build's arrays,
+    and the build reports KDS_ERR_CAPACITY (and goes on to work) where they don't."""
+    import kd_slam2_b200 as kds
+    rng = np.random.default_rng(clusters + pile)
+    xyz = np.repeat(rng.uniform(-40.0, 40.0, (clusters, 3)).astype(np.float32), 20, axis=0)
+    xyz = np.concatenate([rng.permutation(xyz), np.zeros((pile, 3), np.float32)])
+    gen = kds.TreeGeneratorB2003D(leaf_max_points=16, tree_min_good_leaves=1)
+    if fits:
+        O = orc.OTree.build(xyz, None, orc.tree_params(leaf_max_points=16, tree_min_good_leaves=1))
+        G = gen.make_tree(xyz)
+        assert O.accepted == (G is not None)
+        if G is not None:
+            assert_same_tree(O, G)
+        return
+    with pytest.raises(kds.KdsError) as ei:
+        gen.make_tree(xyz)
+    assert ei.value.code == kds.abi.KDS_ERR_CAPACITY
+    assert gen.make_tree(rng.uniform(-40.0, 40.0, (5000, 3)).astype(np.float32)) is not None
+
+
 def test_out_of_range_input_is_rejected_with_status():
     import kd_slam2_b200 as kds
     xyz = np.zeros((100, 3), np.float32)
