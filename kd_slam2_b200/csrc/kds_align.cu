@@ -2060,6 +2060,10 @@ int Runner::run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg
   key.push_back(order_by_size);
   key.push_back(persistent);
   key.push_back(pair_tiles);
+  // two tiles per block: a kind's blocks are not determined by its tiles (3 + 1 tiles of two jobs
+  // make three, 2 + 2 make two)
+  if (pair_tiles)
+    for (int k = 0; k < 3; ++k) { key.push_back(kind_pair_begin[k]); key.push_back(kind_pair_count[k]); }
   if (key != graph_key) {
     // capture only a shape that repeats: a one-off shape (every call of a stream of
     // different scans) costs less launched directly than captured and instantiated

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 import kd_slam2_b200 as kds
+from kd_slam2_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -84,6 +85,44 @@ def test_every_configuration_gives_identical_results(workload, config):
     b.configure(config)
     for _ in range(3):  # direct, graph capture, graph replay
         same(ref, outputs(b.run(jobs, use_graph=True)))
+
+
+@pytest.mark.parametrize("first,then", [((2, 2), (3, 1)), ((3, 1), (2, 2)), ((3, 3, 1), (4, 2, 1))])
+@pytest.mark.parametrize("kind", ["icp", "ct"])
+def test_two_tile_blocks_of_another_split_of_the_same_tiles(workload, first, then, kind):
+    """With two tiles per block, batches of as many jobs, tiles and iterations can need different
+    numbers of blocks: the graph of one must not be replayed for the other."""
+    _, trees = workload
+    cls, code = (kds.CTICPB2003D, kds.abi.KDS_CTICP) if kind == "ct" else (kds.ICPB2003D, kds.abi.KDS_ICP)
+    prm = CT if kind == "ct" else ICP
+    fixed, e = trees[0], trees[1].export()
+    leaf = e["leaves"]
+
+    def moving(tiles):  # a left-deep chain of 128 surfels a tile, the last one not full
+        n = 128 * tiles - 5
+        m, d = np.zeros((2 * n - 1, 3), np.float32), np.tile(np.float32([0, 0, 1]), (2 * n - 1, 1))
+        left, right = np.full(2 * n - 1, -1, np.int32), np.full(2 * n - 1, -1, np.int32)
+        inner = np.arange(0, 2 * n - 2, 2)
+        left[inner], right[inner] = inner + 1, inner + 2
+        m[left < 0], d[left < 0] = e["mean"][np.resize(leaf, n)], e["dir"][np.resize(leaf, n)]
+        return kds.Tree.import_nodes(m, d, left, right)
+    made = {t: moving(t) for t in set(first + then)}
+    a = cls(**prm)
+    X0 = [synth.pose((0.03 * k, 0.02, 0.0), (0.0, 0.0, 0.004 * k)) for k in range(len(first))]
+    alone = {}
+    for t in made:
+        for k, X in enumerate(X0):
+            a.set_fixed(fixed)
+            a.set_moving(made[t])
+            a.set_x(X)
+            a.set_velocities(np.zeros(6))
+            r = a.compute()
+            alone[t, k] = (r, a.get_x().reshape(12), a.velocities(), a.stats["num_inliers"])
+    b = kds.Batch()
+    b.configure(12)  # two tiles per block
+    for tiles in (first, first, first, then, then, then):  # direct, captured, replayed
+        out = b.run([kds.make_job(code, fixed, made[t], a.params, X=X) for t, X in zip(tiles, X0)])
+        same([alone[t, k] for k, t in enumerate(tiles)], outputs(out))
 
 
 def test_autotune_as_first_use_of_the_library(tmp_path):
