@@ -30,6 +30,7 @@
 
 #include "kds_align.cuh"
 #include "kds_internal.cuh"
+#include "kds_rules.h"
 
 namespace kds {
 
@@ -1328,7 +1329,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_linearize_persistent(const JobIn*
 // blocks: 29,000 cycles, of which the tile 12,300 and the step's FP64 chain 13,000).
 constexpr int kClusterThreads = 512;
 constexpr int kClusterGroups = kClusterThreads / kBlock;  // tiles at a time per block, at most
-constexpr int kClusterMax = 16;                           // blocks per cluster (8 is the portable size)
 constexpr int kClusterTiles = 64;
 
 // Shared memory of a block: this, then the warps' partials, the tiles' partials (used in the
@@ -1971,7 +1971,7 @@ bool cluster_fits(const JobIn& J, bool profiling) {
 }
 
 template <int KIND>
-static int launch_cluster(const JobIn& J, const LinDev& L, int stage, int max_blocks, ClusterOut* res,
+static cudaError_t launch_cluster(const JobIn& J, const LinDev& L, int stage, int max_blocks, ClusterOut* res,
                           cudaStream_t s) {
   // as many blocks as tiles, up to the largest cluster that the device schedules: fewer warps
   // per SM to share its issue slots, and more of its L1 per tile for the lower tree levels
@@ -1993,58 +1993,74 @@ static int launch_cluster(const JobIn& J, const LinDev& L, int stage, int max_bl
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  KDS_CK(cudaLaunchKernelEx(&cfg, k_align_cluster<KIND>, J, L, stage, res));
-  count_launch();
-  return KDS_OK;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_align_cluster<KIND>, J, L, stage, res);
+  if (e == cudaSuccess) count_launch();
+  return e;
 }
 
 // Sets the cluster kernels' limits (always to the same values: they belong to the process) and
-// asks for the largest cluster that this device schedules: 16 need its leave, 8 always fit.
+// asks for the largest cluster that this device schedules; 0 for none.
 constexpr int kClusterSmemMax = 200 * 1024;  // 172 KB at 64 CT tiles and 2,047 staged nodes
-static int cluster_setup(int* max_blocks) {
+static int cluster_setup() {
   const void* fs[2] = {(const void*)k_align_cluster<0>, (const void*)k_align_cluster<1>};
-  for (const void* f : fs) {
-    KDS_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax));
-    KDS_CK(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kClusterMax);
-  cfg.blockDim = dim3(kClusterThreads);
-  cfg.dynamicSmemBytes = kClusterSmemMax;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kClusterMax;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  *max_blocks = 8;
-  if (cudaOccupancyMaxActiveClusters(&n, k_align_cluster<1>, &cfg) == cudaSuccess && n > 0) *max_blocks = kClusterMax;
-  else cudaGetLastError();
-  return KDS_OK;
+  for (const void* f : fs)
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+  return largest_cluster([](int blocks) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = kClusterSmemMax;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_align_cluster<1>, &cfg) == cudaSuccess) return n > 0;
+    cudaGetLastError();
+    return false;
+  });
 }
 
-int Runner::run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log) {
-  if (!h_cluster) {
-    KDS_CK(cudaHostAlloc((void**)&h_cluster, sizeof(ClusterOut), cudaHostAllocMapped));
-    memset(h_cluster, 0, sizeof(ClusterOut));
+bool Runner::cluster_ready() {
+  if (cluster_blocks >= 0) return cluster_blocks > 0;
+  cluster_blocks = cluster_setup();
+  if (cluster_blocks == 0) return false;
+  if (cudaHostAlloc((void**)&h_cluster, sizeof(ClusterOut), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&d_cluster, h_cluster, 0) != cudaSuccess) {
+    cudaGetLastError();
+    cluster_blocks = 0;
+    return false;
   }
-  ClusterOut* d = nullptr;
-  KDS_CK(cudaHostGetDevicePointer((void**)&d, h_cluster, 0));
+  memset(h_cluster, 0, sizeof(ClusterOut));
+  return true;
+}
+
+bool Runner::run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log, int* rc) {
+  if (!cluster_ready()) return false;
   J.tile_begin = 0;
   J.tile_count = (J.m_num_leaves + kBlock - 1) / kBlock;
   J.lin_begin = 0;
-  if (!cluster_blocks) {
-    const int rc = cluster_setup(&cluster_blocks);
-    if (rc) { cluster_blocks = 0; return rc; }
+  cudaError_t e = J.kind == 0 ? launch_cluster<0>(J, L, stage_nodes, cluster_blocks, d_cluster, s)
+                              : launch_cluster<1>(J, L, stage_nodes, cluster_blocks, d_cluster, s);
+  if (e != cudaSuccess) {  // not started; an error of the device itself comes back with the next call
+    cudaGetLastError();
+    return false;
   }
-  int rc = J.kind == 0 ? launch_cluster<0>(J, L, stage_nodes, cluster_blocks, d, s)
-                       : launch_cluster<1>(J, L, stage_nodes, cluster_blocks, d, s);
-  if (rc) return rc;
-  KDS_CK(cudaStreamSynchronize(s));
+  e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) {
+    *rc = cuda_status(e, "single alignment", __FILE__, __LINE__);
+    return true;
+  }
   *out = h_cluster->out;
   if (log) log->assign(h_cluster->log, h_cluster->log + kMaxLog);
-  return timeout_status(h_cluster->err);
+  *rc = timeout_status(h_cluster->err);
+  return true;
 }
 
 int Runner::run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg_status) {

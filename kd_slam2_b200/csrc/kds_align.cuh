@@ -140,7 +140,8 @@ struct Runner {
   // (k_linearize_pair); ignored by the persistent form
   int pair_tiles = 0;
   ClusterOut* h_cluster = nullptr;  // results of run_cluster
-  int cluster_blocks = 0;           // largest cluster (0: not asked yet)
+  ClusterOut* d_cluster = nullptr;  // ... as the device sees them
+  int cluster_blocks = -1;          // largest cluster; 0: none, -1: not asked yet
   cudaStream_t side = nullptr;      // launches of a second kind of jobs
   cudaEvent_t fork_ev[2] = {};
   bool smem_attr_set = false;
@@ -162,8 +163,10 @@ struct Runner {
   void enqueue_kind(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status);
   int run(cudaStream_t s, bool use_graph, int32_t* dbg_match, int32_t* dbg_status);
   int fetch(cudaStream_t s, std::vector<JobOut>& outs, std::vector<kds_stats>* logs);
-  // one job in one cluster launch (cluster_fits); waits for it
-  int run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log);
+  // one job in one cluster launch (cluster_fits); waits for it.  Returns false, with nothing run,
+  // where the device has no room for the cluster or its results: then setup, run and fetch.
+  bool run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log, int* rc);
+  bool cluster_ready();
   ~Runner();
 };
 

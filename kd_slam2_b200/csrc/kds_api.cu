@@ -515,16 +515,16 @@ static int run_single(kds_aligner* a, int kind, int mode, int stats_mode, int ma
   }
   cudaStream_t s = a->stream ? a->stream : cudaStreamPerThread;
   std::vector<JobOut> outs(1);
-  if (!dbg_match && cluster_fits(jobs[0], a->runner.profiling)) {
-    rc = a->runner.run_cluster(jobs[0], lins[0], s, &outs[0], &a->log);
-    if (rc && rc != KDS_ERR_TIMEOUT) return rc;
+  if (!dbg_match && cluster_fits(jobs[0], a->runner.profiling) &&
+      a->runner.run_cluster(jobs[0], lins[0], s, &outs[0], &a->log, &rc)) {
+    if (rc && rc != KDS_ERR_TIMEOUT) return rc;  // a timeout still delivers valid outputs
   } else {
     rc = a->runner.setup(jobs, lins, s);
     if (rc) return rc;
     rc = a->runner.run(s, use_graph, dbg_match, dbg_status);
     if (rc) return rc;
     rc = a->runner.fetch(s, outs, mode == KDS_JOB_COMPUTE ? &a->log : nullptr);
-    if (rc && rc != KDS_ERR_TIMEOUT) return rc;  // a timeout still delivers valid outputs
+    if (rc && rc != KDS_ERR_TIMEOUT) return rc;
   }
   a->out = outs[0];
   if (mode == KDS_JOB_COMPUTE) {

@@ -12,4 +12,12 @@ inline bool first_stamp_on_device(int current, int server, int first, int last) 
   return current == server && first == server && last == server;
 }
 
+// Blocks of the largest cluster that the device schedules (fits(n)), 0 for none: 16 where it
+// gives leave, else the portable 8.  A device that is shared or partitioned may have room for
+// neither beside the shared memory that a block needs.
+template <class Fits>
+int largest_cluster(Fits fits) {
+  return fits(16) ? 16 : (fits(8) ? 8 : 0);
+}
+
 }  // namespace kds

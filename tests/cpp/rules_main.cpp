@@ -10,5 +10,9 @@ int main(int argc, char** argv) {
     std::printf("%d\n", kds::first_stamp_on_device(atoi(argv[2]), atoi(argv[3]), atoi(argv[4]), atoi(argv[5])) ? 1 : 0);
     return 0;
   }
+  if (argc == 3 && !strcmp(argv[1], "cluster")) {  // the largest size that fits
+    std::printf("%d\n", kds::largest_cluster([&](int n) { return n <= atoi(argv[2]); }));
+    return 0;
+  }
   return 2;
 }

@@ -30,3 +30,10 @@ def test_first_stamp_kernel_runs_on_the_servers_device_only(rules):
     for current, server, first, last in itertools.product((0, 1), repeat=4):
         same = current == server == first == last
         assert rules("first_stamp", current, server, first, last) == [1 if same else 0]
+
+
+@pytest.mark.parametrize("room,blocks", [(0, 0), (7, 0), (8, 8), (15, 8), (16, 16), (64, 16)])
+def test_alignments_need_no_cluster(rules, room, blocks):
+    """Where the device schedules no cluster the rule says so (and an alignment is launched once
+    per iteration) instead of assuming that the portable size always fits."""
+    assert rules("cluster", room) == [blocks]
