@@ -485,12 +485,6 @@ __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b
 __device__ __forceinline__ double ddot3(double a0, double a1, double a2, double b0, double b1, double b2) {
   return da(dm(a0, b0), da(dm(a1, b1), dm(a2, b2)));
 }
-__device__ void iso_mul_d(const double* A, const double* B, double* C) {
-  for (int i = 0; i < 3; ++i) {
-    for (int j = 0; j < 3; ++j) C[i * 4 + j] = ddot3(A[i * 4], A[i * 4 + 1], A[i * 4 + 2], B[j], B[4 + j], B[8 + j]);
-    C[i * 4 + 3] = da(ddot3(A[i * 4], A[i * 4 + 1], A[i * 4 + 2], B[3], B[7], B[11]), A[i * 4 + 3]);
-  }
-}
 // Canonical FP64 sine/cosine (this project's own, shared with the CPU oracle so that the
 // pose update is bit-identical there): Cody-Waite reduction by pi/2 with a three-part
 // constant (Cody & Waite 1980; parts of 33, 33 and 53 bits, so q * C1 and q * C2 are
@@ -549,92 +543,91 @@ __device__ __forceinline__ void rodrigues_d(const double* w, double* R) {
       R[i * 3 + j] = da(da((i == j) ? 1.0 : 0.0, dm(s, S[i * 3 + j])), dm(omc, s2));
     }
 }
-__device__ void logso3_d(const double* X, double* w) {
-  double tr = X[0] + X[5] + X[10];
-  double ca = fmin(1.0, fmax(-1.0, 0.5 * (tr - 1.0)));
-  double a = acos(ca);
-  double ax[3] = {X[9] - X[6], X[2] - X[8], X[4] - X[1]};
-  double f = (a < 1e-7) ? 0.5 : a / (2.0 * sin(a));
-  for (int i = 0; i < 3; ++i) w[i] = ax[i] * f;
-}
-// dPoseToPoseError (kd/utils/geometry_3d_impl_.h:125-140) in FP64
-__device__ void dpose_d(const double* ZXi, const double* Xm, double* e, double J[6][6]) {
-  double P[12];
-  iso_mul_d(ZXi, Xm, P);
-  for (int i = 0; i < 3; ++i) e[i] = P[i * 4 + 3];
-  logso3_d(P, e + 3);
-  double R[9] = {ZXi[0], ZXi[1], ZXi[2], ZXi[4], ZXi[5], ZXi[6], ZXi[8], ZXi[9], ZXi[10]};
-  double B[12][6];
-  for (int i = 0; i < 12; ++i) for (int j = 0; j < 6; ++j) B[i][j] = 0.0;
-  auto skewmul = [&](const double* v, double* out) {  // out = R * skew(v)
-    double S[9] = {0, -v[2], v[1], v[2], 0, -v[0], -v[1], v[0], 0};
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) out[i * 3 + j] = R[i * 3] * S[j] + R[i * 3 + 1] * S[3 + j] + R[i * 3 + 2] * S[6 + j];
-  };
-  double t[3] = {Xm[3], Xm[7], Xm[11]};
-  double RS[9];
-  skewmul(t, RS);
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) { B[i][j] = R[i * 3 + j]; B[i][3 + j] = -RS[i * 3 + j]; }
-  for (int k = 0; k < 3; ++k) {
-    double col[3] = {Xm[k], Xm[4 + k], Xm[8 + k]};
-    skewmul(col, RS);
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) B[3 + 3 * k + i][3 + j] = -RS[i * 3 + j];
-  }
-  // dlogSO3 of P's rotation (column-major coefficient order)
-  double ax[3] = {P[9] - P[6], P[2] - P[8], P[4] - P[1]};
-  double tr = P[0] + P[5] + P[10];
-  double ca = fmin(1.0, fmax(-1.0, 0.5 * (tr - 1.0)));
-  double a = acos(ca);
-  bool small = a < 1e-7;
-  double f = small ? 0.5 : a / (2.0 * sin(a));
-  double Js[3][9];
-  for (int i = 0; i < 3; ++i) for (int j = 0; j < 9; ++j) Js[i][j] = 0.0;
-  Js[0][5] = f; Js[0][7] = -f;
-  Js[1][6] = f; Js[1][2] = -f;
-  Js[2][1] = f; Js[2][3] = -f;
-  if (!small) {
-    double s = sin(a);
-    double c = (s - a * cos(a)) / (4.0 * s * s * s);
-    for (int k = 0; k < 3; ++k) { Js[k][0] -= c * ax[k]; Js[k][4] -= c * ax[k]; Js[k][8] -= c * ax[k]; }
-  }
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) {
-      double acc = 0.0;
-      if (i < 3) acc = B[i][j];
-      else for (int k = 0; k < 9; ++k) acc += Js[i - 3][k] * B[3 + k][j];
-      J[i][j] = acc;
-    }
-}
-
-// Pose prior (posePriorBuildQuadraticForm, kd/icp/tree_aligner_base_.h:139-152): adds
-// J^T Omega J and J^T Omega e to the pose block.  Single thread, used by the localizer.
-__device__ __noinline__ void add_pose_prior(const JobIn& Jn, const double* X, double* H, double* b, int D) {
-  double e6[6], Jp[6][6];
-  dpose_d(Jn.prior_ZXi, X, e6, Jp);
+// Pose prior (posePriorBuildQuadraticForm, kd/icp/tree_aligner_base_.h:139-152, over
+// dPoseToPoseError, kd/utils/geometry_3d_impl_.h:125-140, in FP64): adds J^T Omega J and
+// J^T Omega e to the pose block.  One warp, an element per lane, with the matrices in t
+// (kPriorDoubles of shared memory).  Bound by the chain of an acos, a sine and four small
+// products.  A single thread with the matrices in local memory spilled under the 64 registers of
+// k_linearize: ten rigid iterations with a prior, launched one by one, took 376 us (290 under
+// 128 registers), now 249; without a prior 216.
+constexpr int kPriorP = 0, kPriorE = 12, kPriorJ = 18;        // Z X^-1 Xm, error, Jacobian
+constexpr int kPriorB = 54, kPriorS = 108;                    // dP's rotation, dlog of it
+constexpr int kPriorOJ = kPriorB, kPriorOe = kPriorB + 36;    // Omega J, Omega e: B is done then
+constexpr int kPriorDoubles = 135;
+__device__ __noinline__ void add_pose_prior(const JobIn& Jn, const double* X, double* H, double* b, int D, double* t,
+                                            int lane) {
+  const double* A = Jn.prior_ZXi;
   const double* Om = Jn.prior_info;
-  double OJ[6][6], Oe[6];
-  for (int i = 0; i < 6; ++i) {
-    for (int j = 0; j < 6; ++j) {
-      double a = 0;
-      for (int k = 0; k < 6; ++k) a += Om[i * 6 + k] * Jp[k][j];
-      OJ[i][j] = a;
-    }
-    double a = 0;
-    for (int k = 0; k < 6; ++k) a += Om[i * 6 + k] * e6[k];
-    Oe[i] = a;
+  if (lane < 12) {
+    const int i = lane >> 2, j = lane & 3;
+    const double d = ddot3(A[i * 4], A[i * 4 + 1], A[i * 4 + 2], X[j], X[4 + j], X[8 + j]);
+    t[kPriorP + lane] = j < 3 ? d : da(d, A[i * 4 + 3]);
   }
-  for (int i = 0; i < 6; ++i) {
-    for (int j = 0; j < 6; ++j) {
-      double a = 0;
-      for (int k = 0; k < 6; ++k) a += Jp[k][i] * OJ[k][j];
-      H[i * D + j] += a;
+  // entry (i, j) of R skew(v), R the rotation of A, v column k of X
+  auto rot_skew = [&](int i, int j, int k) {
+    double m[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const double v = X[4 * ((6 - r - j) % 3) + k];  // the third index; unused where r == j
+      m[r] = A[i * 4 + r] * (r == j ? 0.0 : ((j - r + 3) % 3 == 2 ? v : -v));
     }
-    double a = 0;
-    for (int k = 0; k < 6; ++k) a += Jp[k][i] * Oe[k];
-    b[i] += a;
+    return m[0] + m[1] + m[2];
+  };
+  for (int e = lane; e < 54; e += 32) {  // rows: P's rotation column by column
+    const int r = e / 6, j = e % 6;
+    t[kPriorB + e] = j < 3 ? 0.0 : -rot_skew(r % 3, j - 3, r / 3);
   }
+  __syncwarp();
+  const double* P = t + kPriorP;
+  {
+    const double ca = fmin(1.0, fmax(-1.0, 0.5 * (P[0] + P[5] + P[10] - 1.0)));
+    const double a = acos(ca);
+    const bool small = a < 1e-7;
+    const double f = small ? 0.5 : a / (2.0 * sin(a));
+    auto axis = [&](int i) { return i == 0 ? P[9] - P[6] : (i == 1 ? P[2] - P[8] : P[4] - P[1]); };
+    if (lane < 3) t[kPriorE + lane] = P[lane * 4 + 3];
+    else if (lane < 6) t[kPriorE + lane] = axis(lane - 3) * f;
+    if (lane < 27) {
+      const int i = lane / 9, k = lane % 9;
+      double v = 0.0;
+      if (k == (i == 0 ? 5 : (i == 1 ? 6 : 1))) v = f;
+      if (k == (i == 0 ? 7 : (i == 1 ? 2 : 3))) v = -f;
+      if (!small && (k & 3) == 0) {
+        const double s = sin(a);
+        v -= (s - a * cos(a)) / (4.0 * s * s * s) * axis(i);
+      }
+      t[kPriorS + lane] = v;
+    }
+  }
+  __syncwarp();
+  for (int e = lane; e < 36; e += 32) {
+    const int i = e / 6, j = e % 6;
+    double v = 0.0;
+    if (i >= 3) {
+      for (int k = 0; k < 9; ++k) v += t[kPriorS + (i - 3) * 9 + k] * t[kPriorB + k * 6 + j];
+    } else {
+      v = j < 3 ? A[i * 4 + j] : -rot_skew(i, j - 3, 3);
+    }
+    t[kPriorJ + e] = v;
+  }
+  __syncwarp();
+  const double* J = t + kPriorJ;
+  for (int e = lane; e < 42; e += 32) {
+    const int i = e < 36 ? e / 6 : e - 36, j = e % 6;
+    double v = 0.0;
+    for (int k = 0; k < 6; ++k) v += Om[i * 6 + k] * (e < 36 ? J[k * 6 + j] : t[kPriorE + k]);
+    t[kPriorOJ + e] = v;
+  }
+  static_assert(kPriorOe == kPriorOJ + 36 && kPriorOe + 6 <= kPriorS, "Omega e follows Omega J");
+  __syncwarp();
+  for (int e = lane; e < 42; e += 32) {
+    const int i = e < 36 ? e / 6 : e - 36, j = e % 6;
+    double v = 0.0;
+    for (int k = 0; k < 6; ++k) v += J[k * 6 + i] * (e < 36 ? t[kPriorOJ + k * 6 + j] : t[kPriorOe + k]);
+    if (e < 36) H[i * D + j] += v;
+    else b[i] += v;
+  }
+  __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
@@ -685,6 +678,7 @@ constexpr int kTailState = kTailJob + (int)(sizeof(JobIn) / 8);
 constexpr int kTailDoubles = kTailState + (int)(sizeof(JobState) / 8);
 static_assert(sizeof(JobIn) % 8 == 0 && sizeof(JobState) % 8 == 0, "staged as 8 B words");
 static_assert(kTailDoubles <= kWarps * kPStride, "the step's scratch reuses the warps' partials");
+static_assert(kTailX + kPriorDoubles <= kTailP, "the prior's scratch is where dx and the factor come later");
 static_assert(sizeof(JobIn) / 8 + sizeof(JobState) / 8 + 18 <= kBlock, "one staged word per thread");
 
 // Sum of v(t) over the nt tiles in tile order over four interleaved accumulators; sixteen
@@ -968,7 +962,7 @@ __device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O,
     return;
   }
   if (Jn.prior_enabled) {
-    if (tid == 0) add_pose_prior(Jn, S.X, scr + kTailH, scr + kTailB, D);
+    if (tid < 32) add_pose_prior(Jn, S.X, scr + kTailH, scr + kTailB, D, scr + kTailX, lane);
     __syncthreads();
   }
   if (tid >= 32) {
@@ -1460,10 +1454,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       }
       asm volatile("bar.sync %0, %1;" ::"r"(1), "r"(kBlock) : "memory");
       if (tid < 32) {
-        if (job.prior_enabled) {
-          if (tid == 0) add_pose_prior(Jn, S.X, sm.scr + kTailH, sm.scr + kTailB, D);
-          __syncwarp();
-        }
+        if (job.prior_enabled) add_pose_prior(Jn, S.X, sm.scr + kTailH, sm.scr + kTailB, D, sm.scr + kTailX, lane);
         tail_step<KIND>(Jn, S, sm.out, sm.log, sm.scr, lane, caches, [&]() {
           if (S.done && lane < nblk) *cluster.map_shared_rank(&sm.done, lane) = 1;
           __syncwarp();

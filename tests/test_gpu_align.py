@@ -385,3 +385,55 @@ def test_single_alignment_options(scene):
             X = a.get_x()
             a.compute(stats_mode=True)  # leaves the pose alone
             assert np.array_equal(a.get_x(), X)
+
+
+@pytest.mark.parametrize("kind", ["icp", "ct"])
+@pytest.mark.parametrize("turn", [None, 0.0, 0.3])
+def test_pose_prior_and_statistics_in_both_forms(scene, kind, turn):
+    """A pose prior, and a statistics-only run, in the one-launch form against the launch per
+    iteration (timed launches select it): pose, velocities, H, b, step and statistics equal bit
+    for bit; the pose as close to the oracle's as the order of the prior's terms allows.  turn None:
+    no rotation between the prior and the first pose (the Jacobian's small-angle branch)."""
+    import kd_slam2_b200 as kds
+    from kd_slam2_b200 import synth
+    fx, fs = make_scan(scene, 2510)
+    mx, ms = make_scan(scene, 2511, vel=[6.0, 0, 0, 0, 0, 0.2])
+    G = kds.TreeGeneratorB2003D(leaf_max_points=16)
+    F, M = G.make_tree(fx, fs), G.make_tree(mx, ms)
+    X0 = synth.pose((0.1, -0.05, 0.0), (0.0, 0.0, 0.02))
+    A = np.random.default_rng(5).normal(size=(6, 6))
+    if turn is None:
+        prior = dict(X_ref=synth.pose((0.05, 0.02, 0.01), (0.0, 0.0, 0.02)), Z=synth.pose(), info=50.0 * (A @ A.T))
+    else:
+        prior = dict(X_ref=synth.pose((0.05, 0.02, 0.01), (0.01, -0.02, turn)), Z=synth.pose((0.01, 0.0, 0.02)),
+                     info=50.0 * (A @ A.T))
+    prm = dict(max_error=0.5, max_iterations=8)
+    if kind == "ct":
+        prm["velocity_damping"] = 10.0
+
+    def run(stats_mode, launches):
+        a = (kds.ICPB2003D if kind == "icp" else kds.CTICPB2003D)(**prm)
+        a.set_fixed(F)
+        a.set_moving(M)
+        a.set_x(X0)
+        a.set_pose_prior(**prior)
+        a.set_profiling(launches)
+        ret = a.compute(stats_mode=stats_mode)
+        a.set_profiling(False)
+        assert (a.profile()[1] > 0) == launches  # launches timed: this form ran
+        return ret, a
+    for stats_mode in (False, True):
+        r1, one = run(stats_mode, False)
+        rn, many = run(stats_mode, True)
+        assert r1 == rn and one.stats == many.stats and one.stats_log == many.stats_log
+        for x, y in ((one.get_x(), many.get_x()), (one.velocities(), many.velocities()), (one.H, many.H),
+                     (one.b, many.b), (one.dx, many.dx)):
+            assert np.array_equal(x, y)
+        assert stats_mode == np.array_equal(one.get_x(), X0)
+        if stats_mode:
+            continue
+        O = [orc.OTree.build(x, t, orc.tree_params(leaf_max_points=16)) for x, t in ((fx, fs), (mx, ms))]
+        r = orc.align(orc.KIND_CT if kind == "ct" else orc.KIND_ICP, orc.MODE_MIXED, *O, orc.align_params(**prm), X0,
+                      v0=np.zeros(6) if kind == "ct" else None, prior=(prior["X_ref"], prior["Z"], prior["info"]))
+        dt, dr = pose_err(one.get_x(), r["X"])
+        assert r1 == r["ret"] and dt < POSE_TOL and dr < POSE_TOL
