@@ -915,20 +915,18 @@ __device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nbl
   for (int k = threadIdx.x; k < nblocks; k += blockDim.x) v += bsum[k];
   int total;
   block_scan(v, sm, &total);
-  if (threadIdx.x != 0 || ls->lb >= ls->le) return;
-  const bool fits = 2 * total <= cap - ls->le;
-  ls->lb = ls->le;
-  if (fits) {
-    ls->le += 2 * total;
-  } else {
-    ls->error = 1;
-    ls->max_next = 0;
-  }
-  ls->cur ^= 1;
-  ls->depth += 1;
-  if (ls->depth < kMaxDepth + 1) level_begin[ls->depth] = ls->lb;
-  ls->max_size = ls->max_next;
+  if (threadIdx.x != 0) return;
+  const LevelState x = *ls;  // one round of loads
+  if (x.lb >= x.le) return;
+  const bool fits = 2 * total <= cap - x.le;
+  ls->lb = x.le;
+  ls->le = fits ? x.le + 2 * total : x.le;
+  ls->cur = x.cur ^ 1;
+  ls->depth = x.depth + 1;
+  if (x.depth + 1 < kMaxDepth + 1) level_begin[x.depth + 1] = x.le;
+  ls->max_size = fits ? x.max_next : 0;
   ls->max_next = 0;
+  if (!fits) ls->error = 1;
 }
 
 // The last block of the level's last kernel advances the level (done: a counter that
