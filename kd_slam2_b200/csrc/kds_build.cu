@@ -1598,6 +1598,13 @@ struct DeepNode {
 static_assert(sizeof(DeepNode) == 80, "DeepNode layout");
 static_assert(sizeof(DeepNode) <= kSums * sizeof(U128), "a DeepNode fits the sums slot of one node");
 
+// The sums of a depth's nodes: a subtree of n points has at most max(1, 2 (n / 3)) nodes a depth
+// (two children per split node, which holds at least three points).  First slot of the subtree
+// that is the sub-th of its level and starts at point `start`; deep_sum_slot(N, roots) in all.
+__host__ __device__ __forceinline__ int32_t deep_sum_slot(int64_t start, int32_t sub) {
+  return (int32_t)(2 * start / 3) + sub;
+}
+
 template <int WARPS>
 struct DeepSmem {                             // one group's
   float4 pts[2][DeepForm<WARPS>::kPoints];    // the 16 B point records (w = input index)
@@ -1618,10 +1625,9 @@ struct DeepSmem {                             // one group's
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepForm<WARPS>::kPerSM)
     k_deep_build(BNode* nodes, LevelState* ls, PointBufs B, const U128* mom, ChildSums C, BuildParams P,
-                 double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* ring, int32_t* counts,
-                 int32_t dcap) {
+                 double* root_frame, DeepNode* dn, int32_t dn_cap, int32_t* dn_count, U128* sums, int32_t sum_slots,
+                 int32_t group_slots, int32_t* counts, int32_t dcap) {
   grid_begin();
-  constexpr int kNodes = deep_nodes<WARPS>();
   constexpr int kThreadsG = 32 * WARPS;
   extern __shared__ __align__(16) unsigned char deep_smem_raw[];
   const int lane = threadIdx.x & 31, group = WARPS == 1 ? (int)threadIdx.x >> 5 : 0;
@@ -1639,21 +1645,24 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
   stage_init(sg, lane);
   WarpSums W;
   sums_zero(W);
-  U128* myring = ring + (size_t)gw * 2 * kNodes * kSums;
   const float4* pin = B.p[cur0];
   for (int sub = gw; sub < nroots; sub += nw) {
     const int R = lb + sub;
     const BNode root = nodes[R];
     const int n = root.end - root.start;
     const int pbase = root.start;
+    // the subtree's slots for the sums of one depth's nodes, and of the next one's: its own, or
+    // (group_slots) the group's, whichever are fewer in all
+    U128* const sums0 = sums + (size_t)(group_slots ? gw * group_slots : deep_sum_slot(pbase, sub)) * kSums;
+    U128* const sums1 = sums0 + (size_t)sum_slots * kSums;
     for (int i = tid; i < n; i += kThreadsG) S.pts[0][i] = pin[pbase + i];
     if (tid == 0) {
       S.range[0][0] = (uint32_t)n << 16;
       S.prank[0][0] = -1;
     }
-    if (tid < kSums) {  // the root's sums into the ring
+    if (tid < kSums) {  // the root's sums
       const PendingSums ps = pending_sums(nodes, mom, C, depth0, R, root.parent);
-      myring[tid] = ps.q ? pending_value(ps, tid) : mom[(size_t)R * kSums + tid];
+      sums0[tid] = ps.q ? pending_value(ps, tid) : mom[(size_t)R * kSums + tid];
     }
     sync();
     int cnt = 1, c = 0, base = 0, base_prev = 0;
@@ -1667,7 +1676,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
           break;
         }
       }
-      const U128* psums = myring + (size_t)(d & 1) * kNodes * kSums;
+      const U128* psums = d & 1 ? sums1 : sums0;
       for (int r = tid; r < cnt; r += kThreadsG) {
         const uint32_t rg = S.range[c][r];
         const int st = (int)(rg & 0xffffu), en = (int)(rg >> 16);
@@ -1746,7 +1755,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
         }
         nsplit += total;
       }
-      if (2 * nsplit > kNodes) {  // cannot happen (split nodes hold >= 3 points); refuse rather than overrun
+      if (3 * nsplit > n) {  // cannot happen (split nodes hold >= 3 points); refuse rather than overrun
         if (tid == 0) ls->error = 1;
         break;
       }
@@ -1826,7 +1835,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
             U128 qs = u128_zero();
             for (int k = 0; k < team; ++k) qs = u128_add(qs, S.part[warp + k][lane]);
             const U128 other = u128_sub(psums[(size_t)r * kSums + lane], qs);
-            U128* nxt = myring + (size_t)((d + 1) & 1) * kNodes * kSums;
+            U128* nxt = d & 1 ? sums0 : sums1;
             nxt[(size_t)(2 * q) * kSums + lane] = small_left ? qs : other;
             nxt[(size_t)(2 * q + 1) * kSums + lane] = small_left ? other : qs;
           }
@@ -1883,7 +1892,7 @@ __global__ void __launch_bounds__(32 * WARPS * DeepForm<WARPS>::kGroups, DeepFor
           const int k = lane;
           const U128 ps = psums[(size_t)r * kSums + k];
           const U128 other = u128_sub(ps, qs);
-          U128* nxt = myring + (size_t)((d + 1) & 1) * kNodes * kSums;
+          U128* nxt = d & 1 ? sums0 : sums1;
           nxt[(size_t)(2 * q) * kSums + k] = small_left ? qs : other;
           nxt[(size_t)(2 * q + 1) * kSums + k] = small_left ? other : qs;
         }
@@ -2392,7 +2401,8 @@ struct BuildWs {
   int32_t *big_list, *node_chunk0;
   U128* acc;       // the large roots' sums
   ChildSums accl;  // the smaller children's sums of large nodes, by level parity
-  U128* mom;   // exact sums of every node
+  U128* mom;   // exact sums of every node, and room for the subtree passes
+  U128* mom_end;
   double* ts0;   // per cloud
   double* dt;    // stamps less ts0, input order
   DtSum* dt_tiles;
@@ -2414,6 +2424,15 @@ struct BuildWs {
   int32_t chunk_cap;
 };
 
+// The subtree passes work in the unused end of the sums array, le slots of which are taken: an
+// 80 B record per node to come and two sets of sums of deep_sum_slot(n, roots) nodes (288 B
+// each, 192 B a point) or fewer.  The slots left have 144 B a node, so 64 B a point and what the
+// roots and the nodes above them take has to be added; 72 B a point do for roots of 52 points or
+// more on average (the pass asks the pool where they don't).  A block of the pool beside this
+// workspace, one ring of 396 KB per 16-warp group, was up to 59 MB that no reservation counted.
+// Words of 16 B.
+size_t deep_spare(int64_t n, int R) { return (72 * (size_t)n + 96 * (size_t)R) / 16; }
+
 // Lays the workspace for n points in R clouds out from p (a null base: sizes only); returns its end.
 char* ws_layout(BuildWs& w, char* p, int64_t n, int R) {
   w.cap_nodes = 2 * n + 4096 + 4 * (int64_t)R;
@@ -2434,7 +2453,8 @@ char* ws_layout(BuildWs& w, char* p, int64_t n, int R) {
   w.node_chunk0 = carve<int32_t>(p, w.chunk_cap);
   w.acc = carve<U128>(p, nbig);
   for (int k = 0; k < 2; ++k) w.accl.acc[k] = carve<U128>(p, nbig);
-  w.mom = carve<U128>(p, (size_t)kSums * cn);
+  w.mom = carve<U128>(p, (size_t)kSums * cn + deep_spare(n, R));
+  w.mom_end = w.mom + (size_t)kSums * cn + deep_spare(n, R);
   w.dt = carve<double>(p, n);
   w.dt_tiles = carve<DtSum>(p, n / kDtTile + 1);
   w.off = carve<int64_t>(p, R + 1);
@@ -2485,38 +2505,46 @@ namespace {
 
 // The deep levels of a build whose current level (h, read at the last sync) fits the form:
 // k_deep_build, the depth-major scan of the per-(depth, subtree) node counts, k_deep_place and
-// k_deep_finish.  The node records of the deep levels are staged in the unused part of the
-// sums array (slots from le on).
+// k_deep_finish.  n: the build's points.
 template <int WARPS>
-int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_t s) {
+int deep_pass(BuildWs& w, int64_t n, const BuildParams& P, const LevelState& h, cudaStream_t s) {
   using Form = DeepForm<WARPS>;
   const int lb = h.lb, le = h.le;
   const int nroots = le - lb;
   if (nroots <= 0) return KDS_OK;
   const int dcap = std::max(1, P.max_level - h.depth);
-  DeepNode* dn = reinterpret_cast<DeepNode*>(w.mom + (size_t)le * kSums);
-  const int64_t dn_cap64 = ((w.cap_nodes - le) * (int64_t)(kSums * sizeof(U128))) / (int64_t)sizeof(DeepNode);
-  const int32_t dn_cap = (int32_t)std::min<int64_t>(dn_cap64, INT32_MAX);
   const int grid = (int)std::min<int64_t>((nroots + Form::kGroups - 1) / Form::kGroups, 148 * Form::kPerSM);
-  const size_t ring_n = (size_t)grid * Form::kGroups * 2 * deep_nodes<WARPS>() * kSums;
   const int64_t ncount = (int64_t)dcap * nroots;
   if (ncount > INT32_MAX / 2) { set_error("kds_tree_build: too many deep subtrees"); return KDS_ERR_CAPACITY; }
+  // Records and sums behind the sums in use, counts and offsets in the prune's flags, both free
+  // until the pass is done; a block of the pool in place of what they have no room for.
+  const int64_t dn_cap = w.cap_nodes - le;
+  const int32_t own_slots = deep_sum_slot(n, nroots), all_groups = grid * Form::kGroups * deep_nodes<WARPS>();
+  const int32_t sum_slots = std::min(own_slots, all_groups);
+  const int32_t group_slots = all_groups < own_slots ? deep_nodes<WARPS>() : 0;
+  DeepNode* dn = reinterpret_cast<DeepNode*>(w.mom + (size_t)le * kSums);
+  U128* sums = reinterpret_cast<U128*>(dn + dn_cap);
+  const size_t sum_words = (size_t)2 * kSums * sum_slots;
+  const bool sums_fit = sums + sum_words <= w.mom_end;
   const size_t bc = carve_size<int32_t>(ncount + 64), bt = carve_size<int32_t>(ncount / 4096 + 2),
-               br = carve_size<U128>(ring_n);
+               bk = 2 * bc + bt + 256, br = carve_size<U128>(sum_words);
+  const bool counts_fit = bk <= sizeof(int2) * (size_t)w.cap_nodes;
   void* blk = nullptr;
-  cudaError_t e = cudaMallocAsync(&blk, 2 * bc + bt + 256 + br, s);
+  cudaError_t e = cudaSuccess;
+  if (!sums_fit || !counts_fit) e = cudaMallocAsync(&blk, (sums_fit ? 0 : br) + (counts_fit ? 0 : bk), s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_error("cudaMallocAsync for the deep tree levels failed: %s", cudaGetErrorString(e));
     return KDS_ERR_OOM;
   }
   char* p = (char*)blk;
+  if (!sums_fit) sums = carve<U128>(p, sum_words);
+  if (counts_fit) p = (char*)w.flags;
   int32_t* counts = carve<int32_t>(p, ncount + 64);  // and dn_count behind them: cleared together
   int32_t* dn_count = counts + ncount;
   int32_t* off = carve<int32_t>(p, ncount + 64);
   int32_t* tiles = carve<int32_t>(p, ncount / 4096 + 2);
   int32_t* total = carve<int32_t>(p, 1);
-  U128* ring = carve<U128>(p, ring_n);
   int rc = KDS_OK;
   const size_t smem = sizeof(DeepSmem<WARPS>) * Form::kGroups;
   static std::atomic<bool> attr_set{false};  // a property of the kernel, per process (builds may run on two threads)
@@ -2527,7 +2555,7 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * (ncount + 1), s);
   if (e == cudaSuccess) {
     launch(k_deep_build<WARPS>, grid, 32 * WARPS * Form::kGroups, smem, s, w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame,
-                                                                       dn, dn_cap, dn_count, ring, counts, dcap);
+                                                                       dn, (int32_t)dn_cap, dn_count, sums, sum_slots, group_slots, counts, dcap);
     if (ncount <= kDeepScan) {
       launch(k_deep_scan, 1, 1024, 0, s, w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes,
                                      w.level_begin);
@@ -2536,11 +2564,11 @@ int deep_pass(BuildWs& w, const BuildParams& P, const LevelState& h, cudaStream_
       launch(k_deep_finish, 1, 64, 0, s, w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
     }
     const int pg = (int)std::min<int64_t>(nblk(std::max<int64_t>(w.cap_nodes - le, nroots), kThreads), kGridBlocks * 4);
-    launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, dn_cap, off, dcap, (int32_t)w.cap_nodes,
-           w.alive);
+    launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, (int32_t)dn_cap, off, dcap,
+           (int32_t)w.cap_nodes, w.alive);
     e = cudaGetLastError();
   }
-  cudaFreeAsync(blk, s);
+  if (blk) cudaFreeAsync(blk, s);
   if (e != cudaSuccess) return cuda_status(e, "deep tree levels", __FILE__, __LINE__);
   return rc;
 }
@@ -2716,7 +2744,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
         if (rc) return rc;
       }
       global_levels = hls.depth;
-      rc = by_block ? deep_pass<16>(w, P, hls, s) : deep_pass<1>(w, P, hls, s);
+      rc = by_block ? deep_pass<16>(w, N, P, hls, s) : deep_pass<1>(w, N, P, hls, s);
       if (rc) return rc;
       break;
     }

@@ -158,3 +158,35 @@ def test_device_stamps_equal_host_stamps(trace, take, at):
     a, _, _ = run(trace, inputs=inputs)
     b, _, _ = run(trace, inputs=[(torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()) for x, t in inputs])
     same_results(a, b)
+
+
+@pytest.mark.parametrize("beams,cols", [(16, 1024), (64, 1024), (128, 1024), (128, 2048)])
+def test_build_memory_stays_within_the_reservation(beams, cols):
+    """What a request's build takes from the device's pool at most -- its points, the workspace,
+    the subtree pass, the tree -- is within what admission reserved for it."""
+    import kd_slam2_b200 as kds
+    from conftest import make_scan
+    from cuda.bindings import driver, runtime as rt
+    from kd_slam2_b200 import synth
+    boxes = synth.scene(1001)
+    xyz, st = make_scan(boxes, 77, beams=beams, cols=cols, elev=(-15.0, 15.0) if beams <= 32 else (-22.5, 22.5))
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess
+        return r[-1]
+    pool = ok(rt.cudaDeviceGetDefaultMemPool(ok(rt.cudaGetDevice())))
+    attr = rt.cudaMemPoolAttr
+    srv = kds.Server(tree=TREE, icp=ICP, ct=CT, map_every=100)
+    try:
+        sid = srv.add_stream(make_scan(boxes, 78)[0], len(xyz))
+        ticket = srv.submit(sid, kds.abi.KDS_CTICP, xyz, st, np.eye(3, 4))
+        used = int(ok(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemCurrent)))
+        ok(rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh, driver.cuuint64_t(0)))
+        srv.start()
+        srv.drain(60.0)
+        assert srv.result(ticket)["status"] == 0
+        high = int(ok(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh)))
+        peak = srv.stats()["peak_reserved"]
+    finally:
+        srv.free()
+    assert 0 < high - used <= peak, (high - used, peak)

@@ -108,6 +108,24 @@ def test_degenerate_inputs(scene):
     assert_same_tree(O, G)
 
 
+@pytest.mark.parametrize("clouds,points,extra", [(3000, 9, 0), (4000, 20, 300), (290, 20, 300)])
+def test_many_tiny_clouds(clouds, points, extra):
+    """Subtree passes whose sums, or whose counts, have no room in the build's workspace (very
+    many very small subtrees): the trees equal the oracle's all the same."""
+    import kd_slam2_b200 as kds
+    rng = np.random.default_rng(clouds)
+    sizes = [points] * clouds + ([extra] if extra else [])
+    made = [((rng.normal(size=(n, 3)) * [2.0, 2.0, 0.02] + [12.0, 0, 1.0]).astype(np.float32),
+             np.sort(rng.uniform(0, 0.1, n))) for n in sizes]
+    prm = dict(leaf_max_points=8, leaf_min_points=3, tree_min_good_leaves=1)
+    trees = kds.TreeGeneratorB2003D(**prm).make_trees(made)
+    for i in sorted(set(rng.integers(0, len(made), 60)) | {0, len(made) - 1}):
+        O = orc.OTree.build(*made[i], orc.tree_params(**prm))
+        assert O.accepted == (trees[i] is not None)
+        if O.accepted:
+            assert_same_tree(O, trees[i])
+
+
 @pytest.mark.parametrize("clusters,pile,fits", [
     (60, 0, True),        # a subtree pass from the first level
     (60, 3000, True),     # the pile of equal points keeps the level kernels running to the last level
