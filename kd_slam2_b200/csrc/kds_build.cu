@@ -21,7 +21,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -29,6 +28,7 @@
 #include <vector>
 
 #include "kds_internal.cuh"
+#include "kds_rules.h"
 
 namespace kds {
 
@@ -2547,10 +2547,12 @@ int deep_pass(BuildWs& w, int64_t n, const BuildParams& P, const LevelState& h, 
   int32_t* total = carve<int32_t>(p, 1);
   int rc = KDS_OK;
   const size_t smem = sizeof(DeepSmem<WARPS>) * Form::kGroups;
-  static std::atomic<bool> attr_set{false};  // a property of the kernel, per process (builds may run on two threads)
-  if (!attr_set.load()) {
+  static DeviceSet limits;  // devices with the kernel's limit raised
+  int dev = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && !limits.has(dev)) {
     e = cudaFuncSetAttribute((const void*)k_deep_build<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) attr_set.store(true);
+    if (e == cudaSuccess) limits.add(dev);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * (ncount + 1), s);
   if (e == cudaSuccess) {

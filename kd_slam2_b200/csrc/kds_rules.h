@@ -2,7 +2,24 @@
 // can be checked without a device.
 #pragma once
 
+#include <atomic>
+#include <cstdint>
+
 namespace kds {
+
+// Devices on which something that each one needs has been done (a kernel's limits belong to a
+// device).  Safe with several threads; a device above the 64th is never in it.
+class DeviceSet {
+ public:
+  bool has(int device) const { return in(device) && ((bits_.load() >> device) & 1u); }
+  void add(int device) {
+    if (in(device)) bits_.fetch_or(1ull << device);
+  }
+
+ private:
+  static bool in(int device) { return device >= 0 && device < 64; }
+  std::atomic<uint64_t> bits_{0};
+};
 
 // Whether a request's first stamp is found by a kernel on the calling thread's device: the
 // scratch that the kernel writes is the server's, so the caller, the server and both ends of

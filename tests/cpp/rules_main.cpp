@@ -14,5 +14,13 @@ int main(int argc, char** argv) {
     std::printf("%d\n", kds::largest_cluster([&](int n) { return n <= atoi(argv[2]); }));
     return 0;
   }
+  if (argc > 2 && !strcmp(argv[1], "devices")) {  // per device: was it new?  (added then)
+    kds::DeviceSet set;
+    for (int i = 2; i < argc; ++i) {
+      std::printf("%d\n", set.has(atoi(argv[i])) ? 0 : 1);
+      set.add(atoi(argv[i]));
+    }
+    return 0;
+  }
   return 2;
 }

@@ -37,3 +37,8 @@ def test_alignments_need_no_cluster(rules, room, blocks):
     """Where the device schedules no cluster the rule says so (and an alignment is launched once
     per iteration) instead of assuming that the portable size always fits."""
     assert rules("cluster", room) == [blocks]
+
+
+def test_kernel_limits_are_set_on_every_device(rules):
+    """A limit raised on one device says nothing of the next one."""
+    assert rules("devices", 0, 0, 1, 0, 1, 63, 63, 64, 64, -1, -1) == [1, 0, 1, 0, 0, 1, 0, 1, 1, 1, 1]
