@@ -1660,14 +1660,6 @@ int Runner::reserve(int nj, int nl, int nt) {
 
 void Runner::release() {
   drop_graph();
-  if (side) {
-    for (cudaEvent_t& e : fork_ev) {
-      if (e) cudaEventDestroy(e);
-      e = nullptr;
-    }
-    cudaStreamDestroy(side);
-    side = nullptr;
-  }
   for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
   prof_ev.clear();
   if (block) cudaFree(block);
@@ -1678,6 +1670,31 @@ void Runner::release() {
 Runner::~Runner() {
   release();
   if (h_cluster) cudaFreeHost(h_cluster);
+  for (cudaEvent_t e : fork_ev)
+    if (e) cudaEventDestroy(e);
+  if (side) cudaStreamDestroy(side);
+}
+
+// The second stream and its events, at the priority of s; false where they can't be had.
+bool Runner::side_ready(cudaStream_t s) {
+  int prio = 0;
+  bool ok = cudaStreamGetPriority(s, &prio) == cudaSuccess;
+  if (ok && side && prio != side_priority) {
+    cudaStreamDestroy(side);  // the work on it was joined, and keeps its resources until it is done
+    side = nullptr;
+  }
+  if (ok && !side) {
+    ok = cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, prio) == cudaSuccess;
+    if (!ok) side = nullptr;
+    side_priority = prio;
+  }
+  for (cudaEvent_t& e : fork_ev)
+    if (ok && !e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      e = nullptr;
+      ok = false;
+    }
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 void Runner::drop_graph() {
@@ -1918,15 +1935,11 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
   // The kinds' jobs don't depend on each other: the first kind's iterations run on s, the others'
   // beside them, so that one kind's blocks fill the SMs where the other's last tiles and solves
   // run (a batch of 125 pairs of each kind: 1,735 us one after the other, 1,455 side by side).
-  // In order where each launch is timed, and for one launch a kind: 62 us of kernels give less
-  // than the stream costs to create.
+  // In order where each launch is timed, for one launch a kind (62 us of kernels give less than
+  // the stream costs to create), and where there is no second stream.
   const int first = L[0] ? 0 : (L[1] ? 1 : 2);
-  const bool fork = !profiling && total > L[first] && nmax > 1;
+  const bool fork = !profiling && total > L[first] && nmax > 1 && side_ready(s);
   if (fork) {
-    if (!side) {
-      KDS_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-      for (cudaEvent_t& e : fork_ev) KDS_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
     KDS_CK(cudaEventRecord(fork_ev[0], s));
     KDS_CK(cudaStreamWaitEvent(side, fork_ev[0], 0));
   }

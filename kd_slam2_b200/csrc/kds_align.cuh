@@ -142,7 +142,8 @@ struct Runner {
   ClusterOut* h_cluster = nullptr;  // results of run_cluster
   ClusterOut* d_cluster = nullptr;  // ... as the device sees them
   int cluster_blocks = -1;          // largest cluster; 0: none, -1: not asked yet
-  cudaStream_t side = nullptr;      // launches of a second kind of jobs
+  cudaStream_t side = nullptr;      // launches of a second kind of jobs, at the caller's priority
+  int side_priority = 0;
   cudaEvent_t fork_ev[2] = {};
   bool smem_attr_set = false;
   bool persistent_attr_set = false;
@@ -167,6 +168,7 @@ struct Runner {
   // where the device has no room for the cluster or its results: then setup, run and fetch.
   bool run_cluster(JobIn J, const LinDev& L, cudaStream_t s, JobOut* out, std::vector<kds_stats>* log, int* rc);
   bool cluster_ready();
+  bool side_ready(cudaStream_t s);
   ~Runner();
 };
 

@@ -125,6 +125,21 @@ def test_two_tile_blocks_of_another_split_of_the_same_tiles(workload, first, the
         same([alone[t, k] for k, t in enumerate(tiles)], outputs(out))
 
 
+def test_batches_on_streams_of_other_priorities(workload):
+    """A mixed batch's second stream follows the priority of the caller's: the same results on
+    streams of either priority in turn, and on the default stream."""
+    import torch
+
+    from kd_slam2_b200 import ba
+    wl, trees = workload
+    jobs = ba.jobs(wl, trees, ICP, CT)
+    ref = outputs(kds.Batch().run(jobs, use_graph=False))
+    b = kds.Batch()
+    streams = [torch.cuda.Stream(priority=p).cuda_stream for p in (0, -1)] + [None]
+    for k in range(7):
+        same(ref, outputs(b.run(jobs, use_graph=k % 2 == 1, stream=streams[k % 3])))
+
+
 def test_autotune_as_first_use_of_the_library(tmp_path):
     """In a fresh process, the autotuner's staged configurations opt the kernels into their
     shared memory themselves (no earlier launch did it)."""
