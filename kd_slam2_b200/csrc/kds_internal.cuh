@@ -26,6 +26,9 @@ int cuda_status(cudaError_t e, const char* what, const char* file, int line);
 void count_launch();
 
 inline cudaStream_t as_stream(void* s) { return s ? (cudaStream_t)s : cudaStreamPerThread; }
+// The calling thread's stream of the highest priority on the current device, behind all work
+// that the legacy stream waits for; nullptr where it can't be had.
+cudaStream_t front_stream();
 int ensure_init();
 
 // ---------------------------------------------------------------------------

@@ -104,17 +104,19 @@ __global__ void __launch_bounds__(1024) k_first_stamp(const double* __restrict__
 }
 
 // The first stamp of n device stamps.  Reading the stamps back and searching them on the host took
-// 180 us a request (65,536 points); the kernel and 8 bytes take 40.  On the legacy stream, after
-// the work of every blocking stream, as the copy is.  The copy stays where the caller or the
+// 180 us a request (65,536 points); the kernel and 8 bytes take 40.  After the work of every
+// blocking stream, as the copy is.  The copy stays where the caller or the
 // stamps are on another device than the server's (device; scratch is there) and for pointers
 // whose last element is no device memory.
 int first_stamp(const double* st, int64_t n, int device, double* scratch, double* out) {
   int dev = 0;
   cudaPointerAttributes a, z;
+  cudaStream_t s = nullptr;
   const bool here = scratch && ((uintptr_t)st & 7) == 0 && cudaGetDevice(&dev) == cudaSuccess &&
                     cudaPointerGetAttributes(&a, st) == cudaSuccess &&
                     cudaPointerGetAttributes(&z, st + (n - 1)) == cudaSuccess &&
-                    first_stamp_on_device(dev, device, a.device, z.device) && z.type == cudaMemoryTypeDevice;
+                    first_stamp_on_device(dev, device, a.device, z.device) && z.type == cudaMemoryTypeDevice &&
+                    (s = front_stream()) != nullptr;
   if (!here) {
     cudaGetLastError();
     std::vector<double> hs((size_t)n);
@@ -122,10 +124,11 @@ int first_stamp(const double* st, int64_t n, int device, double* scratch, double
     *out = *std::min_element(hs.begin(), hs.end());
     return KDS_OK;
   }
-  k_first_stamp<<<1, 1024, 0, cudaStreamLegacy>>>(st, n, scratch);
+  k_first_stamp<<<1, 1024, 0, s>>>(st, n, scratch);
   count_launch();
   KDS_CK(cudaGetLastError());
-  KDS_CK(cudaMemcpy(out, scratch, sizeof(double), cudaMemcpyDeviceToHost));
+  KDS_CK(cudaMemcpyAsync(out, scratch, sizeof(double), cudaMemcpyDeviceToHost, s));
+  KDS_CK(cudaStreamSynchronize(s));
   return KDS_OK;
 }
 

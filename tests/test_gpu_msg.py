@@ -98,3 +98,30 @@ def test_message_records_of_all_fields(nodes):
     U = kds.Tree.from_msg(msg)
     assert np.array_equal(U.export()["leaves"], np.flatnonzero(left < 0))
     assert np.array_equal(U.extract_compressed_leaves(), T.extract_compressed_leaves())
+
+
+def test_messages_follow_the_tree_and_other_threads(scene):
+    """A message is written after the work that the tree was given before on the default stream,
+    from threads that come and go (each has its own stream for it)."""
+    import threading
+
+    import kd_slam2_b200 as kds
+    from kd_slam2_b200 import synth
+    xyz, st = make_scan(scene, 4101, beams=64, elev=(-22.5, 22.5))
+    gen = kds.TreeGeneratorB2003D(**TREE)
+    failed = []
+
+    def work(k):
+        T = gen.make_tree(xyz, st)
+        for i in range(8):
+            T.apply_isometry_in_place(synth.pose((0.1 * k, 0.02 * i, 0.0), (0.0, 0.01 * i, 0.02 * k)))
+            m, e = T.to_msg()["nodes"], T.export()
+            if not (np.array_equal(m["mean"], e["mean"]) and np.array_equal(m["direction"], e["dir"])):
+                failed.append((k, i))
+    for _ in range(2):
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not failed
