@@ -2201,25 +2201,6 @@ int launch_admit_slots(const int32_t* d_slots, int n, const JobIn* new_jobs, con
   return KDS_OK;
 }
 
-template <int KIND>
-static void serve_kind(int ntiles, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
-                       const TileDev* tiles, double* partials, cudaStream_t s) {
-  const int stage = stage_room(kServeStage, ntiles, kLinBlocks<KIND>, lin_bytes<KIND>());
-  k_linearize<KIND><<<ntiles, kBlock, stage * sizeof(DNode), s>>>(jobs, states, outs, nullptr, lins, tiles, 0, stage,
-                                                                  partials, nullptr, nullptr, nullptr);
-}
-
-int launch_linearize(int kind, int ntiles, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
-                     const TileDev* tiles, double* partials, cudaStream_t s) {
-  if (ntiles <= 0) return KDS_OK;
-  if (kind == 0) serve_kind<0>(ntiles, jobs, states, outs, lins, tiles, partials, s);
-  else if (kind == 1) serve_kind<1>(ntiles, jobs, states, outs, lins, tiles, partials, s);
-  else serve_kind<2>(ntiles, jobs, states, outs, lins, tiles, partials, s);
-  count_launch();
-  KDS_CK(cudaGetLastError());
-  return KDS_OK;
-}
-
 int launch_linearize_pairs(int kind, int npairs, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
                            const TileDev* tiles, const int2* pairs, double* partials, cudaStream_t s) {
   if (npairs <= 0) return KDS_OK;

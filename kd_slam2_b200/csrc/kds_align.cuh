@@ -197,8 +197,6 @@ constexpr int kTileSurfels = 128;  // moving surfels per tile = threads per k_li
 // Copies n admitted job records into their slots and initialises those jobs.
 int launch_admit_slots(const int32_t* d_slots, int n, const JobIn* new_jobs, const LinDev* new_lins, JobIn* jobs,
                        JobState* states, JobOut* outs, LinDev* lins, cudaStream_t s);
-int launch_linearize(int kind, int ntiles, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,
-                     const TileDev* tiles, double* partials, cudaStream_t s);
 // Two tiles of one (job, fixed entry) per block (k_linearize_pair): pairs[i] = (tile,
 // second tile or -1).
 int launch_linearize_pairs(int kind, int npairs, const JobIn* jobs, JobState* states, JobOut* outs, LinDev* lins,

@@ -747,7 +747,7 @@ __global__ void k_tree_check(const double* sts, const int64_t* off, const unsign
   }
 }
 
-__global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState* ls, int32_t* level_begin) {
+__global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState* ls) {
   grid_begin();
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < R) {
@@ -767,7 +767,6 @@ __global__ void k_init_roots(BNode* nodes, const int64_t* off, int R, LevelState
     ls->cur = 0;
     ls->depth = 0;
     ls->max_next = 0;
-    level_begin[0] = 0;
   }
 }
 
@@ -908,8 +907,7 @@ __global__ void k_decide(BNode* nodes, const LevelState* ls, U128* mom, ChildSum
 // whole block).  Children that don't fit the node arrays have no records: the build has failed,
 // and the levels to come before the host looks are empty (every kernel takes its nodes from
 // [lb, le)).
-__device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nblocks, int32_t cap,
-                                    int32_t* level_begin) {
+__device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nblocks, int32_t cap) {
   __shared__ int sm[32];
   int v = 0;
   for (int k = threadIdx.x; k < nblocks; k += blockDim.x) v += bsum[k];
@@ -923,7 +921,6 @@ __device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nbl
   ls->le = fits ? x.le + 2 * total : x.le;
   ls->cur = x.cur ^ 1;
   ls->depth = x.depth + 1;
-  if (x.depth + 1 < kMaxDepth + 1) level_begin[x.depth + 1] = x.le;
   ls->max_size = fits ? x.max_next : 0;
   ls->max_next = 0;
   if (!fits) ls->error = 1;
@@ -933,7 +930,7 @@ __device__ void level_advance_block(LevelState* ls, const int32_t* bsum, int nbl
 // starts at 0 and is left at 0; nullptr: not the last kernel).  Every block of the
 // calling kernel must reach this.
 __device__ __forceinline__ void advance_if_last(LevelState* ls, const int32_t* bsum, int nblocks, int32_t cap,
-                                                int32_t* level_begin, unsigned* done) {
+                                                unsigned* done) {
   if (!done) return;
   __shared__ int s_last;
   __syncthreads();
@@ -944,7 +941,7 @@ __device__ __forceinline__ void advance_if_last(LevelState* ls, const int32_t* b
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  level_advance_block(ls, bsum, nblocks, cap, level_begin);
+  level_advance_block(ls, bsum, nblocks, cap);
   if (threadIdx.x == 0) *done = 0u;
 }
 
@@ -1004,7 +1001,7 @@ __device__ __forceinline__ void big_count(const Chunk* chunks, const LevelState*
 // us to 329 and 32 keyframes from 2.46 ms to 2.34 (with the large nodes' lists written by
 // k_level_children).
 __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nodes, LevelState* ls, PointBufs B,
-                                                         U128* mom, const int32_t* bsum, int nblocks, int32_t cap, int32_t* level_begin,
+                                                         U128* mom, const int32_t* bsum, int nblocks, int32_t cap,
                                                          unsigned* done, const Chunk* chunks, SegCounts* seg,
                                                          int count_blocks) {
   grid_begin();
@@ -1123,7 +1120,7 @@ __global__ void __launch_bounds__(kThreads, kSmallPerSM) k_small_part(BNode* nod
     }
   }
   if (lane == 0 && maxc > 0) atomicMax(&ls->max_next, maxc);
-  advance_if_last(ls, bsum, nblocks, cap, level_begin, done);
+  advance_if_last(ls, bsum, nblocks, cap, done);
 }
 
 // ---- large nodes ------------------------------------------------------------------
@@ -1340,7 +1337,7 @@ __device__ __forceinline__ int seg_before(const SegCounts& s, int w) {
 // the root, where every warp hits the same words; three blocks per SM spill and take 118 us.
 __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     k_big_scatter(const Chunk* chunks, LevelState* ls, BNode* nodes, PointBufs B, const SegCounts* seg,
-                  const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t cap, int32_t* level_begin,
+                  const int32_t* node_chunk0, ChildSums C, const int32_t* bsum, int nblocks, int32_t cap,
                   unsigned* done) {
   grid_begin();
   __shared__ U128 smm[kSegs][kSums];
@@ -1448,7 +1445,7 @@ __global__ void __launch_bounds__(kThreads, kScatterPerSM)
     }
   }
   if (split) block_add_sums(S, lane, smm, accl + (size_t)big * kSums, per == 1);
-  advance_if_last(ls, bsum, nblocks, cap, level_begin, done);
+  advance_if_last(ls, bsum, nblocks, cap, done);
 }
 
 // ---- children ------------------------------------------------------------------------
@@ -1967,11 +1964,10 @@ __global__ void k_deep_place(BNode* nodes, LevelState* ls, int32_t lb, int32_t l
   }
 }
 
-// One block: the level state after the deep levels (every level done), the begin of each deep
-// level, the depth, and the node capacity check (a thread per depth; one thread for all took
+// One block: the level state after the deep levels (every level done), the depth, and the node capacity check (a thread per depth; one thread for all took
 // 11 us of dependent loads).
 __device__ __forceinline__ void deep_finish(LevelState* ls, int32_t lb, int32_t le, const int32_t* off, int32_t tot,
-                                            int32_t dcap, int32_t cap_nodes, int32_t* level_begin) {
+                                            int32_t dcap, int32_t cap_nodes) {
   __shared__ int s_dmax;  // deepest local depth holding nodes
   const int depth0 = ls->depth;
   const bool failed = ls->error != 0;
@@ -1982,29 +1978,24 @@ __device__ __forceinline__ void deep_finish(LevelState* ls, int32_t lb, int32_t 
   for (int d = 1 + threadIdx.x; d < dcap; d += blockDim.x) {
     const int b = off[(size_t)d * nroots];
     const int e = d + 1 < dcap ? off[(size_t)(d + 1) * nroots] : tot;
-    if (e > b) {
-      atomicMax(&s_dmax, d);
-      if (depth0 + d < kMaxDepth + 1) level_begin[depth0 + d] = le + b;
-    }
+    if (e > b) atomicMax(&s_dmax, d);
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
   if (le + tot > cap_nodes) ls->error = 1;
   ls->depth = depth0 + s_dmax + 1;
   ls->lb = ls->le = le + tot;
-  if (ls->depth < kMaxDepth + 1) level_begin[ls->depth] = ls->lb;
 }
 __global__ void k_deep_finish(LevelState* ls, int32_t lb, int32_t le, const int32_t* off, const int32_t* total,
-                              int32_t dcap, int32_t cap_nodes, int32_t* level_begin) {
+                              int32_t dcap, int32_t cap_nodes) {
   grid_begin();
-  deep_finish(ls, lb, le, off, *total, dcap, cap_nodes, level_begin);
+  deep_finish(ls, lb, le, off, *total, dcap, cap_nodes);
 }
 // The same with the scan of the counts by the one block: up to kDeepScan counts, a run per
 // thread (three scan launches and this otherwise).
 constexpr int kDeepScan = 16384;
 __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, int32_t le, const int32_t* counts,
-                                                    int32_t ncount, int32_t* off, int32_t dcap, int32_t cap_nodes,
-                                                    int32_t* level_begin) {
+                                                    int32_t ncount, int32_t* off, int32_t dcap, int32_t cap_nodes) {
   grid_begin();
   __shared__ int sm[32];
   const int per = (ncount + 1023) / 1024;
@@ -2018,7 +2009,7 @@ __global__ void __launch_bounds__(1024) k_deep_scan(LevelState* ls, int32_t lb, 
     x += counts[i];
   }
   __syncthreads();
-  deep_finish(ls, lb, le, off, tot, dcap, cap_nodes, level_begin);
+  deep_finish(ls, lb, le, off, tot, dcap, cap_nodes);
 }
 
 // ---- prune and per-tree compaction -----------------------------------------------------
@@ -2413,7 +2404,6 @@ struct BuildWs {
   LevelState* ls;
   unsigned* done;  // last-block counter of the level's last kernel
   char* zero_end;
-  int32_t* level_begin;
   int32_t* bsum;
   int32_t* bbig;  // per-block (chunks, large nodes) of the level
   int32_t *cnt, *lcnt, *gp, *lgp, *to, *lto;
@@ -2469,7 +2459,6 @@ char* ws_layout(BuildWs& w, char* p, int64_t n, int R) {
   w.ts0 = carve<double>(p, (size_t)(1 + kRootFrame) * R);
   w.root_frame = w.ts0 + R;
   w.zero_end = p;
-  w.level_begin = carve<int32_t>(p, kMaxDepth + 2);
   w.bsum = carve<int32_t>(p, kLevelBlocks);
   w.bbig = carve<int32_t>(p, 2 * kLevelBlocks);
   w.gp = carve<int32_t>(p, G);
@@ -2559,11 +2548,10 @@ int deep_pass(BuildWs& w, int64_t n, const BuildParams& P, const LevelState& h, 
     launch(k_deep_build<WARPS>, grid, 32 * WARPS * Form::kGroups, smem, s, w.nodes, w.ls, w.B, w.mom, w.accl, P, w.root_frame,
                                                                        dn, (int32_t)dn_cap, dn_count, sums, sum_slots, group_slots, counts, dcap);
     if (ncount <= kDeepScan) {
-      launch(k_deep_scan, 1, 1024, 0, s, w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes,
-                                     w.level_begin);
+      launch(k_deep_scan, 1, 1024, 0, s, w.ls, lb, le, counts, (int32_t)ncount, off, dcap, (int32_t)w.cap_nodes);
     } else {
       rc = scan_exclusive(counts, off, (int32_t)ncount, tiles, total, s);
-      launch(k_deep_finish, 1, 64, 0, s, w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes, w.level_begin);
+      launch(k_deep_finish, 1, 64, 0, s, w.ls, lb, le, off, total, dcap, (int32_t)w.cap_nodes);
     }
     const int pg = (int)std::min<int64_t>(nblk(std::max<int64_t>(w.cap_nodes - le, nroots), kThreads), kGridBlocks * 4);
     launch(k_deep_place, pg, kThreads, 0, s, w.nodes, w.ls, lb, le, dn, dn_count, (int32_t)dn_cap, off, dcap,
@@ -2713,7 +2701,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     launch(k_tree_min, g, kThreads, 0, s, d_st, w.off, w.tsmin);
     launch(k_tree_check, g, kThreads, 0, s, d_st, w.off, w.tsmin, w.ts0, w.dt, w.ls);
   }
-  launch(k_init_roots, (R + 127) / 128, 128, 0, s, w.nodes, w.off, R, w.ls, w.level_begin);
+  launch(k_init_roots, (R + 127) / 128, 128, 0, s, w.nodes, w.off, R, w.ls);
   KDS_CK(cudaGetLastError());
 
   // pinned: [level state | per-tree nodes, leaves, unpruned nodes | ts0 | root frames]
@@ -2789,10 +2777,10 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
       }
       const int count_blocks = big ? cb : 0;
       launch(k_small_part, count_blocks + small_blocks, kThreads, 0, s, w.nodes, w.ls, w.B, w.mom, w.bsum, lvl_blocks,
-             (int32_t)w.cap_nodes, w.level_begin, big ? nullptr : w.done, w.chunks, w.seg, count_blocks);
+             (int32_t)w.cap_nodes, big ? nullptr : w.done, w.chunks, w.seg, count_blocks);
       if (big) {
         launch(k_big_scatter, sb, kThreads, 0, s, w.chunks, w.ls, w.nodes, w.B, w.seg, w.node_chunk0, w.accl, w.bsum,
-                                              lvl_blocks, (int32_t)w.cap_nodes, w.level_begin, w.done);
+                                              lvl_blocks, (int32_t)w.cap_nodes, w.done);
       }
     }
     KDS_CK(cudaGetLastError());
