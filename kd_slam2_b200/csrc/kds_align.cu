@@ -1,6 +1,8 @@
 // Fused ICP / CT-ICP linearization and on-device Gauss-Newton.
 //
-// One launch = one Gauss-Newton iteration for every job of a batch.  A job is one
+// k_linearize: one launch = one Gauss-Newton iteration for every job (of one kind) of a batch.
+// k_linearize_persistent runs all iterations of a batch in one launch, k_align_cluster those of
+// a single alignment, with the same tiles and the same step.  A job is one
 // alignment (ICP_::compute / CTICP_::compute, kd/icp/tree_aligner_base_.h:100-115)
 // or one buildQuadraticForm; it has one moving leaf set and one or more fixed
 // entries (the _fixed_forest of kd/icp/icp_impl_.h:55-71).  The grid is a flat list of
@@ -16,9 +18,9 @@
 //      kd/icp/icp_cuda_impl_.cuh:68-132, kd/cuda/reduce_impl_.cuh:9-78);
 //   3. the last block of a job to finish sums the job's partials in tile order (FP64,
 //      deterministic: the result of a job does not depend on what else is in the
-//      batch), adds the pose prior, solves (H + damping) dx = -b by FP64 LDL^T, applies
-//      X <- expmap(dx) X, v += dx_v, runs the termination test and refreshes the
-//      float caches for the next launch.  No host round trip inside compute().
+//      batch), adds the pose prior, solves (H + damping) dx = -b by an FP64 Cholesky
+//      factorization, applies X <- expmap(dx) X, v += dx_v, runs the termination test and
+//      refreshes the float caches of the next iteration.  No host round trip inside compute().
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -991,8 +993,8 @@ __device__ __noinline__ void job_tail(const JobIn& JnG, JobState& SG, JobOut& O,
 
 // One Gauss-Newton iteration over the tiles [tile0, tile0 + gridDim.x) of one kind.  A descent is
 // a chain of dependent node reads, so a launch with tiles for every SM is bound by the blocks
-// that an SM holds until it is bound by issue: 8 (64 registers; the 18-parameter kind spills
-// there and takes 6), with the tree top staged as far as shared memory leaves room
+// that an SM holds until it is bound by issue: 8 (64 registers, where the 12-parameter kind
+// spills 56 B a thread; the 18-parameter kind spills too much there and takes 6, with 180 B), with the tree top staged as far as shared memory leaves room
 // (stage_room).  4,800 tiles, continuous-time / rigid: 116 / 97 us with 2 blocks and 2,047
 // nodes, 74 / 59 with 4 and 1,023, 61 / 46 with 6 and 511, 58 / 42 with 8 and 255.
 template <int KIND>
@@ -1964,9 +1966,10 @@ int Runner::enqueue(cudaStream_t s, int32_t* dbg_match, int32_t* dbg_status) {
 }
 
 // Whether a job runs as one cluster launch: a COMPUTE job of one fixed entry whose tiles fit
-// the first block's partials, and no per-launch events asked for.  Against a 1.45M-node map,
-// rigid / CT: 154 / 246 us at 1,024 surfels (a launch per iteration: 179 / 295), 167 / 297 at
-// 8,192 (195 / 319).  There the partials end and the blocks begin a second round of tiles,
+// the first block's partials, and no per-launch events asked for.  Against a 1.55M-node map,
+// rigid / CT: 128 / 221 us at 1,024 surfels (a launch per iteration: 176 / 295), 140 / 272 at
+// 8,192 (188 / 321); beside other streams' work the launches wait once each, the cluster once.
+// There the partials end and the blocks begin a second round of tiles,
 // while a launch per iteration still has SMs to spare.
 bool cluster_fits(const JobIn& J, bool profiling) {
   return !profiling && J.mode == KDS_JOB_COMPUTE && (J.kind == 0 || J.kind == 1) && J.lin_count == 1 &&

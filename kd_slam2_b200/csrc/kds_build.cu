@@ -6,9 +6,9 @@
 // reference runs on the CPU only.  The tree is built level by level for all trees of
 // the batch together:
 //   * per-node moments [xx,xy,xz,yy,yz,zz,x,y,z] are exact, order-free 128-bit
-//     fixed-point sums: floor(v * 2^64) of each product of two floats (or double stamp
-//     term) is formed and added in integers, so warps, blocks and atomics may add them in
-//     any order;
+//     fixed-point sums: floor(v * 2^64) of each product of two floats is formed and added in
+//     integers, so warps, blocks and atomics may add them in any order (the stamps' sums,
+//     of dt and dt^2, are differences of such prefix sums over the final point order);
 //   * FP64 covariance, cyclic Jacobi eigensolver, FlatLeafPolicy_ decision
 //     (kd/tree/flat_leaf_policy_.h:52-108) in FP64;
 //   * stable partition by Node_::whichSide in float (kd/tree/node_.h:53-56);
@@ -1614,7 +1614,8 @@ struct DeepSmem {                             // one group's
   U128 part[WARPS][kSums + 1];                // a node's warps: their sums; [kSums].lo: left points
   // mean and direction of the depth's nodes for the partition (one warp reads its records back:
   // its four groups fill the SM's shared memory).  With the next depth's record slots asked
-  // for during the partition, a 12,000-point scan takes 361 us in place of 365.
+  // for during the partition, scans of 12,000 and 23,000 points take 322 and 369 us in place of
+  // 324 and 377 (both builds alternating in one process).
   float plane[WARPS > 1 ? deep_nodes<WARPS>() : 1][6];
   uint8_t split[deep_nodes<WARPS>()];
 };
@@ -2729,7 +2730,7 @@ int tree_build_forest(const float* xyz, const double* stamps, const int64_t* off
     if (by_block || (host_max <= kDeepMax && level_nodes <= kDeepMaxRoots)) {
       // every node of the current level fits one group's shared memory: the rest of every
       // subtree is built there; the host reads the final level state with the counts below
-      if (round == 0) {  // the roots' sums (every root has at most kBig points)
+      if (round == 0) {  // the roots' sums (roots of 1,025 to 2,048 points by their chunks)
         rc = root_sums(w, R, host_max, N, s);
         if (rc) return rc;
       }
